@@ -53,6 +53,7 @@ struct Layer {
 
 // Buffers of the chunked prompt pass: one row per (sequence, position of the chunk).
 struct PrefillWs {
+  void*   block = nullptr;   // the one allocation they all lie in
   int64_t rows = 0;          // capacity
   float*  h = nullptr;       // [rows][H] residual stream
   float*  delta = nullptr;   // [rows][H] output of the last row-parallel GEMM, folded in by the next norm
@@ -61,7 +62,6 @@ struct PrefillWs {
   __half* q16 = nullptr;     // [rows][nq] rotated queries
   ActOut  att;               // [rows][nq]
   ActOut  ffn;               // [rows][f_local]
-  int32_t* tok = nullptr;    // [rows]
 };
 
 struct Model {
@@ -101,7 +101,7 @@ struct Model {
   cudaGraphExec_t step_graph = nullptr;
   bool graph_failed = false;
   int64_t eager_sample_steps = 0;
-  int32_t* prompt = nullptr;  // [T][B]
+  int32_t* prompt = nullptr;  // what a prompt pass indexes by (see prefill_chunked), or [T][B] tokens of the token-by-token pass
   int64_t  prompt_cap = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0.0;
@@ -168,6 +168,7 @@ void destroy(Model* m) {
   tp_symm_free(&m->symm);
   tp_destroy(&m->tp);
   for (void* p : m->allocs) cudaFree(p);
+  if (m->pf.block) cudaFree(m->pf.block);
   for (cudaEvent_t e : m->prof_events) cudaEventDestroy(e);
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
@@ -600,15 +601,34 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
   return step_tail(m, parts, sample, log_tokens, prompt_len, prompt_step);
 }
 
-// h[b] = ws.h[row(b)] + ws.delta[row(b)] for the last prompt position of every sequence: the rows the
-// end of the step (final norm, lm_head, token choice) runs on.
+// h[b] = ws.h[row] + ws.delta[row] for the sequences whose last prompt position lies in the chunk that
+// starts at p0: the rows the end of the step (final norm, lm_head, token choice) runs on.
 __global__ void gather_last_rows_kernel(float* __restrict__ h, const float* __restrict__ src, const float* __restrict__ delta,
-                                        int64_t hidden, int64_t chunk) {
+                                        const int32_t* __restrict__ lens, const int32_t* __restrict__ seq_row0,
+                                        const int32_t* __restrict__ seq_count, int p0, int64_t hidden) {
   pdl_wait();
   pdl_trigger();
-  const int64_t b = blockIdx.x, row = b * chunk + chunk - 1;
+  const int64_t b = blockIdx.x;
+  const int count = seq_count[b];
+  if (count == 0 || lens[b] != p0 + count) return;
+  const int64_t row = seq_row0[b] + count - 1;
   for (int64_t e = threadIdx.x; e < hidden; e += blockDim.x)
     h[b * hidden + e] = __fadd_rn(__ldcg(src + row * hidden + e), __ldcg(delta + row * hidden + e));
+}
+
+// Sequence state before the token choice that ends a prompt pass: a sequence that took a prompt stands at
+// its last prompt position (and is marked in `ends`), an empty prompt leaves length 0 and token 0, a
+// negative length leaves the sequence as it is.
+__global__ void prompt_state_kernel(const int32_t* __restrict__ lens, int32_t* __restrict__ seq_len,
+                                    int32_t* __restrict__ tokens, int32_t* __restrict__ ends, int b) {
+  pdl_wait();
+  pdl_trigger();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= b) return;
+  const int len = lens[i];
+  ends[i] = len > 0 ? 1 : 0;
+  if (len >= 0) seq_len[i] = len > 0 ? len - 1 : 0;
+  if (len == 0) tokens[i] = 0;
 }
 
 bool chunked_prefill_enabled() {
@@ -616,37 +636,60 @@ bool chunked_prefill_enabled() {
   return !(e && (e[0] == 'l' || e[0] == '0'));   // "loop" or "0": prompts run through the decode step token by token
 }
 
+// One block for the buffers of a chunk of up to `rows` rows.  It grows when a later prompt fills a
+// larger chunk than any before it; the old block is freed once the stream has left it.
 logos_status_t prefill_workspace(Model* m, int64_t rows) {
   PrefillWs& w = m->pf;
   if (w.rows >= rows) return LOGOS_OK;
   const logos_llm_config_t& c = m->cfg;
   const int64_t H = c.hidden;
-  auto planes = [&](ActOut* a, int64_t elems) -> logos_status_t {
-    a->mode = c.act_dtype;
-    LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&a->hi), elems * 2));
-    if (c.act_dtype == LOGOS_F32) LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&a->lo), elems * 2));
-    return LOGOS_OK;
+  const bool two = c.act_dtype == LOGOS_F32;
+  int64_t total = 0;
+  auto place = [&](int64_t bytes) {
+    const int64_t at = total;
+    total += (bytes + 255) / 256 * 256;
+    return at;
   };
-  // (a model is given one workspace, sized by the first prompt pass: later passes use chunks that fit it)
-  LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&w.h), rows * H * 4));
-  LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&w.delta), rows * H * 4));
-  LOGOS_TRY(planes(&w.xn, rows * H));
-  LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&w.qkv), rows * m->nqkv * 4));
-  LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&w.q16), rows * m->nq * 2));
-  LOGOS_TRY(planes(&w.att, rows * m->nq));
-  LOGOS_TRY(planes(&w.ffn, rows * m->f_local));
-  LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&w.tok), rows * 4));
+  const int64_t o_h = place(rows * H * 4), o_delta = place(rows * H * 4), o_qkv = place(rows * m->nqkv * 4),
+                o_q16 = place(rows * m->nq * 2);
+  const int64_t widths[3] = {H, m->nq, m->f_local};
+  int64_t o_hi[3], o_lo[3];
+  for (int i = 0; i < 3; ++i) {
+    o_hi[i] = place(rows * widths[i] * 2);
+    o_lo[i] = two ? place(rows * widths[i] * 2) : 0;
+  }
+  char* base = nullptr;
+  if (w.block) {
+    LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
+    cudaFree(w.block);
+    w = PrefillWs();
+  }
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&base), (size_t)total);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc (prompt workspace)");
+  w.block = base;
+  w.h = reinterpret_cast<float*>(base + o_h);
+  w.delta = reinterpret_cast<float*>(base + o_delta);
+  w.qkv = reinterpret_cast<float*>(base + o_qkv);
+  w.q16 = reinterpret_cast<__half*>(base + o_q16);
+  ActOut* planes[3] = {&w.xn, &w.att, &w.ffn};
+  for (int i = 0; i < 3; ++i) {
+    planes[i]->mode = c.act_dtype;
+    planes[i]->hi = reinterpret_cast<__half*>(base + o_hi[i]);
+    planes[i]->lo = two ? reinterpret_cast<__half*>(base + o_lo[i]) : nullptr;
+  }
   w.rows = rows;
   return LOGOS_OK;
 }
 
-// The prompt pass proper: chunks of positions, every sequence's chunk at once (rows = batch x chunk),
-// so that each weight matrix is streamed once per chunk instead of once per token.  Per layer:
-// norm -> qkv GEMM -> RoPE + KV write + causal attention -> o_proj GEMM -> norm -> gate/up GEMM
+// The prompt pass proper: chunks of positions, every sequence's part of the chunk at once, so that each
+// weight matrix is streamed once per chunk instead of once per token.  Rows are packed (sequence,
+// position): a prompt shorter than the chunk's end contributes what it has and nothing after it.  Per
+// layer: norm -> qkv GEMM -> RoPE + KV write + causal attention -> o_proj GEMM -> norm -> gate/up GEMM
 // with SwiGLU -> down GEMM, the same kernels and the same arithmetic as a decode step, on more rows.
-// tokens_host: [B][t].  Leaves the cache filled for positions [0, t), the lengths at t and the
-// token chosen after the last prompt position as the current token.
-logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t) {
+// tokens_host: [B][t]; sequence b takes the first lens[b] of its row (0: an empty prompt, negative: the
+// sequence keeps its state).  Leaves the cache filled for positions [0, lens[b]), the lengths there
+// and the token chosen after the last prompt position as the current token.
+logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, const std::vector<int32_t>& lens) {
   const logos_llm_config_t& c = m->cfg;
   const int64_t B = c.batch, H = c.hidden, D = c.head_dim;
   cudaStream_t st = m->stream;
@@ -654,23 +697,64 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t) 
   // chunk's activations stay inside L2 (LOGOS_B200_PREFILL_ROWS overrides: tests use small chunks)
   int64_t target_rows = 4096;
   if (const char* e = getenv("LOGOS_B200_PREFILL_ROWS")) target_rows = std::max<int64_t>(1, atoll(e));
-  int64_t chunk = std::max<int64_t>(1, target_rows / B);
-  if (m->pf.rows > 0 && chunk * B > m->pf.rows) chunk = std::max<int64_t>(1, m->pf.rows / B);
-  if (chunk > t) chunk = t;
-  if (chunk < 1) chunk = 1;
-  LOGOS_TRY(prefill_workspace(m, B * chunk));
+  struct Chunk { int64_t p0, longest, rows, at; };   // at: its rows' place in the row arrays
+  std::vector<Chunk> chunks;
+  int64_t longest = 0, total_rows = 0, most_rows = 0;
+  for (int64_t b = 0; b < B; ++b) longest = std::max<int64_t>(longest, lens[(size_t)b]);
+  auto rows_of = [&](int64_t p0, int64_t cn) {
+    int64_t r = 0;
+    for (int64_t b = 0; b < B; ++b) r += std::min<int64_t>(std::max<int64_t>(lens[(size_t)b] - p0, 0), cn);
+    return r;
+  };
+  for (int64_t p0 = 0; p0 < longest;) {
+    int64_t lo = 1, hi = longest - p0;   // the largest chunk within the target, at least one position
+    while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) / 2;
+      if (rows_of(p0, mid) <= target_rows) lo = mid; else hi = mid - 1;
+    }
+    chunks.push_back({p0, lo, rows_of(p0, lo), total_rows});
+    total_rows += chunks.back().rows;
+    most_rows = std::max(most_rows, chunks.back().rows);
+    p0 += lo;
+  }
+  if (most_rows > 0) LOGOS_TRY(prefill_workspace(m, most_rows));
+  // everything the kernels index by, in one upload before the first launch: lens [B] | ends [B] | tokens,
+  // sequence and position of every row | row0 [B] and count [B] of every chunk
+  const int64_t need = 2 * B + 3 * total_rows + 2 * B * (int64_t)chunks.size();
+  if (m->prompt_cap < need) {
+    LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->prompt), need * 4));
+    m->prompt_cap = need;
+  }
+  std::vector<int32_t> meta((size_t)need, 0);
+  const int64_t o_ends = B, o_tok = 2 * B, o_seq = o_tok + total_rows, o_pos = o_seq + total_rows, o_chunk = o_pos + total_rows;
+  for (int64_t b = 0; b < B; ++b) meta[(size_t)b] = lens[(size_t)b];
+  for (size_t ci = 0; ci < chunks.size(); ++ci) {
+    const Chunk& ch = chunks[ci];
+    int64_t row = 0;
+    for (int64_t b = 0; b < B; ++b) {
+      const int64_t cnt = std::min<int64_t>(std::max<int64_t>(lens[(size_t)b] - ch.p0, 0), ch.longest);
+      meta[(size_t)(o_chunk + 2 * B * (int64_t)ci + b)] = (int32_t)row;
+      meta[(size_t)(o_chunk + 2 * B * (int64_t)ci + B + b)] = (int32_t)cnt;
+      for (int64_t j = 0; j < cnt; ++j, ++row) {
+        meta[(size_t)(o_tok + ch.at + row)] = tokens_host[b * t + ch.p0 + j];
+        meta[(size_t)(o_seq + ch.at + row)] = (int32_t)b;
+        meta[(size_t)(o_pos + ch.at + row)] = (int32_t)(ch.p0 + j);
+      }
+    }
+  }
+  LOGOS_CUDA_TRY(cudaMemcpyAsync(m->prompt, meta.data(), (size_t)need * 4, cudaMemcpyHostToDevice, st));
+  LOGOS_CUDA_TRY(cudaStreamSynchronize(st));
+  int32_t* const lens_dev = m->prompt;
+  int32_t* const ends_dev = m->prompt + o_ends;
+
   PrefillWs& w = m->pf;
   PdlScope pdl(pdl_enabled());
-  LOGOS_CUDA_TRY(cudaMemsetAsync(m->seq_len, 0, (size_t)B * 4, st));
-  std::vector<int32_t> rows_tok;
-  for (int64_t p0 = 0; p0 < t; p0 += chunk) {
-    const int64_t cn = std::min(chunk, t - p0), M = B * cn;
-    rows_tok.assign((size_t)M, 0);
-    for (int64_t b = 0; b < B; ++b)
-      for (int64_t j = 0; j < cn; ++j) rows_tok[(size_t)(b * cn + j)] = tokens_host[b * t + p0 + j];
-    LOGOS_CUDA_TRY(cudaMemcpyAsync(w.tok, rows_tok.data(), (size_t)M * 4, cudaMemcpyHostToDevice, st));
-    LOGOS_CUDA_TRY(cudaStreamSynchronize(st));   // rows_tok is reused by the next chunk
-    LOGOS_TRY(launch_embed(w.tok, m->embed.q, m->embed.s, w.h, M, H, m->embed.tiled ? 1 : 0, st));
+  for (size_t ci = 0; ci < chunks.size(); ++ci) {
+    const Chunk& ch = chunks[ci];
+    const int64_t M = ch.rows;
+    const int32_t* row0_dev = m->prompt + o_chunk + 2 * B * (int64_t)ci;
+    const int32_t* count_dev = row0_dev + B;
+    LOGOS_TRY(launch_embed(m->prompt + o_tok + ch.at, m->embed.q, m->embed.s, w.h, M, H, m->embed.tiled ? 1 : 0, st));
     auto gemm = [&](const ActOut& a, const Q8Mat& wt, int64_t k, GemmArgs g) -> logos_status_t {
       g.a = a.hi; g.a_lo = a.lo; g.a_dtype = LOGOS_F16; g.lda = k;
       g.q = wt.q; g.s = wt.s; g.q_tiled = wt.tiled;
@@ -692,9 +776,11 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t) 
       }
       {
         PrefillAttnArgs a;
+        a.row_seq = m->prompt + o_seq + ch.at; a.row_pos = m->prompt + o_pos + ch.at;
+        a.seq_row0 = row0_dev; a.seq_count = count_dev; a.rows = M;
         a.qkv = w.qkv; a.qkv_ld = m->nqkv; a.qkv_bias = L.bqkv; a.rope = m->rope; a.q16 = w.q16;
         a.k_cache = L.kc; a.v_cache = L.vc; a.o = w.att;
-        a.b = B; a.h_q = m->hq_local; a.h_kv = m->hkv_local; a.d = D; a.l_max = c.l_max; a.chunk = cn; a.pos0 = p0;
+        a.b = B; a.h_q = m->hq_local; a.h_kv = m->hkv_local; a.d = D; a.l_max = c.l_max; a.chunk = ch.longest; a.pos0 = ch.p0;
         a.scale = 1.0f / sqrtf((float)D);
         a.device = m->device;
         LOGOS_TRY(launch_prefill_attn(a, st));
@@ -720,20 +806,17 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t) 
       }
       LOGOS_TRY(debug_check(m, "prefill layer", l));
     }
-    if (p0 + cn >= t) {
-      // the last position of every sequence: fold the pending delta, then the ordinary end of a step
-      LOGOS_CUDA_TRY(launch_kernel(gather_last_rows_kernel, dim3((unsigned)B), dim3(256), 0, st, m->h, (const float*)w.h,
-                                   (const float*)w.delta, H, cn));
-      LOGOS_TRY(check_launch("gather_last_rows_kernel"));
-    }
+    // the last position of every prompt that ends in this chunk: fold the pending delta
+    LOGOS_CUDA_TRY(launch_kernel(gather_last_rows_kernel, dim3((unsigned)B), dim3(256), 0, st, m->h, (const float*)w.h,
+                                 (const float*)w.delta, (const int32_t*)lens_dev, row0_dev, count_dev, (int)ch.p0, H));
+    LOGOS_TRY(check_launch("gather_last_rows_kernel"));
   }
-  {
-    std::vector<int32_t> len((size_t)B, (int32_t)(t - 1));   // the position the last prompt token sits at
-    LOGOS_CUDA_TRY(cudaMemcpyAsync(m->seq_len, len.data(), (size_t)B * 4, cudaMemcpyHostToDevice, st));
-    LOGOS_CUDA_TRY(cudaStreamSynchronize(st));
-  }
+  // the ordinary end of a step for the sequences that took a prompt
+  LOGOS_CUDA_TRY(launch_kernel(prompt_state_kernel, dim3((unsigned)((B + 127) / 128)), dim3(128), 0, st, (const int32_t*)lens_dev,
+                               m->seq_len, m->tokens, ends_dev, (int)B));
+  LOGOS_TRY(check_launch("prompt_state_kernel"));
   m->launch_counter = 0;
-  LOGOS_TRY(step_tail(m, 0, true, false, nullptr, 0));
+  if (longest > 0) LOGOS_TRY(step_tail(m, 0, true, false, ends_dev, 0));
   LOGOS_CUDA_TRY(cudaStreamSynchronize(st));
   int code = 0;
   LOGOS_TRY(kernel_status_read(m->device, &code, false));
@@ -1013,7 +1096,7 @@ logos_status_t logos_llm_prefill(logos_handle_t model, const int32_t* tokens_hos
     for (int64_t i = 0; i < B * t; ++i)
       if (tokens_host[i] < 0 || tokens_host[i] >= m->cfg.vocab)
         return fail(LOGOS_OUT_OF_BOUNDS, "logos_llm_prefill: token id %d outside the vocabulary", tokens_host[i]);
-    if (chunked_prefill_enabled()) return prefill_chunked(m, tokens_host, t);
+    if (chunked_prefill_enabled()) return prefill_chunked(m, tokens_host, t, std::vector<int32_t>((size_t)B, (int32_t)t));
     if (m->prompt_cap < B * t) {
       LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->prompt), B * t * 4));
       m->prompt_cap = B * t;
@@ -1049,6 +1132,7 @@ logos_status_t logos_llm_prefill_ragged(logos_handle_t model, const int32_t* tok
           return fail(LOGOS_OUT_OF_BOUNDS, "logos_llm_prefill_ragged: token id %d outside the vocabulary",
                       tokens_host[b * t_max + p]);
     }
+    if (chunked_prefill_enabled()) return prefill_chunked(m, tokens_host, t_max, std::vector<int32_t>(lens_host, lens_host + B));
     // device: [longest][B] prompt tokens (0 past a sequence's end), then the [B] lengths
     const int64_t need = (longest + 1) * B;
     if (m->prompt_cap < need) {

@@ -122,16 +122,22 @@ logos_status_t launch_kv_append_rope(__half* k_cache, __half* v_cache, const __h
 void rope_table_host(float* out, int64_t l_max, int64_t d, double theta);
 
 // ---- prompt processing (prefill.cu): RoPE + KV write + causal attention for a chunk of prompt
-// positions [pos0, pos0 + chunk) of every sequence; rows are ordered (sequence, position).
+// positions [pos0, pos0 + chunk) of the sequences whose prompts reach that far; rows are packed and
+// ordered (sequence, position), described by the four device arrays.
 struct PrefillAttnArgs {
-  const float*  qkv = nullptr;       // [b * chunk][qkv_ld] f32: q | k | v heads of a row, un-rotated
+  const int32_t* row_seq = nullptr;   // [rows] sequence of a row
+  const int32_t* row_pos = nullptr;   // [rows] its position
+  const int32_t* seq_row0 = nullptr;  // [b] first row of a sequence
+  const int32_t* seq_count = nullptr; // [b] its rows: at most `chunk`
+  int64_t       rows = 0;
+  const float*  qkv = nullptr;       // [rows][qkv_ld] f32: q | k | v heads of a row, un-rotated
   int64_t       qkv_ld = 0;
   const float*  qkv_bias = nullptr;  // f32 [(Hq + 2 Hkv) * D] or null
   const float*  rope = nullptr;      // [Lmax][D/2][2]
-  __half*       q16 = nullptr;       // scratch [b * chunk][Hq * D]: the rotated queries
+  __half*       q16 = nullptr;       // scratch [rows][Hq * D]: the rotated queries
   __half*       k_cache = nullptr;   // [B][Hkv][Lmax][D]
   __half*       v_cache = nullptr;
-  ActOut        o;                   // planes [b * chunk][Hq * D]
+  ActOut        o;                   // planes [rows][Hq * D]
   int64_t       b = 0, h_q = 0, h_kv = 0, d = 0, l_max = 0, chunk = 0, pos0 = 0;
   float         scale = 1.f;
   int           device = 0;

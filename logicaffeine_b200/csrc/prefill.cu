@@ -14,7 +14,9 @@
 //                             online softmax and output in f32 registers, and feeds the
 //                             probabilities to the second MMA as fp16 high part + residual, as
 //                             the decode kernel does.
-// Rows of the chunk are ordered (sequence, position): row = b * chunk + j.
+// Rows of a chunk are packed and ordered (sequence, position): sequence b contributes rows
+// [row0[b], row0[b] + count[b]) for its positions pos0, pos0 + 1, ...; prompts of different lengths
+// leave no padding rows.
 #include "ops.cuh"
 #include "ptx.cuh"
 
@@ -38,7 +40,9 @@ struct PrefillAttnParams {
   __half*       k_cache; // [B][Hkv][Lmax][D]
   __half*       v_cache;
   ActOut        o;       // planes [rows][Hq * D]
-  int           b, h_q, h_kv, l_max, chunk, pos0;
+  const int32_t* seq_row0;   // [B] first row of a sequence in the chunk
+  const int32_t* seq_count;  // [B] its rows in the chunk (0: it takes no part)
+  int           b, h_q, h_kv, l_max, pos0;
   float         scale_log2;
   int*          status;
 };
@@ -51,13 +55,13 @@ __device__ __forceinline__ uint32_t pack_half2_pf(float a, float b) {
 // One thread per pair (e, e + D/2) of one head of one row.
 __global__ void prefill_rope_kv_kernel(const float* __restrict__ qkv, int64_t ld, const float* __restrict__ bias,
                                        const float* __restrict__ rope, __half* __restrict__ q16,
-                                       __half* __restrict__ k_cache, __half* __restrict__ v_cache, int h_q, int h_kv,
-                                       int d, int l_max, int chunk, int pos0) {
+                                       __half* __restrict__ k_cache, __half* __restrict__ v_cache,
+                                       const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_pos, int h_q,
+                                       int h_kv, int d, int l_max) {
   pdl_wait();
   pdl_trigger();
-  const int row = blockIdx.x;                 // b * chunk + j
-  const int b = row / chunk, j = row - b * chunk;
-  const int pos = pos0 + j;
+  const int row = blockIdx.x;
+  const int b = __ldg(row_seq + row), pos = __ldg(row_pos + row);   // uploaded before the pass began
   const int half_d = d >> 1;
   const float* src = qkv + (int64_t)row * ld;
   const float* tab = rope + (int64_t)pos * half_d * 2;
@@ -114,8 +118,14 @@ gqa_prefill_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int PW = 16 / G;                       // query positions in a warp's 16 rows
   const int qpb = PF_CWARPS * PW;              // query positions of the CTA
   const int kvh = blockIdx.y, b = blockIdx.z;
+  const int count = __ldg(p.seq_count + b);    // the sequence's positions in the chunk (uploaded before the pass)
+  const int row0 = __ldg(p.seq_row0 + b);
   const int j0 = blockIdx.x * qpb;             // first query position of the CTA inside the chunk
-  const int j_end = min(j0 + qpb, p.chunk);    // one past its last
+  if (j0 >= count) {                           // a shorter prompt than the chunk's longest
+    pdl_wait();                                // (a CTA that leaves must not let the grid end before its predecessor)
+    return;
+  }
+  const int j_end = min(j0 + qpb, count);      // one past its last
   // the CTA's last query attends to positions [0, pos0 + j_end): that many tiles are streamed
   const int ntiles = (p.pos0 + j_end + PF_TILE - 1) / PF_TILE;
   const int64_t row_base = ((int64_t)b * p.h_kv + kvh) * p.l_max;
@@ -168,8 +178,8 @@ gqa_prefill_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const int jj = r / G, g = r - jj * G;
     const int j = j0 + warp * PW + jj;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (jj < PW && j < p.chunk)
-      v = __ldcg(reinterpret_cast<const uint4*>(p.q16 + ((int64_t)b * p.chunk + j) * p.h_q * D + (kvh * G + g) * D) + c8);
+    if (jj < PW && j < count)
+      v = __ldcg(reinterpret_cast<const uint4*>(p.q16 + ((int64_t)row0 + j) * p.h_q * D + (kvh * G + g) * D) + c8);
     *reinterpret_cast<uint4*>(qw + r * QS_STRIDE + c8 * 8) = v;
   }
   __syncwarp();
@@ -187,12 +197,12 @@ gqa_prefill_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   for (int h = 0; h < 2; ++h) {
     const int r = g4 + 8 * h, jj = r / G;
     const int j = j0 + warp * PW + jj;
-    lim[h] = (jj < PW && j < p.chunk) ? p.pos0 + j + 1 : 0;
+    lim[h] = (jj < PW && j < count) ? p.pos0 + j + 1 : 0;
   }
   // the furthest position any row of this warp attends to (rows of the warp are uniform per jj)
   int warp_lim = 0;
   {
-    const int j_last = min(j0 + warp * PW + PW, p.chunk);
+    const int j_last = min(j0 + warp * PW + PW, count);
     warp_lim = j_last > j0 + warp * PW ? p.pos0 + j_last : 0;
   }
 
@@ -319,8 +329,8 @@ gqa_prefill_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   for (int h = 0; h < 2; ++h) {
     const int r = g4 + 8 * h, jj = r / G, g = r - jj * G;
     const int j = j0 + warp * PW + jj;
-    if (jj >= PW || j >= p.chunk) continue;
-    const int64_t base = ((int64_t)b * p.chunk + j) * p.h_q * D + (kvh * G + g) * D;
+    if (jj >= PW || j >= count) continue;
+    const int64_t base = ((int64_t)row0 + j) * p.h_q * D + (kvh * G + g) * D;
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) {
       const int col = i * 8 + 2 * t4;
@@ -341,7 +351,7 @@ logos_status_t launch_prefill_attn_t(const PrefillAttnArgs& a, cudaStream_t st) 
   PrefillAttnParams p{};
   p.q16 = a.q16; p.k_cache = a.k_cache; p.v_cache = a.v_cache; p.o = a.o;
   p.b = (int)a.b; p.h_q = (int)a.h_q; p.h_kv = (int)a.h_kv; p.l_max = (int)a.l_max;
-  p.chunk = (int)a.chunk; p.pos0 = (int)a.pos0;
+  p.seq_row0 = a.seq_row0; p.seq_count = a.seq_count; p.pos0 = (int)a.pos0;
   p.scale_log2 = a.scale * 1.4426950408889634f;
   p.status = kernel_status_ptr(a.device);
   if (!p.status) return fail(LOGOS_ERROR, "prefill attention: no kernel status word");
@@ -359,7 +369,7 @@ logos_status_t launch_prefill_attn_t(const PrefillAttnArgs& a, cudaStream_t st) 
 }  // namespace
 
 logos_status_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t st) {
-  if (a.b == 0 || a.chunk == 0 || a.h_q == 0) return LOGOS_OK;
+  if (a.b == 0 || a.rows == 0 || a.h_q == 0) return LOGOS_OK;
   if (a.h_kv <= 0 || a.h_q % a.h_kv) return fail(LOGOS_ERROR, "prefill attention: h_q must be a multiple of h_kv");
   if (a.h_q / a.h_kv > 16) return fail(LOGOS_ERROR, "prefill attention: at most 16 query heads per KV head");
   if (a.pos0 < 0 || a.pos0 + a.chunk > a.l_max)
@@ -367,12 +377,11 @@ logos_status_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t st) {
                 (long long)(a.pos0 + a.chunk), (long long)a.l_max);
   // rotate q and k, write the chunk's K/V rows and the fp16 queries
   {
-    const int64_t rows = a.b * a.chunk;
     const int64_t pairs = (a.h_q + 2 * a.h_kv) * (a.d / 2);
     const int threads = (int)(pairs < 256 ? ((pairs + 31) / 32) * 32 : 256);
-    LOGOS_CUDA_TRY(launch_kernel(prefill_rope_kv_kernel, dim3((unsigned)rows), dim3((unsigned)threads), 0, st, a.qkv,
-                                 a.qkv_ld, a.qkv_bias, a.rope, a.q16, a.k_cache, a.v_cache, (int)a.h_q, (int)a.h_kv,
-                                 (int)a.d, (int)a.l_max, (int)a.chunk, (int)a.pos0));
+    LOGOS_CUDA_TRY(launch_kernel(prefill_rope_kv_kernel, dim3((unsigned)a.rows), dim3((unsigned)threads), 0, st, a.qkv,
+                                 a.qkv_ld, a.qkv_bias, a.rope, a.q16, a.k_cache, a.v_cache, a.row_seq, a.row_pos,
+                                 (int)a.h_q, (int)a.h_kv, (int)a.d, (int)a.l_max));
     count_launch(LK_ELEMWISE);
     LOGOS_TRY(check_launch("prefill_rope_kv_kernel"));
   }
