@@ -48,6 +48,7 @@ struct GemmArgs {
   int64_t       lda = 0;
   const int8_t* q = nullptr;   // [N][K] row-major, or tile-major when q_tiled (launch_q8_retile)
   int           q_tiled = 0;   // tcgen05 kernel only; s is then tile-major too (launch_q8_retile_scales)
+  int           s_tiled = 0;   // row-major q with tile-major s (zero past K): any K that is a multiple of 32
   const float*  s = nullptr;   // [N][K/32]
   void*         c = nullptr;   // [M][N] (or [M][N/2] for EPI_SWIGLU), row stride ldc elements
   int           c_dtype = LOGOS_BF16;  // LOGOS_BF16, LOGOS_F16, LOGOS_F32 or LOGOS_ACT_PLANES

@@ -27,9 +27,12 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ------------------------------------------------------------ mbarrier
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+// The forms on a 32-bit address take the shared-window address: code that walks rings keeps such
+// addresses, since deriving them from generic pointers at every wait costs more than the wait.
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) { mbar_init(smem_u32(bar), count); }
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -40,33 +43,71 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar),
+               "r"((uint32_t)on)
                : "memory");
 }
-// Bounded wait: polls try_wait until the phase completes or about two seconds
-// of SM clock have passed.  Returns false when it gave up; the caller records a
-// status code and leaves.
-constexpr long long kWaitCycles = 4000000000ll;
-__device__ __forceinline__ bool mbar_try(uint32_t bar_addr, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar_addr), "r"(parity)
-      : "memory");
-  return ok != 0;
+// arrives `COUNT` times at once
+template <int COUNT>
+__device__ __forceinline__ void mbar_arrive_n_if(uint32_t bar, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0], %2;\n\t}" ::"r"(bar),
+               "r"((uint32_t)on), "n"(COUNT)
+               : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
+  mbar_arrive_expect_tx(smem_u32(bar), bytes);
+}
+// Bounded waits.  A wait polls until the phase completes or the thread's budget of polls is used up: once
+// *polls is 0 this and every later wait of the thread return at once, so that a loop can look at it once a
+// round instead of after every wait.  What is done in between works on stale data; the caller drops it
+// and reports.  A poll of a barrier that is not ready takes at least 65 cycles, so the budget of one
+// thread lasts for a second of SM clock or longer.  A warp that waits takes issue slots from the warps
+// it waits for: the loop is as few instructions as it can be.
+constexpr uint32_t kWaitPolls = 30000000u;
+#define LOGOS_MBAR_TRY(P, BAR, PH) "mbarrier.try_wait.parity.shared::cta.b64 " P ", [" BAR "], " PH ";\n\t"
+#define LOGOS_MBAR_AGAIN                                                                                     \
+  "@p bra DONE;\n\t"                                                                                         \
+  "setp.ne.u32 s, %0, 0;\n\t"                                                                                \
+  "@s add.u32 %0, %0, -1;\n\t"                                                                               \
+  "@s bra POLL;\n"                                                                                           \
+  "DONE:\n\t}"
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t* polls) {
+  asm volatile("{\n\t.reg .pred p, s;\nPOLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_AGAIN
+               : "+r"(*polls)
+               : "r"(bar), "r"(parity)
+               : "memory");
+}
+// Two or three barriers polled together: their latencies overlap.
+__device__ __forceinline__ void mbar_wait2(uint32_t bar0, uint32_t ph0, uint32_t bar1, uint32_t ph1, uint32_t* polls) {
+  asm volatile("{\n\t.reg .pred p, q, s;\nPOLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_TRY("q", "%3", "%4")
+               "and.pred p, p, q;\n\t" LOGOS_MBAR_AGAIN
+               : "+r"(*polls)
+               : "r"(bar0), "r"(ph0), "r"(bar1), "r"(ph1)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_wait3(uint32_t bar0, uint32_t ph0, uint32_t bar1, uint32_t ph1, uint32_t bar2, uint32_t ph2,
+                                           uint32_t* polls) {
+  asm volatile("{\n\t.reg .pred p, q, r, s;\nPOLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_TRY("q", "%3", "%4")
+               LOGOS_MBAR_TRY("r", "%5", "%6") "and.pred p, p, q;\n\tand.pred p, p, r;\n\t" LOGOS_MBAR_AGAIN
+               : "+r"(*polls)
+               : "r"(bar0), "r"(ph0), "r"(bar1), "r"(ph1), "r"(bar2), "r"(ph2)
+               : "memory");
+}
+// A single wait with a budget of its own; false when it gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  const uint32_t a = smem_u32(bar);
-  if (mbar_try(a, parity)) return true;  // fast path: no clock read
-  const long long start = clock64();
-  for (;;) {
-    if (mbar_try(a, parity)) return true;
-    if (clock64() - start > kWaitCycles) return false;
-  }
+  uint32_t polls = kWaitPolls;
+  mbar_wait(smem_u32(bar), parity, &polls);
+  return polls != 0;
+}
+
+__device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
 }
 
 // ------------------------------------------------------------ TMA (tile mode, no multicast)
@@ -74,52 +115,31 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
 }
 // x = innermost coordinate (elements); x * element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
+__device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_2d_hint(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y,
+__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
+  tma_load_2d(smem_u32(smem_dst), m, smem_u32(bar), x, y);
+}
+__device__ __forceinline__ void tma_load_2d_hint(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar, int x, int y,
                                                  uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint "
       "[%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y),
-      "l"(policy)
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "l"(policy)
       : "memory");
-}
-// Ask L2 to fetch a tile ahead of the TMA load that will want it.
-// ---- TMA stores (shared -> global, bulk async-group completion).  Coordinates past the
-// tensor's extents are clipped by the hardware; x * element size must be a multiple of 16.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* smem_src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem_src)), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* smem_src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// all of this thread's bulk groups have finished READING shared memory (it may be rewritten)
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// all of this thread's bulk groups are complete (their global writes are done)
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-// brings the 128-byte line holding `p` into L2; no register result, no fault on a bad address
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
-               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y)
-               : "memory");
 }
 __device__ __forceinline__ uint64_t policy_evict_first() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t policy_evict_normal() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 __device__ __forceinline__ uint64_t policy_evict_last() {
@@ -175,18 +195,17 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // All MMAs this thread issued so far arrive on `bar` when they complete.
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem desc]; kind::f16 (f16/bf16 inputs, f32 accumulate)
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accumulate) {
+template <bool ACCUMULATE>
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(ACCUMULATE ? 1 : 0)
       : "memory");
 }
 // D[tmem] = A[tmem] * B[smem desc] + D * 2^-SHIFT   (scale-input-d form, f16/tf32 kinds only)
@@ -198,16 +217,6 @@ __device__ __forceinline__ void tc_mma_f16_ts_scaled_d(uint32_t d_tmem, uint32_t
       "setp.ne.b32 p, 1, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%4, %4, %4, %4}, p, %5;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(0), "n"(SHIFT)
-      : "memory");
-}
-// D[tmem] (+)= A[smem desc] * B[smem desc]
-__device__ __forceinline__ void tc_mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -243,10 +252,17 @@ __device__ __forceinline__ void tc_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tc_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
+__device__ __forceinline__ void tc_ld_32x32b_x4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tc_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 // Shared-memory matrix descriptor for a K-major operand tile stored with the

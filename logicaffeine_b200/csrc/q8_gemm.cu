@@ -114,30 +114,6 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partials, int spl
 
 }  // namespace
 
-int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device) {
-  // Work units are (tile of 128 weight rows) x (K split); a CTA's time is a fixed part (pipeline
-  // fill, epilogue: about twelve stage times, measured) plus its K stages, and CTAs run in
-  // rounds of one per SM.  Take the split count with the smallest rounds x (fixed + stages);
-  // ties go to fewer splits (fewer partials to write and fold).
-  // (a row tile for each token tile of 64 is a unit of its own: with many tokens there are enough)
-  const int64_t tiles = ((n + 127) / 128) * ((m + 63) / 64 > 0 ? (m + 63) / 64 : 1);
-  const int64_t stages = k / 128;
-  const int sms = sm_count(device);
-  if (tiles >= sms || stages < 8) return 1;
-  const int64_t fixed = 12;
-  int64_t max_splits = stages / 4;  // at least 4 stages (512 columns) per split
-  if (max_splits > 16) max_splits = 16;
-  int best = 1;
-  int64_t best_cost = INT64_MAX;
-  for (int64_t sp = 1; sp <= max_splits; ++sp) {
-    const int64_t rounds = (tiles * sp + sms - 1) / sms;
-    const int64_t per = (stages + sp - 1) / sp;
-    const int64_t cost = rounds * (fixed + per) * 8 + sp;
-    if (cost < best_cost) { best_cost = cost; best = (int)sp; }
-  }
-  return best;
-}
-
 logos_status_t launch_splitk_reduce(const float* partials, int splits, void* c, int c_dtype, ActOut c_act,
                                     int64_t ldc, const void* aux, int64_t m, int64_t n, int epilogue,
                                     cudaStream_t st) {
@@ -229,24 +205,6 @@ static logos_status_t gemm_abi(logos_handle_t a, logos_handle_t q, logos_handle_
 }
 
 extern "C" {
-
-#ifdef LOGOS_TC_TRACE
-// Development builds only: CTA (0,0,0) of every tcgen05 GEMM launch stores SM-clock timestamps of
-// its pipeline roles per K stage ([stage][16]) into this buffer of at least 64*16 int64; null
-// turns it off.
-__attribute__((visibility("default"))) logos_status_t logos_gemm_trace_buffer(logos_handle_t buf_or_null) {
-  return guarded([&]() -> logos_status_t {
-    if (!buf_or_null) {
-      gemm_set_trace(nullptr);
-      return LOGOS_OK;
-    }
-    long long* p = nullptr;
-    LOGOS_TRY(buf_ptr<long long>(buf_or_null, 64 * 16, "trace", &p));
-    gemm_set_trace(p);
-    return LOGOS_OK;
-  });
-}
-#endif
 
 // f32 activations, f32 output: the form the decode step uses internally (the
 // activations are split into two fp16 planes so the tensor-core product keeps

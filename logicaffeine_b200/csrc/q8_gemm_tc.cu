@@ -1,43 +1,51 @@
-// Q8 GEMM on the 5th-generation tensor cores (tcgen05) for small token counts.
+// Q8 GEMM on the 5th-generation tensor cores (tcgen05).
 //
 //   acc[n, m] = sum_kb s[n,kb] * ( sum_{k in kb} q[n,k] * a[m,k] )
 //
-// The problem is laid out "weights on the M side": one CTA owns 128 weight
-// rows (MMA M = 128, one TMEM lane per row) and MT tokens (MMA N), so the f32
-// scale of a (row, K-block) pair is one scalar per thread when the block's
-// partial sum is drained from tensor memory.
+// "Weights on the M side": a tile is 128 weight rows (MMA M = 128, one TMEM lane per row) and T
+// tokens (MMA N), so the f32 scale of a (row, K block) pair is one scalar per thread when the
+// block's partial sum is drained from tensor memory.  A work unit is a pair of neighbouring row
+// tiles (or a single one, for what full rounds of pairs leave over) x a K split x a token tile: the
+// activation loads of a K stage serve both tiles, which matters because at 64 tokens in two
+// planes they are 32 KB per stage against the 18 KB of weights and scales of a tile, and an SM's
+// L2 port takes about 64 bytes a cycle.
 //
-// Data flow per 128-column K stage (4 Q8 blocks):
-//   TMA  int8 weights [128 rows][128 B], 128-byte swizzle  -> smem ring   (warp 0)
-//   TMA  fp16 activation planes [MT][64] x 2 halves x limbs -> smem ring   (warp 1)
-//   TMA  the stage's f32 scales [128 rows][4]               -> smem ring   (warp 0)
-//   4 converter warps (one per TMEM lane quarter): smem int8 -> fp16 (exact: 0x6400|b trick)
-//        -> tcgen05.st into a TMEM operand ring; the weights never go back to shared memory
-//   2 MMA warps (one per half of a stage): per Q8 block two tcgen05.mma kind::f16 (K=16
-//        each) per plane, A from TMEM, B = activations from smem, into a fresh TMEM
-//        accumulator: first q*lo', then q*hi + D*2^-11 through the MMA's own
-//        accumulator scaling, so hi + lo*2^-11 is recombined on the tensor core
-//   8 drain warps: tcgen05.ld the block's partial sums (two blocks per wait),
-//        acc += s * partial in f32 registers (scales from the shared-memory ring: a global load
-//        under this kernel's own traffic takes several stage times), then the epilogue.
-// A CTA is persistent: it takes work items (tile of 128 weight rows x K split) in turn,
-// and the rings keep running across items, so the next item's weights stream in, are
-// converted and multiplied while the drain warps finish the previous item's epilogue.
-// The epilogue forms the output tile in shared memory in its final type and hands it to
-// one TMA store (split-K partials, plain outputs, SwiGLU into activation planes); other
-// output forms go through a plain loop of global stores.
-// All hand-offs are mbarriers; every wait is bounded and reports through the
-// device status word instead of spinning for ever.
+// Data flow per 128-column K stage (4 Q8 blocks) and tile, in two groups of half a stage:
+//   TMA  int8 weights [128 rows][128 B], 128-byte swizzle, and the stage's scales [128 rows][4]
+//        -> shared-memory rings                                                    (warp 0)
+//   TMA  fp16 activation planes [T][64] of half a stage -> ring                     (warp 1)
+//   4 converter warps (one per TMEM lane quarter): int8 -> fp16 (exact: 0x6400|b trick),
+//        tcgen05.st into the operand ring; the weights never go back to shared memory
+//   MMA warps 2 and 3, one per half: per Q8 block two tcgen05.mma kind::f16 (K = 16 each) per plane, A
+//        from TMEM, B = activations from smem, into a fresh accumulator entry: first q*lo', then
+//        q*hi + D*2^-11 through the MMA's own accumulator scaling, so hi + lo*2^-11 is
+//        recombined on the tensor core
+//   16 drain warps: tcgen05.ld a group's partial sums, acc += s * partial in f32 registers.  Of a pair,
+//        eight warps take one tile each (lane quarter x half of the tokens); a single tile is shared by
+//        all sixteen (lane quarter x quarter of the tokens).  Then the epilogue, straight from
+//        registers: a warp's lanes hold consecutive output columns of a token.
+// A CTA is persistent and the rings keep running across units.  All hand-offs are mbarriers; every
+// wait is bounded and reports through the device status word instead of spinning for ever.
 //
-// HBM roofline: 1.125 bytes per weight (int8 + f32/32); activations and
-// outputs are small next to that at decode batch sizes.
+// What bounds it, in SM cycles (stage traces and micro-measurements on a B200).  A wait for a barrier
+// that is ready costs 65 to 80, a hand-off between two warps 93, an MMA of N = 64 38 with its completion
+// seen ~160 later, tcgen05.ld ~100; FFMA2 issues every 2.3 cycles per scheduler, PRMT and HSUB2 every 2.
+// So a tile's stage at 64 tokens has 430 of FMA pipe, 610 of tensor pipe in two planes and about 730 of
+// HBM time, and everything else is latency: with one accumulator entry per half stage the kernel ran at
+// that entry's round trip (1500 per tile stage, with one plane or two and whatever the ring depths), with
+// eight drain warps at the drain's serial chain (1225).  Hence several entries, two groups of drain
+// warps, few and coarse hand-offs, ring positions kept as 32-bit shared addresses, and registers moved
+// from the other warps to the drain warps.
+//
+// HBM roofline: 1.125 bytes per weight (int8 + f32/32); activations and outputs are small next to
+// that at decode batch sizes.  With many tokens the FMA and tensor pipes are the bound.
 #include "q8_gemm_tc.cuh"
 
 #include "ptx.cuh"
 
-#include <stdlib.h>
-
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 namespace logos {
@@ -46,50 +54,52 @@ namespace {
 
 using namespace ptx;
 
-constexpr int TC_ROWS = 128;     // weight rows per CTA (MMA M)
-constexpr int TC_KSTAGE = 128;   // K per stage
-constexpr int RAW_STAGES = 4;
-constexpr int RAW_PREFETCH = 12;  // L2 prefetch distance of the weight stream, in stages
-constexpr int ACT_STAGES = 3;
-constexpr int TA_STAGES = 4;
-constexpr int TA_LIMB_COLS = 64; // TMEM columns per converted stage and copy: 128 fp16 per row
-constexpr int CONV_WARPS = 4;     // one per TMEM lane quarter
-constexpr int CONV_WARP0 = 4, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS;
-constexpr int TC_THREADS = (DRAIN_WARP0 + 8) * 32;  // 4 single-role warps, converter warps, 8 drain warps
-constexpr int ACC_PAIRS = 2;     // TMEM accumulator ring: each entry holds two Q8 blocks
-constexpr uint32_t TMEM_COLS = 512;
+constexpr int TC_ROWS = 128;     // weight rows per tile (MMA M)
+constexpr int TC_KSTAGE = 128;   // K per stage: one raw slot; a group, an operand or activation slot is half of it
 constexpr int RAW_BYTES = TC_ROWS * TC_KSTAGE;  // 16 KB
-constexpr int SC_STAGES = 12;                   // scale ring: longer than the way from the producer to the drain
 constexpr int SC_BYTES = TC_ROWS * 16;          // four f32 per row and stage
+constexpr int TA_SLOTS = 4;                     // operand ring, in groups
+constexpr int TA_SLOT_COLS = 32;                // TMEM columns of 64 fp16 per row
+constexpr uint32_t TMEM_COLS = 512;
+constexpr int GROUPS = 4;                       // groups of a pair's stage (2 tiles x 2 halves): one set of barriers each
+constexpr int DRAIN_WARP0 = 8;                  // 4 single-role warps, 4 converter warps, 16 drain warps
+constexpr int TC_THREADS = 768;
 
-template <int MT, int LIMBS>
+// Shapes of the rings by token count.  Tensor memory: operand slots x 32 + entries x 2 T columns of the
+// 512; shared memory: raw, activation and scale rings within 227 KB.
+template <int T, int LIMBS>
 struct TcCfg {
-  static constexpr int NB = MT * LIMBS;                 // activation rows staged per stage (planes stacked)
-  static constexpr int TA_COLS = TA_LIMB_COLS;
-  static constexpr int ACC_COL0 = TA_STAGES * TA_COLS;
-  static constexpr int ACT_ATOM_BYTES = NB * 128;       // one 64-column half: NB rows x 128 B
-  static constexpr int ACT_BYTES = 2 * ACT_ATOM_BYTES;
-  static constexpr int EPI_BYTES = MT * TC_ROWS * 4;    // output tile staged for the store: [MT][128] f32 at most
-  static constexpr size_t SMEM_NEED =
-      1024 + (size_t)RAW_STAGES * RAW_BYTES + (size_t)ACT_STAGES * ACT_BYTES + EPI_BYTES + SC_STAGES * SC_BYTES + 1024;
-  // the CTA allocates all of tensor memory, so ask for enough shared memory that only one CTA fits an SM
-  static constexpr size_t SMEM = SMEM_NEED > 120 * 1024 ? SMEM_NEED : 120 * 1024;
-  static_assert(SMEM <= 227 * 1024, "shared memory budget");
-  static_assert(ACC_COL0 + ACC_PAIRS * 2 * MT <= (int)TMEM_COLS, "TMEM budget");
-  static_assert(MT % 16 == 0 && MT <= 64, "MMA N");
-};
-
-// How a finished tile leaves the CTA.
-enum : int {
-  STORE_GENERIC = 0,      // loop of global stores (any epilogue and output type)
-  STORE_TMA_PARTIAL = 1,  // f32 split-K partials [splits][M][N], one 3-D TMA store
-  STORE_TMA_PLAIN = 2,    // f32 / f16 / bf16 [M][ldc], no epilogue, one TMA store
-  STORE_TMA_SWIGLU = 3,   // SwiGLU into fp16 activation planes [M][ldc], one TMA store per plane
+  static constexpr int ENTRIES = T == 96 ? 2 : T == 64 ? 3 : 4;    // accumulator entries, a group (two blocks) each
+  // Blocks per hand-off of accumulators.  One where only two entries fit: each block's columns then go back
+  // to the MMAs as soon as they are read, and the ring turns like four entries.
+  static constexpr int IB = T == 96 ? 1 : 2;
+  static constexpr int PER = 2 / IB;                               // hand-offs per group
+  static constexpr int ACT_BYTES = T * 128 * LIMBS;                // half a stage of activations
+  static constexpr int ACT_SLOTS = T * LIMBS >= 192 ? 4 : T * LIMBS == 128 ? 6 : 8;   // even: a slot belongs to one half
+  static constexpr int RAW_SLOTS_FIT = (225 * 1024 - 2048 - ACT_SLOTS * ACT_BYTES - 5 * SC_BYTES) / (RAW_BYTES + SC_BYTES);
+  static constexpr int RAW_SLOTS = RAW_SLOTS_FIT < 9 ? RAW_SLOTS_FIT : 9;
+  // The scale ring needs no barriers of its own.  A stage's scales count into its raw_full barrier, so whoever
+  // sees the stage's sums sees them; and a slot is written again after the converters have released the raw
+  // slot RAW_SLOTS tile stages before, hence after the MMAs two tile stages before that have started, hence
+  // after the drain has released what was in their accumulator entries: at most five tile stages in all.
+  static constexpr int SC_SLOTS = RAW_SLOTS + 5;
+  static_assert(TA_SLOTS + ENTRIES <= 8, "scale ring");
+  // registers per thread after the split (warpgroups: single roles, converters, drain x 4); the sum stays
+  // within what the block is launched with: 6 warpgroups x 80 (768 threads of an SM's 65536 registers)
+  static constexpr int REGS_MISC = T == 96 ? 40 : 56;
+  static constexpr int REGS_CONV = T == 96 ? 56 : 72;
+  static constexpr int REGS_DRAIN = T == 96 ? 96 : 88;
+  static_assert(REGS_MISC + REGS_CONV + 4 * REGS_DRAIN <= 6 * 80, "register split");
+  static constexpr int ACC_COL0 = TA_SLOTS * TA_SLOT_COLS;
+  static constexpr size_t SMEM = 1024 + (size_t)RAW_SLOTS * RAW_BYTES + (size_t)ACT_SLOTS * ACT_BYTES +
+                                 (size_t)SC_SLOTS * SC_BYTES + 1024;
+  static_assert(SMEM <= 227 * 1024 && SMEM > 114 * 1024, "shared memory: one CTA per SM, since it takes all of tensor memory");
+  static_assert(ACC_COL0 + 2 * ENTRIES * T <= (int)TMEM_COLS, "TMEM budget");
 };
 
 struct TcParams {
   const float* s;
-  int64_t n, k, m;
+  int64_t n, m;
   void* c;
   int c_dtype;
   ActOut c_act;
@@ -99,25 +109,37 @@ struct TcParams {
   float* partials;
   int splits;
   int stages_total;
-  int items;        // (row tile, K split) pairs
-  int mtiles;       // token tiles of MT rows; a work unit is (item, token tile), token tile fastest
-  int store_mode;
-  int tiled;        // weights are tile-major: the map is [row tiles x K tiles x 128][128 B]
+  // Units: `pairs` x splits pair items, then `solos` x splits single tiles, each for mtiles token tiles.
+  int pairs, solos, mtiles, group;
+  int s_tiled;        // scales are [row tile][stage][128 rows][4] (always with tile-major weights)
+  int stream_once;    // one token tile: the weights are not read again
   int* status;
-#ifdef LOGOS_TC_TRACE
-  long long* trace;  // SM-clock timestamps of CTA (0,0,0), first item, [stage][16]
-#endif
 };
 
-// Work item w = (row tile, K split): the splits of a tile are neighbours.
-struct TcItem { int tile, split, st_begin, nst; };
-__device__ __forceinline__ TcItem tc_item(const TcParams& p, int w) {
-  TcItem it;
-  it.tile = w / p.splits;
-  it.split = w - it.tile * p.splits;
-  it.st_begin = (int)(((int64_t)it.split * p.stages_total) / p.splits);
-  it.nst = (int)(((int64_t)(it.split + 1) * p.stages_total) / p.splits) - it.st_begin;
-  return it;
+struct TcUnit {
+  int tile, ntile, split, st_begin, nst, mtile;
+};
+// CTAs that run side by side hold consecutive units: `group` token tiles of a row-tile pair, then the next
+// pair, so that a wave of CTAs covers a near-square part of the output and both operands are
+// shared through L2.
+__device__ __forceinline__ TcUnit tc_unit(const TcParams& p, int u) {
+  TcUnit r;
+  const int pair_units = p.pairs * p.splits * p.mtiles;
+  const bool solo = u >= pair_units;
+  if (solo) u -= pair_units;
+  const int items = (solo ? p.solos : p.pairs) * p.splits;
+  const int g = u / (items * p.group);                       // token-tile group
+  u -= g * items * p.group;
+  const int in_group = min(p.group, p.mtiles - g * p.group);  // the last group may be smaller
+  const int item = u / in_group;
+  r.mtile = g * p.group + (u - item * in_group);
+  const int t = item / p.splits;
+  r.split = item - t * p.splits;
+  r.tile = solo ? 2 * p.pairs + t : 2 * t;
+  r.ntile = solo ? 1 : 2;
+  r.st_begin = r.split * p.stages_total / p.splits;
+  r.nst = (r.split + 1) * p.stages_total / p.splits - r.st_begin;
+  return r;
 }
 
 // First failure wins: code in word 0, where it happened in words 1..5.
@@ -127,18 +149,19 @@ __device__ __forceinline__ void tc_report(int* status, int code, int stage, int 
   }
 }
 
-// Timestamp slot `ev` of stage `i` (development builds with -DLOGOS_TC_TRACE only; CTA 0, its
-// first item, one lane per role).  Compiled out otherwise.
-#ifdef LOGOS_TC_TRACE
-#define TC_TRACE(i, ev)                                                                          \
-  do {                                                                                           \
-    if (trace_on && (i) < 64) p.trace[(i) * 16 + (ev)] = clock64();                              \
-  } while (0)
-#define TC_TRACE_ITEM(w) trace_on = cta0 && (w) == 0
-#else
-#define TC_TRACE(i, ev) do { } while (0)
-#define TC_TRACE_ITEM(w) do { } while (0)
-#endif
+// Position in a ring: slot, and the parity of the pass over it.
+template <int N, int STEP = 1>
+struct Ring {
+  int slot;
+  uint32_t ph;
+  __device__ __forceinline__ explicit Ring(int first = 0, uint32_t phase = 0) : slot(first), ph(phase) {}
+  __device__ __forceinline__ void next() {
+    slot += STEP;
+    const bool wrap = slot >= N;
+    slot = wrap ? slot - N : slot;
+    ph ^= wrap ? 1u : 0u;
+  }
+};
 
 __device__ __forceinline__ float silu_f(float g) { return __fdiv_rn(g, 1.0f + expf(-g)); }
 
@@ -154,8 +177,7 @@ __device__ __forceinline__ float load_aux(const TcParams& p, int64_t i) {
   return reinterpret_cast<const float*>(p.aux)[i];
 }
 
-// two int8 (bytes sel_lo / sel_hi of w ^ 0x80808080, i.e. of q + 128 as unsigned bytes) -> packed
-// fp16 pair, exact
+// two int8 (bytes of w ^ 0x80808080, i.e. of q + 128 as unsigned bytes) -> packed fp16 pair, exact
 __device__ __forceinline__ uint32_t cvt_pair(uint32_t w_xor80, uint32_t selector) {
   uint32_t bits = __byte_perm(w_xor80, 0x64646464u, selector);   // 0x64bb = 1024 + (q + 128)
   __half2 h = *reinterpret_cast<__half2*>(&bits);
@@ -164,496 +186,474 @@ __device__ __forceinline__ uint32_t cvt_pair(uint32_t w_xor80, uint32_t selector
   return *reinterpret_cast<uint32_t*>(&r);
 }
 
-__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-  return r;
-}
-__device__ __forceinline__ uint64_t pack2(float v) { return pack2(__float_as_uint(v), __float_as_uint(v)); }
-// two f32 FMAs in one instruction (sm_100): d = a * b + c on both halves, round to nearest
-__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier; both addresses and the
 // size are multiples of 16
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gmem_src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
+               ::"r"(smem_dst), "l"(gmem_src), "r"(bytes), "r"(bar)
                : "memory");
 }
 
+// N columns of a row into r[0 .. N)
 template <int N>
-__device__ __forceinline__ void tc_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
-  if constexpr (N == 32) tc_ld_32x32b_x32(taddr, r);
-  else if constexpr (N == 16) tc_ld_32x32b_x16(taddr, r);
-  else tc_ld_32x32b_x8(taddr, r);
+__device__ __forceinline__ void tc_ld_cols(uint32_t taddr, uint32_t* r) {
+  if constexpr (N == 32) tc_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(r));
+  else if constexpr (N == 24) {
+    tc_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(r));
+    tc_ld_32x32b_x8(taddr + 16, *reinterpret_cast<uint32_t(*)[8]>(r + 16));
+  } else if constexpr (N == 16) tc_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(r));
+  else if constexpr (N == 8) tc_ld_32x32b_x8(taddr, *reinterpret_cast<uint32_t(*)[8]>(r));
+  else tc_ld_32x32b_x4(taddr, *reinterpret_cast<uint32_t(*)[4]>(r));
+}
+// tcgen05.wait::ld, and the loaded registers tied to this point: no use of them moves above it
+template <int N>
+__device__ __forceinline__ void tc_loaded(uint32_t (&r)[N]) {
+  tc_wait_ld();
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+template <int N>
+__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// sum += s * (columns of a block), two-wide f32 FMAs
+template <int N>
+__device__ __forceinline__ void add_cols(float2* sum, float s, const uint32_t* b) {
+  const float2 s2 = make_float2(s, s);
+#pragma unroll
+  for (int x = 0; x < N / 2; ++x)
+    sum[x] = __ffma2_rn(s2, make_float2(__uint_as_float(b[2 * x]), __uint_as_float(b[2 * x + 1])), sum[x]);
 }
 
-// fp32 -> the value(s) an activation plane pair stores (same rounding as act_store)
-__device__ __forceinline__ void act_split_planes(int mode, float x, __half* h, __half* l) {
-  if (mode == LOGOS_BF16) x = __bfloat162float(__float2bfloat16_rn(x));
-  x = act_clamp(x);
-  *h = __float2half_rn(x);
-  *l = __float2half_rn((x - __half2float(*h)) * 2048.f);
+// HC columns each of the BLKS blocks at `ta` (blocks are T columns apart); `release` runs once all are read.
+template <int HC, int BLKS, int T, class Release>
+__device__ __forceinline__ void drain_blocks(float2* sum, uint32_t ta, const float* s, Release release) {
+  if constexpr (HC * BLKS <= 32) {   // few columns: all of them in one round of latency
+    uint32_t b[HC * BLKS];
+#pragma unroll
+    for (int k = 0; k < BLKS; ++k) tc_ld_cols<HC>(ta + k * T, b + k * HC);
+    tc_loaded(b);
+    release();
+#pragma unroll
+    for (int k = 0; k < BLKS; ++k) add_cols<HC>(sum, s[k], b + k * HC);
+  } else {
+    constexpr int CH = HC <= 32 ? HC : HC / 2;
+#pragma unroll
+    for (int k = 0; k < BLKS; ++k) {
+#pragma unroll
+      for (int c = 0; c < HC / CH; ++c) {
+        uint32_t b[CH];
+        tc_ld_cols<CH>(ta + k * T + c * CH, b);
+        tc_loaded(b);
+        if (k == BLKS - 1 && c == HC / CH - 1) release();
+        add_cols<CH>(sum + c * (CH / 2), s[k], b);
+      }
+    }
+  }
 }
 
-template <int MT, int LIMBS, bool TILED>
+// A thread's HC sums of output column n, tokens m0 ..: a warp stores 32 consecutive columns of a token at a time.
+template <int HC>
+__device__ __forceinline__ void store_tile(const TcParams& p, const float2* acc, int split, int64_t n, int64_t m0, int lane) {
+  const int rows_here = (int)(p.m - m0 < HC ? p.m - m0 : HC);
+  auto at = [&](int e) { return (e & 1) ? acc[e >> 1].y : acc[e >> 1].x; };
+  if (p.splits > 1) {
+    float* dst = p.partials + ((int64_t)split * p.m + m0) * p.n + n;
+    if (n < p.n) {
+#pragma unroll
+      for (int x = 0; x < HC; ++x)
+        if (x < rows_here) dst[x * p.n] = at(x);
+    }
+  } else if (p.epilogue == EPI_SWIGLU) {
+    // rows (2j, 2j+1) are (gate_j, up_j): neighbouring lanes.  The even lane takes the first half of the
+    // tokens, the odd lane the second half.
+    const int par = lane & 1;
+    const int64_t out = n >> 1;
+#pragma unroll
+    for (int x = 0; x < HC / 2; ++x) {
+      const float a = at(x), b = at(x + HC / 2);
+      const float recv = __shfl_xor_sync(0xffffffffu, par ? a : b, 1);
+      const float g = par ? recv : a, up = par ? b : recv;
+      const int mm = par ? x + HC / 2 : x;
+      if (mm < rows_here && (n | 1) < p.n) store_c(p, (m0 + mm) * p.ldc + out, __fmul_rn(silu_f(g), up));
+    }
+  } else if (n < p.n) {
+    if (p.c_dtype == LOGOS_F32 && p.epilogue == EPI_NONE) {
+      float* dst = reinterpret_cast<float*>(p.c) + m0 * p.ldc + n;
+#pragma unroll
+      for (int x = 0; x < HC; ++x)
+        if (x < rows_here) dst[x * p.ldc] = at(x);
+    } else {
+#pragma unroll
+      for (int x = 0; x < HC; ++x)
+        if (x < rows_here) {
+          const int64_t ci = (m0 + x) * p.ldc + n;
+          float v = at(x);
+          if (p.epilogue == EPI_RESIDUAL) v = __fadd_rn(v, load_aux(p, ci));
+          store_c(p, ci, v);
+        }
+    }
+  }
+}
+
+template <int T, int LIMBS, bool TILED>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_ahi,
-                  const __grid_constant__ CUtensorMap map_alo, const __grid_constant__ CUtensorMap map_o0,
-                  const __grid_constant__ CUtensorMap map_o1, const __grid_constant__ CUtensorMap map_s,
+                  const __grid_constant__ CUtensorMap map_alo, const __grid_constant__ CUtensorMap map_s,
                   const TcParams p) {
-  using Cfg = TcCfg<MT, LIMBS>;
-  constexpr int TA_COLS = Cfg::TA_COLS;
-  constexpr int ACC_COL0 = Cfg::ACC_COL0;
+  using Cfg = TcCfg<T, LIMBS>;
+  constexpr int ENTRIES = Cfg::ENTRIES, IB = Cfg::IB, PER = Cfg::PER, ACT_SLOTS = Cfg::ACT_SLOTS, RAW_SLOTS = Cfg::RAW_SLOTS,
+                SC_SLOTS = Cfg::SC_SLOTS;
 
+  // Shared memory by 32-bit window addresses: rings of slots, then the barriers.
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* raw = smem;
-  uint8_t* act = raw + RAW_STAGES * RAW_BYTES;
-  uint8_t* epi = act + ACT_STAGES * Cfg::ACT_BYTES;  // 1024-aligned: all sizes before it are multiples of 1024
-  uint8_t* scl = epi + Cfg::EPI_BYTES;               // scale ring
-  uint64_t* bars = reinterpret_cast<uint64_t*>(scl + SC_STAGES * SC_BYTES);
-  uint64_t* raw_full = bars;                    // [RAW_STAGES]
-  uint64_t* raw_empty = raw_full + RAW_STAGES;  // [RAW_STAGES]
-  uint64_t* act_full = raw_empty + RAW_STAGES;  // [ACT_STAGES]
-  uint64_t* act_empty = act_full + ACT_STAGES;  // [ACT_STAGES]
-  uint64_t* ta_full = act_empty + ACT_STAGES;   // [TA_STAGES]
-  uint64_t* ta_empty = ta_full + TA_STAGES;     // [TA_STAGES]
-  uint64_t* acc_full = ta_empty + TA_STAGES;    // [ACC_PAIRS]
-  uint64_t* acc_empty = acc_full + ACC_PAIRS;   // [ACC_PAIRS]
-  uint64_t* sc_full = acc_empty + ACC_PAIRS;    // [SC_STAGES]
-  uint64_t* sc_empty = sc_full + SC_STAGES;     // [SC_STAGES]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + SC_STAGES);
+  const uint32_t raw = (smem_u32(smem_raw) + 1023u) & ~1023u;       // [RAW_SLOTS] x 16 KB
+  const uint32_t act = raw + RAW_SLOTS * RAW_BYTES;                 // [ACT_SLOTS] x ACT_BYTES
+  const uint32_t scl = act + ACT_SLOTS * Cfg::ACT_BYTES;            // [SC_SLOTS] x 2 KB
+  const uint32_t raw_full = scl + SC_SLOTS * SC_BYTES;              // barriers, 8 bytes each: [RAW_SLOTS]
+  const uint32_t raw_empty = raw_full + 8 * RAW_SLOTS;
+  const uint32_t act_full = raw_empty + 8 * RAW_SLOTS;              // [ACT_SLOTS]
+  const uint32_t act_empty = act_full + 8 * ACT_SLOTS;
+  const uint32_t ta_full = act_empty + 8 * ACT_SLOTS;               // [TA_SLOTS]
+  const uint32_t ta_empty = ta_full + 8 * TA_SLOTS;
+  const uint32_t acc_full = ta_empty + 8 * TA_SLOTS;                // [GROUPS][PER]
+  const uint32_t acc_empty = acc_full + 8 * GROUPS * PER;
+  __shared__ uint32_t tmem_slot;
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  // Work units u = item * mtiles + token tile: CTAs that run side by side hold consecutive units,
-  // i.e. the same weight tile for neighbouring token tiles, so with many tokens (prefill) a
-  // weight tile crosses HBM once and is served to the other token tiles by L2.
-  const int units = p.items * p.mtiles;
-#ifdef LOGOS_TC_TRACE
-  const bool cta0 = p.trace && blockIdx.x == 0;
-  bool trace_on = cta0;
-#endif
 
-  if (tid == 0) TC_TRACE(63, 0);  // kernel entry
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
   // (one thread reads, everyone takes the same decision)
   __shared__ int prior_status;
-  if (tid == 0) prior_status = *reinterpret_cast<volatile int*>(p.status);
-  __syncthreads();
-  if (prior_status != 0) {
-    pdl_wait();  // "this kernel completed" must keep implying "its predecessor did"
-    return;
-  }
-
   if (tid == 0) {
-    for (int i = 0; i < RAW_STAGES; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], CONV_WARPS); }
-    for (int i = 0; i < ACT_STAGES; ++i) { mbar_init(&act_full[i], 1); mbar_init(&act_empty[i], 2); }
-    for (int i = 0; i < TA_STAGES; ++i) { mbar_init(&ta_full[i], CONV_WARPS); mbar_init(&ta_empty[i], 2); }
-    for (int i = 0; i < ACC_PAIRS; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
-    for (int i = 0; i < SC_STAGES; ++i) { mbar_init(&sc_full[i], 1); mbar_init(&sc_empty[i], 8); }
+    prior_status = *reinterpret_cast<volatile int*>(p.status);
+    for (int i = 0; i < RAW_SLOTS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4); }
+    for (int i = 0; i < ACT_SLOTS; ++i) { mbar_init(act_full + 8 * i, 1); mbar_init(act_empty + 8 * i, 1); }
+    for (int i = 0; i < TA_SLOTS; ++i) { mbar_init(ta_full + 8 * i, 4); mbar_init(ta_empty + 8 * i, 1); }
+    for (int i = 0; i < GROUPS * PER; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 16); }
     fence_barrier_init();
+  }
+  if (warp == 1 && lane == 0) {
     prefetch_tensormap(&map_q);
     prefetch_tensormap(&map_ahi);
     if (LIMBS == 2) prefetch_tensormap(&map_alo);
-    if (p.store_mode != STORE_GENERIC) prefetch_tensormap(&map_o0);
-    if (p.store_mode == STORE_TMA_SWIGLU) prefetch_tensormap(&map_o1);
-    if (!TILED) prefetch_tensormap(&map_s);
+    if (!p.s_tiled) prefetch_tensormap(&map_s);
   }
   if (warp == 3) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_alloc(&tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = tmem_slot;
   // Dependent launch: this CTA holds its SM's shared and tensor memory by now, so a successor's
   // CTAs may be scheduled wherever room is left.  Weights and scales are read without waiting
   // for the previous kernel (nothing in a decode step writes them); the activation producer
   // and the drain warps (the only ones that touch what other kernels write) wait first.
   pdl_trigger();
+  // nothing to do on top of an earlier failure
+  const int pair_units = prior_status != 0 ? 0 : p.pairs * p.splits * p.mtiles;
+  const int units = prior_status != 0 ? 0 : (p.pairs + p.solos) * p.splits * p.mtiles;
 
   bool ok = true;
-  if (tid == 0) TC_TRACE(63, 1);  // set-up done
+  uint32_t polls = kWaitPolls;   // see mbar_wait; a new budget every unit
 
-  // Every role walks the same sequence of (item, stage) pairs; `gs` counts stages across items
-  // and alone decides ring slots and barrier phases, so the rings never drain between items.
-  if (warp == 0) {
-    // ------------------------------------------------------------ weight producer
-    if (lane == 0) {
-      const uint64_t pol = policy_evict_first();
-      int gs = 0;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        const int w = u / p.mtiles;
-        const TcItem it = tc_item(p, w);
-        const int n0 = it.tile * TC_ROWS, nst = it.nst, st_begin = it.st_begin;
-        TC_TRACE_ITEM(w);
-        // The smem ring alone (RAW_STAGES x 16 KB per SM) does not cover HBM latency under load:
-        // L2 prefetches run RAW_PREFETCH stages ahead of the TMA loads.  They start only after
-        // the item's first loads are on their way, so that nothing queues in front of those.
-        for (int i = 0; i < nst; ++i, ++gs) {
-          {
-            // the stage's scales, four per row: tile-major they are 2 contiguous KB, row-major a
-            // [128 rows][4] box of the [N][K/32] matrix (rows past N read as zero)
-            const int ss = gs % SC_STAGES;
-            if (!mbar_wait(&sc_empty[ss], ((uint32_t)(gs / SC_STAGES) & 1u) ^ 1u)) { ok = false; tc_report(p.status, 2011, i, nst); break; }
-            mbar_arrive_expect_tx(&sc_full[ss], SC_BYTES);
-            if (TILED)
-              bulk_load(scl + ss * SC_BYTES, p.s + ((int64_t)it.tile * p.stages_total + st_begin + i) * TC_ROWS * 4, SC_BYTES, &sc_full[ss]);
-            else
-              tma_load_2d(scl + ss * SC_BYTES, &map_s, &sc_full[ss], (st_begin + i) * 4, n0);
-          }
-          const int st = gs % RAW_STAGES;
-          const uint32_t ph = (uint32_t)(gs / RAW_STAGES) & 1u;
-          if (!mbar_wait(&raw_empty[st], ph ^ 1u)) { ok = false; tc_report(p.status, 2010, i, nst); break; }
-          TC_TRACE(i, 0);
-          mbar_arrive_expect_tx(&raw_full[st], RAW_BYTES);
-          // row-major weights: tile (n0, stage) of a [N][K] map; tile-major: 128 rows of 128 bytes at
-          // row ((tile * stages + stage) * 128) of a [tiles * stages * 128][128 B] map
-          const int tbase = it.tile * p.stages_total + st_begin;
-          if (TILED) tma_load_2d_hint(raw + st * RAW_BYTES, &map_q, &raw_full[st], 0, (tbase + i) * TC_ROWS, pol);
-          else tma_load_2d_hint(raw + st * RAW_BYTES, &map_q, &raw_full[st], (st_begin + i) * TC_KSTAGE, n0, pol);
-          if (i + 1 >= RAW_STAGES) {
-            // after the first fill: stages RAW_STAGES .. RAW_PREFETCH in one go, then one per stage
-            const int first = (i + 1 == RAW_STAGES) ? RAW_STAGES : i + RAW_PREFETCH;
-            for (int j = first; j <= i + RAW_PREFETCH && j < nst; ++j) {
-              if (TILED) tma_prefetch_l2_2d(&map_q, 0, (tbase + j) * TC_ROWS);
-              else tma_prefetch_l2_2d(&map_q, (st_begin + j) * TC_KSTAGE, n0);
+  // Every role walks the same sequence of groups: units, stages, the unit's tiles, halves.
+  if (warp < 4) {
+    regs_dec<Cfg::REGS_MISC>();
+    if (warp == 0) {
+      // ------------------------------------------------------------ weight and scale producer
+      if (lane == 0) {
+        const uint64_t pol = p.stream_once ? policy_evict_first() : policy_evict_normal();
+        Ring<RAW_SLOTS> r;
+        Ring<SC_SLOTS> c;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+          const TcUnit it = tc_unit(p, u);
+          polls = kWaitPolls;
+          for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
+            for (int j = it.tile; j < it.tile + it.ntile; ++j) {
+              const int block = j * p.stages_total + i;   // of a tile-major array
+              const uint32_t bar = raw_full + 8 * r.slot;
+              mbar_wait(raw_empty + 8 * r.slot, r.ph ^ 1u, &polls);
+              if (polls == 0) { ok = false; tc_report(p.status, 2010, i, it.nst); break; }
+              mbar_arrive_expect_tx(bar, RAW_BYTES + SC_BYTES);
+              // row-major weights: tile (row, stage) of a [N][K] map; tile-major: 128 rows of 128 bytes at
+              // row block * 128 of a [tiles * stages * 128][128 B] map
+              if (TILED) tma_load_2d_hint(raw + r.slot * RAW_BYTES, &map_q, bar, 0, block * TC_ROWS, pol);
+              else tma_load_2d_hint(raw + r.slot * RAW_BYTES, &map_q, bar, i * TC_KSTAGE, j * TC_ROWS, pol);
+              // the stage's scales, four per row: tile-major they are 2 contiguous KB, row-major a
+              // [128 rows][4] box of the [N][K/32] matrix (rows past N read as zero)
+              if (TILED || p.s_tiled) bulk_load(scl + c.slot * SC_BYTES, p.s + (int64_t)block * (TC_ROWS * 4), SC_BYTES, bar);
+              else tma_load_2d(scl + c.slot * SC_BYTES, &map_s, bar, i * 4, j * TC_ROWS);
+              r.next();
+              c.next();
             }
           }
         }
       }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ activation producer
-    if (lane == 0) {
-      pdl_wait();  // the activations are the previous kernel's output
-      const uint64_t pol = policy_evict_last();
-      int gs = 0;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        const int w = u / p.mtiles;
-        const int m0 = (u - w * p.mtiles) * MT;
-        const TcItem it = tc_item(p, w);
-        const int nst = it.nst, st_begin = it.st_begin;
-        TC_TRACE_ITEM(w);
-        for (int i = 0; i < nst; ++i, ++gs) {
-          const int st = gs % ACT_STAGES;
-          const uint32_t ph = (uint32_t)(gs / ACT_STAGES) & 1u;
-          if (!mbar_wait(&act_empty[st], ph ^ 1u)) { ok = false; tc_report(p.status, 2020, i, nst); break; }
-          TC_TRACE(i, 1);
-          mbar_arrive_expect_tx(&act_full[st], Cfg::ACT_BYTES);
-          uint8_t* sb = act + st * Cfg::ACT_BYTES;
-          const int x = (st_begin + i) * TC_KSTAGE;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            tma_load_2d_hint(sb + h * Cfg::ACT_ATOM_BYTES, &map_ahi, &act_full[st], x + h * 64, (int)m0, pol);
-            if (LIMBS == 2)
-              tma_load_2d_hint(sb + h * Cfg::ACT_ATOM_BYTES + MT * 128, &map_alo, &act_full[st], x + h * 64, (int)m0, pol);
+    } else if (warp == 1) {
+      // ------------------------------------------------------------ activation producer
+      if (lane == 0) {
+        pdl_wait();  // the activations are the previous kernel's output
+        const uint64_t pol = policy_evict_last();
+        Ring<ACT_SLOTS> r;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+          const TcUnit it = tc_unit(p, u);
+          polls = kWaitPolls;
+          const int m0 = it.mtile * T;
+          for (int h = 2 * it.st_begin; h < 2 * (it.st_begin + it.nst); ++h) {
+            mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &polls);
+            if (polls == 0) { ok = false; tc_report(p.status, 2020, h, it.nst); break; }
+            const uint32_t bar = act_full + 8 * r.slot, sb = act + r.slot * Cfg::ACT_BYTES;
+            mbar_arrive_expect_tx(bar, Cfg::ACT_BYTES);
+            tma_load_2d_hint(sb, &map_ahi, bar, h * 64, m0, pol);
+            if (LIMBS == 2) tma_load_2d_hint(sb + T * 128, &map_alo, bar, h * 64, m0, pol);
+            r.next();
           }
         }
       }
-    }
-  } else if (warp == 2 || warp == 3) {
-    // ------------------------------------------------------------ MMA issuers
-    // Two warps, one per half of a stage: warp 2 issues the first pair of Q8 blocks of every
-    // stage, warp 3 the second.  What bounds the kernel is the round trip of an accumulator entry
-    // (MMAs execute -> completion seen by the drain -> tcgen05.ld -> entry released -> next
-    // stage's MMAs), so the two pairs' round trips run side by side; and every barrier is
-    // waited on, phase after phase, by the same warp, which the odd/even phase test needs.
-    // A warp runs its loop with all lanes (addresses and descriptors stay warp-uniform) and one
-    // elected lane issues the tcgen05 instructions.  A pair owns accumulator ring entry `pr`.
-    constexpr int NSPLIT = 1;   // an M=128, K=16 MMA costs the same at N=32 and N=64: one MMA per block and plane
-    constexpr int MN = MT;      // tokens per MMA (MMA N, a multiple of 16)
-    constexpr uint32_t idesc = make_idesc_f16(0, 0, TC_ROWS, MN);
-    static_assert(ACC_PAIRS == 2, "one accumulator ring entry per MMA warp");
-    const int pr = warp - 2;
-    int gs = 0;
-    int as = 0;           // slot and phase of the activation ring, counted
-    uint32_t aph = 0;
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-      const int w = u / p.mtiles;
-      const int nst = tc_item(p, w).nst;
-      TC_TRACE_ITEM(w);
-      for (int i = 0; i < nst && ok; ++i, ++gs) {
-        const int ts = gs % TA_STAGES;
-        const uint32_t tph = (uint32_t)(gs / TA_STAGES) & 1u;
-        if (!mbar_wait(&ta_full[ts], tph)) { ok = false; if (lane == 0) tc_report(p.status, 2031, i, nst); break; }
-        if (lane == 0 && pr == 0) TC_TRACE(i, 2);
-        if (!mbar_wait(&act_full[as], aph)) { ok = false; if (lane == 0) tc_report(p.status, 2032, i, nst); break; }
-        const uint32_t act_base = smem_u32(act + as * Cfg::ACT_BYTES);
-        const uint32_t sph = (uint32_t)gs & 1u;
-        if (pr == 1 && lane == 0) TC_TRACE(i, 11);
-        if (!mbar_wait(&acc_empty[pr], sph ^ 1u)) { ok = false; if (lane == 0) tc_report(p.status, 2033, i, nst); break; }
-        if (pr == 1 && lane == 0) TC_TRACE(i, 12);
-        tc_fence_after();
-        if (elect_one()) {
-          // Per block: d = q * lo' first, then d = q * hi + d * 2^-11 (the residual plane is folded
-          // in by the accumulator scaling of the MMA itself, from one copy of the weights).
-          // The two blocks' chains are issued interleaved (measured neutral: the pipe runs
-          // dependent and independent accumulations at the same rate).
+    } else {
+      // ------------------------------------------------------------ MMA issuers, one warp per half of a stage
+      // A warp runs its loop with all lanes, so that addresses and descriptors stay warp-uniform (with one lane
+      // alone the issue of a group took three times as long), and one elected lane issues the tcgen05
+      // instructions.  The barriers a group needs are polled together: one round of latency, not three.
+      // Barrier sets follow the groups modulo GROUPS and accumulator entries modulo ENTRIES; a warp meets the
+      // same sets phase after phase, which the parity test needs.
+      constexpr uint32_t idesc = make_idesc_f16(0, 0, TC_ROWS, T);
+      const int half = warp - 2;
+      const uint64_t bdesc_first = make_desc_sw128(act);
+      Ring<ACT_SLOTS, 2> ra(half);
+      Ring<TA_SLOTS, 2> rt(half);
+      Ring<GROUPS, 2> rf(half);                                              // the group's own barriers
+      Ring<GROUPS, 2> re((half + GROUPS - ENTRIES) % GROUPS, 1u);            // those of the entry's previous group
+      Ring<ENTRIES, 2> rd(half % ENTRIES);                                   // the entry
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const TcUnit it = tc_unit(p, u);
+        polls = kWaitPolls;
+        for (int i = 0; i < it.nst; ++i) {
+          const uint64_t bdesc0 = bdesc_first + (uint32_t)(ra.slot * (Cfg::ACT_BYTES >> 4));   // start address field: no carry out of it
+          for (int j = 0; j < it.ntile; ++j) {
+            const uint32_t free_bar = acc_empty + 8 * PER * re.slot;
+            if (j == 0) mbar_wait3(act_full + 8 * ra.slot, ra.ph, ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
+            else mbar_wait2(ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
+            tc_fence_after();
+            const uint32_t d0 = tmem_base + Cfg::ACC_COL0 + rd.slot * 2 * T;
+            const uint32_t a0 = tmem_base + rt.slot * TA_SLOT_COLS;
 #pragma unroll
-          for (int u = 0; u < 2 * LIMBS; ++u) {
-#pragma unroll
-            for (int bb = 0; bb < 2; ++bb) {
-#pragma unroll
-              for (int hh = 0; hh < NSPLIT; ++hh) {
-                const int blk = 2 * pr + bb;
-                const uint32_t d = tmem_base + ACC_COL0 + blk * MT + hh * MN;
-                const int l = (LIMBS == 2) ? 1 - (u >> 1) : 0, j = u & 1;
-                const int kk = blk * 2 + j;  // K=16 step inside the stage
-                const uint32_t a = tmem_base + ts * TA_COLS + kk * 8;
-                const uint64_t bdesc = make_desc_sw128(act_base + (kk >> 2) * Cfg::ACT_ATOM_BYTES + l * MT * 128 +
-                                                       hh * MN * 128 + (kk & 3) * 32);
-                if (LIMBS == 2 && u == 2) tc_mma_f16_ts_scaled_d<11>(d, a, bdesc, idesc);
-                else tc_mma_f16_ts(d, a, bdesc, idesc, (uint32_t)(u != 0));
+            for (int k = 0; k < PER; ++k) {
+              if (k > 0) {
+                mbar_wait(free_bar + 8 * k, re.ph, &polls);
+                tc_fence_after();
               }
+              if (elect_one()) {
+                // Per block: d = q * lo' first, then d = q * hi + d * 2^-11 (the residual plane is folded in by the
+                // accumulator scaling of the MMA itself, from one copy of the weights).
+#pragma unroll
+                for (int v = 0; v < 2 * LIMBS; ++v) {
+#pragma unroll
+                  for (int b = 0; b < IB; ++b) {
+                    const int bb = k * IB + b;
+                    const int l = (LIMBS == 2) ? 1 - (v >> 1) : 0;
+                    const int kk = bb * 2 + (v & 1);     // K = 16 step inside the half stage
+                    const uint64_t bdesc = bdesc0 + (uint32_t)((l * T * 128 + kk * 32) >> 4);
+                    if (LIMBS == 2 && v == 2) tc_mma_f16_ts_scaled_d<11>(d0 + bb * T, a0 + kk * 8, bdesc, idesc);
+                    else if (v == 0) tc_mma_f16_ts<false>(d0 + bb * T, a0 + kk * 8, bdesc, idesc);
+                    else tc_mma_f16_ts<true>(d0 + bb * T, a0 + kk * 8, bdesc, idesc);
+                  }
+                }
+                tc_commit(acc_full + 8 * (PER * rf.slot + k));
+                if (k == PER - 1) {
+                  tc_commit(ta_empty + 8 * rt.slot);
+                  if (j + 1 == it.ntile) tc_commit(act_empty + 8 * ra.slot);   // free once these MMAs have completed
+                }
+              }
+              __syncwarp();
             }
+            rt.next();
+            rf.next();
+            re.next();
+            rd.next();
           }
-          if (pr == 1) TC_TRACE(i, 13);
-          tc_commit(&acc_full[pr]);
-          // the stage's operands are free once both warps' MMAs have completed
-          tc_commit(&ta_empty[ts]);
-          tc_commit(&act_empty[as]);
+          ra.next();
+          if (polls == 0) {
+            if (lane == 0) tc_report(p.status, 2030, i, it.nst);
+            ok = false;
+            break;
+          }
         }
-        __syncwarp();
-        if (lane == 0 && pr == 0) TC_TRACE(i, 4);
-        if (++as == ACT_STAGES) { as = 0; aph ^= 1u; }
       }
     }
-
-  } else if (warp >= CONV_WARP0 && warp < DRAIN_WARP0) {
+  } else if (warp < DRAIN_WARP0) {
     // ------------------------------------------------------------ converters: int8 smem -> fp16 TMEM
-    // One or two warps per lane quarter; each converts its share of the stage's eight 16-byte
-    // chunks per row.
+    regs_dec<Cfg::REGS_CONV>();
     const int qd = warp & 3;
-    const int chalf = (warp - CONV_WARP0) >> 2;
     const uint32_t row = qd * 32 + lane;
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16);
-    int gs = 0;
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-      const int w = u / p.mtiles;
-      const int nst = tc_item(p, w).nst;
-      TC_TRACE_ITEM(w);
-      for (int i = 0; i < nst; ++i, ++gs) {
-        const int rs = gs % RAW_STAGES, ts = gs % TA_STAGES;
-        const uint32_t rph = (uint32_t)(gs / RAW_STAGES) & 1u, tph = (uint32_t)(gs / TA_STAGES) & 1u;
-        if (!mbar_wait(&raw_full[rs], rph)) { ok = false; if (lane == 0) tc_report(p.status, 2041, i, nst); break; }
-        if (warp == CONV_WARP0 && lane == 0) TC_TRACE(i, 5);
-        if (!mbar_wait(&ta_empty[ts], tph ^ 1u)) { ok = false; if (lane == 0) tc_report(p.status, 2042, i, nst); break; }
-        if (warp == CONV_WARP0 && lane == 0) TC_TRACE(i, 6);
-        tc_fence_after();
-        const uint8_t* rb = raw + rs * RAW_BYTES;
+    // the row's 16-byte chunks: chunk c sits at c ^ (row & 7) (128-byte swizzle)
+    uint32_t off[8];
 #pragma unroll
-        for (int cc = 0; cc < 32 / CONV_WARPS; ++cc) {
-          const int c = chalf * (32 / CONV_WARPS) + cc;
-          const uint4 wv = *reinterpret_cast<const uint4*>(rb + swz128(row, c));
-          uint32_t r[8];
-          const uint32_t ws[4] = {wv.x, wv.y, wv.z, wv.w};
-          if (TILED) {  // tile-major weights are stored as q + 128 already (compile-time branch: two
-                        // copies of this loop in one kernel cost 10 % of its speed)
+    for (int c = 0; c < 8; ++c) off[c] = swz128(row, c);
+    auto load_half = [&](uint4 (&wv)[4], uint32_t rb, int h) {
 #pragma unroll
-            for (int wi = 0; wi < 4; ++wi) {
-              r[2 * wi] = cvt_pair(ws[wi], 0x4140);
-              r[2 * wi + 1] = cvt_pair(ws[wi], 0x4342);
-            }
-          } else {
+      for (int c = 0; c < 4; ++c) wv[c] = lds_v4(rb + off[h * 4 + c]);
+    };
+    auto convert = [&](uint32_t (&o)[32], const uint4 (&wv)[4]) {
 #pragma unroll
-            for (int wi = 0; wi < 4; ++wi) {
-              const uint32_t u = ws[wi] ^ 0x80808080u;
-              r[2 * wi] = cvt_pair(u, 0x4140);
-              r[2 * wi + 1] = cvt_pair(u, 0x4342);
-            }
-          }
-          tc_st_32x32b_x8(t_lane + ts * TA_COLS + c * 8, r);
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t ws[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
+#pragma unroll
+        for (int wi = 0; wi < 4; ++wi) {
+          const uint32_t w = TILED ? ws[wi] : ws[wi] ^ 0x80808080u;   // tile-major bytes hold q + 128 already
+          o[c * 8 + 2 * wi] = cvt_pair(w, 0x4140);
+          o[c * 8 + 2 * wi + 1] = cvt_pair(w, 0x4342);
         }
+      }
+    };
+    auto store_half = [&](const uint32_t (&o)[32], int slot) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        tc_st_32x32b_x16(t_lane + slot * TA_SLOT_COLS + c * 16, *reinterpret_cast<const uint32_t(*)[16]>(&o[c * 16]));
+    };
+    Ring<RAW_SLOTS> r;
+    Ring<TA_SLOTS, 2> a(0, 1u);   // a stage takes slots a and a + 1
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const TcUnit it = tc_unit(p, u);
+      polls = kWaitPolls;
+      const int count = it.nst * it.ntile;
+      for (int i = 0; i < count && ok; ++i) {
+        const uint32_t rb = raw + r.slot * RAW_BYTES;
+        uint4 wv[4];
+        uint32_t o[32];
+        mbar_wait2(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, &polls);
+        tc_fence_after();
+        load_half(wv, rb, 0);
+        convert(o, wv);
+        store_half(o, a.slot);
+        load_half(wv, rb, 1);             // the second half is converted while the first one is stored
+        convert(o, wv);
         tc_wait_st();
-        if (warp == CONV_WARP0 && lane == 0) TC_TRACE(i, 7);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&raw_empty[rs]);
-          mbar_arrive(&ta_full[ts]);
+        mbar_arrive_if(ta_full + 8 * a.slot, lane == 0);
+        mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
+        mbar_wait(ta_empty + 8 * (a.slot + 1), a.ph, &polls);
+        tc_fence_after();
+        store_half(o, a.slot + 1);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_if(ta_full + 8 * (a.slot + 1), lane == 0);
+        a.next();
+        r.next();
+        if (polls == 0) {
+          if (lane == 0) tc_report(p.status, 2040, i, count);
+          ok = false;
         }
       }
     }
-
-  } else if (warp >= DRAIN_WARP0) {
+  } else {
     // ------------------------------------------------------------ drain + epilogue
-    // Two warps per lane quarter, each owning half of the token columns.  Blocks are taken two
-    // at a time so one tcgen05.wait::ld covers both loads: the TMEM read latency, not the
-    // arithmetic, is what bounds this role.
+    regs_inc<Cfg::REGS_DRAIN>();
     const int qd = warp & 3;
-    const int half = (warp - DRAIN_WARP0) >> 2;
-    constexpr int HC = MT / 2;  // token columns per drain warp
-    const int nl = qd * 32 + lane;  // row of the tile this thread drains
-    const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16) + ACC_COL0 + half * HC;
-    const int et = tid - DRAIN_WARP0 * 32;  // 0..255 among the drain warps
+    const int g = (warp - DRAIN_WARP0) >> 3;        // the tile of a pair
+    const int th = ((warp - DRAIN_WARP0) >> 2) & 1;
+    const int nl = qd * 32 + lane;                  // row of the tile this thread drains
+    const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16) + Cfg::ACC_COL0;
+    const uint32_t s_lane = scl + nl * 16;
     pdl_wait();  // before any write to global memory (nothing to drain before the activations are in anyway)
-    bool stored = false;  // thread et == 0: a TMA store of this CTA may still be reading the staging tile
-    int gs = 0;
-    int ss = 0;           // slot and phase of the scale ring (SC_STAGES is not a power of two: counted, not divided)
-    uint32_t sph = 0;
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-      const int w = u / p.mtiles;
-      const int64_t m0 = (int64_t)(u - w * p.mtiles) * MT;
-      const int64_t rows_here = (p.m - m0 < MT) ? (p.m - m0) : MT;
-      const TcItem it = tc_item(p, w);
-      const int nst = it.nst;
-      const int64_t n0 = (int64_t)it.tile * TC_ROWS;
-      TC_TRACE_ITEM(w);
-      uint64_t acc2[HC / 2];  // packed f32 pairs: the drain arithmetic uses two-wide f32 FMAs
+    int ent = (2 * g) % ENTRIES;   // entry of the next group
+    int rc = g;                    // scale slot of the next stage
+    uint32_t ph = 0;               // parity of the barriers' next phase: all of them go through one phase a pair stage
+    auto step = [](int& v, int by, int n) {
+      v += by;
+      if (v >= n) v -= n;
+    };
+    // one group: the blocks of a half stage, `hs` the stage's two scales for it
+    auto drain_group = [&](auto hc, float2* sum, uint32_t col, int grp, const float* hs, auto arrivals) {
 #pragma unroll
-      for (int j = 0; j < HC / 2; ++j) acc2[j] = 0ull;
-      for (int i = 0; i < nst && ok; ++i, ++gs) {
-        // the stage's four scales of this row, from the ring
-        if (!mbar_wait(&sc_full[ss], sph)) { ok = false; if (lane == 0) tc_report(p.status, 2051, i, nst); break; }
-        const float4 sc4 = *reinterpret_cast<const float4*>(scl + ss * SC_BYTES + nl * 16);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sc_empty[ss]);
-        if (++ss == SC_STAGES) { ss = 0; sph ^= 1u; }
-        const float scs[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
-        const uint32_t fph = (uint32_t)gs & 1u;
-#pragma unroll
-        for (int pr = 0; pr < 2; ++pr) {
-          if (!mbar_wait(&acc_full[pr], fph)) { ok = false; if (lane == 0) tc_report(p.status, 2050, i, nst); break; }
-          if (warp == DRAIN_WARP0 && lane == 0 && pr == 0) TC_TRACE(i, 8);
-          tc_fence_after();
-          uint32_t b0[HC], b1[HC];
-          tc_ld_cols<HC>(t_lane + (pr * 2) * MT, b0);
-          tc_ld_cols<HC>(t_lane + (pr * 2 + 1) * MT, b1);
-          tc_wait_ld();
-          if (warp == DRAIN_WARP0 && lane == 0) TC_TRACE(i, pr == 0 ? 9 : 14);
-#ifdef LOGOS_TC_TRACE
-          if (trace_on && lane == 0 && i < 64)  // the last of the eight drain warps to get here
-            atomicMax(reinterpret_cast<unsigned long long*>(&p.trace[i * 16 + (pr == 0 ? 3 : 15)]), (unsigned long long)clock64());
-#endif
+      for (int k = 0; k < PER; ++k) {
+        const uint32_t bar = 8 * (PER * grp + k);
+        if (k > 0) mbar_wait(acc_full + bar, ph, &polls);   // (the first hand-off: waited for by the caller)
+        tc_fence_after();
+        drain_blocks<hc, IB, T>(sum, t_lane + col + ent * 2 * T + k * IB * T, hs + k * IB, [&] {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[pr]);
-          const uint64_t sc0 = pack2(scs[2 * pr]), sc1 = pack2(scs[2 * pr + 1]);
-#pragma unroll
-          for (int j = 0; j < HC / 2; ++j) {
-            acc2[j] = ffma2(sc0, pack2(b0[2 * j], b0[2 * j + 1]), acc2[j]);
-            acc2[j] = ffma2(sc1, pack2(b1[2 * j], b1[2 * j + 1]), acc2[j]);
-          }
-          if (warp == DRAIN_WARP0 && lane == 0 && pr == 0) TC_TRACE(i, 10);
-        }
+          mbar_arrive_n_if<arrivals>(acc_empty + bar, lane == 0);
+        });
       }
-      if (warp == DRAIN_WARP0 && lane == 0) TC_TRACE(63, 2);  // main loop of the first item done
+    };
+    constexpr std::integral_constant<int, T / 2> half_cols{};
+    constexpr std::integral_constant<int, T / 4> quarter_cols{};
+    constexpr std::integral_constant<int, 1> one{};
+    constexpr std::integral_constant<int, 2> two{};   // eight warps stand for sixteen arrivals
 
-      // ---- epilogue.  The tile goes to shared memory in the form it will have in global
-      // memory, and one thread hands it to the TMA; the next item's stages are already being
-      // loaded, converted and multiplied meanwhile.  The staging tile is free again once the
-      // previous store has read it.
-      if (et == 0 && stored) bulk_wait_read_all();
-      int all_ok;
-      asm volatile(
-          "{\n\t.reg .pred q, r;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred r, 2, 256, q;\n\tselp.u32 %0, 1, 0, r;\n\t}"
-          : "=r"(all_ok)
-          : "r"((uint32_t)ok)
-          : "memory");  // the eight drain warps agree on leaving
-      if (!all_ok) { ok = false; break; }
-      // element x (0..HC-1) of this thread's row: token half * HC + x
-#define TC_ACC(x) __uint_as_float((uint32_t)(((x) & 1) ? (acc2[(x) >> 1] >> 32) : acc2[(x) >> 1]))
-      const int mode = p.store_mode;
-      if (mode == STORE_TMA_SWIGLU) {
-        // rows (2j, 2j+1) of the tile are (gate_j, up_j): neighbouring lanes.  The even lane
-        // takes the first half of this warp's tokens, the odd lane the second half.
-        __half* eh = reinterpret_cast<__half*>(epi);   // [MT][64] hi plane
-        __half* el = eh + MT * (TC_ROWS / 2);           // [MT][64] lo plane
-        const int par = lane & 1, jj = nl >> 1;
+    int u = blockIdx.x;
+    for (; u < pair_units && ok; u += gridDim.x) {
+      const TcUnit it = tc_unit(p, u);
+      polls = kWaitPolls;
+      float2 acc[T / 4];
 #pragma unroll
-        for (int t = 0; t < HC / 2; ++t) {
-          const float a = TC_ACC(t), b = TC_ACC(t + HC / 2);
-          const float recv = __shfl_xor_sync(0xffffffffu, par ? a : b, 1);
-          const float mine = par ? b : a;
-          const float g = par ? recv : mine, u = par ? mine : recv;
-          const int mm = half * HC + (par ? t + HC / 2 : t);
-          __half h, l;
-          act_split_planes(p.c_act.mode, __fmul_rn(silu_f(g), u), &h, &l);
-          eh[mm * (TC_ROWS / 2) + jj] = h;
-          el[mm * (TC_ROWS / 2) + jj] = l;
-        }
-      } else if (mode == STORE_TMA_PLAIN && p.c_dtype != LOGOS_F32) {
-        __half* e16 = reinterpret_cast<__half*>(epi);  // [MT][128] f16 or bf16
-#pragma unroll
-        for (int x = 0; x < HC; ++x) {
-          const float v = TC_ACC(x);
-          if (p.c_dtype == LOGOS_F16) e16[(half * HC + x) * TC_ROWS + nl] = __float2half_rn(v);
-          else reinterpret_cast<__nv_bfloat16*>(e16)[(half * HC + x) * TC_ROWS + nl] = __float2bfloat16_rn(v);
-        }
-      } else {
-        float* e32 = reinterpret_cast<float*>(epi);    // [MT][128] f32
-#pragma unroll
-        for (int x = 0; x < HC; ++x) e32[(half * HC + x) * TC_ROWS + nl] = TC_ACC(x);
+      for (int x = 0; x < T / 4; ++x) acc[x] = make_float2(0.f, 0.f);
+      for (int i = 0; i < it.nst && polls != 0; ++i) {
+        mbar_wait(acc_full + 8 * PER * (2 * g), ph, &polls);
+        const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
+        const float s[4] = {__uint_as_float(sc.x), __uint_as_float(sc.y), __uint_as_float(sc.z), __uint_as_float(sc.w)};
+        drain_group(half_cols, acc, th * (T / 2), 2 * g, s, two);
+        step(ent, 1 % ENTRIES, ENTRIES);
+        mbar_wait(acc_full + 8 * PER * (2 * g + 1), ph, &polls);
+        drain_group(half_cols, acc, th * (T / 2), 2 * g + 1, s + 2, two);
+        step(ent, 3 % ENTRIES, ENTRIES);            // past the other tile's two groups
+        step(rc, 2, SC_SLOTS);
+        ph ^= 1u;
       }
-#undef TC_ACC
-      if (mode != STORE_GENERIC) fence_proxy_async_smem();
-      if (warp == DRAIN_WARP0 && lane == 0) TC_TRACE(63, 5);  // staged
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (mode != STORE_GENERIC) {
-        if (et == 0) {
-          if (mode == STORE_TMA_PARTIAL) {
-            tma_store_3d(&map_o0, epi, (int)n0, (int)m0, it.split);
-          } else if (mode == STORE_TMA_PLAIN) {
-            tma_store_2d(&map_o0, epi, (int)n0, (int)m0);
-          } else {
-            tma_store_2d(&map_o0, epi, (int)(n0 >> 1), (int)m0);
-            if (p.c_act.mode == LOGOS_F32) tma_store_2d(&map_o1, epi + MT * TC_ROWS, (int)(n0 >> 1), (int)m0);
-          }
-          bulk_commit();
-          stored = true;
-        }
-      } else {
-        const float* stage_c = reinterpret_cast<const float*>(epi);
-        if (p.splits <= 1 && p.epilogue == EPI_SWIGLU) {
-          // rows (2j, 2j+1) of the tile are (gate_j, up_j): 64 outputs per token
-          const int64_t out0 = n0 >> 1;
-          const int64_t outs = ((p.n - n0 < TC_ROWS ? p.n - n0 : TC_ROWS)) >> 1;
-#pragma unroll 4
-          for (int e = et; e < MT * (TC_ROWS / 2); e += 256) {
-            const int mm = e / (TC_ROWS / 2), jj = e % (TC_ROWS / 2);
-            if (mm < rows_here && jj < outs) {
-              const float g = stage_c[mm * TC_ROWS + 2 * jj], u = stage_c[mm * TC_ROWS + 2 * jj + 1];
-              store_c(p, (m0 + mm) * p.ldc + out0 + jj, __fmul_rn(silu_f(g), u));
-            }
-          }
-        } else {
-          const int64_t cols_here = (p.n - n0 < TC_ROWS) ? (p.n - n0) : TC_ROWS;
-#pragma unroll 4
-          for (int e = et; e < MT * TC_ROWS; e += 256) {
-            const int mm = e / TC_ROWS, nn = e % TC_ROWS;
-            if (mm < rows_here && nn < cols_here) {
-              float v = stage_c[mm * TC_ROWS + nn];
-              if (p.splits > 1) {
-                p.partials[((int64_t)it.split * p.m + m0 + mm) * p.n + n0 + nn] = v;
-              } else {
-                const int64_t ci = (m0 + mm) * p.ldc + n0 + nn;
-                if (p.epilogue == EPI_RESIDUAL) v = __fadd_rn(v, load_aux(p, ci));
-                store_c(p, ci, v);
-              }
-            }
-          }
-        }
+      if (polls == 0) {
+        if (lane == 0) tc_report(p.status, 2050, 0, it.nst);
+        ok = false;
+        break;
       }
-      if (warp == DRAIN_WARP0 && lane == 0) TC_TRACE(63, 3);  // first item's stores issued
+      store_tile<T / 2>(p, acc, it.split, (int64_t)(it.tile + g) * TC_ROWS + nl, (int64_t)it.mtile * T + th * (T / 2), lane);
     }
-    // global writes of the TMA stores are complete before the CTA ends
-    if (et == 0 && stored) bulk_wait_all();
+    // From here on a warp waits for barriers that only the other tile's warps have followed so far: once all have
+    // come this far, their phases of the pair units are over.  (Every drain warp passes here exactly once.)
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    ent = (ent + 2 * ENTRIES - 2 * g) % ENTRIES;
+    rc = (rc + SC_SLOTS - g) % SC_SLOTS;
+    int sp = 0;                                     // stage parity: groups 2 sp, 2 sp + 1
+    for (; u < units && ok; u += gridDim.x) {
+      const TcUnit it = tc_unit(p, u);
+      polls = kWaitPolls;
+      float2 acc[T / 8];
+#pragma unroll
+      for (int x = 0; x < T / 8; ++x) acc[x] = make_float2(0.f, 0.f);
+      const uint32_t col = (2 * g + th) * (T / 4);
+      for (int i = 0; i < it.nst && polls != 0; ++i) {
+        mbar_wait(acc_full + 8 * PER * (2 * sp), ph, &polls);
+        const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
+        const float s[4] = {__uint_as_float(sc.x), __uint_as_float(sc.y), __uint_as_float(sc.z), __uint_as_float(sc.w)};
+        drain_group(quarter_cols, acc, col, 2 * sp, s, one);
+        step(ent, 1, ENTRIES);
+        mbar_wait(acc_full + 8 * PER * (2 * sp + 1), ph, &polls);
+        drain_group(quarter_cols, acc, col, 2 * sp + 1, s + 2, one);
+        step(ent, 1, ENTRIES);
+        step(rc, 1, SC_SLOTS);
+        ph ^= (uint32_t)sp;
+        sp ^= 1;
+      }
+      if (polls == 0) {
+        if (lane == 0) tc_report(p.status, 2051, 0, it.nst);
+        ok = false;
+        break;
+      }
+      store_tile<T / 4>(p, acc, it.split, (int64_t)it.tile * TC_ROWS + nl, (int64_t)it.mtile * T + col, lane);
+    }
   }
 
   tc_fence_before();
   __syncthreads();
-#ifdef LOGOS_TC_TRACE
-  if (tid == 0) { trace_on = cta0; TC_TRACE(63, 4); }
-#endif
   if (warp == 3) {
     __syncwarp();
     tc_fence_after();
@@ -662,10 +662,6 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 }
 
 // ---------------------------------------------------------------- host side
-#ifdef LOGOS_TC_TRACE
-long long* g_trace = nullptr;  // set through logos_gemm_trace_buffer; null = tracing off
-#endif
-
 struct MapKey {
   const void* base;
   uint64_t d0, d1, d2, pitch1, pitch2;
@@ -714,109 +710,149 @@ logos_status_t cached_map(CUtensorMap* out, const void* base, CUtensorMapDataTyp
 
 namespace {
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+// How a product is cut up: tokens per tile, K splits, and the row tiles that run in pairs and alone.
+struct TcPlan {
+  int t, splits, pairs, solos;
+};
 
-template <int MT, int LIMBS>
-logos_status_t launch_t(const GemmArgs& g, cudaStream_t st) {
-  using Cfg = TcCfg<MT, LIMBS>;
-  CUtensorMap mq, mhi, mlo, mo0, mo1, ms;
+// Cycles of one K stage of a pair and of a single tile, by tokens per tile (timings of this kernel), of the
+// pipeline fill plus the last epilogue, and of a unit's epilogue.
+struct TcCost {
+  int t, pair, solo;
+};
+constexpr TcCost kCosts[] = {{16, 1450, 760}, {32, 1450, 760}, {64, 1500, 860}, {96, 1900, 1100}};
+constexpr int kFillCycles = 6000, kUnitCycles = 700;
+
+// The slowest CTA's time when `pairs` pair items and `solos` single tiles run round robin on g CTAs.
+int64_t plan_cycles(const TcCost& c, int64_t pairs, int64_t solos, int64_t sp, int64_t mt, int64_t stages, int64_t g) {
+  const int64_t pu = pairs * sp * mt, total = (pairs + solos) * sp * mt;
+  const int64_t per = (stages + sp - 1) / sp;
+  const int64_t tp = per * c.pair + kUnitCycles, ts = per * c.solo + kUnitCycles;
+  int64_t worst = 0;
+  for (int64_t cta : {(int64_t)0, pu % g, pu % g - 1, total % g - 1}) {
+    if (cta < 0 || cta >= g) continue;
+    const int64_t np = pu > cta ? (pu - cta + g - 1) / g : 0, nt = total > cta ? (total - cta + g - 1) / g : 0;
+    worst = std::max(worst, np * tp + (nt - np) * ts);
+  }
+  return worst + kFillCycles;
+}
+
+TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int sms) {
+  const int64_t tl = (n + TC_ROWS - 1) / TC_ROWS, stages = (k + TC_KSTAGE - 1) / TC_KSTAGE;
+  TcPlan best{16, 1, 0, (int)tl};
+  int64_t best_cost = INT64_MAX;
+  for (const TcCost& c : kCosts) {
+    // fewer tokens than half a larger tile never pay for it
+    if (c.t < 64 && m > c.t) continue;
+    if (c.t > 16 && m <= c.t / 2 && c.t <= 64) continue;
+    if (c.t == 96 && m <= 64) continue;
+    const int64_t mt = (m + c.t - 1) / c.t;
+    int64_t sp_lo = 1, sp_hi = 1;
+    if (forced_splits > 0) sp_lo = sp_hi = forced_splits;
+    else if (tl * mt < sms && stages >= 8) sp_hi = std::min<int64_t>(16, stages / 4);   // at least 4 stages (512 columns) per split
+    for (int64_t sp = sp_lo; sp <= sp_hi; ++sp) {
+      const int64_t full_rounds = tl * sp * mt / (2 * sms);
+      const int64_t cand[3] = {0, tl / 2, std::min<int64_t>(tl / 2, full_rounds * sms / (sp * mt))};
+      for (int64_t pairs : cand) {
+        int64_t cost = plan_cycles(c, pairs, tl - 2 * pairs, sp, mt, stages, sms);
+        // partial sums are written and read back through L2 (about 4.4 KB per cycle) and folded by one more kernel
+        if (sp > 1) cost += 2000 + 8 * sp * m * n / 4400;
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = TcPlan{c.t, (int)sp, (int)pairs, (int)(tl - 2 * pairs)};
+        }
+      }
+    }
+  }
+  return best;
+}
+
+// Plans are pure functions of the shape: the last ones of a thread are kept.
+TcPlan plan_for(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int device) {
+  struct Entry {
+    int64_t m = -1, n = 0, k = 0, sp = 0;
+    int device = 0;
+    TcPlan plan{};
+  };
+  thread_local Entry cache[64];
+  const uint64_t h = ((uint64_t)m * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)n * 0xBF58476D1CE4E5B9ull) ^ ((uint64_t)k * 0x94D049BB133111EBull) ^
+                     (uint64_t)forced_splits;
+  Entry& e = cache[(h ^ (h >> 29)) >> 7 & 63];
+  if (e.m != m || e.n != n || e.k != k || e.sp != forced_splits || e.device != device) {
+    e.m = m; e.n = n; e.k = k; e.sp = forced_splits; e.device = device;
+    e.plan = make_plan(m, n, k, forced_splits, sm_count(device));
+  }
+  return e.plan;
+}
+
+template <int T, int LIMBS>
+logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) {
+  using Cfg = TcCfg<T, LIMBS>;
+  CUtensorMap mq, mhi, mlo, ms;
+  const int64_t stages = (g.k + TC_KSTAGE - 1) / TC_KSTAGE, tiles = (g.n + TC_ROWS - 1) / TC_ROWS;
   if (g.q_tiled) {
-    const uint64_t rows = (uint64_t)((g.n + TC_ROWS - 1) / TC_ROWS) * (uint64_t)(g.k / TC_KSTAGE) * TC_ROWS;
+    const uint64_t rows = (uint64_t)tiles * (uint64_t)stages * TC_ROWS;
     LOGOS_TRY(cached_map(&mq, g.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, TC_KSTAGE, rows, TC_KSTAGE, TC_KSTAGE, TC_ROWS));
   } else {
     LOGOS_TRY(cached_map(&mq, g.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)g.k, (uint64_t)g.n, (uint64_t)g.k, TC_KSTAGE, TC_ROWS));
   }
-  LOGOS_TRY(cached_map(&mhi, g.a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)g.k, (uint64_t)g.m, (uint64_t)g.lda * 2, 64, MT));
+  LOGOS_TRY(cached_map(&mhi, g.a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)g.k, (uint64_t)g.m, (uint64_t)g.lda * 2, 64, T));
   if (LIMBS == 2)
-    LOGOS_TRY(cached_map(&mlo, g.a_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)g.k, (uint64_t)g.m, (uint64_t)g.lda * 2, 64, MT));
+    LOGOS_TRY(cached_map(&mlo, g.a_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)g.k, (uint64_t)g.m, (uint64_t)g.lda * 2, 64, T));
   else
     mlo = mhi;
   ms = mhi;
-  if (!g.q_tiled)
+  const bool s_tiled = g.q_tiled || g.s_tiled;
+  if (!s_tiled)
     LOGOS_TRY(cached_map(&ms, g.s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)(g.k / 32), (uint64_t)g.n, (uint64_t)(g.k / 32) * 4, 4,
                          TC_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE));
   TcParams p{};
-  p.s = g.s; p.n = g.n; p.k = g.k; p.m = g.m;
+  p.s = g.s; p.n = g.n; p.m = g.m;
   p.c = g.c; p.c_dtype = g.c_dtype; p.c_act = g.c_act; p.ldc = g.ldc; p.aux = g.aux; p.epilogue = g.epilogue;
   p.partials = g.partials;
-  p.tiled = g.q_tiled;
-  p.splits = g.splits > 1 ? g.splits : 1;
-  p.stages_total = (int)(g.k / TC_KSTAGE);
-  const int64_t tiles = (g.n + TC_ROWS - 1) / TC_ROWS;
-  if (tiles * p.splits > INT32_MAX) return fail(LOGOS_OUT_OF_BOUNDS, "q8_gemm: too many work items");
-  p.items = (int)(tiles * p.splits);
+  p.splits = plan.splits;
+  p.stages_total = (int)stages;
+  p.s_tiled = s_tiled;
+  const int64_t mtiles = (g.m + T - 1) / T;
+  const int64_t units = (int64_t)(plan.pairs + plan.solos) * plan.splits * mtiles;
+  if (units > INT32_MAX / 4 || tiles * stages > INT32_MAX / TC_ROWS) return fail(LOGOS_OUT_OF_BOUNDS, "q8_gemm: too many work units");
+  p.pairs = plan.pairs;
+  p.solos = plan.solos;
+  p.mtiles = (int)mtiles;
+  const int64_t groups = (mtiles + 11) / 12;   // about 12 token tiles x 12 row tiles of 256 run side by side
+  p.group = (int)((mtiles + groups - 1) / groups);
+  p.stream_once = mtiles == 1;
   p.status = kernel_status_ptr(g.device);
-#ifdef LOGOS_TC_TRACE
-  p.trace = g_trace;
-  if (g_trace) {
-    // optional filter: trace only launches whose grid has this many row tiles
-    static const char* f = getenv("LOGOS_B200_TRACE_TILES");
-    if (f && atoi(f) != (int)tiles) p.trace = nullptr;
-  }
-#endif
   if (!p.status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   if (p.splits > p.stages_total) return fail(LOGOS_ERROR, "q8_gemm: more K splits than 128-column stages");
 
-  // How the tile is stored: through the TMA where the destination allows a tensor map
-  // (16-byte aligned base and row pitch), else by a loop of plain stores.
-  static const bool no_tma_store = getenv("LOGOS_B200_GEMM_PLAIN_STORES") != nullptr;
-  p.store_mode = STORE_GENERIC;
-  mo0 = mq;
-  mo1 = mq;
-  if (no_tma_store) {
-  } else if (p.splits > 1) {
-    if (aligned16(g.partials) && g.n % 4 == 0) {
-      LOGOS_TRY(cached_map(&mo0, g.partials, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)g.n, (uint64_t)g.m,
-                           (uint64_t)g.n * 4, TC_ROWS, MT, CU_TENSOR_MAP_SWIZZLE_NONE, (uint64_t)p.splits,
-                           (uint64_t)g.m * g.n * 4));
-      p.store_mode = STORE_TMA_PARTIAL;
-    }
-  } else if (g.epilogue == EPI_NONE &&
-             (g.c_dtype == LOGOS_F32 || g.c_dtype == LOGOS_F16 || g.c_dtype == LOGOS_BF16)) {
-    const uint32_t eb = g.c_dtype == LOGOS_F32 ? 4 : 2;
-    const CUtensorMapDataType dt = g.c_dtype == LOGOS_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                   : g.c_dtype == LOGOS_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                            : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    if (aligned16(g.c) && (g.ldc * eb) % 16 == 0) {
-      LOGOS_TRY(cached_map(&mo0, g.c, dt, eb, (uint64_t)g.n, (uint64_t)g.m, (uint64_t)g.ldc * eb, TC_ROWS, MT,
-                           CU_TENSOR_MAP_SWIZZLE_NONE));
-      p.store_mode = STORE_TMA_PLAIN;
-    }
-  } else if (g.epilogue == EPI_SWIGLU && g.c_dtype == LOGOS_ACT_PLANES && g.n % 2 == 0) {
-    const bool two = g.c_act.mode == LOGOS_F32;
-    if (aligned16(g.c_act.hi) && (!two || aligned16(g.c_act.lo)) && (g.ldc * 2) % 16 == 0) {
-      LOGOS_TRY(cached_map(&mo0, g.c_act.hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)(g.n / 2), (uint64_t)g.m,
-                           (uint64_t)g.ldc * 2, TC_ROWS / 2, MT, CU_TENSOR_MAP_SWIZZLE_NONE));
-      if (two)
-        LOGOS_TRY(cached_map(&mo1, g.c_act.lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)(g.n / 2),
-                             (uint64_t)g.m, (uint64_t)g.ldc * 2, TC_ROWS / 2, MT, CU_TENSOR_MAP_SWIZZLE_NONE));
-      p.store_mode = STORE_TMA_SWIGLU;
-    }
-  }
-
-  auto kernel = g.q_tiled ? q8_gemm_tc_kernel<MT, LIMBS, true> : q8_gemm_tc_kernel<MT, LIMBS, false>;
+  auto kernel = g.q_tiled ? q8_gemm_tc_kernel<T, LIMBS, true> : q8_gemm_tc_kernel<T, LIMBS, false>;
   LOGOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
   // persistent CTAs: one per SM at most, each takes units blockIdx.x, blockIdx.x + gridDim.x, ...
   const int sms = sm_count(g.device);
-  const int64_t mtiles = (g.m + MT - 1) / MT;
-  if ((int64_t)p.items * mtiles > INT32_MAX) return fail(LOGOS_OUT_OF_BOUNDS, "q8_gemm: too many work units");
-  p.mtiles = (int)mtiles;
-  const int64_t units = (int64_t)p.items * mtiles;
   dim3 grid((unsigned)(units < sms ? units : sms), 1u, 1u);
-  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(TC_THREADS), Cfg::SMEM, st, mq, mhi, mlo, mo0, mo1, ms, p));
+  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(TC_THREADS), Cfg::SMEM, st, mq, mhi, mlo, ms, p));
   count_launch(LK_GEMM_TC);
   return check_launch("q8_gemm_tc_kernel");
 }
 
-}  // namespace
+template <int LIMBS>
+logos_status_t launch_plan(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) {
+  switch (plan.t) {
+    case 16: return launch_t<16, LIMBS>(g, plan, st);
+    case 32: return launch_t<32, LIMBS>(g, plan, st);
+    case 64: return launch_t<64, LIMBS>(g, plan, st);
+    default: return launch_t<96, LIMBS>(g, plan, st);
+  }
+}
 
-#ifdef LOGOS_TC_TRACE
-void gemm_set_trace(long long* buf) { g_trace = buf; }
-#endif
+}  // namespace
 
 bool gemm_tc_applicable(const GemmArgs& g) {
   if (g.a_dtype != LOGOS_F16) return false;
-  if (g.k < TC_KSTAGE || g.k % TC_KSTAGE) return false;
+  if (g.k < TC_KSTAGE || g.k % 32) return false;
+  // K of whole stages, or scales in the tile-major form: the row-major box needs rows of 16-byte multiples
+  if (g.k % TC_KSTAGE && !g.q_tiled && !g.s_tiled) return false;
   if (g.m < 1 || g.n < 1) return false;
   if (g.lda % 8) return false;
   if ((reinterpret_cast<uintptr_t>(g.a) & 15u) || (reinterpret_cast<uintptr_t>(g.a_lo) & 15u) ||
@@ -825,11 +861,11 @@ bool gemm_tc_applicable(const GemmArgs& g) {
   return true;
 }
 
+int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device) { return plan_for(m, n, k, 0, device).splits; }
+
 logos_status_t launch_q8_gemm_tc(const GemmArgs& g, cudaStream_t st) {
-  const bool two = g.a_lo != nullptr;
-  if (g.m <= 16) return two ? launch_t<16, 2>(g, st) : launch_t<16, 1>(g, st);
-  if (g.m <= 32) return two ? launch_t<32, 2>(g, st) : launch_t<32, 1>(g, st);
-  return two ? launch_t<64, 2>(g, st) : launch_t<64, 1>(g, st);
+  const TcPlan plan = plan_for(g.m, g.n, g.k, g.splits > 1 ? g.splits : 1, g.device);
+  return g.a_lo ? launch_plan<2>(g, plan, st) : launch_plan<1>(g, plan, st);
 }
 
 }  // namespace logos
