@@ -338,14 +338,51 @@ tp_residual_rmsnorm_kernel(float* __restrict__ h, const TpFusedArgs t, int parts
   }
 }
 
-__global__ void bf16_to_f16_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ y, int64_t count) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) y[i] = __float2half_rn(act_clamp(__bfloat162float(x[i])));
-}
-
-__global__ void act_split_kernel(const float* __restrict__ x, ActOut o, int64_t count) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) act_store(o, i, x[i]);
+// See launch_gemm_prep.  Eight activations a thread (K is a multiple of 32, so rows and planes stay 16-byte
+// aligned), then four scales a thread: one row of a K tile.
+template <bool BF16>
+__global__ void __launch_bounds__(256)
+gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const float* __restrict__ s, float* __restrict__ tiled,
+                 int64_t n, int64_t kb, int64_t ktiles, int64_t act_blocks) {
+  pdl_trigger();
+  if ((int64_t)blockIdx.x < act_blocks) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= count8) return;
+    float x[8];
+    if (BF16) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a) + i);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[2 * j] = __uint_as_float(w[j] << 16);
+        x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+      }
+    } else {
+      const float4 v0 = __ldg(reinterpret_cast<const float4*>(a) + 2 * i), v1 = __ldg(reinterpret_cast<const float4*>(a) + 2 * i + 1);
+      x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
+      x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
+    }
+    __half hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float c = act_clamp(x[j]);
+      hi[j] = __float2half_rn(c);
+      lo[j] = __float2half_rn((c - __half2float(hi[j])) * 2048.f);
+    }
+    reinterpret_cast<uint4*>(o.hi)[i] = *reinterpret_cast<const uint4*>(hi);
+    if (o.mode == LOGOS_F32) reinterpret_cast<uint4*>(o.lo)[i] = *reinterpret_cast<const uint4*>(lo);
+    return;
+  }
+  const int64_t i = ((int64_t)blockIdx.x - act_blocks) * 256 + threadIdx.x;   // (row, K tile), K tile fastest
+  const int64_t row = i / ktiles, kt = i - row * ktiles;
+  if (row >= n) return;
+  float4 v;
+  const float* src = s + row * kb + kt * 4;
+  v.x = __ldg(src);
+  v.y = kt * 4 + 1 < kb ? __ldg(src + 1) : 0.f;
+  v.z = kt * 4 + 2 < kb ? __ldg(src + 2) : 0.f;
+  v.w = kt * 4 + 3 < kb ? __ldg(src + 3) : 0.f;
+  reinterpret_cast<float4*>(tiled)[((row >> 7) * ktiles + kt) * 128 + (row & 127)] = v;
 }
 
 // Order-preserving map of a float onto unsigned integers, and back.
@@ -482,18 +519,19 @@ logos_status_t launch_embed(const int32_t* tokens, const int8_t* q, const float*
   return check_launch("embed_kernel");
 }
 
-logos_status_t launch_bf16_to_f16(const __nv_bfloat16* x, __half* y, int64_t count, cudaStream_t st) {
-  if (count == 0) return LOGOS_OK;
-  bf16_to_f16_kernel<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(x, y, count);
+logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t count, const float* s,
+                                float* tiled_or_null, int64_t n, int64_t k, cudaStream_t st) {
+  if (count % 8 || (reinterpret_cast<uintptr_t>(a) & 15u))
+    return fail(LOGOS_ERROR, "gemm_prep: activations must be 16-byte aligned and a multiple of 8");
+  const int64_t count8 = count / 8, ktiles = (k + 127) / 128;
+  const int64_t act_blocks = (count8 + 255) / 256, scale_blocks = tiled_or_null ? (n * ktiles + 255) / 256 : 0;
+  const dim3 grid((unsigned)(act_blocks + scale_blocks));
+  if (a_dtype == LOGOS_BF16)
+    gemm_prep_kernel<true><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks);
+  else
+    gemm_prep_kernel<false><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks);
   count_launch(LK_ELEMWISE);
-  return check_launch("bf16_to_f16_kernel");
-}
-
-logos_status_t launch_act_split(const float* x, ActOut o, int64_t count, cudaStream_t st) {
-  if (count == 0) return LOGOS_OK;
-  act_split_kernel<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(x, o, count);
-  count_launch(LK_ELEMWISE);
-  return check_launch("act_split_kernel");
+  return check_launch("gemm_prep_kernel");
 }
 
 logos_status_t launch_residual_rmsnorm(float* h, const float* delta, int parts, int64_t part_stride,

@@ -180,10 +180,12 @@ struct TpFusedArgs {
 };
 logos_status_t launch_tp_residual_rmsnorm(float* h, const TpFusedArgs& t, int parts, int64_t part_stride, const float* g,
                                           int64_t rows, int64_t hidden, float eps, int device, cudaStream_t st);
-// bf16 [count] -> fp16 plane (exact inside fp16's normal range, saturating outside)
-logos_status_t launch_bf16_to_f16(const __nv_bfloat16* x, __half* y, int64_t count, cudaStream_t st);
-// f32 [count] -> activation planes
-logos_status_t launch_act_split(const float* x, ActOut o, int64_t count, cudaStream_t st);
+// What a stand-alone product needs before it starts, in one launch: `count` activations (LOGOS_BF16 or LOGOS_F32)
+// into planes (mode LOGOS_F16: one plane, exact for bf16 inside fp16's normal range, saturating outside;
+// LOGOS_F32: two), and, where tiled_or_null is set, scales [n][k/32] into the tile-major form
+// [row tile][K tile][128 rows][4], zero past K (rows past n are left alone: their products are dropped).
+logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t count, const float* s,
+                                float* tiled_or_null, int64_t n, int64_t k, cudaStream_t st);
 // Sampling state of a model, in device memory so that a captured step follows changes to it.
 struct SamplingParams {
   float inv_temperature;  // 1 / T

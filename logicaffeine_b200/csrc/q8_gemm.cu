@@ -1,9 +1,9 @@
 // Q8 GEMM front: C[m,n] = sum_kb s[n,kb] * sum_k A[m,k] * q[n,k].
 //
 // Dispatch between two kernels:
-//   * q8_gemm_tc.cu — the tcgen05 / TMA kernel used for every shape the decode
-//     step produces (K a multiple of 128, N a multiple of 128, M <= 256);
-//   * the SIMT kernel below — any other shape, and the on-device cross-check
+//   * q8_gemm_tc.cu — the tcgen05 / TMA kernel: K of at least 128, 16-byte aligned operands, and K a
+//     multiple of 128 or scales in the tile-major form (the stand-alone operators bring them there);
+//   * the SIMT kernel below — anything else, and the on-device cross-check
 //     the tests hold the tensor-core kernel against.
 // Plus the split-K reduction + epilogue kernel shared by both.
 #include "ops.cuh"
@@ -146,6 +146,61 @@ logos_status_t launch_q8_gemm(const GemmArgs& g, cudaStream_t st) {
 
 using namespace logos;
 
+// The stand-alone operators' way to the tensor-core kernel: activations into fp16 planes (and, where K is not
+// a multiple of 128, scales into the tile-major form) by one small kernel, then the product, then the
+// fold of the K splits.  The launches after the first are dependent ones: each kernel sets up, and the
+// product fetches its first weights, while the one before it finishes.  Nothing here writes weights, and the
+// first kernel is an ordinary launch, so what ran before in the stream has ended.
+static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) {
+  const void* src = g.a;
+  const int src_dtype = g.a_dtype;
+  const int64_t stages = (g.k + 127) / 128;
+  const bool retile = g.k % 128 != 0;
+  const int splits = gemm_pick_splits(g.m, g.n, g.k, g.device);
+  auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
+  const int64_t plane_bytes = up(g.m * g.k * 2);
+  const int64_t scale_bytes = retile ? up((g.n + 127) / 128 * stages * 2048) : 0;
+  const int64_t part_bytes = splits > 1 ? (int64_t)splits * g.m * g.n * (int64_t)sizeof(float) : 0;
+  void* scratch = nullptr;
+  LOGOS_TRY(scratch_get(g.device, 0, (two_planes ? 2 : 1) * plane_bytes + scale_bytes + part_bytes, &scratch));
+  char* at = static_cast<char*>(scratch);
+  ActOut planes;
+  planes.hi = reinterpret_cast<__half*>(at);
+  planes.lo = two_planes ? reinterpret_cast<__half*>(at + plane_bytes) : nullptr;
+  planes.mode = two_planes ? LOGOS_F32 : LOGOS_F16;
+  at += (two_planes ? 2 : 1) * plane_bytes;
+  float* tiled = retile ? reinterpret_cast<float*>(at) : nullptr;
+  at += scale_bytes;
+  LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m * g.k, g.s, tiled, g.n, g.k, st));
+  g.a = planes.hi;
+  g.a_lo = planes.lo;
+  g.a_dtype = LOGOS_F16;
+  if (retile) {
+    g.s = tiled;
+    g.s_tiled = 1;
+  }
+  PdlScope pdl(true);
+  if (splits <= 1) return launch_q8_gemm(g, st);
+  GemmArgs gp = g;
+  gp.splits = splits;
+  gp.partials = reinterpret_cast<float*>(at);
+  gp.epilogue = EPI_NONE;
+  gp.c = nullptr;
+  gp.c_dtype = LOGOS_F32;
+  gp.aux = nullptr;
+  LOGOS_TRY(launch_q8_gemm(gp, st));
+  return launch_splitk_reduce(gp.partials, splits, g.c, g.c_dtype, ActOut(), g.ldc, g.aux, g.m, g.n, g.epilogue, st);
+}
+
+// Whether the operands of a stand-alone call can go to the tensor-core kernel once prepared (the planes and, where
+// needed, the scales are scratch of the library's own then).
+static bool gemm_tensor_takes(GemmArgs g) {
+  g.a_dtype = LOGOS_F16;
+  g.a = g.a_lo = nullptr;
+  g.s_tiled = g.k % 128 != 0;
+  return gemm_tc_applicable(g);
+}
+
 static logos_status_t gemm_abi(logos_handle_t a, logos_handle_t q, logos_handle_t s, logos_handle_t c, int64_t m,
                                int64_t n, int64_t k, int32_t epilogue, logos_handle_t aux, void* stream,
                                int force_simt) {
@@ -177,31 +232,10 @@ static logos_status_t gemm_abi(logos_handle_t a, logos_handle_t q, logos_handle_
   g.device = dev;
   g.force_simt = force_simt;
   cudaStream_t st = as_stream(stream);
-  if (force_simt) return launch_q8_gemm(g, st);
   // Tensor-core path: the kernel multiplies fp16 planes.  A bf16 value is exactly
   // representable in fp16 inside fp16's normal range, so one plane is enough.
-  GemmArgs t = g;
-  t.a_dtype = LOGOS_F16;
-  t.a = reinterpret_cast<const void*>(uintptr_t(16));  // placeholder so applicability can be asked first
-  if (!gemm_tc_applicable(t)) return launch_q8_gemm(g, st);
-  int splits = gemm_pick_splits(m, n, k, dev);
-  void* scratch = nullptr;
-  int64_t plane_bytes = ((m * k * 2 + 255) / 256) * 256;
-  int64_t part_bytes = splits > 1 ? (int64_t)splits * m * n * (int64_t)sizeof(float) : 0;
-  LOGOS_TRY(scratch_get(dev, 0, plane_bytes + part_bytes, &scratch));
-  __half* plane = reinterpret_cast<__half*>(scratch);
-  LOGOS_TRY(launch_bf16_to_f16(ap, plane, m * k, st));
-  t.a = plane;
-  if (splits > 1) {
-    GemmArgs gp = t;
-    gp.splits = splits;
-    gp.partials = reinterpret_cast<float*>(static_cast<char*>(scratch) + plane_bytes);
-    gp.epilogue = EPI_NONE;
-    gp.c = nullptr;
-    LOGOS_TRY(launch_q8_gemm(gp, st));
-    return launch_splitk_reduce(gp.partials, splits, cp, LOGOS_BF16, ActOut(), n_out, xp, m, n, epilogue, st);
-  }
-  return launch_q8_gemm(t, st);
+  if (force_simt || !gemm_tensor_takes(g)) return launch_q8_gemm(g, st);
+  return gemm_tensor(g, false, st);
 }
 
 extern "C" {
@@ -229,30 +263,8 @@ logos_status_t logos_q8_gemm_f32(logos_handle_t a, logos_handle_t q, logos_handl
     g.c = cp; g.c_dtype = LOGOS_F32; g.ldc = n;
     g.m = m; g.n = n; g.k = k;
     g.device = dev;
-    GemmArgs t = g;
-    t.a_dtype = LOGOS_F16;
-    t.a = reinterpret_cast<const void*>(uintptr_t(16));
-    if (m == 0 || n == 0 || !gemm_tc_applicable(t)) return launch_q8_gemm(g, st);
-    int splits = gemm_pick_splits(m, n, k, dev);
-    int64_t plane_bytes = ((m * k * 2 + 255) / 256) * 256;
-    int64_t part_bytes = splits > 1 ? (int64_t)splits * m * n * (int64_t)sizeof(float) : 0;
-    void* scratch = nullptr;
-    LOGOS_TRY(scratch_get(dev, 0, 2 * plane_bytes + part_bytes, &scratch));
-    ActOut planes;
-    planes.hi = reinterpret_cast<__half*>(scratch);
-    planes.lo = reinterpret_cast<__half*>(static_cast<char*>(scratch) + plane_bytes);
-    planes.mode = LOGOS_F32;
-    LOGOS_TRY(launch_act_split(ap, planes, m * k, st));
-    t.a = planes.hi;
-    t.a_lo = planes.lo;
-    if (splits > 1) {
-      t.splits = splits;
-      t.partials = reinterpret_cast<float*>(static_cast<char*>(scratch) + 2 * plane_bytes);
-      t.c = nullptr;
-      LOGOS_TRY(launch_q8_gemm(t, st));
-      return launch_splitk_reduce(t.partials, splits, cp, LOGOS_F32, ActOut(), n, nullptr, m, n, EPI_NONE, st);
-    }
-    return launch_q8_gemm(t, st);
+    if (!gemm_tensor_takes(g)) return launch_q8_gemm(g, st);
+    return gemm_tensor(g, true, st);
   });
 }
 

@@ -14,7 +14,7 @@
 //   TMA  int8 weights [128 rows][128 B], 128-byte swizzle, and the stage's scales [128 rows][4]
 //        -> shared-memory rings                                                    (warp 0)
 //   TMA  fp16 activation planes [T][64] of half a stage -> ring                     (warp 1)
-//   4 converter warps (one per TMEM lane quarter): int8 -> fp16 (exact: 0x6400|b trick),
+//   4 or 8 converter warps (one or two per TMEM lane quarter): int8 -> fp16 (exact: 0x6400|b trick),
 //        tcgen05.st into the operand ring; the weights never go back to shared memory
 //   MMA warps 2 and 3, one per half: per Q8 block two tcgen05.mma kind::f16 (K = 16 each) per plane, A
 //        from TMEM, B = activations from smem, into a fresh accumulator entry: first q*lo', then
@@ -61,17 +61,20 @@ constexpr int SC_BYTES = TC_ROWS * 16;          // four f32 per row and stage
 constexpr int TA_SLOTS = 4;                     // operand ring, in groups
 constexpr int TA_SLOT_COLS = 32;                // TMEM columns of 64 fp16 per row
 constexpr uint32_t TMEM_COLS = 512;
-constexpr int GROUPS = 4;                       // groups of a pair's stage (2 tiles x 2 halves): one set of barriers each
-constexpr int DRAIN_WARP0 = 8;                  // 4 single-role warps, 4 converter warps, 16 drain warps
-constexpr int TC_THREADS = 768;
+// Barrier sets of the accumulators: group n hands off through set n % GROUPS, over entry n % ENTRIES.  The MMA warp
+// of one half may wait for releases of the other half's groups (odd ENTRIES).  Those run at most one pair stage
+// (four groups) ahead of it, because the drain takes the halves in turn; with eight sets a set cannot go
+// through a second phase unseen, which the parity test could not tell from none (with four it could).
+constexpr int GROUPS = 8;
+constexpr int CONV_WARP0 = 4;                   // 4 single-role warps, 4 or 8 converter warps, 16 drain warps
 
 // Shapes of the rings by token count.  Tensor memory: operand slots x 32 + entries x 2 T columns of the
 // 512; shared memory: raw, activation and scale rings within 227 KB.
 template <int T, int LIMBS>
 struct TcCfg {
-  static constexpr int ENTRIES = T == 96 ? 2 : T == 64 ? 3 : 4;    // accumulator entries, a group (two blocks) each
-  // Blocks per hand-off of accumulators.  One where only two entries fit: each block's columns then go back
-  // to the MMAs as soon as they are read, and the ring turns like four entries.
+  // Accumulator entries, a group (two blocks) each, and blocks per hand-off: one where only two entries fit, so
+  // that each block's columns go back to the MMAs as soon as they are read.
+  static constexpr int ENTRIES = T == 96 ? 2 : T == 64 ? 3 : 4;
   static constexpr int IB = T == 96 ? 1 : 2;
   static constexpr int PER = 2 / IB;                               // hand-offs per group
   static constexpr int ACT_BYTES = T * 128 * LIMBS;                // half a stage of activations
@@ -83,18 +86,26 @@ struct TcCfg {
   // slot RAW_SLOTS tile stages before, hence after the MMAs two tile stages before that have started, hence
   // after the drain has released what was in their accumulator entries: at most five tile stages in all.
   static constexpr int SC_SLOTS = RAW_SLOTS + 5;
-  static_assert(TA_SLOTS + ENTRIES <= 8, "scale ring");
+  // Converter warpgroups: one for both halves of a stage, or one for each.  Two halve the chain of waits, loads,
+  // conversion and tcgen05.st that one has to walk twice a stage (about a thousand cycles), but leave the
+  // others 72 registers a thread at launch instead of 80: measured 47.2 against 53.7 us at 64 tokens x 37888 x
+  // 3584 in one plane, 101 against 97 us at 64 x 55296 x 5120 in two, 1041 against 985 us at 96 tokens a tile.
+  static constexpr int CONV_WGS = T == 64 && LIMBS == 1 ? 2 : 1;
+  static constexpr int DRAIN_WARP0 = CONV_WARP0 + 4 * CONV_WGS;
+  static constexpr int THREADS = (DRAIN_WARP0 + 16) * 32;
   // registers per thread after the split (warpgroups: single roles, converters, drain x 4); the sum stays
-  // within what the block is launched with: 6 warpgroups x 80 (768 threads of an SM's 65536 registers)
-  static constexpr int REGS_MISC = T == 96 ? 40 : 56;
-  static constexpr int REGS_CONV = T == 96 ? 56 : 72;
+  // within what the block is launched with: 6 warpgroups x 80 or 7 x 72 of an SM's 65536 registers
+  static constexpr int REGS_LAUNCH = CONV_WGS == 1 ? 80 : 72;
   static constexpr int REGS_DRAIN = T == 96 ? 96 : 88;
-  static_assert(REGS_MISC + REGS_CONV + 4 * REGS_DRAIN <= 6 * 80, "register split");
+  static constexpr int REGS_MISC = CONV_WGS == 2 || T == 96 ? 40 : 56;
+  static constexpr int REGS_CONV = CONV_WGS == 1 ? (T == 96 ? 56 : 72) : (T == 96 ? 40 : 56);
+  static_assert(REGS_MISC + CONV_WGS * REGS_CONV + 4 * REGS_DRAIN <= (5 + CONV_WGS) * REGS_LAUNCH, "register split");
   static constexpr int ACC_COL0 = TA_SLOTS * TA_SLOT_COLS;
   static constexpr size_t SMEM = 1024 + (size_t)RAW_SLOTS * RAW_BYTES + (size_t)ACT_SLOTS * ACT_BYTES +
                                  (size_t)SC_SLOTS * SC_BYTES + 1024;
   static_assert(SMEM <= 227 * 1024 && SMEM > 114 * 1024, "shared memory: one CTA per SM, since it takes all of tensor memory");
-  static_assert(ACC_COL0 + 2 * ENTRIES * T <= (int)TMEM_COLS, "TMEM budget");
+  static constexpr int ENTRY_COLS = 2 * T;
+  static_assert(ACC_COL0 + ENTRIES * ENTRY_COLS <= (int)TMEM_COLS, "TMEM budget");
 };
 
 struct TcParams {
@@ -112,6 +123,7 @@ struct TcParams {
   // Units: `pairs` x splits pair items, then `solos` x splits single tiles, each for mtiles token tiles.
   int pairs, solos, mtiles, group;
   int s_tiled;        // scales are [row tile][stage][128 rows][4] (always with tile-major weights)
+  int wait_scales;    // the scales are the previous kernel's output too
   int stream_once;    // one token tile: the weights are not read again
   int* status;
 };
@@ -298,13 +310,13 @@ __device__ __forceinline__ void store_tile(const TcParams& p, const float2* acc,
 }
 
 template <int T, int LIMBS, bool TILED>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(TcCfg<T, LIMBS>::THREADS, 1)
 q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_ahi,
                   const __grid_constant__ CUtensorMap map_alo, const __grid_constant__ CUtensorMap map_s,
                   const TcParams p) {
   using Cfg = TcCfg<T, LIMBS>;
   constexpr int ENTRIES = Cfg::ENTRIES, IB = Cfg::IB, PER = Cfg::PER, ACT_SLOTS = Cfg::ACT_SLOTS, RAW_SLOTS = Cfg::RAW_SLOTS,
-                SC_SLOTS = Cfg::SC_SLOTS;
+                SC_SLOTS = Cfg::SC_SLOTS, DRAIN_WARP0 = Cfg::DRAIN_WARP0;
 
   // Shared memory by 32-bit window addresses: rings of slots, then the barriers.
   extern __shared__ uint8_t smem_raw[];
@@ -330,7 +342,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __shared__ int prior_status;
   if (tid == 0) {
     prior_status = *reinterpret_cast<volatile int*>(p.status);
-    for (int i = 0; i < RAW_SLOTS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4); }
+    for (int i = 0; i < RAW_SLOTS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4 * Cfg::CONV_WGS); }
     for (int i = 0; i < ACT_SLOTS; ++i) { mbar_init(act_full + 8 * i, 1); mbar_init(act_empty + 8 * i, 1); }
     for (int i = 0; i < TA_SLOTS; ++i) { mbar_init(ta_full + 8 * i, 4); mbar_init(ta_empty + 8 * i, 1); }
     for (int i = 0; i < GROUPS * PER; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 16); }
@@ -368,6 +380,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     if (warp == 0) {
       // ------------------------------------------------------------ weight and scale producer
       if (lane == 0) {
+        if (p.wait_scales) pdl_wait();
         const uint64_t pol = p.stream_once ? policy_evict_first() : policy_evict_normal();
         Ring<RAW_SLOTS> r;
         Ring<SC_SLOTS> c;
@@ -421,34 +434,29 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       // A warp runs its loop with all lanes, so that addresses and descriptors stay warp-uniform (with one lane
       // alone the issue of a group took three times as long), and one elected lane issues the tcgen05
       // instructions.  The barriers a group needs are polled together: one round of latency, not three.
-      // Barrier sets follow the groups modulo GROUPS and accumulator entries modulo ENTRIES; a warp meets the
-      // same sets phase after phase, which the parity test needs.
       constexpr uint32_t idesc = make_idesc_f16(0, 0, TC_ROWS, T);
       const int half = warp - 2;
       const uint64_t bdesc_first = make_desc_sw128(act);
       Ring<ACT_SLOTS, 2> ra(half);
       Ring<TA_SLOTS, 2> rt(half);
-      Ring<GROUPS, 2> rf(half);                                              // the group's own barriers
-      Ring<GROUPS, 2> re((half + GROUPS - ENTRIES) % GROUPS, 1u);            // those of the entry's previous group
-      Ring<ENTRIES, 2> rd(half % ENTRIES);                                   // the entry
+      Ring<GROUPS, 2> rf(half);                                    // the group's own barriers
+      Ring<GROUPS, 2> re((half + GROUPS - ENTRIES) % GROUPS, 1u);  // those of the entry's previous group
+      Ring<ENTRIES, 2> rd(half % ENTRIES);                         // the entry
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const TcUnit it = tc_unit(p, u);
         polls = kWaitPolls;
         for (int i = 0; i < it.nst; ++i) {
           const uint64_t bdesc0 = bdesc_first + (uint32_t)(ra.slot * (Cfg::ACT_BYTES >> 4));   // start address field: no carry out of it
           for (int j = 0; j < it.ntile; ++j) {
-            const uint32_t free_bar = acc_empty + 8 * PER * re.slot;
-            if (j == 0) mbar_wait3(act_full + 8 * ra.slot, ra.ph, ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
-            else mbar_wait2(ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
-            tc_fence_after();
-            const uint32_t d0 = tmem_base + Cfg::ACC_COL0 + rd.slot * 2 * T;
             const uint32_t a0 = tmem_base + rt.slot * TA_SLOT_COLS;
+            const uint32_t free_bar = acc_empty + 8 * PER * re.slot, full_bar = acc_full + 8 * PER * rf.slot;
 #pragma unroll
             for (int k = 0; k < PER; ++k) {
-              if (k > 0) {
-                mbar_wait(free_bar + 8 * k, re.ph, &polls);
-                tc_fence_after();
-              }
+              if (k > 0) mbar_wait(free_bar + 8 * k, re.ph, &polls);
+              else if (j == 0) mbar_wait3(act_full + 8 * ra.slot, ra.ph, ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
+              else mbar_wait2(ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
+              tc_fence_after();
+              const uint32_t d0 = tmem_base + Cfg::ACC_COL0 + rd.slot * Cfg::ENTRY_COLS + k * IB * T;
               if (elect_one()) {
                 // Per block: d = q * lo' first, then d = q * hi + d * 2^-11 (the residual plane is folded in by the
                 // accumulator scaling of the MMA itself, from one copy of the weights).
@@ -456,16 +464,15 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 for (int v = 0; v < 2 * LIMBS; ++v) {
 #pragma unroll
                   for (int b = 0; b < IB; ++b) {
-                    const int bb = k * IB + b;
                     const int l = (LIMBS == 2) ? 1 - (v >> 1) : 0;
-                    const int kk = bb * 2 + (v & 1);     // K = 16 step inside the half stage
+                    const int kk = (k * IB + b) * 2 + (v & 1);     // K = 16 step inside the half stage
                     const uint64_t bdesc = bdesc0 + (uint32_t)((l * T * 128 + kk * 32) >> 4);
-                    if (LIMBS == 2 && v == 2) tc_mma_f16_ts_scaled_d<11>(d0 + bb * T, a0 + kk * 8, bdesc, idesc);
-                    else if (v == 0) tc_mma_f16_ts<false>(d0 + bb * T, a0 + kk * 8, bdesc, idesc);
-                    else tc_mma_f16_ts<true>(d0 + bb * T, a0 + kk * 8, bdesc, idesc);
+                    if (LIMBS == 2 && v == 2) tc_mma_f16_ts_scaled_d<11>(d0 + b * T, a0 + kk * 8, bdesc, idesc);
+                    else if (v == 0) tc_mma_f16_ts<false>(d0 + b * T, a0 + kk * 8, bdesc, idesc);
+                    else tc_mma_f16_ts<true>(d0 + b * T, a0 + kk * 8, bdesc, idesc);
                   }
                 }
-                tc_commit(acc_full + 8 * (PER * rf.slot + k));
+                tc_commit(full_bar + 8 * k);
                 if (k == PER - 1) {
                   tc_commit(ta_empty + 8 * rt.slot);
                   if (j + 1 == it.ntile) tc_commit(act_empty + 8 * ra.slot);   // free once these MMAs have completed
@@ -491,62 +498,66 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // ------------------------------------------------------------ converters: int8 smem -> fp16 TMEM
     regs_dec<Cfg::REGS_CONV>();
     const int qd = warp & 3;
+    const int first = Cfg::CONV_WGS == 2 ? (warp - CONV_WARP0) >> 2 : 0;   // the group's (first) half
     const uint32_t row = qd * 32 + lane;
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16);
-    // the row's 16-byte chunks: chunk c sits at c ^ (row & 7) (128-byte swizzle)
-    uint32_t off[8];
+    // the row's 16-byte chunks of a half: chunk c sits at c ^ (row & 7) (128-byte swizzle); the second half's
+    // chunks differ in bit 6 of the address
+    uint32_t off[4];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) off[c] = swz128(row, c);
-    auto load_half = [&](uint4 (&wv)[4], uint32_t rb, int h) {
+    for (int c = 0; c < 4; ++c) off[c] = raw + swz128(row, first * 4 + c);
+    auto load_half = [&](uint4 (&wv)[4], int slot, uint32_t flip) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) wv[c] = lds_v4(rb + off[h * 4 + c]);
+      for (int c = 0; c < 4; ++c) wv[c] = lds_v4((off[c] ^ flip) + slot * RAW_BYTES);
     };
-    auto convert = [&](uint32_t (&o)[32], const uint4 (&wv)[4]) {
+    auto convert_store = [&](const uint4 (&wv)[4], uint32_t t_dst) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint32_t ws[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
+      for (int c2 = 0; c2 < 2; ++c2) {
+        uint32_t o[16];
 #pragma unroll
-        for (int wi = 0; wi < 4; ++wi) {
-          const uint32_t w = TILED ? ws[wi] : ws[wi] ^ 0x80808080u;   // tile-major bytes hold q + 128 already
-          o[c * 8 + 2 * wi] = cvt_pair(w, 0x4140);
-          o[c * 8 + 2 * wi + 1] = cvt_pair(w, 0x4342);
+        for (int c = 0; c < 2; ++c) {
+          const uint4 w4 = wv[c2 * 2 + c];
+          const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+          for (int wi = 0; wi < 4; ++wi) {
+            const uint32_t w = TILED ? ws[wi] : ws[wi] ^ 0x80808080u;   // tile-major bytes hold q + 128 already
+            o[c * 8 + 2 * wi] = cvt_pair(w, 0x4140);
+            o[c * 8 + 2 * wi + 1] = cvt_pair(w, 0x4342);
+          }
         }
+        tc_st_32x32b_x16(t_dst + c2 * 16, o);
       }
     };
-    auto store_half = [&](const uint32_t (&o)[32], int slot) {
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-        tc_st_32x32b_x16(t_lane + slot * TA_SLOT_COLS + c * 16, *reinterpret_cast<const uint32_t(*)[16]>(&o[c * 16]));
+    auto stored = [&](uint32_t bar) {
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      mbar_arrive_if(bar, lane == 0);
     };
     Ring<RAW_SLOTS> r;
-    Ring<TA_SLOTS, 2> a(0, 1u);   // a stage takes slots a and a + 1
+    Ring<TA_SLOTS, 2> a(first, 1u);
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
       polls = kWaitPolls;
       const int count = it.nst * it.ntile;
       for (int i = 0; i < count && ok; ++i) {
-        const uint32_t rb = raw + r.slot * RAW_BYTES;
         uint4 wv[4];
-        uint32_t o[32];
         mbar_wait2(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, &polls);
         tc_fence_after();
-        load_half(wv, rb, 0);
-        convert(o, wv);
-        store_half(o, a.slot);
-        load_half(wv, rb, 1);             // the second half is converted while the first one is stored
-        convert(o, wv);
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        mbar_arrive_if(ta_full + 8 * a.slot, lane == 0);
-        mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
-        mbar_wait(ta_empty + 8 * (a.slot + 1), a.ph, &polls);
-        tc_fence_after();
-        store_half(o, a.slot + 1);
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        mbar_arrive_if(ta_full + 8 * (a.slot + 1), lane == 0);
+        load_half(wv, r.slot, 0u);
+        convert_store(wv, t_lane + a.slot * TA_SLOT_COLS);
+        if (Cfg::CONV_WGS == 2) {
+          mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
+          stored(ta_full + 8 * a.slot);
+        } else {
+          load_half(wv, r.slot, 64u);
+          stored(ta_full + 8 * a.slot);
+          mbar_wait(ta_empty + 8 * (a.slot + 1), a.ph, &polls);
+          tc_fence_after();
+          convert_store(wv, t_lane + (a.slot + 1) * TA_SLOT_COLS);
+          mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
+          stored(ta_full + 8 * (a.slot + 1));
+        }
         a.next();
         r.next();
         if (polls == 0) {
@@ -565,25 +576,36 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16) + Cfg::ACC_COL0;
     const uint32_t s_lane = scl + nl * 16;
     pdl_wait();  // before any write to global memory (nothing to drain before the activations are in anyway)
-    int ent = (2 * g) % ENTRIES;   // entry of the next group
-    int rc = g;                    // scale slot of the next stage
-    uint32_t ph = 0;               // parity of the barriers' next phase: all of them go through one phase a pair stage
+    int ent = (2 * g) % ENTRIES;     // entry of the next group
+    int rc = g;                      // scale slot of the next stage
+    int grp = 2 * g;                 // barrier set of the next stage's first group, and the parity of its phase
+    uint32_t ph = 0;
     auto step = [](int& v, int by, int n) {
       v += by;
       if (v >= n) v -= n;
     };
-    // one group: the blocks of a half stage, `hs` the stage's two scales for it
-    auto drain_group = [&](auto hc, float2* sum, uint32_t col, int grp, const float* hs, auto arrivals) {
+    // one stage of a tile, from this warp's first column `col` on
+    auto drain_stage = [&](auto hc, float2* sum, uint32_t col, auto arrivals) {
+      float s[4];
 #pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const uint32_t bar = 8 * (PER * grp + k);
-        if (k > 0) mbar_wait(acc_full + bar, ph, &polls);   // (the first hand-off: waited for by the caller)
-        tc_fence_after();
-        drain_blocks<hc, IB, T>(sum, t_lane + col + ent * 2 * T + k * IB * T, hs + k * IB, [&] {
-          tc_fence_before();
-          __syncwarp();
-          mbar_arrive_n_if<arrivals>(acc_empty + bar, lane == 0);
-        });
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t at = t_lane + col + ent * Cfg::ENTRY_COLS;
+        step(ent, 1, ENTRIES);
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const uint32_t bar = 8 * (PER * (grp + h) + k);
+          mbar_wait(acc_full + bar, ph, &polls);
+          tc_fence_after();
+          if (h == 0 && k == 0) {
+            const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
+            s[0] = __uint_as_float(sc.x); s[1] = __uint_as_float(sc.y); s[2] = __uint_as_float(sc.z); s[3] = __uint_as_float(sc.w);
+          }
+          drain_blocks<hc, IB, T>(sum, at + k * IB * T, s + h * 2 + k * IB, [&] {
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_n_if<arrivals>(acc_empty + bar, lane == 0);
+          });
+        }
       }
     };
     constexpr std::integral_constant<int, T / 2> half_cols{};
@@ -599,16 +621,11 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
       for (int x = 0; x < T / 4; ++x) acc[x] = make_float2(0.f, 0.f);
       for (int i = 0; i < it.nst && polls != 0; ++i) {
-        mbar_wait(acc_full + 8 * PER * (2 * g), ph, &polls);
-        const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
-        const float s[4] = {__uint_as_float(sc.x), __uint_as_float(sc.y), __uint_as_float(sc.z), __uint_as_float(sc.w)};
-        drain_group(half_cols, acc, th * (T / 2), 2 * g, s, two);
-        step(ent, 1 % ENTRIES, ENTRIES);
-        mbar_wait(acc_full + 8 * PER * (2 * g + 1), ph, &polls);
-        drain_group(half_cols, acc, th * (T / 2), 2 * g + 1, s + 2, two);
-        step(ent, 3 % ENTRIES, ENTRIES);            // past the other tile's two groups
+        drain_stage(half_cols, acc, th * (T / 2), two);
+        step(ent, 2 % ENTRIES, ENTRIES);            // past the other tile's two groups
         step(rc, 2, SC_SLOTS);
-        ph ^= 1u;
+        grp ^= 4;
+        ph ^= (uint32_t)(grp < 4);
       }
       if (polls == 0) {
         if (lane == 0) tc_report(p.status, 2050, 0, it.nst);
@@ -622,7 +639,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     asm volatile("bar.sync 1, 512;" ::: "memory");
     ent = (ent + 2 * ENTRIES - 2 * g) % ENTRIES;
     rc = (rc + SC_SLOTS - g) % SC_SLOTS;
-    int sp = 0;                                     // stage parity: groups 2 sp, 2 sp + 1
+    grp -= 2 * g;
     for (; u < units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
       polls = kWaitPolls;
@@ -631,17 +648,10 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       for (int x = 0; x < T / 8; ++x) acc[x] = make_float2(0.f, 0.f);
       const uint32_t col = (2 * g + th) * (T / 4);
       for (int i = 0; i < it.nst && polls != 0; ++i) {
-        mbar_wait(acc_full + 8 * PER * (2 * sp), ph, &polls);
-        const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
-        const float s[4] = {__uint_as_float(sc.x), __uint_as_float(sc.y), __uint_as_float(sc.z), __uint_as_float(sc.w)};
-        drain_group(quarter_cols, acc, col, 2 * sp, s, one);
-        step(ent, 1, ENTRIES);
-        mbar_wait(acc_full + 8 * PER * (2 * sp + 1), ph, &polls);
-        drain_group(quarter_cols, acc, col, 2 * sp + 1, s + 2, one);
-        step(ent, 1, ENTRIES);
+        drain_stage(quarter_cols, acc, col, one);
         step(rc, 1, SC_SLOTS);
-        ph ^= (uint32_t)sp;
-        sp ^= 1;
+        step(grp, 2, GROUPS);
+        ph ^= (uint32_t)(grp == 0);
       }
       if (polls == 0) {
         if (lane == 0) tc_report(p.status, 2051, 0, it.nst);
@@ -813,6 +823,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   p.splits = plan.splits;
   p.stages_total = (int)stages;
   p.s_tiled = s_tiled;
+  p.wait_scales = g.s_tiled;
   const int64_t mtiles = (g.m + T - 1) / T;
   const int64_t units = (int64_t)(plan.pairs + plan.solos) * plan.splits * mtiles;
   if (units > INT32_MAX / 4 || tiles * stages > INT32_MAX / TC_ROWS) return fail(LOGOS_OUT_OF_BOUNDS, "q8_gemm: too many work units");
@@ -831,7 +842,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   // persistent CTAs: one per SM at most, each takes units blockIdx.x, blockIdx.x + gridDim.x, ...
   const int sms = sm_count(g.device);
   dim3 grid((unsigned)(units < sms ? units : sms), 1u, 1u);
-  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(TC_THREADS), Cfg::SMEM, st, mq, mhi, mlo, ms, p));
+  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, st, mq, mhi, mlo, ms, p));
   count_launch(LK_GEMM_TC);
   return check_launch("q8_gemm_tc_kernel");
 }

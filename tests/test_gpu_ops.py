@@ -127,6 +127,36 @@ def test_q8_gemm_epilogues(llm, oracle, golden, simt):
     assert np.mean(c2 != O.q8_gemm(a, q, s, 2)) < 0.01
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (1, 128, 160),        # K a tail of one Q8 block past a whole stage: scales brought to the tile-major form
+    (17, 5000, 1056),     # a last row tile of 8 rows, a tail of 32 columns
+    (64, 3584, 2368),     # K splits and a tail of 64 columns
+    (65, 300, 256),       # the first count past one 64-token tile
+    (96, 384, 384),       # one full 96-token tile, an odd number of row tiles
+    (97, 130, 992),       # a second token tile of one token, two rows in the last row tile
+    (64, 55196, 256),     # pairs of row tiles first, then single ones, on the same CTAs
+    (200, 20000, 128),    # several token tiles of 96, one stage
+])
+def test_q8_gemm_tiles_tails_and_units(llm, oracle, m, n, k):
+    """Edges of the tensor-core kernel's tiles and work units, f32 and bf16, against the oracle; repeated
+    calls give the same bits (the kernel's sums have a fixed order)."""
+    O = oracle
+    a = O.synth_fill(O.F32, 2, 6, 10, 0, m * k, 0.0, 1.0).reshape(m, k)
+    q = O.synth_fill(O.I8, 0, 6, 11, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 6, 12, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    before = llm.launchCounts()["q8_gemm_tc"]
+    c = llm.q8GemmF32Host(a, q, s)
+    assert llm.launchCounts()["q8_gemm_tc"] == before + 1
+    # f32 sums over k terms in another order: about sqrt(k) roundings of 2^-24, and planes of 22 bits
+    assert rel_l2(c, O.q8_gemm_f32(a, O.F32, q, s)) < 2e-6
+    for _ in range(3):
+        assert np.array_equal(llm.q8GemmF32Host(a, q, s), c)
+    ab = O.f32_to_bf16(a)
+    got, want = O.bf16_to_f32(llm.q8GemmHost(ab, q, s)), O.q8_gemm_f32(ab, O.BF16, q, s)
+    assert rel_l2(got, want) < 3e-3     # bf16 results: half a last place is 2^-9 of the value
+    assert llm.kernelStatus() == 0
+
+
 def test_q8_gemm_config1_slice(llm, oracle):
     """Config 1 shapes (M=64, K=3584) on a 2048-row slice of N, both kernels."""
     O = oracle
