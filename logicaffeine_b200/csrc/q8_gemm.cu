@@ -9,6 +9,8 @@
 #include "ops.cuh"
 #include "q8_gemm_tc.cuh"
 
+#include <algorithm>
+
 namespace logos {
 
 namespace {
@@ -113,6 +115,29 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partials, int spl
 }
 
 }  // namespace
+
+// K splits: a unit's time is a fixed part (pipeline fill, epilogue: about twelve stage times, measured) plus its K
+// stages, and units run in rounds of one per SM.  The split count with the smallest rounds x (fixed + stages);
+// ties go to fewer splits (fewer partials to write and fold).  A row tile for each token tile of 64 is a
+// unit of its own: with many tokens there are enough.  The split count is also what fixes the order of a
+// sum, so that the same shape gives the same bits whatever the kernel's tiles.
+int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device) {
+  const int64_t tiles = ((n + 127) / 128) * std::max<int64_t>((m + 63) / 64, 1);
+  const int64_t stages = k / 128;
+  const int sms = sm_count(device);
+  if (tiles >= sms || stages < 8) return 1;
+  const int64_t fixed = 12;
+  const int64_t max_splits = std::min<int64_t>(stages / 4, 16);   // at least 4 stages (512 columns) per split
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int64_t sp = 1; sp <= max_splits; ++sp) {
+    const int64_t rounds = (tiles * sp + sms - 1) / sms;
+    const int64_t per = (stages + sp - 1) / sp;
+    const int64_t cost = rounds * (fixed + per) * 8 + sp;
+    if (cost < best_cost) { best_cost = cost; best = (int)sp; }
+  }
+  return best;
+}
 
 logos_status_t launch_splitk_reduce(const float* partials, int splits, void* c, int c_dtype, ActOut c_act,
                                     int64_t ldc, const void* aux, int64_t m, int64_t n, int epilogue,

@@ -726,12 +726,13 @@ struct TcPlan {
 };
 
 // Cycles of one K stage of a pair and of a single tile, by tokens per tile (timings of this kernel), of the
-// pipeline fill plus the last epilogue, and of a unit's epilogue.
+// pipeline fill plus the last epilogue, and of a unit's epilogue.  They decide only who computes what: the
+// order of a sum depends on the K splits alone.
 struct TcCost {
   int t, pair, solo;
 };
-constexpr TcCost kCosts[] = {{16, 1450, 760}, {32, 1450, 760}, {64, 1500, 860}, {96, 1900, 1100}};
-constexpr int kFillCycles = 6000, kUnitCycles = 700;
+constexpr TcCost kCosts[] = {{16, 1760, 1065}, {32, 1900, 1090}, {64, 2550, 1400}, {96, 3300, 1900}};
+constexpr int kFillCycles = 8000, kUnitCycles = 700;
 
 // The slowest CTA's time when `pairs` pair items and `solos` single tiles run round robin on g CTAs.
 int64_t plan_cycles(const TcCost& c, int64_t pairs, int64_t solos, int64_t sp, int64_t mt, int64_t stages, int64_t g) {
@@ -747,9 +748,9 @@ int64_t plan_cycles(const TcCost& c, int64_t pairs, int64_t solos, int64_t sp, i
   return worst + kFillCycles;
 }
 
-TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int sms) {
+TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms) {
   const int64_t tl = (n + TC_ROWS - 1) / TC_ROWS, stages = (k + TC_KSTAGE - 1) / TC_KSTAGE;
-  TcPlan best{16, 1, 0, (int)tl};
+  TcPlan best{16, (int)sp, 0, (int)tl};
   int64_t best_cost = INT64_MAX;
   for (const TcCost& c : kCosts) {
     // fewer tokens than half a larger tile never pay for it
@@ -757,20 +758,13 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int sms
     if (c.t > 16 && m <= c.t / 2 && c.t <= 64) continue;
     if (c.t == 96 && m <= 64) continue;
     const int64_t mt = (m + c.t - 1) / c.t;
-    int64_t sp_lo = 1, sp_hi = 1;
-    if (forced_splits > 0) sp_lo = sp_hi = forced_splits;
-    else if (tl * mt < sms && stages >= 8) sp_hi = std::min<int64_t>(16, stages / 4);   // at least 4 stages (512 columns) per split
-    for (int64_t sp = sp_lo; sp <= sp_hi; ++sp) {
-      const int64_t full_rounds = tl * sp * mt / (2 * sms);
-      const int64_t cand[3] = {0, tl / 2, std::min<int64_t>(tl / 2, full_rounds * sms / (sp * mt))};
-      for (int64_t pairs : cand) {
-        int64_t cost = plan_cycles(c, pairs, tl - 2 * pairs, sp, mt, stages, sms);
-        // partial sums are written and read back through L2 (about 4.4 KB per cycle) and folded by one more kernel
-        if (sp > 1) cost += 2000 + 8 * sp * m * n / 4400;
-        if (cost < best_cost) {
-          best_cost = cost;
-          best = TcPlan{c.t, (int)sp, (int)pairs, (int)(tl - 2 * pairs)};
-        }
+    const int64_t full_rounds = tl * sp * mt / (2 * sms);
+    const int64_t cand[3] = {0, tl / 2, std::min<int64_t>(tl / 2, full_rounds * sms / (sp * mt))};
+    for (int64_t pairs : cand) {
+      const int64_t cost = plan_cycles(c, pairs, tl - 2 * pairs, sp, mt, stages, sms);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = TcPlan{c.t, (int)sp, (int)pairs, (int)(tl - 2 * pairs)};
       }
     }
   }
@@ -778,7 +772,7 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int sms
 }
 
 // Plans are pure functions of the shape: the last ones of a thread are kept.
-TcPlan plan_for(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int device) {
+TcPlan plan_for(int64_t m, int64_t n, int64_t k, int64_t splits, int device) {
   struct Entry {
     int64_t m = -1, n = 0, k = 0, sp = 0;
     int device = 0;
@@ -786,11 +780,11 @@ TcPlan plan_for(int64_t m, int64_t n, int64_t k, int64_t forced_splits, int devi
   };
   thread_local Entry cache[64];
   const uint64_t h = ((uint64_t)m * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)n * 0xBF58476D1CE4E5B9ull) ^ ((uint64_t)k * 0x94D049BB133111EBull) ^
-                     (uint64_t)forced_splits;
+                     (uint64_t)splits;
   Entry& e = cache[(h ^ (h >> 29)) >> 7 & 63];
-  if (e.m != m || e.n != n || e.k != k || e.sp != forced_splits || e.device != device) {
-    e.m = m; e.n = n; e.k = k; e.sp = forced_splits; e.device = device;
-    e.plan = make_plan(m, n, k, forced_splits, sm_count(device));
+  if (e.m != m || e.n != n || e.k != k || e.sp != splits || e.device != device) {
+    e.m = m; e.n = n; e.k = k; e.sp = splits; e.device = device;
+    e.plan = make_plan(m, n, k, splits, sm_count(device));
   }
   return e.plan;
 }
@@ -871,8 +865,6 @@ bool gemm_tc_applicable(const GemmArgs& g) {
     return false;
   return true;
 }
-
-int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device) { return plan_for(m, n, k, 0, device).splits; }
 
 logos_status_t launch_q8_gemm_tc(const GemmArgs& g, cudaStream_t st) {
   const TcPlan plan = plan_for(g.m, g.n, g.k, g.splits > 1 ? g.splits : 1, g.device);
