@@ -344,13 +344,22 @@ template <bool BF16>
 __global__ void __launch_bounds__(256)
 gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const float* __restrict__ s, float* __restrict__ tiled,
                  int64_t n, int64_t kb, int64_t ktiles, int64_t act_blocks) {
+  // count8: groups of eight of the planes; rows of the planes are whole K tiles, rows of `a` kb * 32 values
   pdl_trigger();
   if ((int64_t)blockIdx.x < act_blocks) {
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= count8) return;
-    float x[8];
-    if (BF16) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a) + i);
+    float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int64_t src = i;                      // group of eight of `a`
+    bool inside = true;
+    if (tiled) {                          // K is not a multiple of 128: zeros fill the last K tile
+      const int64_t row = i / (ktiles * 16), g = i - row * (ktiles * 16);
+      src = row * (kb * 4) + g;
+      inside = g < kb * 4;
+    }
+    if (!inside) {
+    } else if (BF16) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a) + src);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -358,7 +367,7 @@ gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const flo
         x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
       }
     } else {
-      const float4 v0 = __ldg(reinterpret_cast<const float4*>(a) + 2 * i), v1 = __ldg(reinterpret_cast<const float4*>(a) + 2 * i + 1);
+      const float4 v0 = __ldg(reinterpret_cast<const float4*>(a) + 2 * src), v1 = __ldg(reinterpret_cast<const float4*>(a) + 2 * src + 1);
       x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
       x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
     }
@@ -519,11 +528,11 @@ logos_status_t launch_embed(const int32_t* tokens, const int8_t* q, const float*
   return check_launch("embed_kernel");
 }
 
-logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t count, const float* s,
+logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t m, const float* s,
                                 float* tiled_or_null, int64_t n, int64_t k, cudaStream_t st) {
-  if (count % 8 || (reinterpret_cast<uintptr_t>(a) & 15u))
-    return fail(LOGOS_ERROR, "gemm_prep: activations must be 16-byte aligned and a multiple of 8");
-  const int64_t count8 = count / 8, ktiles = (k + 127) / 128;
+  if (k % 32 || (reinterpret_cast<uintptr_t>(a) & 15u))
+    return fail(LOGOS_ERROR, "gemm_prep: K must be a multiple of 32 and the activations 16-byte aligned");
+  const int64_t ktiles = (k + 127) / 128, count8 = m * ktiles * 16;
   const int64_t act_blocks = (count8 + 255) / 256, scale_blocks = tiled_or_null ? (n * ktiles + 255) / 256 : 0;
   const dim3 grid((unsigned)(act_blocks + scale_blocks));
   if (a_dtype == LOGOS_BF16)

@@ -302,8 +302,10 @@ logos_status_t build(Model* m, const void* nccl_id) {
   LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->h), B * H * 4));
   auto planes = [&](ActOut* a, int64_t elems) -> logos_status_t {
     a->mode = c.act_dtype;
-    LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&a->hi), elems * 2));
-    if (c.act_dtype == LOGOS_F32) LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&a->lo), elems * 2));
+    const int64_t plane = (elems * 2 + 255) / 256 * 256;   // one allocation: the GEMM's tensor map spans both planes
+    const bool two = c.act_dtype == LOGOS_F32;
+    LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&a->hi), two ? 2 * plane : plane));
+    if (two) a->lo = a->hi + plane / 2;
     return LOGOS_OK;
   };
   LOGOS_TRY(planes(&m->xn, B * H));

@@ -45,7 +45,7 @@ struct GemmArgs {
   const void*   a = nullptr;   // activations [M][K], row stride lda elements
   const __half* a_lo = nullptr;  // second fp16 plane (see act.cuh); only with a_dtype LOGOS_F16
   int           a_dtype = LOGOS_BF16;  // LOGOS_F16 plane(s), LOGOS_BF16 or LOGOS_F32
-  int64_t       lda = 0;
+  int64_t       lda = 0;       // tcgen05 kernel: at least ceil128(k), zeros past k; a_lo after a
   const int8_t* q = nullptr;   // [N][K] row-major, or tile-major when q_tiled (launch_q8_retile)
   int           q_tiled = 0;   // tcgen05 kernel only; s is then tile-major too (launch_q8_retile_scales)
   int           s_tiled = 0;   // row-major q with tile-major s (zero past K): any K that is a multiple of 32
@@ -180,11 +180,12 @@ struct TpFusedArgs {
 };
 logos_status_t launch_tp_residual_rmsnorm(float* h, const TpFusedArgs& t, int parts, int64_t part_stride, const float* g,
                                           int64_t rows, int64_t hidden, float eps, int device, cudaStream_t st);
-// What a stand-alone product needs before it starts, in one launch: `count` activations (LOGOS_BF16 or LOGOS_F32)
-// into planes (mode LOGOS_F16: one plane, exact for bf16 inside fp16's normal range, saturating outside;
-// LOGOS_F32: two), and, where tiled_or_null is set, scales [n][k/32] into the tile-major form
+// What a stand-alone product needs before it starts, in one launch: activations [m][k] (LOGOS_BF16 or LOGOS_F32)
+// into planes whose rows are whole K tiles (ceil128(k), zero past k; mode LOGOS_F16: one plane, exact for bf16
+// inside fp16's normal range, saturating outside; LOGOS_F32: two), and, where K is not a multiple of 128
+// (tiled_or_null set then and only then), scales [n][k/32] into the tile-major form
 // [row tile][K tile][128 rows][4], zero past K (rows past n are left alone: their products are dropped).
-logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t count, const float* s,
+logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t m, const float* s,
                                 float* tiled_or_null, int64_t n, int64_t k, cudaStream_t st);
 // Sampling state of a model, in device memory so that a captured step follows changes to it.
 struct SamplingParams {

@@ -183,7 +183,8 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   const bool retile = g.k % 128 != 0;
   const int splits = gemm_pick_splits(g.m, g.n, g.k, g.device);
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
-  const int64_t plane_bytes = up(g.m * g.k * 2);
+  const int64_t lda = stages * 128;
+  const int64_t plane_bytes = up(g.m * lda * 2);
   const int64_t scale_bytes = retile ? up((g.n + 127) / 128 * stages * 2048) : 0;
   const int64_t part_bytes = splits > 1 ? (int64_t)splits * g.m * g.n * (int64_t)sizeof(float) : 0;
   void* scratch = nullptr;
@@ -196,7 +197,8 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   at += (two_planes ? 2 : 1) * plane_bytes;
   float* tiled = retile ? reinterpret_cast<float*>(at) : nullptr;
   at += scale_bytes;
-  LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m * g.k, g.s, tiled, g.n, g.k, st));
+  LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, st));
+  g.lda = lda;
   g.a = planes.hi;
   g.a_lo = planes.lo;
   g.a_dtype = LOGOS_F16;
@@ -222,6 +224,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
 static bool gemm_tensor_takes(GemmArgs g) {
   g.a_dtype = LOGOS_F16;
   g.a = g.a_lo = nullptr;
+  g.lda = (g.k + 127) / 128 * 128;
   g.s_tiled = g.k % 128 != 0;
   return gemm_tc_applicable(g);
 }

@@ -13,17 +13,17 @@
 // Data flow per 128-column K stage (4 Q8 blocks) and tile, in two groups of half a stage:
 //   TMA  int8 weights [128 rows][128 B], 128-byte swizzle, and the stage's scales [128 rows][4]
 //        -> shared-memory rings                                                    (warp 0)
-//   TMA  fp16 activation planes [T][64] of half a stage -> ring                     (warp 1)
-//   4 or 8 converter warps (one or two per TMEM lane quarter): int8 -> fp16 (exact: 0x6400|b trick),
+//   TMA  fp16 activation planes of the stage [planes][2 halves][T][64] -> ring, one 4-D copy (warp 1)
+//   4 converter warps (one per TMEM lane quarter): int8 -> fp16 (exact: 0x6400|b trick),
 //        tcgen05.st into the operand ring; the weights never go back to shared memory
 //   MMA warps 2 and 3, one per half: per Q8 block two tcgen05.mma kind::f16 (K = 16 each) per plane, A
 //        from TMEM, B = activations from smem, into a fresh accumulator entry: first q*lo', then
 //        q*hi + D*2^-11 through the MMA's own accumulator scaling, so hi + lo*2^-11 is
 //        recombined on the tensor core
-//   16 drain warps: tcgen05.ld a group's partial sums, acc += s * partial in f32 registers.  Of a pair,
-//        eight warps take one tile each (lane quarter x half of the tokens); a single tile is shared by
-//        all sixteen (lane quarter x quarter of the tokens).  Then the epilogue, straight from
-//        registers: a warp's lanes hold consecutive output columns of a token.
+//   16 drain warps (8 up to 32 tokens): tcgen05.ld a group's partial sums, acc += s * partial in f32
+//        registers.  Of a pair, half of the warps take one tile each (lane quarter x a share of the tokens);
+//        a single tile is shared by all.  Then the epilogue, straight from registers: a warp's lanes
+//        hold consecutive output columns of a token.
 // A CTA is persistent and the rings keep running across units.  All hand-offs are mbarriers; every
 // wait is bounded and reports through the device status word instead of spinning for ever.
 //
@@ -66,7 +66,7 @@ constexpr uint32_t TMEM_COLS = 512;
 // (four groups) ahead of it, because the drain takes the halves in turn; with eight sets a set cannot go
 // through a second phase unseen, which the parity test could not tell from none (with four it could).
 constexpr int GROUPS = 8;
-constexpr int CONV_WARP0 = 4;                   // 4 single-role warps, 4 or 8 converter warps, 16 drain warps
+constexpr int CONV_WARP0 = 4, DRAIN_WARP0 = 8;  // 4 single-role warps, 4 converter warps, then the drain warps
 
 // Shapes of the rings by token count.  Tensor memory: operand slots x 32 + entries x 2 T columns of the
 // 512; shared memory: raw, activation and scale rings within 227 KB.
@@ -74,32 +74,35 @@ template <int T, int LIMBS>
 struct TcCfg {
   // Accumulator entries, a group (two blocks) each, and blocks per hand-off: one where only two entries fit, so
   // that each block's columns go back to the MMAs as soon as they are read.
-  static constexpr int ENTRIES = T == 96 ? 2 : T == 64 ? 3 : 4;
+  static constexpr int ENTRIES = T == 96 ? 2 : T == 64 ? 3 : T == 32 ? 4 : 8;
+  static_assert(ENTRIES <= GROUPS, "a barrier set belongs to one group in flight");
   static constexpr int IB = T == 96 ? 1 : 2;
   static constexpr int PER = 2 / IB;                               // hand-offs per group
-  static constexpr int ACT_BYTES = T * 128 * LIMBS;                // half a stage of activations
-  static constexpr int ACT_SLOTS = T * LIMBS >= 192 ? 4 : T * LIMBS == 128 ? 6 : 8;   // even: a slot belongs to one half
-  static constexpr int RAW_SLOTS_FIT = (225 * 1024 - 2048 - ACT_SLOTS * ACT_BYTES - 5 * SC_BYTES) / (RAW_BYTES + SC_BYTES);
-  static constexpr int RAW_SLOTS = RAW_SLOTS_FIT < 9 ? RAW_SLOTS_FIT : 9;
+  static constexpr int ACT_BYTES = 2 * T * 128 * LIMBS;            // a stage of activations
+  static constexpr int ACT_SLOTS = T * LIMBS >= 192 ? 2 : T * LIMBS == 128 ? 3 : T * LIMBS >= 64 ? 4 : 6;
   // The scale ring needs no barriers of its own.  A stage's scales count into its raw_full barrier, so whoever
-  // sees the stage's sums sees them; and a slot is written again after the converters have released the raw
-  // slot RAW_SLOTS tile stages before, hence after the MMAs two tile stages before that have started, hence
-  // after the drain has released what was in their accumulator entries: at most five tile stages in all.
-  static constexpr int SC_SLOTS = RAW_SLOTS + 5;
-  // Converter warpgroups: one for both halves of a stage, or one for each.  Two halve the chain of waits, loads,
-  // conversion and tcgen05.st that one has to walk twice a stage (about a thousand cycles), but leave the
-  // others 72 registers a thread at launch instead of 80: measured 47.2 against 53.7 us at 64 tokens x 37888 x
-  // 3584 in one plane, 101 against 97 us at 64 x 55296 x 5120 in two, 1041 against 985 us at 96 tokens a tile.
-  static constexpr int CONV_WGS = T == 64 && LIMBS == 1 ? 2 : 1;
-  static constexpr int DRAIN_WARP0 = CONV_WARP0 + 4 * CONV_WGS;
-  static constexpr int THREADS = (DRAIN_WARP0 + 16) * 32;
-  // registers per thread after the split (warpgroups: single roles, converters, drain x 4); the sum stays
-  // within what the block is launched with: 6 warpgroups x 80 or 7 x 72 of an SM's 65536 registers
-  static constexpr int REGS_LAUNCH = CONV_WGS == 1 ? 80 : 72;
-  static constexpr int REGS_DRAIN = T == 96 ? 96 : 88;
-  static constexpr int REGS_MISC = CONV_WGS == 2 || T == 96 ? 40 : 56;
-  static constexpr int REGS_CONV = CONV_WGS == 1 ? (T == 96 ? 56 : 72) : (T == 96 ? 40 : 56);
-  static_assert(REGS_MISC + CONV_WGS * REGS_CONV + 4 * REGS_DRAIN <= (5 + CONV_WGS) * REGS_LAUNCH, "register split");
+  // sees the stage's sums sees them.  The scales of tile stage n are written once the converters have released
+  // stage n - RAW_SLOTS; by then its operand slots were free, so the MMAs of stage n - RAW_SLOTS - TA_SLOTS / 2
+  // were complete; those could start once the drain had released what was in their entries, the groups ENTRIES
+  // before, so (ENTRIES + 1) / 2 stages further back everything has been read.
+  static constexpr int SC_MORE = TA_SLOTS / 2 + (ENTRIES + 1) / 2 + 1;   // (and one to spare)
+  static constexpr int RAW_SLOTS_FIT = (225 * 1024 - 2048 - ACT_SLOTS * ACT_BYTES - SC_MORE * SC_BYTES) / (RAW_BYTES + SC_BYTES);
+  static constexpr int RAW_SLOTS = RAW_SLOTS_FIT < 9 ? RAW_SLOTS_FIT : 9;
+  static constexpr int SC_SLOTS = RAW_SLOTS + SC_MORE;
+  // Drain warpgroups: up to 32 tokens there is little to drain, and two groups (all tokens of a tile per warp) take
+  // a whole stage in one round of latency; from 64 on the drain needs sixteen warps and the registers.  One
+  // converter group: every further warp costs its own waits and ring steps, and issue slots are what the
+  // kernel runs short of (0.64 of them were taken with sixteen converter warps at 16 tokens).
+  static constexpr int DRAIN_WGS = T <= 32 ? 2 : 4;
+  static constexpr int WGS = 2 + DRAIN_WGS;
+  static constexpr int THREADS = WGS * 128;
+  // registers per thread after the split (warpgroups: single roles, converters, drain); the sum stays within
+  // what the block is launched with: an SM's 65536 registers over its threads, in steps of 8
+  static constexpr int REGS_LAUNCH = 65536 / THREADS / 8 * 8;
+  static constexpr int REGS_DRAIN = T <= 32 ? 168 : T == 96 ? 96 : 88;
+  static constexpr int REGS_MISC = T == 96 ? 40 : 56;
+  static constexpr int REGS_CONV = T <= 32 ? 96 : T == 96 ? 56 : 72;
+  static_assert(REGS_MISC + REGS_CONV + DRAIN_WGS * REGS_DRAIN <= WGS * REGS_LAUNCH, "register split");
   static constexpr int ACC_COL0 = TA_SLOTS * TA_SLOT_COLS;
   static constexpr size_t SMEM = 1024 + (size_t)RAW_SLOTS * RAW_BYTES + (size_t)ACT_SLOTS * ACT_BYTES +
                                  (size_t)SC_SLOTS * SC_BYTES + 1024;
@@ -139,18 +142,28 @@ __device__ __forceinline__ TcUnit tc_unit(const TcParams& p, int u) {
   const int pair_units = p.pairs * p.splits * p.mtiles;
   const bool solo = u >= pair_units;
   if (solo) u -= pair_units;
-  const int items = (solo ? p.solos : p.pairs) * p.splits;
-  const int g = u / (items * p.group);                       // token-tile group
-  u -= g * items * p.group;
-  const int in_group = min(p.group, p.mtiles - g * p.group);  // the last group may be smaller
-  const int item = u / in_group;
-  r.mtile = g * p.group + (u - item * in_group);
-  const int t = item / p.splits;
-  r.split = item - t * p.splits;
+  int item = u;
+  r.mtile = 0;
+  if (p.mtiles > 1) {
+    const int items = (solo ? p.solos : p.pairs) * p.splits;
+    const int g = u / (items * p.group);                       // token-tile group
+    u -= g * items * p.group;
+    const int in_group = min(p.group, p.mtiles - g * p.group);  // the last group may be smaller
+    item = u / in_group;
+    r.mtile = g * p.group + (u - item * in_group);
+  }
+  int t = item;
+  r.split = 0;
+  r.st_begin = 0;
+  r.nst = p.stages_total;
+  if (p.splits > 1) {   // (a division takes a hundred cycles, and every role of a CTA starts with this)
+    t = item / p.splits;
+    r.split = item - t * p.splits;
+    r.st_begin = r.split * p.stages_total / p.splits;
+    r.nst = (r.split + 1) * p.stages_total / p.splits - r.st_begin;
+  }
   r.tile = solo ? 2 * p.pairs + t : 2 * t;
   r.ntile = solo ? 1 : 2;
-  r.st_begin = r.split * p.stages_total / p.splits;
-  r.nst = (r.split + 1) * p.stages_total / p.splits - r.st_begin;
   return r;
 }
 
@@ -177,12 +190,6 @@ struct Ring {
 
 __device__ __forceinline__ float silu_f(float g) { return __fdiv_rn(g, 1.0f + expf(-g)); }
 
-__device__ __forceinline__ void store_c(const TcParams& p, int64_t i, float v) {
-  if (p.c_dtype == LOGOS_ACT_PLANES) act_store(p.c_act, i, v);
-  else if (p.c_dtype == LOGOS_F16) reinterpret_cast<__half*>(p.c)[i] = __float2half_rn(v);
-  else if (p.c_dtype == LOGOS_BF16) reinterpret_cast<__nv_bfloat16*>(p.c)[i] = __float2bfloat16_rn(v);
-  else reinterpret_cast<float*>(p.c)[i] = v;
-}
 __device__ __forceinline__ float load_aux(const TcParams& p, int64_t i) {
   if (p.c_dtype == LOGOS_F16) return __half2float(reinterpret_cast<const __half*>(p.aux)[i]);
   if (p.c_dtype == LOGOS_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.aux)[i]);
@@ -241,7 +248,7 @@ __device__ __forceinline__ void add_cols(float2* sum, float s, const uint32_t* b
 // HC columns each of the BLKS blocks at `ta` (blocks are T columns apart); `release` runs once all are read.
 template <int HC, int BLKS, int T, class Release>
 __device__ __forceinline__ void drain_blocks(float2* sum, uint32_t ta, const float* s, Release release) {
-  if constexpr (HC * BLKS <= 32) {   // few columns: all of them in one round of latency
+  if constexpr (HC * BLKS <= (T <= 32 ? 64 : 32)) {   // few columns: all of them in one round of latency
     uint32_t b[HC * BLKS];
 #pragma unroll
     for (int k = 0; k < BLKS; ++k) tc_ld_cols<HC>(ta + k * T, b + k * HC);
@@ -266,57 +273,79 @@ __device__ __forceinline__ void drain_blocks(float2* sum, uint32_t ta, const flo
 }
 
 // A thread's HC sums of output column n, tokens m0 ..: a warp stores 32 consecutive columns of a token at a time.
+// What is chosen at run time (output form, whether all tokens exist) is chosen once, and a row's address is the
+// last one's plus the stride: with both inside the loop the epilogue of one tile took 5800 cycles.
+template <int ROWS, class Put>
+__device__ __forceinline__ void each_row(int rows, Put put) {
+  if (rows >= ROWS) {
+#pragma unroll
+    for (int x = 0; x < ROWS; ++x) put(x);
+  } else {
+#pragma unroll
+    for (int x = 0; x < ROWS; ++x)
+      if (x < rows) put(x);
+  }
+}
+template <int ROWS, class Value>
+__device__ __forceinline__ void put_rows(const TcParams& p, int64_t at, int rows, Value value) {
+  const int64_t ld = p.ldc;
+  if (p.c_dtype == LOGOS_F32) {
+    float* d = reinterpret_cast<float*>(p.c) + at;
+    each_row<ROWS>(rows, [&](int x) { *d = value(x); d += ld; });
+  } else if (p.c_dtype == LOGOS_BF16) {
+    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.c) + at;
+    each_row<ROWS>(rows, [&](int x) { *d = __float2bfloat16_rn(value(x)); d += ld; });
+  } else if (p.c_dtype == LOGOS_F16) {
+    __half* d = reinterpret_cast<__half*>(p.c) + at;
+    each_row<ROWS>(rows, [&](int x) { *d = __float2half_rn(value(x)); d += ld; });
+  } else {
+    ActOut o = p.c_act;
+    o.hi += at;
+    if (o.mode == LOGOS_F32) o.lo += at;
+    each_row<ROWS>(rows, [&](int x) { act_store(o, 0, value(x)); o.hi += ld; o.lo += ld; });
+  }
+}
 template <int HC>
 __device__ __forceinline__ void store_tile(const TcParams& p, const float2* acc, int split, int64_t n, int64_t m0, int lane) {
-  const int rows_here = (int)(p.m - m0 < HC ? p.m - m0 : HC);
-  auto at = [&](int e) { return (e & 1) ? acc[e >> 1].y : acc[e >> 1].x; };
+  const int rows = (int)(p.m - m0 < HC ? p.m - m0 : HC);
+  auto sum = [&](int e) { return (e & 1) ? acc[e >> 1].y : acc[e >> 1].x; };
   if (p.splits > 1) {
-    float* dst = p.partials + ((int64_t)split * p.m + m0) * p.n + n;
-    if (n < p.n) {
-#pragma unroll
-      for (int x = 0; x < HC; ++x)
-        if (x < rows_here) dst[x * p.n] = at(x);
-    }
+    float* d = p.partials + ((int64_t)split * p.m + m0) * p.n + n;
+    if (n < p.n) each_row<HC>(rows, [&](int x) { *d = sum(x); d += p.n; });
   } else if (p.epilogue == EPI_SWIGLU) {
     // rows (2j, 2j+1) are (gate_j, up_j): neighbouring lanes.  The even lane takes the first half of the
     // tokens, the odd lane the second half.
-    const int par = lane & 1;
-    const int64_t out = n >> 1;
+    const int par = lane & 1, first = par * (HC / 2);
+    float g[HC / 2];
 #pragma unroll
     for (int x = 0; x < HC / 2; ++x) {
-      const float a = at(x), b = at(x + HC / 2);
+      const float a = sum(x), b = sum(x + HC / 2);
       const float recv = __shfl_xor_sync(0xffffffffu, par ? a : b, 1);
-      const float g = par ? recv : a, up = par ? b : recv;
-      const int mm = par ? x + HC / 2 : x;
-      if (mm < rows_here && (n | 1) < p.n) store_c(p, (m0 + mm) * p.ldc + out, __fmul_rn(silu_f(g), up));
+      g[x] = __fmul_rn(silu_f(par ? recv : a), par ? b : recv);
     }
+    if ((n | 1) < p.n) put_rows<HC / 2>(p, (m0 + first) * p.ldc + (n >> 1), rows - first, [&](int x) { return g[x]; });
   } else if (n < p.n) {
-    if (p.c_dtype == LOGOS_F32 && p.epilogue == EPI_NONE) {
-      float* dst = reinterpret_cast<float*>(p.c) + m0 * p.ldc + n;
-#pragma unroll
-      for (int x = 0; x < HC; ++x)
-        if (x < rows_here) dst[x * p.ldc] = at(x);
+    const int64_t at = m0 * p.ldc + n;
+    if (p.epilogue == EPI_RESIDUAL) {
+      int64_t i = at;
+      put_rows<HC>(p, at, rows, [&](int x) {
+        const float v = __fadd_rn(sum(x), load_aux(p, i));
+        i += p.ldc;
+        return v;
+      });
     } else {
-#pragma unroll
-      for (int x = 0; x < HC; ++x)
-        if (x < rows_here) {
-          const int64_t ci = (m0 + x) * p.ldc + n;
-          float v = at(x);
-          if (p.epilogue == EPI_RESIDUAL) v = __fadd_rn(v, load_aux(p, ci));
-          store_c(p, ci, v);
-        }
+      put_rows<HC>(p, at, rows, [&](int x) { return sum(x); });
     }
   }
 }
 
 template <int T, int LIMBS, bool TILED>
 __global__ void __launch_bounds__(TcCfg<T, LIMBS>::THREADS, 1)
-q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_ahi,
-                  const __grid_constant__ CUtensorMap map_alo, const __grid_constant__ CUtensorMap map_s,
-                  const TcParams p) {
+q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_a,
+                  const __grid_constant__ CUtensorMap map_s, const TcParams p) {
   using Cfg = TcCfg<T, LIMBS>;
   constexpr int ENTRIES = Cfg::ENTRIES, IB = Cfg::IB, PER = Cfg::PER, ACT_SLOTS = Cfg::ACT_SLOTS, RAW_SLOTS = Cfg::RAW_SLOTS,
-                SC_SLOTS = Cfg::SC_SLOTS, DRAIN_WARP0 = Cfg::DRAIN_WARP0;
+                SC_SLOTS = Cfg::SC_SLOTS;
 
   // Shared memory by 32-bit window addresses: rings of slots, then the barriers.
   extern __shared__ uint8_t smem_raw[];
@@ -340,18 +369,23 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
   // (one thread reads, everyone takes the same decision)
   __shared__ int prior_status;
-  if (tid == 0) {
-    prior_status = *reinterpret_cast<volatile int*>(p.status);
-    for (int i = 0; i < RAW_SLOTS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4 * Cfg::CONV_WGS); }
-    for (int i = 0; i < ACT_SLOTS; ++i) { mbar_init(act_full + 8 * i, 1); mbar_init(act_empty + 8 * i, 1); }
-    for (int i = 0; i < TA_SLOTS; ++i) { mbar_init(ta_full + 8 * i, 4); mbar_init(ta_empty + 8 * i, 1); }
-    for (int i = 0; i < GROUPS * PER; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 16); }
+  constexpr int NBARS = 2 * (RAW_SLOTS + ACT_SLOTS + TA_SLOTS + GROUPS * PER);
+  static_assert(NBARS <= 128, "one barrier a thread");
+  if (warp >= CONV_WARP0 && tid - CONV_WARP0 * 32 < NBARS) {
+    const int i = tid - CONV_WARP0 * 32;
+    const uint32_t bar = raw_full + 8 * i;
+    uint32_t count = 1;                                             // TMA and tcgen05.commit arrive once
+    if (bar >= raw_empty && bar < act_full) count = 4;              // the converter warps
+    else if (bar >= ta_full && bar < ta_empty) count = 4;
+    else if (bar >= act_empty && bar < ta_full) count = 2;          // a commit of each MMA warp
+    else if (bar >= acc_empty) count = 4 * Cfg::DRAIN_WGS;          // the drain warps
+    mbar_init(bar, count);
     fence_barrier_init();
   }
+  if (tid == 0) prior_status = *reinterpret_cast<volatile int*>(p.status);
   if (warp == 1 && lane == 0) {
     prefetch_tensormap(&map_q);
-    prefetch_tensormap(&map_ahi);
-    if (LIMBS == 2) prefetch_tensormap(&map_alo);
+    prefetch_tensormap(&map_a);
     if (!p.s_tiled) prefetch_tensormap(&map_s);
   }
   if (warp == 3) {
@@ -379,20 +413,23 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     regs_dec<Cfg::REGS_MISC>();
     if (warp == 0) {
       // ------------------------------------------------------------ weight and scale producer
-      if (lane == 0) {
-        if (p.wait_scales) pdl_wait();
-        const uint64_t pol = p.stream_once ? policy_evict_first() : policy_evict_normal();
-        Ring<RAW_SLOTS> r;
-        Ring<SC_SLOTS> c;
-        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-          const TcUnit it = tc_unit(p, u);
-          polls = kWaitPolls;
-          for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
-            for (int j = it.tile; j < it.tile + it.ntile; ++j) {
-              const int block = j * p.stages_total + i;   // of a tile-major array
-              const uint32_t bar = raw_full + 8 * r.slot;
-              mbar_wait(raw_empty + 8 * r.slot, r.ph ^ 1u, &polls);
-              if (polls == 0) { ok = false; tc_report(p.status, 2010, i, it.nst); break; }
+      // The single-role warps run their loops with all lanes and issue from one elected lane: addresses and
+      // descriptors stay in uniform registers.  Under a plain `lane == 0` branch a TMA instruction took its
+      // thread about 230 cycles (a stage's four activation loads 1100, more than the stage itself) and a group
+      // of MMAs three times as long.
+      if (p.wait_scales) pdl_wait();
+      const uint64_t pol = p.stream_once ? policy_evict_first() : policy_evict_normal();
+      Ring<RAW_SLOTS> r;
+      Ring<SC_SLOTS> c;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const TcUnit it = tc_unit(p, u);
+        polls = kWaitPolls;
+        for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
+          for (int j = it.tile; j < it.tile + it.ntile; ++j) {
+            const int block = j * p.stages_total + i;   // of a tile-major array
+            const uint32_t bar = raw_full + 8 * r.slot;
+            mbar_wait(raw_empty + 8 * r.slot, r.ph ^ 1u, &polls);
+            if (elect_one()) {
               mbar_arrive_expect_tx(bar, RAW_BYTES + SC_BYTES);
               // row-major weights: tile (row, stage) of a [N][K] map; tile-major: 128 rows of 128 bytes at
               // row block * 128 of a [tiles * stages * 128][128 B] map
@@ -402,42 +439,48 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               // [128 rows][4] box of the [N][K/32] matrix (rows past N read as zero)
               if (TILED || p.s_tiled) bulk_load(scl + c.slot * SC_BYTES, p.s + (int64_t)block * (TC_ROWS * 4), SC_BYTES, bar);
               else tma_load_2d(scl + c.slot * SC_BYTES, &map_s, bar, i * 4, j * TC_ROWS);
-              r.next();
-              c.next();
             }
+            __syncwarp();
+            r.next();
+            c.next();
+          }
+          if (polls == 0) {
+            if (lane == 0) tc_report(p.status, 2010, i, it.nst);
+            ok = false;
           }
         }
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------ activation producer
-      if (lane == 0) {
-        pdl_wait();  // the activations are the previous kernel's output
-        const uint64_t pol = policy_evict_last();
-        Ring<ACT_SLOTS> r;
-        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-          const TcUnit it = tc_unit(p, u);
-          polls = kWaitPolls;
-          const int m0 = it.mtile * T;
-          for (int h = 2 * it.st_begin; h < 2 * (it.st_begin + it.nst); ++h) {
-            mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &polls);
-            if (polls == 0) { ok = false; tc_report(p.status, 2020, h, it.nst); break; }
-            const uint32_t bar = act_full + 8 * r.slot, sb = act + r.slot * Cfg::ACT_BYTES;
+      pdl_wait();  // the activations are the previous kernel's output
+      const uint64_t pol = policy_evict_last();
+      Ring<ACT_SLOTS> r;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const TcUnit it = tc_unit(p, u);
+        polls = kWaitPolls;
+        const int m0 = it.mtile * T;
+        for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
+          const uint32_t bar = act_full + 8 * r.slot;
+          mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &polls);
+          if (elect_one()) {
             mbar_arrive_expect_tx(bar, Cfg::ACT_BYTES);
-            tma_load_2d_hint(sb, &map_ahi, bar, h * 64, m0, pol);
-            if (LIMBS == 2) tma_load_2d_hint(sb + T * 128, &map_alo, bar, h * 64, m0, pol);
-            r.next();
+            tma_load_4d_hint(act + r.slot * Cfg::ACT_BYTES, &map_a, bar, 0, m0, 2 * i, 0, pol);
+          }
+          __syncwarp();
+          r.next();
+          if (polls == 0) {
+            if (lane == 0) tc_report(p.status, 2020, i, it.nst);
+            ok = false;
           }
         }
       }
     } else {
       // ------------------------------------------------------------ MMA issuers, one warp per half of a stage
-      // A warp runs its loop with all lanes, so that addresses and descriptors stay warp-uniform (with one lane
-      // alone the issue of a group took three times as long), and one elected lane issues the tcgen05
-      // instructions.  The barriers a group needs are polled together: one round of latency, not three.
+      // The barriers a group needs are polled together: one round of latency, not three.
       constexpr uint32_t idesc = make_idesc_f16(0, 0, TC_ROWS, T);
       const int half = warp - 2;
-      const uint64_t bdesc_first = make_desc_sw128(act);
-      Ring<ACT_SLOTS, 2> ra(half);
+      const uint64_t bdesc_first = make_desc_sw128(act + half * T * 128);
+      Ring<ACT_SLOTS> ra;
       Ring<TA_SLOTS, 2> rt(half);
       Ring<GROUPS, 2> rf(half);                                    // the group's own barriers
       Ring<GROUPS, 2> re((half + GROUPS - ENTRIES) % GROUPS, 1u);  // those of the entry's previous group
@@ -466,7 +509,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                   for (int b = 0; b < IB; ++b) {
                     const int l = (LIMBS == 2) ? 1 - (v >> 1) : 0;
                     const int kk = (k * IB + b) * 2 + (v & 1);     // K = 16 step inside the half stage
-                    const uint64_t bdesc = bdesc0 + (uint32_t)((l * T * 128 + kk * 32) >> 4);
+                    const uint64_t bdesc = bdesc0 + (uint32_t)((l * 2 * T * 128 + kk * 32) >> 4);
                     if (LIMBS == 2 && v == 2) tc_mma_f16_ts_scaled_d<11>(d0 + b * T, a0 + kk * 8, bdesc, idesc);
                     else if (v == 0) tc_mma_f16_ts<false>(d0 + b * T, a0 + kk * 8, bdesc, idesc);
                     else tc_mma_f16_ts<true>(d0 + b * T, a0 + kk * 8, bdesc, idesc);
@@ -498,66 +541,49 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // ------------------------------------------------------------ converters: int8 smem -> fp16 TMEM
     regs_dec<Cfg::REGS_CONV>();
     const int qd = warp & 3;
-    const int first = Cfg::CONV_WGS == 2 ? (warp - CONV_WARP0) >> 2 : 0;   // the group's (first) half
     const uint32_t row = qd * 32 + lane;
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16);
-    // the row's 16-byte chunks of a half: chunk c sits at c ^ (row & 7) (128-byte swizzle); the second half's
-    // chunks differ in bit 6 of the address
+    // the row's eight 16-byte chunks: chunk c sits at c ^ (row & 7) (128-byte swizzle)
     uint32_t off[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) off[c] = raw + swz128(row, first * 4 + c);
-    auto load_half = [&](uint4 (&wv)[4], int slot, uint32_t flip) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) wv[c] = lds_v4((off[c] ^ flip) + slot * RAW_BYTES);
-    };
-    auto convert_store = [&](const uint4 (&wv)[4], uint32_t t_dst) {
-#pragma unroll
-      for (int c2 = 0; c2 < 2; ++c2) {
-        uint32_t o[16];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const uint4 w4 = wv[c2 * 2 + c];
-          const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-          for (int wi = 0; wi < 4; ++wi) {
-            const uint32_t w = TILED ? ws[wi] : ws[wi] ^ 0x80808080u;   // tile-major bytes hold q + 128 already
-            o[c * 8 + 2 * wi] = cvt_pair(w, 0x4140);
-            o[c * 8 + 2 * wi + 1] = cvt_pair(w, 0x4342);
-          }
-        }
-        tc_st_32x32b_x16(t_dst + c2 * 16, o);
-      }
-    };
-    auto stored = [&](uint32_t bar) {
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      mbar_arrive_if(bar, lane == 0);
-    };
+    for (int c = 0; c < 4; ++c) off[c] = raw + swz128(row, c);   // chunk c + 4: bit 6 of the address flipped
     Ring<RAW_SLOTS> r;
-    Ring<TA_SLOTS, 2> a(first, 1u);
+    Ring<TA_SLOTS, 2> a(0, 1u);   // a stage takes slots a and a + 1
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
       polls = kWaitPolls;
       const int count = it.nst * it.ntile;
       for (int i = 0; i < count && ok; ++i) {
-        uint4 wv[4];
-        mbar_wait2(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, &polls);
+        // everything the stage needs in one wait, all its loads together, one wait for its stores: a round of
+        // latency costs as much as fifty instructions
+        mbar_wait3(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, ta_empty + 8 * (a.slot + 1), a.ph, &polls);
         tc_fence_after();
-        load_half(wv, r.slot, 0u);
-        convert_store(wv, t_lane + a.slot * TA_SLOT_COLS);
-        if (Cfg::CONV_WGS == 2) {
-          mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
-          stored(ta_full + 8 * a.slot);
-        } else {
-          load_half(wv, r.slot, 64u);
-          stored(ta_full + 8 * a.slot);
-          mbar_wait(ta_empty + 8 * (a.slot + 1), a.ph, &polls);
-          tc_fence_after();
-          convert_store(wv, t_lane + (a.slot + 1) * TA_SLOT_COLS);
-          mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
-          stored(ta_full + 8 * (a.slot + 1));
+        uint4 wv[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) wv[c] = lds_v4((off[c & 3] ^ (c & 4 ? 64u : 0u)) + r.slot * RAW_BYTES);
+        const uint32_t t_dst = t_lane + a.slot * TA_SLOT_COLS;
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) {
+          uint32_t o[32];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const uint4 w4 = wv[c2 * 4 + c];
+            const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int wi = 0; wi < 4; ++wi) {
+              const uint32_t w = TILED ? ws[wi] : ws[wi] ^ 0x80808080u;   // tile-major bytes hold q + 128 already
+              o[c * 8 + 2 * wi] = cvt_pair(w, 0x4140);
+              o[c * 8 + 2 * wi + 1] = cvt_pair(w, 0x4342);
+            }
+          }
+          tc_st_32x32b_x32(t_dst + c2 * 32, o);
         }
+        mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_if(ta_full + 8 * a.slot, lane == 0);
+        mbar_arrive_if(ta_full + 8 * (a.slot + 1), lane == 0);
         a.next();
         r.next();
         if (polls == 0) {
@@ -570,8 +596,10 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // ------------------------------------------------------------ drain + epilogue
     regs_inc<Cfg::REGS_DRAIN>();
     const int qd = warp & 3;
-    const int g = (warp - DRAIN_WARP0) >> 3;        // the tile of a pair
-    const int th = ((warp - DRAIN_WARP0) >> 2) & 1;
+    constexpr int DW = 4 * Cfg::DRAIN_WGS;
+    constexpr int SHARE = Cfg::DRAIN_WGS / 2;       // warps that share a lane quarter of a tile of a pair
+    const int g = (warp - DRAIN_WARP0) / (DW / 2);  // the tile of a pair
+    const int th = ((warp - DRAIN_WARP0) >> 2) % SHARE;
     const int nl = qd * 32 + lane;                  // row of the tile this thread drains
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16) + Cfg::ACC_COL0;
     const uint32_t s_lane = scl + nl * 16;
@@ -587,41 +615,65 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // one stage of a tile, from this warp's first column `col` on
     auto drain_stage = [&](auto hc, float2* sum, uint32_t col, auto arrivals) {
       float s[4];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t at = t_lane + col + ent * Cfg::ENTRY_COLS;
+      auto scales = [&] {
+        const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
+        s[0] = __uint_as_float(sc.x); s[1] = __uint_as_float(sc.y); s[2] = __uint_as_float(sc.z); s[3] = __uint_as_float(sc.w);
+      };
+      if constexpr (T <= 32 && 4 * hc <= 64) {   // few columns: the whole stage in one round of latency
+        const uint32_t at0 = t_lane + col + ent * Cfg::ENTRY_COLS;
         step(ent, 1, ENTRIES);
+        const uint32_t at1 = t_lane + col + ent * Cfg::ENTRY_COLS;
+        step(ent, 1, ENTRIES);
+        mbar_wait2(acc_full + 8 * grp, ph, acc_full + 8 * (grp + 1), ph, &polls);
+        tc_fence_after();
+        uint32_t b[4 * hc];
+        tc_ld_cols<hc>(at0, b);
+        tc_ld_cols<hc>(at0 + T, b + hc);
+        tc_ld_cols<hc>(at1, b + 2 * hc);
+        tc_ld_cols<hc>(at1 + T, b + 3 * hc);
+        scales();
+        tc_loaded(b);
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_n_if<arrivals>(acc_empty + 8 * grp, lane == 0);
+        mbar_arrive_n_if<arrivals>(acc_empty + 8 * (grp + 1), lane == 0);
 #pragma unroll
-        for (int k = 0; k < PER; ++k) {
-          const uint32_t bar = 8 * (PER * (grp + h) + k);
-          mbar_wait(acc_full + bar, ph, &polls);
-          tc_fence_after();
-          if (h == 0 && k == 0) {
-            const uint4 sc = lds_v4(s_lane + rc * SC_BYTES);
-            s[0] = __uint_as_float(sc.x); s[1] = __uint_as_float(sc.y); s[2] = __uint_as_float(sc.z); s[3] = __uint_as_float(sc.w);
+        for (int k = 0; k < 4; ++k) add_cols<hc>(sum, s[k], b + k * hc);
+      } else {
+        if (PER == 1) mbar_wait2(acc_full + 8 * grp, ph, acc_full + 8 * (grp + 1), ph, &polls);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t at = t_lane + col + ent * Cfg::ENTRY_COLS;
+          step(ent, 1, ENTRIES);
+#pragma unroll
+          for (int k = 0; k < PER; ++k) {
+            const uint32_t bar = 8 * (PER * (grp + h) + k);
+            if (PER > 1) mbar_wait(acc_full + bar, ph, &polls);
+            if (PER > 1 || h == 0) tc_fence_after();
+            if (h == 0 && k == 0) scales();
+            drain_blocks<hc, IB, T>(sum, at + k * IB * T, s + h * 2 + k * IB, [&] {
+              tc_fence_before();
+              __syncwarp();
+              mbar_arrive_n_if<arrivals>(acc_empty + bar, lane == 0);
+            });
           }
-          drain_blocks<hc, IB, T>(sum, at + k * IB * T, s + h * 2 + k * IB, [&] {
-            tc_fence_before();
-            __syncwarp();
-            mbar_arrive_n_if<arrivals>(acc_empty + bar, lane == 0);
-          });
         }
       }
     };
-    constexpr std::integral_constant<int, T / 2> half_cols{};
-    constexpr std::integral_constant<int, T / 4> quarter_cols{};
+    constexpr std::integral_constant<int, T / SHARE> pair_cols{};
+    constexpr std::integral_constant<int, T / Cfg::DRAIN_WGS> solo_cols{};
     constexpr std::integral_constant<int, 1> one{};
-    constexpr std::integral_constant<int, 2> two{};   // eight warps stand for sixteen arrivals
+    constexpr std::integral_constant<int, 2> two{};   // half of the drain warps stand for all of them
 
     int u = blockIdx.x;
     for (; u < pair_units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
       polls = kWaitPolls;
-      float2 acc[T / 4];
+      float2 acc[pair_cols / 2];
 #pragma unroll
-      for (int x = 0; x < T / 4; ++x) acc[x] = make_float2(0.f, 0.f);
+      for (int x = 0; x < pair_cols / 2; ++x) acc[x] = make_float2(0.f, 0.f);
       for (int i = 0; i < it.nst && polls != 0; ++i) {
-        drain_stage(half_cols, acc, th * (T / 2), two);
+        drain_stage(pair_cols, acc, th * pair_cols, two);
         step(ent, 2 % ENTRIES, ENTRIES);            // past the other tile's two groups
         step(rc, 2, SC_SLOTS);
         grp ^= 4;
@@ -632,23 +684,23 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         ok = false;
         break;
       }
-      store_tile<T / 2>(p, acc, it.split, (int64_t)(it.tile + g) * TC_ROWS + nl, (int64_t)it.mtile * T + th * (T / 2), lane);
+      store_tile<pair_cols>(p, acc, it.split, (int64_t)(it.tile + g) * TC_ROWS + nl, (int64_t)it.mtile * T + th * pair_cols, lane);
     }
     // From here on a warp waits for barriers that only the other tile's warps have followed so far: once all have
     // come this far, their phases of the pair units are over.  (Every drain warp passes here exactly once.)
-    asm volatile("bar.sync 1, 512;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
     ent = (ent + 2 * ENTRIES - 2 * g) % ENTRIES;
     rc = (rc + SC_SLOTS - g) % SC_SLOTS;
     grp -= 2 * g;
     for (; u < units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
       polls = kWaitPolls;
-      float2 acc[T / 8];
+      float2 acc[solo_cols / 2];
 #pragma unroll
-      for (int x = 0; x < T / 8; ++x) acc[x] = make_float2(0.f, 0.f);
-      const uint32_t col = (2 * g + th) * (T / 4);
+      for (int x = 0; x < solo_cols / 2; ++x) acc[x] = make_float2(0.f, 0.f);
+      const uint32_t col = (SHARE * g + th) * solo_cols;
       for (int i = 0; i < it.nst && polls != 0; ++i) {
-        drain_stage(quarter_cols, acc, col, one);
+        drain_stage(solo_cols, acc, col, one);
         step(rc, 1, SC_SLOTS);
         step(grp, 2, GROUPS);
         ph ^= (uint32_t)(grp == 0);
@@ -658,7 +710,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         ok = false;
         break;
       }
-      store_tile<T / 4>(p, acc, it.split, (int64_t)it.tile * TC_ROWS + nl, (int64_t)it.mtile * T + col, lane);
+      store_tile<solo_cols>(p, acc, it.split, (int64_t)it.tile * TC_ROWS + nl, (int64_t)it.mtile * T + col, lane);
     }
   }
 
@@ -672,36 +724,29 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 }
 
 // ---------------------------------------------------------------- host side
+// What a tensor map is a function of: address, extents, pitches and box.  Maps are encoded once and kept.
 struct MapKey {
   const void* base;
-  uint64_t d0, d1, d2, pitch1, pitch2;
-  uint32_t box0, box1, elem, swizzle;
+  uint64_t d0, d1, d2, d3, p1, p2, p3;
+  uint32_t b0, b1, b2, b3, elem, swizzle;
   bool operator==(const MapKey& o) const {
-    return base == o.base && d0 == o.d0 && d1 == o.d1 && d2 == o.d2 && pitch1 == o.pitch1 && pitch2 == o.pitch2 &&
-           box0 == o.box0 && box1 == o.box1 && elem == o.elem && swizzle == o.swizzle;
+    return base == o.base && d0 == o.d0 && d1 == o.d1 && d2 == o.d2 && d3 == o.d3 && p1 == o.p1 && p2 == o.p2 && p3 == o.p3 &&
+           b0 == o.b0 && b1 == o.b1 && b2 == o.b2 && b3 == o.b3 && elem == o.elem && swizzle == o.swizzle;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     uint64_t h = reinterpret_cast<uint64_t>(k.base);
-    for (uint64_t v : {k.d0, k.d1, k.d2, k.pitch1, k.pitch2, ((uint64_t)k.box0 << 32) | k.box1,
+    for (uint64_t v : {k.d0, k.d1, k.d2, k.d3, k.p1, k.p2, k.p3, ((uint64_t)k.b0 << 32) | k.b1, ((uint64_t)k.b2 << 32) | k.b3,
                        ((uint64_t)k.elem << 32) | k.swizzle})
       h = h * 0x9E3779B97F4A7C15ull + v;
-    return (size_t)h;
+    return (size_t)(h ^ (h >> 29));
   }
 };
 
-}  // namespace
-
-// Tensor maps are pure functions of (address, shape, box): encode once, reuse.  d2 == 0 asks
-// for a 2-D map [d1][d0] with the given swizzle; otherwise a 3-D map [d2][d1][d0], box depth 1,
-// no swizzle.
-logos_status_t cached_map(CUtensorMap* out, const void* base, CUtensorMapDataType dt, uint32_t elem, uint64_t d0,
-                          uint64_t d1, uint64_t pitch1, uint32_t box0, uint32_t box1, CUtensorMapSwizzle swizzle,
-                          uint64_t d2, uint64_t pitch2) {
+logos_status_t map_cached(CUtensorMap* out, const MapKey& key, CUtensorMapDataType dt) {   // d2 == 0: two dimensions
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  MapKey key{base, d0, d1, d2, pitch1, pitch2, box0, box1, elem, (uint32_t)swizzle};
   {
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
@@ -710,13 +755,34 @@ logos_status_t cached_map(CUtensorMap* out, const void* base, CUtensorMapDataTyp
       return LOGOS_OK;
     }
   }
-  if (d2 == 0) LOGOS_TRY(make_tensor_map_2d(out, base, dt, elem, d0, d1, pitch1, box0, box1, swizzle));
-  else LOGOS_TRY(make_tensor_map_3d(out, base, dt, elem, d0, d1, d2, pitch1, pitch2, box0, box1, 1));
+  if (key.d2 == 0) {
+    LOGOS_TRY(make_tensor_map_2d(out, key.base, dt, key.elem, key.d0, key.d1, key.p1, key.b0, key.b1, (CUtensorMapSwizzle)key.swizzle));
+  } else {
+    const uint64_t dims[4] = {key.d0, key.d1, key.d2, key.d3}, pitch[3] = {key.p1, key.p2, key.p3};
+    const uint32_t box[4] = {key.b0, key.b1, key.b2, key.b3};
+    LOGOS_TRY(make_tensor_map_4d(out, key.base, dt, key.elem, dims, pitch, box, (CUtensorMapSwizzle)key.swizzle));
+  }
   std::lock_guard<std::mutex> lk(mu);
   if (cache.size() > 8192) cache.clear();
   cache[key] = *out;
   return LOGOS_OK;
 }
+
+}  // namespace
+
+logos_status_t cached_map(CUtensorMap* out, const void* base, CUtensorMapDataType dt, uint32_t elem, uint64_t d0,
+                          uint64_t d1, uint64_t pitch1, uint32_t box0, uint32_t box1, CUtensorMapSwizzle swizzle) {
+  return map_cached(out, MapKey{base, d0, d1, 0, 0, pitch1, 0, 0, box0, box1, 0, 0, elem, (uint32_t)swizzle}, dt);
+}
+
+namespace {
+
+logos_status_t cached_map_4d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, uint64_t d0, uint64_t d1, uint64_t d2,
+                             uint64_t d3, uint64_t p1, uint64_t p2, uint64_t p3, uint32_t b1, uint32_t b2, uint32_t b3) {
+  return map_cached(out, MapKey{base, d0, d1, d2, d3, p1, p2, p3, (uint32_t)d0, b1, b2, b3, 2, (uint32_t)CU_TENSOR_MAP_SWIZZLE_128B}, dt);
+}
+
+}  // namespace
 
 namespace {
 
@@ -792,7 +858,7 @@ TcPlan plan_for(int64_t m, int64_t n, int64_t k, int64_t splits, int device) {
 template <int T, int LIMBS>
 logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) {
   using Cfg = TcCfg<T, LIMBS>;
-  CUtensorMap mq, mhi, mlo, ms;
+  CUtensorMap mq, ma, ms;
   const int64_t stages = (g.k + TC_KSTAGE - 1) / TC_KSTAGE, tiles = (g.n + TC_ROWS - 1) / TC_ROWS;
   if (g.q_tiled) {
     const uint64_t rows = (uint64_t)tiles * (uint64_t)stages * TC_ROWS;
@@ -800,12 +866,11 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   } else {
     LOGOS_TRY(cached_map(&mq, g.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)g.k, (uint64_t)g.n, (uint64_t)g.k, TC_KSTAGE, TC_ROWS));
   }
-  LOGOS_TRY(cached_map(&mhi, g.a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)g.k, (uint64_t)g.m, (uint64_t)g.lda * 2, 64, T));
-  if (LIMBS == 2)
-    LOGOS_TRY(cached_map(&mlo, g.a_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)g.k, (uint64_t)g.m, (uint64_t)g.lda * 2, 64, T));
-  else
-    mlo = mhi;
-  ms = mhi;
+  // [planes][halves of a stage][tokens][64]: the planes lie at any multiple of 16 bytes from each other
+  LOGOS_TRY(cached_map_4d(&ma, g.a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 64, (uint64_t)g.m, (uint64_t)(2 * stages), LIMBS,
+                          (uint64_t)g.lda * 2, 128, LIMBS == 2 ? (uint64_t)(reinterpret_cast<const char*>(g.a_lo) - static_cast<const char*>(g.a)) : 128,
+                          T, 2, LIMBS));
+  ms = ma;
   const bool s_tiled = g.q_tiled || g.s_tiled;
   if (!s_tiled)
     LOGOS_TRY(cached_map(&ms, g.s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)(g.k / 32), (uint64_t)g.n, (uint64_t)(g.k / 32) * 4, 4,
@@ -836,7 +901,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   // persistent CTAs: one per SM at most, each takes units blockIdx.x, blockIdx.x + gridDim.x, ...
   const int sms = sm_count(g.device);
   dim3 grid((unsigned)(units < sms ? units : sms), 1u, 1u);
-  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, st, mq, mhi, mlo, ms, p));
+  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, st, mq, ma, ms, p));
   count_launch(LK_GEMM_TC);
   return check_launch("q8_gemm_tc_kernel");
 }
@@ -859,7 +924,8 @@ bool gemm_tc_applicable(const GemmArgs& g) {
   // K of whole stages, or scales in the tile-major form: the row-major box needs rows of 16-byte multiples
   if (g.k % TC_KSTAGE && !g.q_tiled && !g.s_tiled) return false;
   if (g.m < 1 || g.n < 1) return false;
-  if (g.lda % 8) return false;
+  if (g.lda % 8 || g.lda < (g.k + TC_KSTAGE - 1) / TC_KSTAGE * TC_KSTAGE) return false;   // whole stages, zero past K
+  if (g.a_lo && reinterpret_cast<uintptr_t>(g.a_lo) <= reinterpret_cast<uintptr_t>(g.a)) return false;
   if ((reinterpret_cast<uintptr_t>(g.a) & 15u) || (reinterpret_cast<uintptr_t>(g.a_lo) & 15u) ||
       (reinterpret_cast<uintptr_t>(g.q) & 15u) || (reinterpret_cast<uintptr_t>(g.s) & 15u))
     return false;
