@@ -236,16 +236,16 @@ LOGOS_API logos_status_t logos_gqa_decode_attn(logos_handle_t q, logos_handle_t 
  * that the kernel's persistent grid cuts go to a fixed 6 MiB array inside the library image
  * instead of library-allocated scratch, so every GPU that loads the library holds those 6 MiB
  * until the process exits.  What the kernel needs depends on the GPU, not on the shape: two
- * slots of 16 * (d + 2) floats and a 16-byte descriptor per CTA, two CTAs per SM (4.7 MiB on a
- * 148-SM B200 at d = 128);
- * a GPU with so many SMs that this exceeds the array is refused with LOGOS_OUT_OF_BOUNDS and
+ * slots of 16 * (d + 2) floats per CTA, two CTAs per SM (4.7 MiB on a
+ * 148-SM B200 at d = 128), and a counter per (sequence, KV head) pair in the last MiB;
+ * a GPU with so many SMs, or a call with so many pairs, that this exceeds the array is refused with LOGOS_OUT_OF_BOUNDS and
  * a message giving both sizes, and so is a call with more than 2048 sequences (the limit of
- * both attention entry points: a CTA keeps one tile count per sequence in shared memory).
+ * both attention entry points: a CTA keeps the lengths in shared memory).
  * The call itself makes no
  * cudaMalloc / cudaFree.  The first call on a device looks up the array's device address;
  * make that first call outside any stream capture.  All calls share the one array and one
  * status word.  Nothing is cleared between calls: the partials are always written before
- * they are read, and the status word is zero until a bounded wait inside the kernel gives up,
+ * they are read, the counters return to zero, and the status word is zero until a bounded wait inside the kernel gives up,
  * after which calls on this entry point leave `o` untouched until logos_kernel_status has
  * reported and cleared the code (call logos_kernel_status once at start-up if it must not
  * allocate later).  Two calls that overlap on the GPU race on the array: keep calls on this

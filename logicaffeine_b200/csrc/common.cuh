@@ -86,6 +86,19 @@ logos_status_t buf_ptr(logos_handle_t h, int64_t elems, const char* name, T** ou
 // captured decode step points at is owned by the model.
 logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out);
 
+// Arrival counters of the stand-alone attention calls, one block per device, zeroed when it is allocated; the kernels
+// leave them at zero.  Ordered like scratch_get's blocks.
+logos_status_t counters_get(int32_t device, int64_t bytes, void** out);
+// Counters that someone else owns (a model): a kernel that gave up leaves them in the middle of a count, so
+// counters_reset zeroes all of a device's once such a failure has been read.
+void counters_register(int32_t device, void* ptr, int64_t bytes);
+void counters_unregister(void* ptr);
+logos_status_t counters_reset(int32_t device);
+
+// cudaFuncAttributeMaxDynamicSharedMemorySize of `kernel` on the current device, raised to `bytes` once instead of
+// on every launch.
+logos_status_t allow_smem(const void* kernel, int device, int bytes);
+
 int sm_count(int device);
 
 // Per-device status word in device memory: kernels store a non-zero code when

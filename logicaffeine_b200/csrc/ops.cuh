@@ -111,11 +111,13 @@ struct AttnArgs {
   // point at memory another caller can outgrow).
   void*         ext_scratch = nullptr;
   int64_t       ext_scratch_bytes = 0;
+  void*         ext_arrive = nullptr;      // with ext_scratch: b * h_kv + 1 counters, zero before the first call
+  int64_t       ext_arrive_bytes = 0;
   int*          ext_status = nullptr;
 };
 logos_status_t launch_gqa_decode_attn(const AttnArgs& a, cudaStream_t st);
 // Bytes of split-KV scratch a call with these extents (b, h_q, h_kv, d, l_max, device) needs:
-// what a caller that passes ext_scratch has to provide.
+// what a caller that passes ext_scratch has to provide (the counters come on top).
 int64_t attn_scratch_bytes(const AttnArgs& a);
 logos_status_t launch_kv_append_rope(__half* k_cache, __half* v_cache, const __half* k_new, const __half* v_new,
                                      const float* rope, int32_t* seq_len, int64_t b, int64_t h_kv, int64_t d,

@@ -897,7 +897,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   if (p.splits > p.stages_total) return fail(LOGOS_ERROR, "q8_gemm: more K splits than 128-column stages");
 
   auto kernel = g.q_tiled ? q8_gemm_tc_kernel<T, LIMBS, true> : q8_gemm_tc_kernel<T, LIMBS, false>;
-  LOGOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
+  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), g.device, (int)Cfg::SMEM));
   // persistent CTAs: one per SM at most, each takes units blockIdx.x, blockIdx.x + gridDim.x, ...
   const int sms = sm_count(g.device);
   dim3 grid((unsigned)(units < sms ? units : sms), 1u, 1u);

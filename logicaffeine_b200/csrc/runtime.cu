@@ -142,6 +142,77 @@ logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out) 
   return LOGOS_OK;
 }
 
+namespace {
+struct Counters {
+  int32_t device;
+  void*   ptr;
+  int64_t bytes;
+  bool    own;     // the library's block of the device (the latest one)
+};
+std::mutex g_counters_mu;
+std::vector<Counters> g_counters;
+}  // namespace
+
+logos_status_t counters_get(int32_t device, int64_t bytes, void** out) {
+  std::lock_guard<std::mutex> lk(g_counters_mu);
+  int64_t have = 0;
+  for (const Counters& c : g_counters)
+    if (c.own && c.device == device && c.bytes > have) {
+      have = c.bytes;
+      *out = c.ptr;
+    }
+  if (have >= bytes) return LOGOS_OK;
+  const int64_t want = ((bytes > 2 * have ? bytes : 2 * have) + 4095) & ~int64_t(4095);
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, (size_t)want);   // an outgrown block stays: launches already enqueued may use it
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc (arrival counters)");
+  e = cudaMemset(p, 0, (size_t)want);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return cuda_fail(e, "cudaMemset (arrival counters)");
+  }
+  LOGOS_CUDA_TRY(cudaDeviceSynchronize());        // zero before a launch on any stream (once per growth)
+  g_counters.push_back({device, p, want, true});
+  *out = p;
+  return LOGOS_OK;
+}
+void counters_register(int32_t device, void* ptr, int64_t bytes) {
+  std::lock_guard<std::mutex> lk(g_counters_mu);
+  g_counters.push_back({device, ptr, bytes, false});
+}
+void counters_unregister(void* ptr) {
+  std::lock_guard<std::mutex> lk(g_counters_mu);
+  for (size_t i = 0; i < g_counters.size(); ++i)
+    if (g_counters[i].ptr == ptr) {
+      g_counters.erase(g_counters.begin() + (long)i);
+      return;
+    }
+}
+logos_status_t counters_reset(int32_t device) {
+  std::lock_guard<std::mutex> lk(g_counters_mu);
+  for (const Counters& c : g_counters)
+    if (c.device == device) LOGOS_CUDA_TRY(cudaMemset(c.ptr, 0, (size_t)c.bytes));
+  return LOGOS_OK;
+}
+
+logos_status_t allow_smem(const void* kernel, int device, int bytes) {
+  struct Seen {
+    const void* kernel;
+    int device, bytes;
+  };
+  thread_local std::vector<Seen> seen;   // a few kernels: a scan is cheaper than any lock
+  for (Seen& s : seen)
+    if (s.kernel == kernel && s.device == device) {
+      if (s.bytes >= bytes) return LOGOS_OK;
+      LOGOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      s.bytes = bytes;
+      return LOGOS_OK;
+    }
+  LOGOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  seen.push_back({kernel, device, bytes});
+  return LOGOS_OK;
+}
+
 int sm_count(int device) {
   static std::mutex mu;
   static std::unordered_map<int, int> cache;

@@ -111,7 +111,10 @@ logos_status_t kernel_status_read(int device, int* out, bool clear) {
     set_last_error("device-side wait gave up: code " + std::to_string(words[0]) + " block (" + std::to_string(words[1]) +
                    "," + std::to_string(words[2]) + ") stage " + std::to_string(words[3]) + " of " +
                    std::to_string(words[4]) + " warp " + std::to_string(words[5]));
-    if (clear) LOGOS_CUDA_TRY(cudaMemset(p, 0, sizeof(words)));
+    if (clear) {
+      LOGOS_TRY(counters_reset(device));
+      LOGOS_CUDA_TRY(cudaMemset(p, 0, sizeof(words)));
+    }
   }
   return LOGOS_OK;
 }

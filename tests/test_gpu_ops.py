@@ -252,6 +252,35 @@ def test_gqa_decode_attn_fused_kv_bit_exact(llm, oracle, b, hq, hkv, d, lmax, le
     assert rel_l2(o, ref) < 1e-3
 
 
+@pytest.mark.parametrize("b,hq,hkv,d,lmax,lens", [
+    (1, 2, 1, 64, 64 * 200, [64 * 200 - 2]),           # one pair cut into more parts than the list holds
+    (1, 12, 2, 128, 64 * 70, [64 * 66 - 1]),           # more shares than tiles: some hold none
+    (2, 16, 1, 64, 64 * 64, [64 * 63, 0]),             # 64 parts beside a pair of one tile
+    (40, 32, 8, 128, 200, [(37 * i) % 199 for i in range(40)]),   # more pairs than shares: whole and cut ones
+])
+def test_gqa_decode_attn_cut_pairs_fold_the_same_every_time(llm, oracle, b, hq, hkv, d, lmax, lens):
+    O = oracle
+    q, kn, vn, kc, vc, seq = _attn_inputs(O, b, hq, hkv, d, lmax, lens, seed=4)
+    tab = O.rope_table(lmax, d, 1e6)
+    scale = 1.0 / np.sqrt(d)
+    dq, dkn, dvn, dkc, dvc, dtab, dseq = (_dev(llm, x) for x in (q, kn, vn, kc, vc, tab, seq))
+    do = llm.DeviceBuffer(b * hq * d * 2)
+    for _ in range(2):   # the second call finds the arrival counters and the lengths as the first left them
+        llm.gqaDecodeAttnFused(dq, dkn, dvn, dkc, dvc, dtab, dseq, do, b, hq, hkv, d, lmax, scale)
+        o = O.f16_to_f32(do.download(np.uint16, (b, hq, d)))
+        ref = O.f16_to_f32(O.gqa_decode_attn_fused(q, kn, vn, kc, vc, tab, seq, scale))
+        assert llm.kernelStatus() == 0
+        assert np.array_equal(dseq.download(np.int32, (b,)), seq)
+        # both sides round to fp16 (2^-11 relative at most, each); the sums before it differ by some f32 roundings
+        assert rel_l2(o, ref) < 1e-3
+    # nothing appended: the same inputs again and again, bit for bit
+    llm.gqaDecodeAttn(dq, dkc, dvc, dseq, do, b, hq, hkv, d, lmax, scale)
+    first = do.download(np.uint16, (b, hq, d))
+    for _ in range(20):
+        llm.gqaDecodeAttn(dq, dkc, dvc, dseq, do, b, hq, hkv, d, lmax, scale)
+    assert np.array_equal(do.download(np.uint16, (b, hq, d)), first)
+
+
 def test_gqa_decode_attn_config2_full_size(llm, oracle):
     """Config 2 as BASELINE.json states it: batch 32, 28 query / 4 KV heads, head_dim 128, 4096
     cached positions, one token appended per sequence with RoPE theta 1e6: the KV cache after the
