@@ -1,28 +1,26 @@
 // Q8 GEMV: y[n] = sum_kb s[n,kb] * sum_{k in kb} q[n,k] * x[k].
 //
-// HBM-bound: 1.125 bytes of weights per multiply-add, so the kernel is a
-// coalesced stream.  One warp owns one row at a time; every lane issues 128-bit
-// read-only loads of 16 consecutive int8 (a half block), so a warp covers 512
-// columns per load and keeps eight such loads in flight.  int8 -> f32 uses
-// the 2^23 mantissa trick (one byte-permute and one subtract), the half-block
-// dot product is scaled by its block's f32 scale in registers, and the row sum
-// is a warp-shuffle reduction.  x lives in shared memory, laid out so the
-// four 128-bit reads a lane needs are bank-conflict free.
+// HBM-bound: 1.125 bytes of weights per multiply-add, so the kernel is a coalesced stream that must
+// not stop while the products are computed.  Every warp owns a ring of three 2 KiB stages of weights
+// (with their scales) in shared memory and fills it itself with asynchronous copies: a lane copies
+// the bytes that it will use, so nothing wider than the warp ever waits, and an SM keeps up to 100 KiB
+// in flight whatever its warps compute.  int8 -> f32 uses the 2^23 mantissa trick (one byte-permute
+// and one subtract), the half-block dot product is scaled by its block's f32 scale in registers, and
+// the row sum is a warp-shuffle reduction.  x lives in shared memory, laid out so that the four
+// 128-bit reads a lane needs are bank-conflict free; a warp takes two rows at a time, because a row at
+// a time needs four bytes of x for a byte of weights from the same port.
 #include "ops.cuh"
+
+#include <algorithm>
 
 namespace logos {
 
 namespace {
 
-constexpr int GEMV_WARPS = 8;
-
-__device__ __forceinline__ uint4 ldg_nc_v4(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
+constexpr int GEMV_DEPTH = 3;                     // stages of a warp's ring
+constexpr int GEMV_WARPS = 24, GEMV_FEW_WARPS = 16;  // a CTA has; one CTA fills an SM
+constexpr int GEMV_STAGE = 2048 + 64 * 4;         // 128 chunks of 16 weights, 64 scales
+constexpr int GEMV_SMEM = 227 * 1024;
 
 // byte `sel` of the bias-flipped word -> exact float value of the int8
 __device__ __forceinline__ float byte_to_f32(uint32_t w_xor80, uint32_t selector) {
@@ -45,86 +43,117 @@ __device__ __forceinline__ float dot4(uint32_t w, float4 x, float acc) {
 // the same j of consecutive chunks touch consecutive 16-byte slots.
 __device__ __forceinline__ int xs4_index(int chunk, int j) { return (chunk >> 5) * 128 + j * 32 + (chunk & 31); }
 
-// A warp owns one row.  For each super-chunk of 4096 columns a lane first issues
-// all of its eight 128-bit weight loads (and the eight scales), and only then
-// waits for x to be staged, so the HBM stream starts at the first instruction.
-// What decides the speed is the bytes an SM keeps in flight: the launch bound caps the
-// kernel at 64 registers so that four CTAs share an SM (128 KB of loads in flight, and the
-// 512 CTAs of a 4096-row matrix are one wave); with three CTAs per SM the same code
-// measured 3.2 instead of 3.4 TB/s at 4096 x 4096 and 4.05 instead of 4.3 TB/s at
-// 152064 x 5120.
-template <bool X_IN_SMEM>
-__global__ void __launch_bounds__(GEMV_WARPS * 32, 4)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// A warp takes R neighbouring rows (a group); groups go round the CTAs first, so that a small matrix still
+// uses every SM.  The ring runs on from one group to the next.  Measured before (eight loads a lane in flight in
+// registers, four CTAs an SM) -> now: 152064 x 5120 197 -> 148 us (5.9 TB/s), 151936 x 896 72 -> 37 us,
+// 27648 x 5120 43 -> 33 us, 5120 x 27648 154 -> 41 us, 300 x 16384 13.6 -> 8.3 us.  Four rows at a time
+// measured 166 us on the first, one row 164 us.
+template <int R, bool X_IN_SMEM>
+__global__ void __launch_bounds__(GEMV_WARPS * 32, 1)
 q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const float* __restrict__ x,
                float* __restrict__ y, int64_t n, int64_t k) {
+  constexpr int U = 4 / R;   // chunks of a row that a lane has in a stage
   extern __shared__ float4 xs4[];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  const int warp = tid >> 5;
+  const int warp = tid >> 5, warps = blockDim.x >> 5;
   const int chunks = (int)(k >> 4);  // 16-element chunks per row
-  const int64_t kb_per_row = k >> 5;
+  const int kb = (int)(k >> 5);
+  const int xchunks = X_IN_SMEM ? (chunks + 31) / 32 * 32 : 0;
+  uint8_t* ring = reinterpret_cast<uint8_t*>(xs4 + xchunks * 4) + warp * (GEMV_DEPTH * GEMV_STAGE);
+  const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
   // Dependent launch: the weights are read before the previous kernel of the stream has
   // finished (the caller's scope promises nothing in it writes them); x and y wait for it.
   pdl_trigger();
-  bool waited = false;
-  bool x_ready = !X_IN_SMEM;
-  for (int64_t row0 = (int64_t)blockIdx.x * GEMV_WARPS; row0 < n; row0 += (int64_t)gridDim.x * GEMV_WARPS) {
-    const int64_t row = row0 + warp;
-    const bool row_ok = row < n;
-    const uint4* qr = reinterpret_cast<const uint4*>(q + (row_ok ? row : 0) * k);
-    const float* sr = s + (row_ok ? row : 0) * kb_per_row;
-    float acc = 0.f;
-    for (int c0 = 0; c0 < chunks; c0 += 256) {
-      uint4 w[8];
-      float sc[8];
+  const int64_t groups = (n + R - 1) / R, step = (int64_t)gridDim.x * warps;
+  int64_t lg = blockIdx.x + (int64_t)gridDim.x * warp;   // the load cursor
+  int lc = 0, lslot = 0;
+  // the next stage; a row past the end repeats the last one.  Always a commit group, so that the waits count right
+  auto load = [&]() {
+    if (lg < groups) {
+      const uint32_t at = ring_a + lslot * GEMV_STAGE;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        int c = c0 + lane + 32 * u;
-        if (row_ok && c < chunks) {
-          w[u] = ldg_nc_v4(qr + c);
-          sc[u] = __ldg(sr + (c >> 1));
-        } else {
-          w[u] = make_uint4(0x0, 0x0, 0x0, 0x0);
-          sc[u] = 0.f;
+      for (int r = 0; r < R; ++r) {
+        const int64_t row = min(lg * R + r, n - 1);
+        const int8_t* qr = q + row * k;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = lc + 32 * u + lane;
+          if (c < chunks) cp_async16(at + (r * U + u) * 512 + lane * 16, qr + (int64_t)c * 16);
         }
       }
-      if (!waited) {
-        pdl_wait();
-        waited = true;
-      }
-      if (!x_ready) {
-        const float4* xg = reinterpret_cast<const float4*>(x);
-        for (int i = tid; i < chunks * 4; i += GEMV_WARPS * 32) {
-          int c = i >> 2, j = i & 3;
-          xs4[xs4_index(c, j)] = __ldcg(xg + i);
-        }
-        __syncthreads();
-        x_ready = true;
-      }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        int c = c0 + lane + 32 * u;
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h, r = i / (16 * U), blk = (lc >> 1) + i % (16 * U);
+        if (blk < kb) cp_async4(at + 2048 + i * 4, s + min(lg * R + r, n - 1) * kb + blk);
+      }
+      lc += 32 * U;
+      if (lc >= chunks) {
+        lc = 0;
+        lg += step;
+      }
+      lslot = lslot + 1 == GEMV_DEPTH ? 0 : lslot + 1;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < GEMV_DEPTH - 1; ++i) load();
+  pdl_wait();
+  if (X_IN_SMEM) {
+    const float4* xg = reinterpret_cast<const float4*>(x);
+    for (int i = tid; i < chunks * 4; i += blockDim.x) xs4[xs4_index(i >> 2, i & 3)] = __ldcg(xg + i);
+    __syncthreads();
+  }
+  int slot = 0;
+  for (int64_t g = blockIdx.x + (int64_t)gridDim.x * warp; g < groups; g += step) {
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int c0 = 0; c0 < chunks; c0 += 32 * U) {
+      __syncwarp();   // every lane is done with the stage that the next load overwrites
+      load();
+      asm volatile("cp.async.wait_group %0;" ::"n"(GEMV_DEPTH - 1) : "memory");
+      __syncwarp();
+      const uint8_t* st = ring + slot * GEMV_STAGE;
+      slot = slot + 1 == GEMV_DEPTH ? 0 : slot + 1;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c = c0 + 32 * u + lane;
         if (c < chunks) {
-          float4 x0, x1, x2, x3;
-          if (X_IN_SMEM) {
-            x0 = xs4[xs4_index(c, 0)]; x1 = xs4[xs4_index(c, 1)];
-            x2 = xs4[xs4_index(c, 2)]; x3 = xs4[xs4_index(c, 3)];
-          } else {
-            const float4* xg = reinterpret_cast<const float4*>(x) + c * 4;
-            x0 = __ldcg(xg); x1 = __ldcg(xg + 1); x2 = __ldcg(xg + 2); x3 = __ldcg(xg + 3);
+          uint4 w[R];
+          float p[R];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            w[r] = *reinterpret_cast<const uint4*>(st + (r * U + u) * 512 + lane * 16);
+            p[r] = 0.f;
           }
-          float p = 0.f;
-          p = dot4(w[u].x, x0, p);
-          p = dot4(w[u].y, x1, p);
-          p = dot4(w[u].z, x2, p);
-          p = dot4(w[u].w, x3, p);
-          acc = fmaf(sc[u], p, acc);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 xv = X_IN_SMEM ? xs4[xs4_index(c, j)] : __ldcg(reinterpret_cast<const float4*>(x) + (int64_t)c * 4 + j);
+#pragma unroll
+            for (int r = 0; r < R; ++r) p[r] = dot4(j == 0 ? w[r].x : j == 1 ? w[r].y : j == 2 ? w[r].z : w[r].w, xv, p[r]);
+          }
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const float sc = *reinterpret_cast<const float*>(st + 2048 + (r * 16 * U + 16 * u + (lane >> 1)) * 4);
+            acc[r] = fmaf(sc, p[r], acc[r]);
+          }
         }
       }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0 && row_ok) y[row] = acc;
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+      if (lane == 0 && g * R + r < n) y[g * R + r] = acc[r];
+    }
   }
 }
 
@@ -138,18 +167,20 @@ logos_status_t launch_q8_gemv(const int8_t* q, const float* s, const float* x, f
     LOGOS_CUDA_TRY(cudaMemsetAsync(y, 0, sizeof(float) * n, st));
     return LOGOS_OK;
   }
-  int64_t ctas = (n + GEMV_WARPS - 1) / GEMV_WARPS;
-  int64_t cap = (int64_t)sm_count(device) * 8;
-  int grid = (int)(ctas < cap ? ctas : cap);
-  // x padded to whole groups of 32 chunks (512 floats)
-  size_t smem = (size_t)((k / 16 + 31) / 32) * 128 * sizeof(float4);
-  if (smem <= 96 * 1024) {
-    if (smem > 48 * 1024)
-      LOGOS_CUDA_TRY(cudaFuncSetAttribute(q8_gemv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    LOGOS_CUDA_TRY(launch_kernel(q8_gemv_kernel<true>, dim3((unsigned)grid), dim3(GEMV_WARPS * 32), smem, st, q, s, x, y, n, k));
-  } else {
-    LOGOS_CUDA_TRY(launch_kernel(q8_gemv_kernel<false>, dim3((unsigned)grid), dim3(GEMV_WARPS * 32), 0, st, q, s, x, y, n, k));
-  }
+  // two rows a warp unless that would leave more than half of the warps without any; the larger CTA where x fits
+  // beside its rings (K up to 16384), past K = 29696 x stays in global memory
+  const int64_t sms = sm_count(device);
+  const int rows = n <= sms * GEMV_WARPS ? 1 : 2;
+  const int64_t groups = (n + rows - 1) / rows;
+  const int64_t xb = (k / 16 + 31) / 32 * 128 * (int64_t)sizeof(float4);
+  auto ring = [](int warps) { return (int64_t)warps * GEMV_DEPTH * GEMV_STAGE; };
+  const int warps = ring(GEMV_WARPS) + xb <= GEMV_SMEM ? GEMV_WARPS : GEMV_FEW_WARPS;
+  const bool in_smem = ring(warps) + xb <= GEMV_SMEM;
+  auto kern = rows == 2 ? (in_smem ? q8_gemv_kernel<2, true> : q8_gemv_kernel<2, false>)
+                        : (in_smem ? q8_gemv_kernel<1, true> : q8_gemv_kernel<1, false>);
+  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kern), device, GEMV_SMEM));
+  LOGOS_CUDA_TRY(launch_kernel(kern, dim3((unsigned)std::min(groups, sms)), dim3(warps * 32), (size_t)(ring(warps) + (in_smem ? xb : 0)),
+                               st, q, s, x, y, n, k));
   count_launch(LK_GEMV);
   return check_launch("q8_gemv_kernel");
 }

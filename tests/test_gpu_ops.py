@@ -186,6 +186,24 @@ def test_q8_gemm_config1_full_size(llm, oracle):
     assert (np.abs(c).max(axis=0) > 0).all() and (np.abs(c).max(axis=1) > 0).all()
 
 
+@pytest.mark.parametrize("n,k", [
+    (1, 32), (5, 544), (149, 2080),       # less than a stage; columns and rows that end inside one
+    (3552, 128), (3553, 96), (7109, 544),  # one row a warp up to 24 warps on each of 148 SMs, then two
+    (300, 16384), (301, 16416),           # x beside the larger CTA's rings, and the smaller one's
+    (9, 29696), (9, 29728),               # x in shared memory, and in global
+])
+def test_q8_gemv_edges(llm, oracle, n, k):
+    O = oracle
+    q = O.synth_fill(O.I8, 0, 5, 1, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 5, 2, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    x = O.synth_fill(O.F32, 2, 5, 3, 0, k, 0.0, 1.0)
+    y = llm.q8GemvHost(q, s, x)
+    w = q.astype(np.float64) * np.repeat(s.astype(np.float64), 32, axis=1)
+    # f32 sums of k terms in any order: k roundings of at most 2^-24 of the sum of magnitudes
+    bound = k * 2.0 ** -24 * (np.abs(w) @ np.abs(x.astype(np.float64)))
+    assert (np.abs(y - w @ x.astype(np.float64)) <= bound).all()
+
+
 def _attn_inputs(O, b, hq, hkv, d, lmax, lens, seed=0):
     kc = O.synth_fill(O.F16, 2, seed, 20, 0, b * hkv * lmax * d, 0.0, 1.0).reshape(b, hkv, lmax, d)
     vc = O.synth_fill(O.F16, 2, seed, 21, 0, b * hkv * lmax * d, 0.0, 1.0).reshape(b, hkv, lmax, d)
