@@ -111,6 +111,22 @@ def test_synth_kv_matches_oracle_and_decodes(llm, oracle):
     ref.close()
 
 
+@pytest.mark.parametrize("vocab", [5, 37, 1001, 4096, 16389])   # fewer than a cluster's CTAs, ragged shares, ragged vectors
+def test_token_choice_of_any_vocabulary(llm, oracle, vocab):
+    """From the same logits the GPU chooses the oracle's token: greedy, sampled, and over the k largest."""
+    cfg = dict(SMALL, vocab=vocab)
+    gpu = llm.Llm(act_dtype=llm.F32, **cfg)
+    gpu.setTokens(np.arange(cfg["batch"], dtype=np.int32) % vocab)
+    settings = [(0.0, 0)] + [(1.5, k) for k in (0, 1, 3, vocab - 1, vocab)]
+    for step, (temperature, top_k) in enumerate(settings):
+        gpu.setSampling(temperature, 11, top_k=top_k)
+        got = gpu.decodeStep()
+        want = oracle.sample_rows(gpu.readLogits(), temperature, 11, np.full(cfg["batch"], step), top_k=top_k)
+        assert np.array_equal(got, want), (temperature, top_k)
+    assert llm.kernelStatus() == 0
+    gpu.free()
+
+
 def test_temperature_sampling_tokens_match_the_oracle(llm, oracle):
     """Gumbel-max on the seeded generator: the draw is a pure function of (seed, sequence,
     position), so the GPU (eager first step, then the replayed graph) and the oracle pick the
