@@ -114,6 +114,27 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partials, int spl
   store_out(c, c_dtype, mm * ldc + nn, v, c_act);
 }
 
+// c = staged sums + residual, bf16; HBM-bound, eight elements a thread.
+__global__ void __launch_bounds__(256) residual_kernel(const float* __restrict__ sums, const __nv_bfloat16* aux, __nv_bfloat16* c, int64_t count) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
+  const bool vec = i + 8 <= count && !((reinterpret_cast<uintptr_t>(aux) | reinterpret_cast<uintptr_t>(c)) & 15u);
+  if (vec) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(sums + i)), b = __ldcg(reinterpret_cast<const float4*>(sums + i) + 1);
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const uint4 r = *reinterpret_cast<const uint4*>(aux + i);
+    const __nv_bfloat16* rh = reinterpret_cast<const __nv_bfloat16*>(&r);
+    uint4 o;
+    __nv_bfloat16* oh = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) oh[j] = __float2bfloat16_rn(__fadd_rn(v[j], __bfloat162float(rh[j])));
+    *reinterpret_cast<uint4*>(c + i) = o;
+  } else {
+    for (int64_t j = i; j < count && j < i + 8; ++j) c[j] = __float2bfloat16_rn(__fadd_rn(__ldcg(sums + j), __bfloat162float(aux[j])));
+  }
+}
+
 }  // namespace
 
 // K splits: a unit's time is a fixed part (pipeline fill, epilogue: about twelve stage times, measured) plus its K
@@ -186,7 +207,11 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   const int64_t lda = stages * 128;
   const int64_t plane_bytes = up(g.m * lda * 2);
   const int64_t scale_bytes = retile ? up((g.n + 127) / 128 * stages * 2048) : 0;
-  const int64_t part_bytes = splits > 1 ? (int64_t)splits * g.m * g.n * (int64_t)sizeof(float) : 0;
+  // The product kernel loads a residual row after row, which an SM with several tiles to do waits for every time: from
+  // the second token tile on the sums are staged in f32 and a kernel of its own adds the residual (2048 x 37888 x 3584:
+  // 1365 -> 1075 us, the same bits).  Beyond 512 MB of sums the library's scratch is not worth it.
+  const bool staged = g.epilogue == EPI_RESIDUAL && splits <= 1 && g.m > 96 && g.m * g.n <= (128ll << 20);
+  const int64_t part_bytes = staged ? g.m * g.n * (int64_t)sizeof(float) : splits > 1 ? (int64_t)splits * g.m * g.n * (int64_t)sizeof(float) : 0;
   void* scratch = nullptr;
   LOGOS_TRY(scratch_get(g.device, 0, (two_planes ? 2 : 1) * plane_bytes + scale_bytes + part_bytes, &scratch));
   char* at = static_cast<char*>(scratch);
@@ -207,8 +232,20 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     g.s_tiled = 1;
   }
   PdlScope pdl(true);
-  if (splits <= 1) return launch_q8_gemm(g, st);
+  if (splits <= 1 && !staged) return launch_q8_gemm(g, st);
   GemmArgs gp = g;
+  if (staged) {
+    gp.c = at;
+    gp.c_dtype = LOGOS_F32;
+    gp.epilogue = EPI_NONE;
+    gp.aux = nullptr;
+    LOGOS_TRY(launch_q8_gemm(gp, st));
+    LOGOS_CUDA_TRY(launch_kernel(residual_kernel, dim3((unsigned)((g.m * g.n + 2047) / 2048)), dim3(256), 0, st,
+                                 reinterpret_cast<const float*>(at), reinterpret_cast<const __nv_bfloat16*>(g.aux),
+                                 reinterpret_cast<__nv_bfloat16*>(g.c), g.m * g.n));
+    count_launch(LK_ELEMWISE);
+    return check_launch("residual_kernel");
+  }
   gp.splits = splits;
   gp.partials = reinterpret_cast<float*>(at);
   gp.epilogue = EPI_NONE;

@@ -204,6 +204,20 @@ def test_q8_gemv_edges(llm, oracle, n, k):
     assert (np.abs(y - w @ x.astype(np.float64)) <= bound).all()
 
 
+@pytest.mark.parametrize("m,n,k", [(96, 19000, 256), (97, 19001, 256), (193, 19004, 160), (100, 200, 128)])
+def test_q8_gemm_residual_of_several_token_tiles(llm, oracle, m, n, k):
+    """Past one token tile the residual is added by a kernel of its own: ends of its vectors, and of the rule."""
+    O = oracle
+    a, q, s = _gemm_inputs(O, m, n, k, seed=6)
+    aux = O.f32_to_bf16(O.synth_fill(O.F32, 2, 6, 13, 0, m * n, 0.0, 1.0).reshape(m, n))
+    c = llm.q8GemmHost(a, q, s, epilogue=1, aux=aux)
+    ref = O.q8_gemm(a, q, s, 1, aux)
+    assert llm.kernelStatus() == 0
+    # f32 sums of k terms in another order, then one rounding to bf16: last-place differences of few elements
+    assert np.mean(c != ref) < 0.01
+    assert rel_l2(O.bf16_to_f32(c), O.bf16_to_f32(ref)) < 1e-3
+
+
 def _attn_inputs(O, b, hq, hkv, d, lmax, lens, seed=0):
     kc = O.synth_fill(O.F16, 2, seed, 20, 0, b * hkv * lmax * d, 0.0, 1.0).reshape(b, hkv, lmax, d)
     vc = O.synth_fill(O.F16, 2, seed, 21, 0, b * hkv * lmax * d, 0.0, 1.0).reshape(b, hkv, lmax, d)
