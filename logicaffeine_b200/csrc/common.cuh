@@ -96,7 +96,7 @@ void counters_unregister(void* ptr);
 logos_status_t counters_reset(int32_t device);
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize of `kernel` on the current device, raised to `bytes` once instead of
-// on every launch.
+// on every launch; never lowered, whichever threads call.
 logos_status_t allow_smem(const void* kernel, int device, int bytes);
 
 int sm_count(int device);

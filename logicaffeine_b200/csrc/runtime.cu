@@ -196,20 +196,24 @@ logos_status_t counters_reset(int32_t device) {
 }
 
 logos_status_t allow_smem(const void* kernel, int device, int bytes) {
-  struct Seen {
+  // One limit per kernel and device for every thread of the process, so only a larger request may set it: kept per
+  // thread, a thread's first small call lowered what another thread's launches rely on.
+  struct Allowed {
     const void* kernel;
     int device, bytes;
   };
-  thread_local std::vector<Seen> seen;   // a few kernels: a scan is cheaper than any lock
-  for (Seen& s : seen)
-    if (s.kernel == kernel && s.device == device) {
-      if (s.bytes >= bytes) return LOGOS_OK;
+  static std::mutex mu;
+  static std::vector<Allowed> allowed;   // a few kernels: a scan is enough
+  std::lock_guard<std::mutex> lk(mu);
+  for (Allowed& a : allowed)
+    if (a.kernel == kernel && a.device == device) {
+      if (a.bytes >= bytes) return LOGOS_OK;
       LOGOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      s.bytes = bytes;
+      a.bytes = bytes;
       return LOGOS_OK;
     }
   LOGOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  seen.push_back({kernel, device, bytes});
+  allowed.push_back({kernel, device, bytes});
   return LOGOS_OK;
 }
 

@@ -2,6 +2,8 @@
 oracle on the same seeded inputs.  Integer, index and KV-cache results are
 compared bit for bit; f32-accumulated results within a relative L2 error of
 1e-3 (the stated tolerance; observed values are around 1e-6)."""
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -311,6 +313,32 @@ def test_gqa_decode_attn_cut_pairs_fold_the_same_every_time(llm, oracle, b, hq, 
     for _ in range(20):
         llm.gqaDecodeAttn(dq, dkc, dvc, dseq, do, b, hq, hkv, d, lmax, scale)
     assert np.array_equal(do.download(np.uint16, (b, hq, d)), first)
+
+
+def test_gqa_decode_attn_batches_of_several_threads(llm, oracle):
+    """Each thread's calls go on working whatever batch sizes the other threads have: the kernel's shared-memory limit,
+    which grows with the batch, belongs to the process."""
+    O = oracle
+    hq, hkv, d, lmax = 4, 2, 64, 70
+    scale = 1.0 / np.sqrt(d)
+    wants, gots = {}, []
+    for b in (64, 1):
+        q, _, _, kc, vc, seq = _attn_inputs(O, b, hq, hkv, d, lmax, [(17 * i) % 70 for i in range(1, b + 1)], seed=9)
+        wants[b] = (q, kc, vc, seq, O.f16_to_f32(O.gqa_decode_attn(q, kc, vc, seq, scale)))
+
+    def call(b):
+        q, kc, vc, seq, _ = wants[b]
+        do = llm.DeviceBuffer(b * hq * d * 2)
+        llm.gqaDecodeAttn(*(_dev(llm, x) for x in (q, kc, vc, seq)), do, b, hq, hkv, d, lmax, scale)
+        gots.append((b, O.f16_to_f32(do.download(np.uint16, (b, hq, d)))))
+
+    with ThreadPoolExecutor(1) as one, ThreadPoolExecutor(1) as other:
+        one.submit(call, 64).result()
+        other.submit(call, 1).result()
+        one.submit(call, 64).result()
+    assert [b for b, _ in gots] == [64, 1, 64]
+    for b, o in gots:
+        assert rel_l2(o, wants[b][-1]) < 1e-3   # both sides round to fp16
 
 
 def test_gqa_decode_attn_config2_full_size(llm, oracle):
