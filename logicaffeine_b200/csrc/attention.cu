@@ -23,9 +23,9 @@
 //   * a pair that lies inside one share is normalised and written by that CTA; the parts of a pair
 //     that was cut are merged, in the fixed order of their shares, by the CTA that finishes the
 //     last of them (a kernel of its own for this cost a launch and a start-up);
-//   * a small batch is bound by the chain from the predecessor's end to the output: what is older
-//     than the step (lengths, cached rows) is read, and the work cut, before the wait for the
-//     predecessor; every row of the query and the new K/V is one round of loads; the fold is three.
+//   * a small batch is bound by the chain from the predecessor's end to the output: in a decode step
+//     what is older than it (lengths, cached rows) is read, and the work cut, before the wait for
+//     the predecessor (AttnArgs::early_reads); every row of the query and the new K/V is one round of loads; the fold is three.
 // Measured, before -> after these two: 32 sequences of 4096, 28/4 heads of 128: 69.3 -> 62.2 us
 // (6.4 TB/s); seven ragged sequences 18.4 -> 14.3 us; a decode step of the 0.5B shape at batch 16
 // 954 -> 887 us (24 layers).
@@ -79,6 +79,7 @@ struct AttnParams {
   // (the counters wrap by themselves).
   unsigned*     arrive;
   int           bump;     // the last CTA to finish advances the lengths
+  int           early_reads;   // see AttnArgs
   void*         o;        // [B][Hq][D]
   int           o_dtype;
   ActOut        o_act;
@@ -272,8 +273,10 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int G = p.h_q / p.h_kv;
   auto tiles_of = [&](int b) { return (attn_len_eff(p, s_len[b]) + ATT_TILE - 1) / ATT_TILE; };
 
-  // The lengths and the cached rows are older than the step, so reading them, cutting the work and loading the first
-  // tiles overlap the predecessor's end; only what reads the query and the new K/V rows waits.
+  // In a decode step the lengths and the cached rows are older than the step, so reading them, cutting the work and
+  // loading the first tiles overlap the predecessor's end, and only what reads the query and the new K/V rows waits.
+  // Elsewhere the predecessor may write any of them: everything waits.
+  if (!p.early_reads) pdl_wait();
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
   // (one thread reads, everyone takes the same decision)
   __shared__ int prior_status;
@@ -801,6 +804,7 @@ logos_status_t launch_attn_t(const AttnArgs& a, cudaStream_t st) {
   p.part_ml = p.part_o + (int64_t)shares * 2 * 16 * D;
   p.arrive = reinterpret_cast<unsigned*>(arrive);
   p.bump = a.bump_seq_len;
+  p.early_reads = a.early_reads;
   p.o = a.o; p.o_dtype = a.o_dtype; p.o_act = a.o_act;
   p.b = (int)a.b; p.h_q = (int)a.h_q; p.h_kv = (int)a.h_kv; p.l_max = (int)a.l_max;
   p.shares = shares;

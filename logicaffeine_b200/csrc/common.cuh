@@ -124,7 +124,8 @@ static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStre
 // work that depends on nothing (barrier set-up, tensor-memory allocation, fetching WEIGHTS, which
 // nothing in a decode step writes) and then block in pdl_wait() until the previous kernel has
 // completed and its writes are visible.  The contract every kernel of the step keeps:
-//   * no read or write of anything another kernel of the step writes before pdl_wait();
+//   * before pdl_wait() no write, and no read of anything that a kernel still running can write: weights only, and
+//     in a decode step the lengths and cached rows, whose writers are over by then (AttnArgs::early_reads);
 //   * at least the threads that do such accesses call pdl_wait(), and every path through the
 //     kernel has some thread calling it (so "this kernel completed" implies "its predecessor did");
 //   * pdl_trigger() after the point where a successor's CTAs may take up SM resources.

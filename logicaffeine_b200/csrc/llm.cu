@@ -544,8 +544,11 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
   const int64_t B = c.batch, H = c.hidden, D = c.head_dim;
   cudaStream_t st = m->stream;
   m->launch_counter = 0;
-  // Every kernel of a step keeps the dependent-launch contract (common.cuh): weights are the
-  // only thing a kernel touches before it has waited for its predecessor.
+  // Every kernel of a step keeps the dependent-launch contract (common.cuh): before it has waited for its
+  // predecessor a kernel touches weights only, and the attention the lengths and cached rows too.  What writes those
+  // (the end of the step before, or this step's attention of another layer, another cache) is over when
+  // the attention starts: the norm before the qkv product waits for its predecessor before it lets
+  // anything start, and the predecessor (embedding or down product) is later than they are.
   PdlScope pdl(pdl_enabled());
   {
     ProfScope ps(m, PROF_ELEMWISE);
@@ -580,6 +583,7 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
       }
       a.k_cache = L.kc; a.v_cache = L.vc; a.rope = m->rope; a.seq_len = m->seq_len;
       a.bump_seq_len = 0;
+      a.early_reads = true;
       a.o_dtype = LOGOS_ACT_PLANES; a.o_act = m->att;
       a.b = B; a.h_q = m->hq_local; a.h_kv = m->hkv_local; a.d = D; a.l_max = c.l_max;
       a.scale = 1.0f / sqrtf((float)D);

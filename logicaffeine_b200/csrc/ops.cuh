@@ -114,6 +114,10 @@ struct AttnArgs {
   void*         ext_arrive = nullptr;      // with ext_scratch: b * h_kv + 1 counters, zero before the first call
   int64_t       ext_arrive_bytes = 0;
   int*          ext_status = nullptr;
+  // Lengths and cached rows may be read before the previous kernel of the stream has completed.  Only for a caller
+  // that knows every kernel which writes them to be over by then, as a decode step does; in a scope of the
+  // library's user they can be what that very kernel writes.
+  bool          early_reads = false;
 };
 logos_status_t launch_gqa_decode_attn(const AttnArgs& a, cudaStream_t st);
 // Bytes of split-KV scratch a call with these extents (b, h_q, h_kv, d, l_max, device) needs:

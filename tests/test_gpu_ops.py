@@ -443,3 +443,47 @@ def test_gemv_chain_in_a_dependent_launch_scope(llm, oracle):
         assert np.array_equal(y_.download(np.float32, (n,)), w)
     for b in [dq, ds] + dx + dy:
         b.free()
+
+
+def _sequences_in_a_scope(llm, O, scoped):
+    """Attention calls whose inputs the calls before them write, on one stream: what is left of each sequence."""
+    b, hq, hkv, d, lmax, n, k = 6, 14, 2, 64, 700, 512, 4096
+    lens = [0, 63, 64, 400, 690, 127]
+    q, kn, vn, kc, vc, seq = _attn_inputs(O, b, hq, hkv, d, lmax, lens, seed=12)
+    tab = O.rope_table(lmax, d, 1e6)
+    scale = 1.0 / np.sqrt(d)
+    dw = [_dev(llm, x) for x in (O.synth_fill(O.I8, 0, 5, 31, 0, n * k), O.synth_fill(O.F32, 1, 5, 32, 0, n * (k // 32), 1e-3, 1e-2),
+                                 O.synth_fill(O.F32, 2, 5, 33, 0, k, 0.0, 1.0))]
+    dy = llm.DeviceBuffer(n * 4)
+    left = []
+    for between in ("nothing", "gemv", "append"):
+        dq, dkn, dvn, dkc, dvc, dtab, dseq = (_dev(llm, x) for x in (q, kn, vn, kc, vc, tab, seq))
+        outs = [llm.DeviceBuffer(b * hq * d * 2) for _ in range(8)]
+        llm.devSync()
+        prev = llm.dependentLaunchScope(scoped)
+        try:
+            for do in outs:
+                if between == "append":
+                    llm.kvAppendRope(dkc, dvc, dkn, dvn, dtab, dseq, b, hkv, d, lmax)
+                    llm.gqaDecodeAttn(dq, dkc, dvc, dseq, do, b, hq, hkv, d, lmax, scale)
+                    continue
+                llm.gqaDecodeAttnFused(dq, dkn, dvn, dkc, dvc, dtab, dseq, do, b, hq, hkv, d, lmax, scale)
+                if between == "gemv":
+                    llm.q8Gemv(*dw, dy, n, k)
+        finally:
+            llm.dependentLaunchScope(prev)
+        llm.devSync()
+        left.append([do.download(np.uint16, (b, hq, d)) for do in outs] + [dkc.download(np.uint16, kc.shape),
+                    dvc.download(np.uint16, vc.shape), dseq.download(np.int32, (b,))])
+    assert llm.kernelStatus() == 0
+    return left
+
+
+def test_attention_in_a_dependent_launch_scope(llm, oracle):
+    """A scope only promises that nothing writes weights: lengths and cache rows that the call before an attention call
+    wrote, or one two calls before it behind a kernel that lets its successor start early, are waited for."""
+    plain = _sequences_in_a_scope(llm, oracle, False)
+    for _ in range(3):
+        for got, want in zip(_sequences_in_a_scope(llm, oracle, True), plain):
+            for g, w in zip(got, want):
+                assert np.array_equal(g, w)
