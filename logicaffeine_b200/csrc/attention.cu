@@ -280,7 +280,8 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
   // (one thread reads, everyone takes the same decision)
   __shared__ int prior_status;
-  __shared__ int s_last;
+  __shared__ int s_bump;   // this CTA is the last to have its lengths
+  __shared__ int s_last;   // this CTA wrote a pair's last part (the consumers' own: the producer may still look at s_bump)
   __shared__ MergeScratch s_merge;
   if (tid == 0) {
     prior_status = *reinterpret_cast<volatile int*>(p.status);
@@ -335,9 +336,9 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         for (int e = tid; e < p.h_q * D; e += ATT_CTHREADS) store_out(p, (int64_t)b * p.h_q * D + e, 0.f);
   // everyone has its lengths by now: the last CTA to come by advances them
   if (p.bump) {
-    if (tid == 0) s_last = arrive_inc(p.arrive + p.b * p.h_kv, gridDim.x - 1) == gridDim.x - 1;
+    if (tid == 0) s_bump = arrive_inc(p.arrive + p.b * p.h_kv, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();
-    if (s_last)
+    if (s_bump)
       for (int b = tid; b < p.b; b += ATT_THREADS) {
         const int len = __ldcg(p.seq_len + b);
         if (len < p.l_max) p.seq_len[b] = len + 1;
