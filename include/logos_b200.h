@@ -237,8 +237,8 @@ LOGOS_API logos_status_t logos_gqa_decode_attn(logos_handle_t q, logos_handle_t 
  * instead of library-allocated scratch, so every GPU that loads the library holds those 6 MiB
  * until the process exits.  What the kernel needs depends on the GPU, not on the shape: two
  * slots of 16 * (d + 2) floats per CTA, two CTAs per SM (4.7 MiB on a
- * 148-SM B200 at d = 128), and a counter per (sequence, KV head) pair in the last MiB;
- * a GPU with so many SMs, or a call with so many pairs, that this exceeds the array is refused with LOGOS_OUT_OF_BOUNDS and
+ * 148-SM B200 at d = 128), and 4 KiB of counters;
+ * a GPU with so many SMs that this exceeds the array is refused with LOGOS_OUT_OF_BOUNDS and
  * a message giving both sizes, and so is a call with more than 2048 sequences (the limit of
  * both attention entry points: a CTA keeps the lengths in shared memory).
  * The call itself makes no

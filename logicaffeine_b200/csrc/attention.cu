@@ -35,6 +35,7 @@
 
 #include <math.h>
 
+#include <algorithm>
 #include <mutex>
 
 namespace logos {
@@ -75,8 +76,8 @@ struct AttnParams {
   // at most two: slot 0 for a part that begins at the share's first tile, slot 1 otherwise.
   float*        part_o;   // [shares][2][16][D]   unnormalised outputs
   float*        part_ml;  // [shares][2][16][2]   their (max, sum)
-  // Arrivals: [B * Hkv] parts written of each pair, then CTAs that are done.  Zero before and after every launch
-  // (the counters wrap by themselves).
+  // Arrivals: [shares] parts written of the pair that the end of a share cuts (one pair at most, whatever their
+  // number), then CTAs that are done.  Zero before and after every launch (the counters wrap by themselves).
   unsigned*     arrive;
   int           bump;     // the last CTA to finish advances the lengths
   int           early_reads;   // see AttnArgs
@@ -336,7 +337,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         for (int e = tid; e < p.h_q * D; e += ATT_CTHREADS) store_out(p, (int64_t)b * p.h_q * D + e, 0.f);
   // everyone has its lengths by now: the last CTA to come by advances them
   if (p.bump) {
-    if (tid == 0) s_bump = arrive_inc(p.arrive + p.b * p.h_kv, gridDim.x - 1) == gridDim.x - 1;
+    if (tid == 0) s_bump = arrive_inc(p.arrive + p.shares, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();
     if (s_bump)
       for (int b = tid; b < p.b; b += ATT_THREADS) {
@@ -702,7 +703,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // with no more shares than tiles every share in between holds some; with more, each holds one at most
         const unsigned parts = p.shares <= total ? (unsigned)(share_last - share_first + 1) : (unsigned)tiles_b;
         // (the barrier above put all of this CTA's part before the releasing increment)
-        if (ctid == 0) s_last = arrive_inc(p.arrive + b * p.h_kv + kvh, parts - 1) == parts - 1;
+        if (ctid == 0) s_last = arrive_inc(p.arrive + share_first, parts - 1) == parts - 1;
         asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
         if (s_last) {
           merge_parts<D>(p, s_merge, b, kvh, share_first, share_last, share_begin(share_first, total, p.shares) == pair_g0 ? 0 : 1, total);
@@ -753,7 +754,7 @@ size_t attn_smem_bytes(int64_t batch) {
 int attn_shares(const AttnArgs& a) {
   const int sms = sm_count(a.device);
   const int64_t tiles_max = (a.l_max + ATT_TILE - 1) / ATT_TILE;
-  int64_t g = 2ll * sms;   // two CTAs of about 113 KB of shared memory fit an SM
+  int64_t g = std::min<int64_t>(2 * sms, ATT_COUNTER_BYTES / sizeof(unsigned) - 1);   // two CTAs of about 113 KB of shared memory fit an SM
   // With no more (sequence, KV head) pairs than CTAs, a whole number of shares per pair: where the
   // sequences are equally long every share boundary then falls on a pair boundary or cuts a pair
   // into equal pieces, and a CTA stages one pair's query instead of two (measured 4-8 % on the
@@ -777,19 +778,15 @@ logos_status_t launch_attn_t(const AttnArgs& a, cudaStream_t st) {
 
   // parts of cut pairs, then the arrival counters, which have to be zero when the first launch comes
   const int64_t part_bytes = (int64_t)shares * 2 * 16 * (D + 2) * (int64_t)sizeof(float);
-  const int64_t arrive_bytes = (a.b * a.h_kv + 1) * (int64_t)sizeof(unsigned);
   void* scratch = a.ext_scratch;
   void* arrive = a.ext_arrive;
   if (a.ext_scratch) {
     if (part_bytes > a.ext_scratch_bytes)
       return fail(LOGOS_OUT_OF_BOUNDS, "attention: this shape needs %lld bytes of split-KV scratch, the fixed scratch holds %lld",
                   (long long)part_bytes, (long long)a.ext_scratch_bytes);
-    if (arrive_bytes > a.ext_arrive_bytes)
-      return fail(LOGOS_OUT_OF_BOUNDS, "attention: this shape needs %lld bytes of arrival counters, the fixed scratch holds %lld",
-                  (long long)arrive_bytes, (long long)a.ext_arrive_bytes);
   } else {
     LOGOS_TRY(scratch_get(a.device, 1, part_bytes, &scratch));
-    LOGOS_TRY(counters_get(a.device, arrive_bytes, &arrive));
+    LOGOS_TRY(counters_get(a.device, ATT_COUNTER_BYTES, &arrive));
   }
 
   AttnParams p{};
@@ -863,9 +860,8 @@ logos_status_t launch_kv_append_rope(__half* k_cache, __half* v_cache, const __h
 // Scratch that lives in the library image instead of coming from cudaMalloc: every GPU
 // that loads the library holds these 6 MiB (+ one status word) until the process exits.
 // The kernel needs two part slots of 16 x (D + 2) floats per CTA of its persistent grid (two
-// CTAs per SM): 4.7 MiB on a 148-SM B200 at D = 128; the 5 MiB before the counters provide for 157 SMs.
-// The counters of 262143 (sequence, KV head) pairs take the last MiB.
-constexpr int64_t kStaticScratchBytes = 6ll << 20, kStaticArriveBytes = 1ll << 20;
+// CTAs per SM): 4.7 MiB on a 148-SM B200 at D = 128; what is left before the counters provides for 188 SMs.
+constexpr int64_t kStaticScratchBytes = 6ll << 20;
 static __device__ __align__(256) unsigned char g_static_attn_scratch[kStaticScratchBytes];
 static __device__ __align__(256) int g_static_attn_status[8];
 
@@ -918,7 +914,7 @@ logos_status_t static_attn_status_read(int device, int words_out[8], bool clear,
   LOGOS_CUDA_TRY(cudaMemcpy(words_out, sa.status, sizeof(int) * 8, cudaMemcpyDeviceToHost));
   if (clear && words_out[0] != 0) {
     // a kernel that gave up leaves arrivals uncounted
-    LOGOS_CUDA_TRY(cudaMemset(static_cast<char*>(sa.scratch) + kStaticScratchBytes - kStaticArriveBytes, 0, kStaticArriveBytes));
+    LOGOS_CUDA_TRY(cudaMemset(static_cast<char*>(sa.scratch) + kStaticScratchBytes - ATT_COUNTER_BYTES, 0, ATT_COUNTER_BYTES));
     LOGOS_CUDA_TRY(cudaMemset(sa.status, 0, sizeof(int) * 8));
   }
   *used = true;
@@ -958,9 +954,8 @@ logos_status_t logos_gqa_decode_attn_fixed_scratch(logos_handle_t q, logos_handl
     a.q_f16 = qp; a.k_cache = kc; a.v_cache = vc; a.seq_len = sl; a.o = op; a.o_dtype = LOGOS_F16;
     a.b = b; a.h_q = h_q; a.h_kv = h_kv; a.d = d; a.l_max = l_max; a.scale = softmax_scale; a.device = dev;
     a.ext_scratch = sa.scratch;
-    a.ext_scratch_bytes = kStaticScratchBytes - kStaticArriveBytes;
+    a.ext_scratch_bytes = kStaticScratchBytes - ATT_COUNTER_BYTES;
     a.ext_arrive = static_cast<char*>(sa.scratch) + a.ext_scratch_bytes;
-    a.ext_arrive_bytes = kStaticArriveBytes;
     a.ext_status = sa.status;
     return launch_gqa_decode_attn(a, st);
   });

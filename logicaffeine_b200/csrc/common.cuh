@@ -86,8 +86,8 @@ logos_status_t buf_ptr(logos_handle_t h, int64_t elems, const char* name, T** ou
 // captured decode step points at is owned by the model.
 logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out);
 
-// Arrival counters of the stand-alone attention calls, one block per device, zeroed when it is allocated; the kernels
-// leave them at zero.  Ordered like scratch_get's blocks.
+// Arrival counters of the stand-alone attention calls, one block per device (every call asks for the same size), zeroed
+// when it is allocated; the kernels leave them at zero.  Ordered like scratch_get's blocks.
 logos_status_t counters_get(int32_t device, int64_t bytes, void** out);
 // Counters that someone else owns (a model): a kernel that gave up leaves them in the middle of a count, so
 // counters_reset zeroes all of a device's once such a failure has been read.

@@ -85,7 +85,6 @@ struct Model {
   void*  attn_scratch = nullptr;  // split-KV partials of the attention kernel: owned here, so the captured step
   int64_t attn_scratch_bytes = 0; // never points at the library's shared scratch
   void*  attn_arrive = nullptr;   // its arrival counters
-  int64_t attn_arrive_bytes = 0;
   // tensor parallelism with peer-addressable memory: partials, xn planes and flag words live in
   // one block per rank that every rank maps; the all-reduce is folded into residual + RMSNorm
   TpSymm symm;
@@ -360,10 +359,9 @@ logos_status_t build(Model* m, const void* nccl_id) {
     a.b = B; a.h_q = m->hq_local; a.h_kv = m->hkv_local; a.d = D; a.l_max = c.l_max; a.device = m->device;
     m->attn_scratch_bytes = attn_scratch_bytes(a);
     LOGOS_TRY(dmalloc(m, &m->attn_scratch, m->attn_scratch_bytes));
-    m->attn_arrive_bytes = (B * m->hkv_local + 1) * (int64_t)sizeof(unsigned);
-    LOGOS_TRY(dmalloc(m, &m->attn_arrive, m->attn_arrive_bytes));
-    LOGOS_CUDA_TRY(cudaMemsetAsync(m->attn_arrive, 0, (size_t)m->attn_arrive_bytes, m->stream));
-    counters_register(m->device, m->attn_arrive, m->attn_arrive_bytes);
+    LOGOS_TRY(dmalloc(m, &m->attn_arrive, ATT_COUNTER_BYTES));
+    LOGOS_CUDA_TRY(cudaMemsetAsync(m->attn_arrive, 0, ATT_COUNTER_BYTES, m->stream));
+    counters_register(m->device, m->attn_arrive, ATT_COUNTER_BYTES);
   }
   LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->logits), B * c.vocab * 4));
   m->history_cap = c.l_max;
@@ -589,7 +587,7 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
       a.scale = 1.0f / sqrtf((float)D);
       a.device = m->device;
       a.ext_scratch = m->attn_scratch; a.ext_scratch_bytes = m->attn_scratch_bytes;
-      a.ext_arrive = m->attn_arrive; a.ext_arrive_bytes = m->attn_arrive_bytes;
+      a.ext_arrive = m->attn_arrive;
       LOGOS_TRY(launch_gqa_decode_attn(a, st));
       m->launch_counter += 1;
     }

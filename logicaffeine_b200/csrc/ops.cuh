@@ -71,6 +71,8 @@ int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device);
 bool gemm_tc_applicable(const GemmArgs& g);
 
 // ---- attention (attention.cu)
+// The attention kernel's arrival counters, whatever the call's extents: one per CTA of its persistent grid and one more
+constexpr int64_t ATT_COUNTER_BYTES = 4096;
 struct AttnArgs {
   // query: either f16 [B][Hq][D] (q_f16) or f32 rows inside a wider matrix
   // (q_f32, row stride q_ld floats per sequence, head h at column h*D).
@@ -111,8 +113,7 @@ struct AttnArgs {
   // point at memory another caller can outgrow).
   void*         ext_scratch = nullptr;
   int64_t       ext_scratch_bytes = 0;
-  void*         ext_arrive = nullptr;      // with ext_scratch: b * h_kv + 1 counters, zero before the first call
-  int64_t       ext_arrive_bytes = 0;
+  void*         ext_arrive = nullptr;      // with ext_scratch: ATT_COUNTER_BYTES of counters, zero before the first call
   int*          ext_status = nullptr;
   // Lengths and cached rows may be read before the previous kernel of the stream has completed.  Only for a caller
   // that knows every kernel which writes them to be over by then, as a decode step does; in a scope of the

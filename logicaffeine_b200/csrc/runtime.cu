@@ -147,7 +147,7 @@ struct Counters {
   int32_t device;
   void*   ptr;
   int64_t bytes;
-  bool    own;     // the library's block of the device (the latest one)
+  bool    own;     // the library's block of the device
 };
 std::mutex g_counters_mu;
 std::vector<Counters> g_counters;
@@ -155,24 +155,21 @@ std::vector<Counters> g_counters;
 
 logos_status_t counters_get(int32_t device, int64_t bytes, void** out) {
   std::lock_guard<std::mutex> lk(g_counters_mu);
-  int64_t have = 0;
   for (const Counters& c : g_counters)
-    if (c.own && c.device == device && c.bytes > have) {
-      have = c.bytes;
+    if (c.own && c.device == device) {
       *out = c.ptr;
+      return LOGOS_OK;
     }
-  if (have >= bytes) return LOGOS_OK;
-  const int64_t want = ((bytes > 2 * have ? bytes : 2 * have) + 4095) & ~int64_t(4095);
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, (size_t)want);   // an outgrown block stays: launches already enqueued may use it
+  cudaError_t e = cudaMalloc(&p, (size_t)bytes);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc (arrival counters)");
-  e = cudaMemset(p, 0, (size_t)want);
+  e = cudaMemset(p, 0, (size_t)bytes);
   if (e != cudaSuccess) {
     cudaFree(p);
     return cuda_fail(e, "cudaMemset (arrival counters)");
   }
-  LOGOS_CUDA_TRY(cudaDeviceSynchronize());        // zero before a launch on any stream (once per growth)
-  g_counters.push_back({device, p, want, true});
+  LOGOS_CUDA_TRY(cudaDeviceSynchronize());        // zero before a launch on any stream
+  g_counters.push_back({device, p, bytes, true});
   *out = p;
   return LOGOS_OK;
 }

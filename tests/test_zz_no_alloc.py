@@ -70,3 +70,18 @@ def test_fixed_scratch_refuses_what_does_not_fit(llm):
     assert e.value.status == 4 and "2048" in str(e.value)
     for x in (q, cache, seq):
         x.free()
+
+
+def test_fixed_scratch_takes_any_number_of_pairs(llm):
+    """What the kernel needs depends on the GPU alone: 2048 sequences of 128 KV heads, one position each, whose output is
+    that position's V row (the softmax of one score is 1)."""
+    b, h, d, lmax = 2048, 128, 64, 1
+    q, kc, vc, o = (llm.DeviceBuffer(b * h * d * 2) for _ in range(4))
+    for i, x in enumerate((q, kc, vc)):
+        llm.synthFill(x, llm.F16, 2, 7, i, 0, b * h * d, 0.0, 1.0)
+    seq = llm.DeviceBuffer.from_host(np.full(b, 1, np.int32))
+    llm.gqaDecodeAttnFixedScratch(q, kc, vc, seq, o, b, h, h, d, lmax, 0.125)
+    assert np.array_equal(o.download(np.uint16, (b, h, d)), vc.download(np.uint16, (b, h, d)))
+    assert llm.kernelStatus() == 0
+    for x in (q, kc, vc, o, seq):
+        x.free()
