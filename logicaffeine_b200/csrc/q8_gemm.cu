@@ -197,6 +197,8 @@ using namespace logos;
 // fold of the K splits.  The launches after the first are dependent ones: each kernel sets up, and the
 // product fetches its first weights, while the one before it finishes.  Nothing here writes weights, and the
 // first kernel is an ordinary launch, so what ran before in the stream has ended.
+constexpr int64_t STAGED_BYTES = 64ll << 20;   // sums staged at a time, see below: half of L2
+
 static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) {
   const void* src = g.a;
   const int src_dtype = g.a_dtype;
@@ -207,11 +209,13 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   const int64_t lda = stages * 128;
   const int64_t plane_bytes = up(g.m * lda * 2);
   const int64_t scale_bytes = retile ? up((g.n + 127) / 128 * stages * 2048) : 0;
-  // The product kernel loads a residual row after row, which an SM with several tiles to do waits for every time: from
-  // the second token tile on the sums are staged in f32 and a kernel of its own adds the residual (2048 x 37888 x 3584:
-  // 1365 -> 1075 us, the same bits).  Beyond 512 MB of sums the library's scratch is not worth it.
-  const bool staged = g.epilogue == EPI_RESIDUAL && splits <= 1 && g.m > 96 && g.m * g.n <= (128ll << 20);
-  const int64_t part_bytes = staged ? g.m * g.n * (int64_t)sizeof(float) : splits > 1 ? (int64_t)splits * g.m * g.n * (int64_t)sizeof(float) : 0;
+  // The product kernel loads a residual row after row, which an SM with several tiles to do waits for every time: with
+  // more tokens than its largest tile the sums are staged in f32 and a kernel of its own adds the residual, the same
+  // bits.  A few token tiles at a time, so that the scratch stays small and the sums in L2.
+  const int64_t stage_rows = STAGED_BYTES / (g.n * (int64_t)sizeof(float)) / 96 * 96;
+  const bool staged = g.epilogue == EPI_RESIDUAL && splits <= 1 && g.m > 96 && stage_rows > 0;
+  const int64_t part_rows = staged ? std::min(g.m, stage_rows) : splits > 1 ? splits * g.m : 0;
+  const int64_t part_bytes = part_rows * g.n * (int64_t)sizeof(float);
   void* scratch = nullptr;
   LOGOS_TRY(scratch_get(g.device, 0, (two_planes ? 2 : 1) * plane_bytes + scale_bytes + part_bytes, &scratch));
   char* at = static_cast<char*>(scratch);
@@ -235,16 +239,23 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   if (splits <= 1 && !staged) return launch_q8_gemm(g, st);
   GemmArgs gp = g;
   if (staged) {
-    gp.c = at;
     gp.c_dtype = LOGOS_F32;
     gp.epilogue = EPI_NONE;
     gp.aux = nullptr;
-    LOGOS_TRY(launch_q8_gemm(gp, st));
-    LOGOS_CUDA_TRY(launch_kernel(residual_kernel, dim3((unsigned)((g.m * g.n + 2047) / 2048)), dim3(256), 0, st,
-                                 reinterpret_cast<const float*>(at), reinterpret_cast<const __nv_bfloat16*>(g.aux),
-                                 reinterpret_cast<__nv_bfloat16*>(g.c), g.m * g.n));
-    count_launch(LK_ELEMWISE);
-    return check_launch("residual_kernel");
+    gp.c = at;
+    for (int64_t m0 = 0; m0 < g.m; m0 += stage_rows) {
+      gp.m = std::min(stage_rows, g.m - m0);
+      gp.a = planes.hi + m0 * lda;
+      gp.a_lo = two_planes ? planes.lo + m0 * lda : nullptr;
+      LOGOS_TRY(launch_q8_gemm(gp, st));
+      const int64_t count = gp.m * g.n;
+      LOGOS_CUDA_TRY(launch_kernel(residual_kernel, dim3((unsigned)((count + 2047) / 2048)), dim3(256), 0, st,
+                                   reinterpret_cast<const float*>(at), reinterpret_cast<const __nv_bfloat16*>(g.aux) + m0 * g.n,
+                                   reinterpret_cast<__nv_bfloat16*>(g.c) + m0 * g.n, count));
+      count_launch(LK_ELEMWISE);
+      LOGOS_TRY(check_launch("residual_kernel"));
+    }
+    return LOGOS_OK;
   }
   gp.splits = splits;
   gp.partials = reinterpret_cast<float*>(at);

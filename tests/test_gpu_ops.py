@@ -2,6 +2,10 @@
 oracle on the same seeded inputs.  Integer, index and KV-cache results are
 compared bit for bit; f32-accumulated results within a relative L2 error of
 1e-3 (the stated tolerance; observed values are around 1e-6)."""
+import os
+import subprocess
+import sys
+import textwrap
 from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
@@ -218,6 +222,40 @@ def test_q8_gemm_residual_of_several_token_tiles(llm, oracle, m, n, k):
     # f32 sums of k terms in another order, then one rounding to bf16: last-place differences of few elements
     assert np.mean(c != ref) < 0.01
     assert rel_l2(O.bf16_to_f32(c), O.bf16_to_f32(ref)) < 1e-3
+
+
+def _in_a_process_of_its_own(code):
+    """Runs `code` after the imports it needs in a fresh process, whose library scratch is empty."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    head = "import sys; sys.path[:0] = [%r, %r]\nimport numpy as np\nfrom logicaffeine_b200 import llm\n" % (here, os.path.dirname(here))
+    r = subprocess.run([sys.executable, "-c", head + textwrap.dedent(code)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+@pytest.mark.parametrize("m,n", [(2048, 37888), (4100, 33000)])   # 310 MB of sums, and more than 2^27 of them
+def test_q8_gemm_residual_keeps_little_scratch(llm, m, n):
+    _in_a_process_of_its_own("""
+        m, n, k = %d, %d, 128
+        q, s = llm.DeviceBuffer(n * k), llm.DeviceBuffer(n * (k // 32) * 4)
+        a, x, c, want = llm.DeviceBuffer(m * k * 2), llm.DeviceBuffer(m * n * 2), llm.DeviceBuffer(m * n * 2), llm.DeviceBuffer(m * n * 2)
+        llm.synthFill(q, llm.I8, 0, 3, 1, 0, n * k)
+        llm.synthFill(s, llm.F32, 1, 3, 2, 0, n * (k // 32), 1e-3, 1e-2)
+        llm.synthFill(a, llm.BF16, 2, 3, 3, 0, m * k)
+        llm.synthFill(x, llm.BF16, 2, 3, 4, 0, m * n)
+        llm.q8Gemm(a, q, s, c, 1, 128, k)     # loads the kernels
+        llm.q8GemmSimt(a, q, s, want, m, n, k, 1, x)
+        assert llm.kernelStatus() == 0
+        before, _ = llm.devMemInfo()
+        llm.q8Gemm(a, q, s, c, m, n, k, 1, x)
+        llm.devSync()
+        after, _ = llm.devMemInfo()
+        assert before - after <= 80 << 20, before - after    # 64 MB of sums, the activation plane, rounding
+        got, want = c.download(np.uint16, (m, n)), want.download(np.uint16, (m, n))
+        assert np.mean(got != want) < 0.01     # last places: f32 sums in another order, then one rounding to bf16
+        f = lambda b: (b.astype(np.uint32) << 16).view(np.float32)
+        assert np.abs(f(got) - f(want)).max() <= 2.0 ** -7 * np.abs(f(want)).max()
+        assert llm.kernelStatus() == 0
+    """ % (m, n))
 
 
 def _attn_inputs(O, b, hq, hkv, d, lmax, lens, seed=0):
