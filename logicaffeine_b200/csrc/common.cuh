@@ -85,6 +85,9 @@ logos_status_t buf_ptr(logos_handle_t h, int64_t elems, const char* name, T** ou
 // capture; outgrown blocks are kept until the process exits.  A model never uses it: what a
 // captured decode step points at is owned by the model.
 logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out);
+// The same for a caller that can do without: false, and no error, if the block would have to grow while `st` is being
+// captured, or there is no memory left for it.
+bool scratch_try(int32_t device, int slot, int64_t bytes, cudaStream_t st, void** out);
 
 // Arrival counters of the stand-alone attention calls, one block per device (every call asks for the same size), zeroed
 // when it is allocated; the kernels leave them at zero.  Ordered like scratch_get's blocks.

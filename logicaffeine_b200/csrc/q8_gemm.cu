@@ -213,11 +213,25 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   // more tokens than its largest tile the sums are staged in f32 and a kernel of its own adds the residual, the same
   // bits.  A few token tiles at a time, so that the scratch stays small and the sums in L2.
   const int64_t stage_rows = STAGED_BYTES / (g.n * (int64_t)sizeof(float)) / 96 * 96;
-  const bool staged = g.epilogue == EPI_RESIDUAL && splits <= 1 && g.m > 96 && stage_rows > 0;
+  bool staged = g.epilogue == EPI_RESIDUAL && splits <= 1 && g.m > 96 && stage_rows > 0;
   const int64_t part_rows = staged ? std::min(g.m, stage_rows) : splits > 1 ? splits * g.m : 0;
   const int64_t part_bytes = part_rows * g.n * (int64_t)sizeof(float);
+  const int64_t own_bytes = (two_planes ? 2 : 1) * plane_bytes + scale_bytes;
   void* scratch = nullptr;
-  LOGOS_TRY(scratch_get(g.device, 0, (two_planes ? 2 : 1) * plane_bytes + scale_bytes + part_bytes, &scratch));
+  if (retile || staged) {
+    // neither form is worth failing for: the CUDA-core kernel needs no scratch, and the residual can be added
+    // in the product
+    if (!scratch_try(g.device, 0, own_bytes + part_bytes, st, &scratch)) {
+      if (retile) {
+        g.force_simt = 1;
+        return launch_q8_gemm(g, st);
+      }
+      staged = false;
+      LOGOS_TRY(scratch_get(g.device, 0, own_bytes, &scratch));
+    }
+  } else {
+    LOGOS_TRY(scratch_get(g.device, 0, own_bytes + part_bytes, &scratch));
+  }
   char* at = static_cast<char*>(scratch);
   ActOut planes;
   planes.hi = reinterpret_cast<__half*>(at);

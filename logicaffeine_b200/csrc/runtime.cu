@@ -109,37 +109,64 @@ logos_status_t buf_resolve(logos_handle_t h, int64_t offset, int64_t need, const
   return LOGOS_OK;
 }
 
-logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out) {
-  std::lock_guard<std::mutex> lk(g_scratch_mu);
-  uint64_t key = (static_cast<uint64_t>(static_cast<uint32_t>(device)) << 8) | static_cast<uint64_t>(slot);
-  Scratch& s = g_scratch[key];
-  if (s.bytes < bytes) {
-    int prev = 0;
-    LOGOS_CUDA_TRY(cudaGetDevice(&prev));
-    LOGOS_CUDA_TRY(cudaSetDevice(device));
-    // An outgrown block is never freed: kernels already enqueued (on any stream) may still
-    // write to it.  Growing at least geometrically bounds what the retired blocks hold to the
-    // size of the live one.
-    int64_t want = bytes > 2 * s.bytes ? bytes : 2 * s.bytes;
-    want = (want + 255) & ~int64_t(255);
-    void* fresh = nullptr;
-    cudaError_t e = cudaMalloc(&fresh, want);
-    if (e != cudaSuccess && want > bytes) {  // no room for the doubled block: take what is needed
-      cudaGetLastError();
-      want = (bytes + 255) & ~int64_t(255);
-      e = cudaMalloc(&fresh, want);
-    }
-    if (e != cudaSuccess) {
-      cudaSetDevice(prev);
-      return cuda_fail(e, "cudaMalloc (library scratch)");
-    }
+namespace {
+// The block of a device's slot, grown if it is smaller than `bytes`; a failure is left for the caller to word.
+cudaError_t scratch_grow(int32_t device, Scratch& s, int64_t bytes) {
+  int prev = 0;
+  cudaError_t e = cudaGetDevice(&prev);
+  if (e == cudaSuccess) e = cudaSetDevice(device);
+  if (e != cudaSuccess) return e;
+  // An outgrown block is never freed: kernels already enqueued (on any stream) may still
+  // write to it.  Growing at least geometrically bounds what the retired blocks hold to the
+  // size of the live one.
+  int64_t want = bytes > 2 * s.bytes ? bytes : 2 * s.bytes;
+  want = (want + 255) & ~int64_t(255);
+  void* fresh = nullptr;
+  e = cudaMalloc(&fresh, want);
+  if (e != cudaSuccess && want > bytes) {  // no room for the doubled block: take what is needed
+    cudaGetLastError();
+    want = (bytes + 255) & ~int64_t(255);
+    e = cudaMalloc(&fresh, want);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // reported by the return value; the launches that follow check for errors of their own
+  } else {
     if (s.ptr) s.retired.push_back(s.ptr);
     s.ptr = fresh;
     s.bytes = want;
-    LOGOS_CUDA_TRY(cudaSetDevice(prev));
+  }
+  const cudaError_t back = cudaSetDevice(prev);
+  return e != cudaSuccess ? e : back;
+}
+Scratch& scratch_of(int32_t device, int slot) {   // under g_scratch_mu
+  return g_scratch[(static_cast<uint64_t>(static_cast<uint32_t>(device)) << 8) | static_cast<uint64_t>(slot)];
+}
+}  // namespace
+
+logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out) {
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  Scratch& s = scratch_of(device, slot);
+  if (s.bytes < bytes) {
+    const cudaError_t e = scratch_grow(device, s, bytes);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc (library scratch)");
   }
   *out = s.ptr;
   return LOGOS_OK;
+}
+
+bool scratch_try(int32_t device, int slot, int64_t bytes, cudaStream_t st, void** out) {
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  Scratch& s = scratch_of(device, slot);
+  if (s.bytes < bytes) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (capture != cudaStreamCaptureStatusNone || scratch_grow(device, s, bytes) != cudaSuccess) return false;
+  }
+  *out = s.ptr;
+  return true;
 }
 
 namespace {

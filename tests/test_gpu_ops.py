@@ -258,6 +258,57 @@ def test_q8_gemm_residual_keeps_little_scratch(llm, m, n):
     """ % (m, n))
 
 
+def test_q8_gemm_of_any_k_without_room_for_scratch(llm):
+    """K that is no multiple of 128 takes the tensor cores where the library has scratch for it, and goes on without: as
+    the first call inside a capture, and when the memory is spent.  So does a residual of many tokens."""
+    _in_a_process_of_its_own("""
+        import torch
+        def inputs(m, n, k):
+            a, q, s, c = (llm.DeviceBuffer(b) for b in (m * k * 4, n * k, n * (k // 32) * 4, m * n * 4))
+            llm.synthFill(a, llm.F32, 2, 3, 3, 0, m * k)
+            llm.synthFill(q, llm.I8, 0, 3, 1, 0, n * k)
+            llm.synthFill(s, llm.F32, 1, 3, 2, 0, n * (k // 32), 1e-3, 1e-2)
+            return a, q, s, c
+        def check(a, q, s, c, m, n, k):
+            w = q.download(np.int8, (n, k)).astype(np.float64) * np.repeat(s.download(np.float32, (n, k // 32)).astype(np.float64), 32, axis=1)
+            for r in {0, m // 2, m - 1}:
+                x = a.download(np.float32, (k,), r * k * 4).astype(np.float64)
+                y = c.download(np.float32, (n,), r * n * 4)
+                # f32 sums of k terms in any order: k roundings of at most 2^-24 of the sum of magnitudes
+                assert (np.abs(y - w @ x) <= k * 2.0 ** -24 * (np.abs(w) @ np.abs(x))).all()
+        m, n, k = 3, 40, 160
+        bufs = inputs(m, n, k)
+        warm = [llm.DeviceBuffer(x) for x in (32 * 2, 32, 4, 2)]
+        llm.q8GemmSimt(*warm, 1, 1, 32)
+        llm.devSync()
+        st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            llm.q8GemmF32(*bufs, m, n, k, stream=st.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        check(*bufs, m, n, k)
+        # with little memory left: 48 MB where 0.9 GB of planes are wanted, and 64 MB of staged sums
+        m, n, k = 4096, 64, 27616
+        bufs = inputs(m, n, k)
+        rm, rn, rk = 2048, 37888, 128
+        ra, rq, rs, rc, rx, want = (llm.DeviceBuffer(x) for x in (rm * rk * 2, rn * rk, rn * (rk // 32) * 4, rm * rn * 2, rm * rn * 2, rm * rn * 2))
+        llm.synthFill(rq, llm.I8, 0, 3, 1, 0, rn * rk)
+        llm.synthFill(rs, llm.F32, 1, 3, 2, 0, rn * (rk // 32), 1e-3, 1e-2)
+        llm.synthFill(ra, llm.BF16, 2, 3, 3, 0, rm * rk)
+        llm.synthFill(rx, llm.BF16, 2, 3, 4, 0, rm * rn)
+        llm.q8GemmSimt(ra, rq, rs, want, rm, rn, rk, 1, rx)
+        llm.q8Gemm(ra, rq, rs, rc, 97, 128, rk, 0)      # loads the kernel of large tiles and its plane
+        assert llm.kernelStatus() == 0
+        rest = llm.DeviceBuffer(llm.devMemInfo()[0] - (48 << 20))
+        llm.q8GemmF32(*bufs, m, n, k)
+        check(*bufs, m, n, k)
+        llm.q8Gemm(ra, rq, rs, rc, rm, rn, rk, 1, rx)
+        got, want = rc.download(np.uint16, (rm, rn)), want.download(np.uint16, (rm, rn))
+        assert np.mean(got != want) < 0.01     # last places: f32 sums in another order, then one rounding to bf16
+        assert llm.kernelStatus() == 0
+    """)
+
+
 def _attn_inputs(O, b, hq, hkv, d, lmax, lens, seed=0):
     kc = O.synth_fill(O.F16, 2, seed, 20, 0, b * hkv * lmax * d, 0.0, 1.0).reshape(b, hkv, lmax, d)
     vc = O.synth_fill(O.F16, 2, seed, 21, 0, b * hkv * lmax * d, 0.0, 1.0).reshape(b, hkv, lmax, d)
