@@ -304,7 +304,9 @@ LOGOS_API logos_status_t logos_llm_prefill(logos_handle_t model, const int32_t* 
  * current token is the one chosen after its last prompt token (token 0 for an empty prompt);
  * decode steps then run all sequences in lock step, each at its own position.
  * lens_host[b] == -1 leaves sequence b as it is (cache, length, current token): a finished
- * sequence's slot takes a new prompt while the others of the running batch keep their state. */
+ * sequence's slot takes a new prompt while the others of the running batch keep their state.
+ * Logits: those after a sequence's last prompt token; zero after an empty prompt; those of its
+ * last step for a sequence left as it is.  (If no sequence has a prompt, nothing is computed.) */
 LOGOS_API logos_status_t logos_llm_prefill_ragged(logos_handle_t model, const int32_t* tokens_host, int64_t t_max,
                                                   const int32_t* lens_host);
 /* Fill the KV cache for positions [0,t) with seeded N(0,1) fp16 values instead

@@ -302,6 +302,7 @@ logos_status_t build(Model* m, const void* nccl_id) {
     m->max_splits = s1 > s2 ? s1 : s2;
   }
   LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->h), B * H * 4));
+  LOGOS_CUDA_TRY(cudaMemsetAsync(m->h, 0, (size_t)(B * H * 4), m->stream));   // a prompt pass may read rows that no step wrote
   auto planes = [&](ActOut* a, int64_t elems) -> logos_status_t {
     a->mode = c.act_dtype;
     const int64_t plane = (elems * 2 + 255) / 256 * 256;   // one allocation: the GEMM's tensor map spans both planes
@@ -628,16 +629,20 @@ __global__ void gather_last_rows_kernel(float* __restrict__ h, const float* __re
     h[b * hidden + e] = __fadd_rn(__ldcg(src + row * hidden + e), __ldcg(delta + row * hidden + e));
 }
 
-// Sequence state before the token choice that ends a prompt pass: a sequence that took a prompt stands at
-// its last prompt position (and is marked in `ends`), an empty prompt leaves length 0 and token 0, a
-// negative length leaves the sequence as it is.
+// Sequence state before the token choice that ends a prompt pass, a CTA a sequence: one that took a prompt stands at
+// its last prompt position (and is marked in `ends`), an empty prompt leaves length 0, token 0 and a residual row
+// of zeros (hence logits of zero instead of those of the slot's last owner), a negative length leaves the
+// sequence as it is, its residual row, hence its last logits, included.
 __global__ void prompt_state_kernel(const int32_t* __restrict__ lens, int32_t* __restrict__ seq_len,
-                                    int32_t* __restrict__ tokens, int32_t* __restrict__ ends, int b) {
+                                    int32_t* __restrict__ tokens, int32_t* __restrict__ ends, float* __restrict__ h,
+                                    int64_t hidden) {
   pdl_wait();
   pdl_trigger();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= b) return;
+  const int64_t i = blockIdx.x;
   const int len = lens[i];
+  if (len == 0)
+    for (int64_t e = threadIdx.x; e < hidden; e += blockDim.x) h[i * hidden + e] = 0.f;
+  if (threadIdx.x != 0) return;
   ends[i] = len > 0 ? 1 : 0;
   if (len >= 0) seq_len[i] = len > 0 ? len - 1 : 0;
   if (len == 0) tokens[i] = 0;
@@ -824,8 +829,8 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
     LOGOS_TRY(check_launch("gather_last_rows_kernel"));
   }
   // the ordinary end of a step for the sequences that took a prompt
-  LOGOS_CUDA_TRY(launch_kernel(prompt_state_kernel, dim3((unsigned)((B + 127) / 128)), dim3(128), 0, st, (const int32_t*)lens_dev,
-                               m->seq_len, m->tokens, ends_dev, (int)B));
+  LOGOS_CUDA_TRY(launch_kernel(prompt_state_kernel, dim3((unsigned)B), dim3(128), 0, st, (const int32_t*)lens_dev,
+                               m->seq_len, m->tokens, ends_dev, m->h, H));
   LOGOS_TRY(check_launch("prompt_state_kernel"));
   m->launch_counter = 0;
   if (longest > 0) LOGOS_TRY(step_tail(m, 0, true, false, ends_dev, 0));

@@ -230,6 +230,28 @@ def test_ragged_prompts_tokens_lengths_and_kv(llm, oracle):
     ref.close()
 
 
+def test_ragged_prompts_logits_of_every_sequence(llm, oracle):
+    """Logits after prompts of different lengths: a sequence's own, zero after an empty prompt, the last step's where the
+    sequence was left as it is, zero where there was no step yet."""
+    toks = np.arange(SMALL["batch"] * 5, dtype=np.int32).reshape(SMALL["batch"], 5)
+    gpu = llm.Llm(**SMALL)
+    gpu.prefillRagged(toks, [3, 0, -1, 2])
+    assert not gpu.readLogits()[1:3].any()
+    gpu.prefill(toks)
+    gpu.decodeSteps(3)
+    before = gpu.readLogits()
+    gpu.prefillRagged(toks[:, ::-1], [3, 0, -1, 2])
+    after = gpu.readLogits()
+    assert not after[1].any()
+    assert np.array_equal(after[2], before[2])
+    alone = llm.Llm(**dict(SMALL, batch=1))
+    for b, n in ((0, 3), (3, 2)):
+        alone.prefill(toks[b:b + 1, ::-1][:, :n])
+        assert rel_l2(after[b], alone.readLogits()[0]) < 1e-4
+    gpu.free()
+    alone.free()
+
+
 @pytest.mark.parametrize("temperature", [0.0, 1.0])
 def test_decode_past_a_full_cache(llm, oracle, temperature):
     """The maximum size: once a sequence fills its cache (length == l_max) a step appends nothing,
