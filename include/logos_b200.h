@@ -294,8 +294,9 @@ LOGOS_API logos_status_t logos_llm_create(const logos_llm_config_t* cfg, const v
 LOGOS_API logos_status_t logos_llm_get_config(logos_handle_t model, logos_llm_config_t* cfg_out);
 /* Process t prompt tokens per sequence ([B][T] row-major, host) and fill the KV
  * cache; sequence lengths become t.  Starts from an empty cache.  The prompt runs in chunks of
- * positions, every sequence's chunk through a layer at once (about 4096 rows; the first call
- * allocates the chunk's workspace), with the decode step's arithmetic: weights
+ * positions, every sequence's chunk through a layer at once (about 4096 rows, fewer where there is
+ * no memory for their workspace, which a prompt that is larger than those before it
+ * allocates or enlarges), with the decode step's arithmetic: weights
  * are streamed once per chunk, not once per token.  LOGOS_B200_PREFILL=loop in the environment
  * selects the token-by-token pass through the decode step instead (for logos_llm_prefill_ragged too). */
 LOGOS_API logos_status_t logos_llm_prefill(logos_handle_t model, const int32_t* tokens_host, int64_t t);

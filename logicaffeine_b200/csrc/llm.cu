@@ -171,6 +171,7 @@ void destroy(Model* m) {
   if (m->attn_arrive) counters_unregister(m->attn_arrive);
   for (void* p : m->allocs) cudaFree(p);
   if (m->pf.block) cudaFree(m->pf.block);
+  if (m->prompt) cudaFree(m->prompt);
   for (cudaEvent_t e : m->prof_events) cudaEventDestroy(e);
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
@@ -653,36 +654,77 @@ bool chunked_prefill_enabled() {
   return !(e && (e[0] == 'l' || e[0] == '0'));   // "loop" or "0": prompts run through the decode step token by token
 }
 
-// One block for the buffers of a chunk of up to `rows` rows.  It grows when a later prompt fills a
-// larger chunk than any before it; the old block is freed once the stream has left it.
-logos_status_t prefill_workspace(Model* m, int64_t rows) {
+// Device words that prompts are indexed by (Model::prompt): grown at least geometrically, what is outgrown is freed once
+// the stream has left it.
+logos_status_t prompt_words(Model* m, int64_t need) {
+  if (m->prompt_cap >= need) return LOGOS_OK;
+  int64_t want = std::max(need, 2 * m->prompt_cap);
+  if (m->prompt) {
+    LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
+    cudaFree(m->prompt);
+    m->prompt = nullptr;
+    m->prompt_cap = 0;
+  }
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->prompt), (size_t)want * 4);
+  if (e != cudaSuccess && want > need) {
+    cudaGetLastError();
+    want = need;
+    e = cudaMalloc(reinterpret_cast<void**>(&m->prompt), (size_t)want * 4);
+  }
+  if (e != cudaSuccess) {
+    m->prompt = nullptr;
+    cudaGetLastError();
+    return cuda_fail(e, "cudaMalloc (prompt words)");
+  }
+  m->prompt_cap = want;
+  return LOGOS_OK;
+}
+
+// One block for the buffers of a chunk of up to `rows` rows.  When a later prompt fills a larger chunk than any before
+// it, it grows at least geometrically, up to `most` rows unless more are needed; the old block is freed once the
+// stream has left it.
+logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
   PrefillWs& w = m->pf;
   if (w.rows >= rows) return LOGOS_OK;
   const logos_llm_config_t& c = m->cfg;
   const int64_t H = c.hidden;
   const bool two = c.act_dtype == LOGOS_F32;
-  int64_t total = 0;
-  auto place = [&](int64_t bytes) {
-    const int64_t at = total;
-    total += (bytes + 255) / 256 * 256;
-    return at;
-  };
-  const int64_t o_h = place(rows * H * 4), o_delta = place(rows * H * 4), o_qkv = place(rows * m->nqkv * 4),
-                o_q16 = place(rows * m->nq * 2);
   const int64_t widths[3] = {H, m->nq, m->f_local};
-  int64_t o_hi[3], o_lo[3];
-  for (int i = 0; i < 3; ++i) {
-    o_hi[i] = place(rows * widths[i] * 2);
-    o_lo[i] = two ? place(rows * widths[i] * 2) : 0;
-  }
-  char* base = nullptr;
+  int64_t total = 0, o_h = 0, o_delta = 0, o_qkv = 0, o_q16 = 0, o_hi[3], o_lo[3];
+  auto lay_out = [&](int64_t n) {
+    total = 0;
+    auto place = [&](int64_t bytes) {
+      const int64_t at = total;
+      total += (bytes + 255) / 256 * 256;
+      return at;
+    };
+    o_h = place(n * H * 4);
+    o_delta = place(n * H * 4);
+    o_qkv = place(n * m->nqkv * 4);
+    o_q16 = place(n * m->nq * 2);
+    for (int i = 0; i < 3; ++i) {
+      o_hi[i] = place(n * widths[i] * 2);
+      o_lo[i] = two ? place(n * widths[i] * 2) : 0;
+    }
+  };
+  int64_t want = std::max(rows, std::min(2 * w.rows, most));
   if (w.block) {
     LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
     cudaFree(w.block);
     w = PrefillWs();
   }
+  char* base = nullptr;
+  lay_out(want);
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&base), (size_t)total);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc (prompt workspace)");
+  if (e != cudaSuccess && want > rows) {
+    cudaGetLastError();
+    lay_out(want = rows);
+    e = cudaMalloc(reinterpret_cast<void**>(&base), (size_t)total);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_fail(e, "cudaMalloc (prompt workspace)");
+  }
   w.block = base;
   w.h = reinterpret_cast<float*>(base + o_h);
   w.delta = reinterpret_cast<float*>(base + o_delta);
@@ -694,7 +736,7 @@ logos_status_t prefill_workspace(Model* m, int64_t rows) {
     planes[i]->hi = reinterpret_cast<__half*>(base + o_hi[i]);
     planes[i]->lo = two ? reinterpret_cast<__half*>(base + o_lo[i]) : nullptr;
   }
-  w.rows = rows;
+  w.rows = want;
   return LOGOS_OK;
 }
 
@@ -723,25 +765,36 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
     for (int64_t b = 0; b < B; ++b) r += std::min<int64_t>(std::max<int64_t>(lens[(size_t)b] - p0, 0), cn);
     return r;
   };
-  for (int64_t p0 = 0; p0 < longest;) {
-    int64_t lo = 1, hi = longest - p0;   // the largest chunk within the target, at least one position
-    while (lo < hi) {
-      const int64_t mid = (lo + hi + 1) / 2;
-      if (rows_of(p0, mid) <= target_rows) lo = mid; else hi = mid - 1;
+  auto cut = [&] {
+    chunks.clear();
+    total_rows = most_rows = 0;
+    for (int64_t p0 = 0; p0 < longest;) {
+      int64_t lo = 1, hi = longest - p0;   // the largest chunk within the target, at least one position
+      while (lo < hi) {
+        const int64_t mid = (lo + hi + 1) / 2;
+        if (rows_of(p0, mid) <= target_rows) lo = mid; else hi = mid - 1;
+      }
+      chunks.push_back({p0, lo, rows_of(p0, lo), total_rows});
+      total_rows += chunks.back().rows;
+      most_rows = std::max(most_rows, chunks.back().rows);
+      p0 += lo;
     }
-    chunks.push_back({p0, lo, rows_of(p0, lo), total_rows});
-    total_rows += chunks.back().rows;
-    most_rows = std::max(most_rows, chunks.back().rows);
-    p0 += lo;
+  };
+  cut();
+  while (most_rows > 0) {
+    const logos_status_t got = prefill_workspace(m, most_rows, target_rows);
+    if (got == LOGOS_OK) break;
+    // no room for chunks of this size: smaller ones, down to a position at a time
+    const int64_t before = most_rows;
+    if (got != LOGOS_MEMORY_EXHAUSTED) return got;
+    target_rows = most_rows / 2;
+    cut();
+    if (most_rows >= before) return got;
   }
-  if (most_rows > 0) LOGOS_TRY(prefill_workspace(m, most_rows));
   // everything the kernels index by, in one upload before the first launch: lens [B] | ends [B] | tokens,
   // sequence and position of every row | row0 [B] and count [B] of every chunk
   const int64_t need = 2 * B + 3 * total_rows + 2 * B * (int64_t)chunks.size();
-  if (m->prompt_cap < need) {
-    LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->prompt), need * 4));
-    m->prompt_cap = need;
-  }
+  LOGOS_TRY(prompt_words(m, need));
   std::vector<int32_t> meta((size_t)need, 0);
   const int64_t o_ends = B, o_tok = 2 * B, o_seq = o_tok + total_rows, o_pos = o_seq + total_rows, o_chunk = o_pos + total_rows;
   for (int64_t b = 0; b < B; ++b) meta[(size_t)b] = lens[(size_t)b];
@@ -1114,10 +1167,7 @@ logos_status_t logos_llm_prefill(logos_handle_t model, const int32_t* tokens_hos
       if (tokens_host[i] < 0 || tokens_host[i] >= m->cfg.vocab)
         return fail(LOGOS_OUT_OF_BOUNDS, "logos_llm_prefill: token id %d outside the vocabulary", tokens_host[i]);
     if (chunked_prefill_enabled()) return prefill_chunked(m, tokens_host, t, std::vector<int32_t>((size_t)B, (int32_t)t));
-    if (m->prompt_cap < B * t) {
-      LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->prompt), B * t * 4));
-      m->prompt_cap = B * t;
-    }
+    LOGOS_TRY(prompt_words(m, B * t));
     std::vector<int32_t> tr((size_t)(B * t));
     for (int64_t b = 0; b < B; ++b)
       for (int64_t p = 0; p < t; ++p) tr[(size_t)(p * B + b)] = tokens_host[b * t + p];
@@ -1152,10 +1202,7 @@ logos_status_t logos_llm_prefill_ragged(logos_handle_t model, const int32_t* tok
     if (chunked_prefill_enabled()) return prefill_chunked(m, tokens_host, t_max, std::vector<int32_t>(lens_host, lens_host + B));
     // device: [longest][B] prompt tokens (0 past a sequence's end), then the [B] lengths
     const int64_t need = (longest + 1) * B;
-    if (m->prompt_cap < need) {
-      LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->prompt), need * 4));
-      m->prompt_cap = need;
-    }
+    LOGOS_TRY(prompt_words(m, need));
     std::vector<int32_t> tr((size_t)need, 0);
     for (int64_t b = 0; b < B; ++b) {
       for (int64_t p = 0; p < lens_host[b]; ++p) tr[(size_t)(p * B + b)] = tokens_host[b * t_max + p];

@@ -252,6 +252,41 @@ def test_ragged_prompts_logits_of_every_sequence(llm, oracle):
     alone.free()
 
 
+def test_prompts_that_grow_keep_no_outgrown_memory(llm, oracle):
+    cfg = dict(SMALL, layers=1, hidden=128, h_q=2, h_kv=1, ffn=128, vocab=64, l_max=4000, batch=8)
+    gpu = llm.Llm(**cfg)
+    gpu.prefill(np.zeros((8, 512), np.int32))   # a full chunk: the workspace has its size from here on
+    before, _ = llm.devMemInfo()
+    for t in range(600, 4001, 50):
+        gpu.prefill(np.full((8, t), t % 64, np.int32))
+    after, _ = llm.devMemInfo()
+    # three words a row, at most twice the largest prompt's, in blocks of the driver's 2 MB
+    assert before - after <= 4 << 20, before - after
+    assert (gpu.readSeqLen() == 4000).all()
+    gpu.free()
+
+
+def test_a_longer_prompt_with_little_memory_left(llm, oracle):
+    """A prompt for whose chunks there is no memory runs in smaller ones, and one after it in large ones again."""
+    cfg = dict(SMALL, layers=1, hidden=1024, h_q=8, h_kv=2, head_dim=128, ffn=8192, batch=1, l_max=2100)
+    toks = (np.arange(2048, dtype=np.int32) * 37 % cfg["vocab"]).reshape(1, 2048)
+    gpu = llm.Llm(**cfg)
+    gpu.prefill(toks[:, :2048])
+    want = gpu.readLogits()
+    gpu.free()
+    gpu = llm.Llm(**cfg)
+    gpu.prefill(toks[:, :16])
+    rest = llm.DeviceBuffer(llm.devMemInfo()[0] - (24 << 20))   # 2048 rows take about 117 MB
+    gpu.prefill(toks)
+    got = gpu.readLogits()
+    rest.free()
+    assert rel_l2(got, want) < 1e-4
+    gpu.prefill(toks)
+    assert np.array_equal(gpu.readLogits(), want)
+    assert llm.kernelStatus() == 0
+    gpu.free()
+
+
 @pytest.mark.parametrize("temperature", [0.0, 1.0])
 def test_decode_past_a_full_cache(llm, oracle, temperature):
     """The maximum size: once a sequence fills its cache (length == l_max) a step appends nothing,
