@@ -134,6 +134,8 @@ static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStre
 //   * pdl_trigger() after the point where a successor's CTAs may take up SM resources.
 // Outside a scope the launch is an ordinary one and both calls are no-ops.
 bool pdl_active();
+// LOGOS_B200_PDL=0 in the environment: the library opens no scopes of its own
+bool pdl_enabled();
 struct PdlScope {
   bool prev;
   explicit PdlScope(bool on);

@@ -472,7 +472,6 @@ logos_status_t gemm_partials(Model* m, const ActOut& a, const Q8Mat& w, int* spl
 }
 
 bool debug_sync();
-bool pdl_enabled();
 logos_status_t debug_check(Model* m, const char* what, int64_t layer) {
   if (!debug_sync()) return LOGOS_OK;
   LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
@@ -901,15 +900,6 @@ bool debug_sync() {
   if (v < 0) {
     const char* e = getenv("LOGOS_B200_DEBUG_SYNC");
     v = (e && e[0] == '1') ? 1 : 0;
-  }
-  return v == 1;
-}
-
-bool pdl_enabled() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("LOGOS_B200_PDL");
-    v = (e && e[0] == '0') ? 0 : 1;
   }
   return v == 1;
 }

@@ -249,7 +249,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     g.s = tiled;
     g.s_tiled = 1;
   }
-  PdlScope pdl(true);
+  PdlScope pdl(pdl_active() || pdl_enabled());
   if (splits <= 1 && !staged) return launch_q8_gemm(g, st);
   GemmArgs gp = g;
   if (staged) {

@@ -66,6 +66,13 @@ void count_launch(int kind, int64_t n) { g_launches[kind].fetch_add(n, std::memo
 
 thread_local bool g_pdl = false;
 bool pdl_active() { return g_pdl; }
+bool pdl_enabled() {
+  static const bool on = [] {
+    const char* e = getenv("LOGOS_B200_PDL");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
 PdlScope::PdlScope(bool on) : prev(g_pdl) { g_pdl = on; }
 PdlScope::~PdlScope() { g_pdl = prev; }
 
