@@ -50,7 +50,7 @@ constexpr int ATT_CWARPS = 4;
 constexpr int ATT_CTHREADS = ATT_CWARPS * 32;
 constexpr int ATT_THREADS = (ATT_CWARPS + 1) * 32;
 constexpr int ATT_BOX_BYTES = 64 * 128;  // 64 rows x 128 bytes
-constexpr int ATT_MAX_BATCH = 2048;      // sequences whose tile counts a CTA keeps in shared memory
+constexpr int ATT_MAX_BATCH = 2048;      // sequences whose lengths a CTA keeps in shared memory
 
 struct AttnParams {
   const __half* q_f16;
@@ -145,11 +145,12 @@ __device__ __forceinline__ void store_out4(const AttnParams& p, int64_t oi, floa
 // normaliser are computed once by a warp, and the threads then sum the parts' output rows with all their loads
 // independent of one another: a fold is three rounds of global loads whatever the number of parts.  A
 // pair cut into more than ATT_MERGE_PARTS shares goes through a plain loop.
+// The lists lie where the query was staged, which nothing reads any more.
 constexpr int ATT_MERGE_PARTS = 64;
 struct MergeScratch {
   int   row0[ATT_MERGE_PARTS];    // first of the 16 rows of each part that holds tiles
-  float w[ATT_MERGE_PARTS][16];   // weight of a part for a query row, and its sum
-  float sum[ATT_MERGE_PARTS][16];
+  float w[ATT_MERGE_PARTS][16];   // weight of a part for a query row
+  float sum[ATT_CWARPS][ATT_MERGE_PARTS];   // the parts' sums for the row that a warp is at
   float l[16];                    // the row's normaliser
   int   np;
 };
@@ -212,16 +213,17 @@ __device__ __forceinline__ void merge_parts(const AttnParams& p, MergeScratch& m
       const int pi = lane + 32 * j;
       if (pi < np) {
         ms.w[pi][r] = exp2f(ml[j].x - muse);
-        ms.sum[pi][r] = ml[j].y;
+        ms.sum[warp][pi] = ml[j].y;
       }
     }
     __syncwarp();
     if (lane == 0) {
       float L = 0.f;
 #pragma unroll 4
-      for (int pi = 0; pi < np; ++pi) L = fmaf(ms.sum[pi][r], ms.w[pi][r], L);
+      for (int pi = 0; pi < np; ++pi) L = fmaf(ms.sum[warp][pi], ms.w[pi][r], L);
       ms.l[r] = L;
     }
+    __syncwarp();   // the next row's sums go where these are
   }
   asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
   // four neighbouring elements a thread, four parts' loads in flight: a part at a time took a round of latency
@@ -246,13 +248,33 @@ __device__ __forceinline__ void merge_parts(const AttnParams& p, MergeScratch& m
   }
 }
 
+// Dynamic shared memory of a CTA: the ring, the staged query, the appended rows and the warps' (max, sum), whose place
+// the fold's lists take over, the barriers, then by sequence the tiles before it and its last tile.
+template <int D>
+struct AttnSmem {
+  static constexpr int QS_STRIDE = D + 8;  // halfs; +16 bytes keeps ldmatrix rows on distinct banks
+  static constexpr int STAGE_BYTES = 2 * (D / 64) * ATT_BOX_BYTES;
+  static constexpr int STAGED = 16 * QS_STRIDE * 2 + 2 * D * 2 + ATT_CWARPS * 16 * 2 * 4;
+  static constexpr int WORK = ((STAGED > (int)sizeof(MergeScratch) ? STAGED : (int)sizeof(MergeScratch)) + 15) / 16 * 16;
+  static constexpr int BARS = 2 * ATT_STAGES * 8;
+  static constexpr int FLAGS = 16;
+  static constexpr int bytes(int batch) {
+    return 1024 + ATT_STAGES * STAGE_BYTES + WORK + BARS + FLAGS + (batch + 1) * 4 + batch;
+  }
+};
+// An SM has 228 KB and keeps 1 KB of it for each CTA.  With one CTA an SM the grid takes two rounds: 512 sequences of
+// 1024 positions, 28/4 heads of 128, 240 us against 181.
+static_assert(2 * (AttnSmem<128>::bytes(ATT_MAX_BATCH) + 1024) <= 228 * 1024, "two CTAs fit an SM whatever the batch");
+static_assert(2 * (AttnSmem<64>::bytes(ATT_MAX_BATCH) + 1024) <= 228 * 1024, "two CTAs fit an SM whatever the batch");
+
 template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        const AttnParams p) {
   constexpr int NBOX = D / 64;
-  constexpr int STAGE_BYTES = 2 * NBOX * ATT_BOX_BYTES;
-  constexpr int QS_STRIDE = D + 8;  // halfs; +16 bytes keeps ldmatrix rows on distinct banks
+  using Smem = AttnSmem<D>;
+  constexpr int STAGE_BYTES = Smem::STAGE_BYTES;
+  constexpr int QS_STRIDE = Smem::QS_STRIDE;
   constexpr int KSTEPS = D / 16;
   static_assert(STAGE_BYTES >= ATT_CWARPS * 16 * D * 4, "a ring stage doubles as the scratch that combines the warps");
 
@@ -263,16 +285,22 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   __half* new_k = qs + 16 * QS_STRIDE;                               // [D]
   __half* new_v = new_k + D;                                         // [D]
   float* mml = reinterpret_cast<float*>(new_v + D);                  // [warp][16][2]
-  uint64_t* bar_full = reinterpret_cast<uint64_t*>(mml + ATT_CWARPS * 16 * 2);
+  MergeScratch& s_merge = *reinterpret_cast<MergeScratch*>(qs);      // in place of all of these, once a pair is done
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(qs) + Smem::WORK);
   uint64_t* bar_empty = bar_full + ATT_STAGES;
-  int32_t* s_len = reinterpret_cast<int32_t*>(bar_empty + ATT_STAGES);    // [B] lengths, read once
-  int32_t* s_pref = s_len + p.b;                                         // [B + 1] tiles before it
+  int& prior_status = *reinterpret_cast<int*>(bar_empty + ATT_STAGES);
+  int& s_bump = *(&prior_status + 1);   // this CTA is the last to have its lengths
+  int& s_last = *(&prior_status + 2);   // this CTA wrote a pair's last part (the consumers' own: the producer may still look at s_bump)
+  int32_t* s_pref = &prior_status + 4;                               // [B + 1] tiles before it
+  uint8_t* s_tail = reinterpret_cast<uint8_t*>(s_pref + p.b + 1);    // [B] positions that its last tile lacks; FULL: the length is l_max or more
+  constexpr int FULL = 128;
+  static_assert(ATT_TILE <= FULL, "a tile's positions beside the flag");
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int G = p.h_q / p.h_kv;
-  auto tiles_of = [&](int b) { return (attn_len_eff(p, s_len[b]) + ATT_TILE - 1) / ATT_TILE; };
+  auto tiles_of = [&](int b) { return s_pref[b + 1] - s_pref[b]; };
 
   // In a decode step the lengths and the cached rows are older than the step, so reading them, cutting the work and
   // loading the first tiles overlap the predecessor's end, and only what reads the query and the new K/V rows waits.
@@ -280,10 +308,6 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   if (!p.early_reads) pdl_wait();
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
   // (one thread reads, everyone takes the same decision)
-  __shared__ int prior_status;
-  __shared__ int s_bump;   // this CTA is the last to have its lengths
-  __shared__ int s_last;   // this CTA wrote a pair's last part (the consumers' own: the producer may still look at s_bump)
-  __shared__ MergeScratch s_merge;
   if (tid == 0) {
     prior_status = *reinterpret_cast<volatile int*>(p.status);
     for (int i = 0; i < ATT_STAGES; ++i) {
@@ -294,7 +318,12 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     prefetch_tensormap(&map_k);
     prefetch_tensormap(&map_v);
   }
-  for (int b = tid; b < p.b; b += ATT_THREADS) s_len[b] = __ldcg(p.seq_len + b);
+  for (int b = tid; b < p.b; b += ATT_THREADS) {
+    const int len0 = __ldcg(p.seq_len + b), len_eff = attn_len_eff(p, len0);
+    const int tiles = (len_eff + ATT_TILE - 1) / ATT_TILE;
+    s_pref[b] = tiles;
+    s_tail[b] = (uint8_t)((tiles * ATT_TILE - len_eff) | (len0 >= p.l_max ? FULL : 0));
+  }
   __syncthreads();
   if (prior_status != 0) {
     pdl_wait();
@@ -305,7 +334,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     int run = 0;
     for (int i = 0; i < per; ++i) {
       const int b = lane * per + i;
-      if (b < p.b) run += tiles_of(b);
+      if (b < p.b) run += s_pref[b];
     }
     int incl = run;
 #pragma unroll
@@ -317,8 +346,9 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     for (int i = 0; i < per; ++i) {
       const int b = lane * per + i;
       if (b < p.b) {
+        const int tiles = s_pref[b];
         s_pref[b] = acc;
-        acc += tiles_of(b);
+        acc += tiles;
       }
     }
     if (lane == 31) s_pref[p.b] = incl;
@@ -410,8 +440,8 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       const int share_last = share_of_tile(pair_g0 + tiles_b - 1, total, p.shares);
       const bool whole = share_first == share_last;   // the pair lies inside this share: write the result itself
       const int slot = g == g_lo ? 0 : 1;
-      const int len0 = s_len[b];
-      const int len_eff = attn_len_eff(p, len0);
+      const int len_eff = tiles_b * ATT_TILE - (s_tail[b] & (FULL - 1));
+      const int len0 = (s_tail[b] & FULL) ? p.l_max : p.fused ? len_eff - 1 : len_eff;   // up to l_max
       const int64_t row_base = ((int64_t)b * p.h_kv + kvh) * p.l_max;
       const int pos_new = len0;  // where the appended row goes
       const bool append = p.fused && len0 < p.l_max;
@@ -744,17 +774,11 @@ __global__ void kv_append_rope_kernel(__half* k_cache, __half* v_cache, const __
   }
 }
 
-template <int D>
-size_t attn_smem_bytes(int64_t batch) {
-  return 1024 + (size_t)ATT_STAGES * 2 * (D / 64) * ATT_BOX_BYTES + (size_t)16 * (D + 8) * 2 + (size_t)2 * D * 2 +
-         (size_t)ATT_CWARPS * 16 * 2 * 4 + 2 * ATT_STAGES * 8 + (size_t)(2 * batch + 1) * 4 + 64;
-}
-
 // The persistent grid: the tile sequence is cut into this many shares, one per CTA.
 int attn_shares(const AttnArgs& a) {
   const int sms = sm_count(a.device);
   const int64_t tiles_max = (a.l_max + ATT_TILE - 1) / ATT_TILE;
-  int64_t g = std::min<int64_t>(2 * sms, ATT_COUNTER_BYTES / sizeof(unsigned) - 1);   // two CTAs of about 113 KB of shared memory fit an SM
+  int64_t g = std::min<int64_t>(2 * sms, ATT_COUNTER_BYTES / sizeof(unsigned) - 1);   // two CTAs of up to 113 KB of shared memory fit an SM (AttnSmem)
   // With no more (sequence, KV head) pairs than CTAs, a whole number of shares per pair: where the
   // sequences are equally long every share boundary then falls on a pair boundary or cuts a pair
   // into equal pieces, and a CTA stages one pair's query instead of two (measured 4-8 % on the
@@ -810,9 +834,9 @@ logos_status_t launch_attn_t(const AttnArgs& a, cudaStream_t st) {
   p.status = a.ext_status ? a.ext_status : kernel_status_ptr(a.device);
   if (!p.status) return fail(LOGOS_ERROR, "attention: no kernel status word");
 
-  const size_t smem = attn_smem_bytes<D>(a.b);
-  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(gqa_decode_attn_kernel<D>), a.device, (int)smem));
-  LOGOS_CUDA_TRY(launch_kernel(gqa_decode_attn_kernel<D>, dim3((unsigned)shares), dim3(ATT_THREADS), smem, st, mk, mv, p));
+  const int smem = AttnSmem<D>::bytes((int)a.b);
+  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(gqa_decode_attn_kernel<D>), a.device, smem));
+  LOGOS_CUDA_TRY(launch_kernel(gqa_decode_attn_kernel<D>, dim3((unsigned)shares), dim3(ATT_THREADS), (size_t)smem, st, mk, mv, p));
   count_launch(LK_ATTN);
   return check_launch("gqa_decode_attn_kernel");
 }
