@@ -61,47 +61,85 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   mbar_arrive_expect_tx(smem_u32(bar), bytes);
 }
-// Bounded waits.  A wait polls until the phase completes or the thread's budget of polls is used up: once
-// *polls is 0 this and every later wait of the thread return at once, so that a loop can look at it once a
-// round instead of after every wait.  What is done in between works on stale data; the caller drops it
-// and reports.  A poll of a barrier that is not ready takes at least 65 cycles, so the budget of one
-// thread lasts for a second of SM clock or longer.  A warp that waits takes issue slots from the warps
-// it waits for: the loop is as few instructions as it can be.
-constexpr uint32_t kWaitPolls = 30000000u;
+// Bounded waits: one to two periods of the upper half of the SM clock, two to four and a half seconds at 1.9 GHz.  The
+// limit is of time, since a poll that finds its phase open takes anything from 65 cycles to the 7800 for which
+// the hardware suspends the thread (measured on a B200): a number of polls that outlasts the short ones bounds the
+// long ones by minutes.  The clock is read once in 32 failed polls: an arrival that does not end the phase wakes the
+// thread too, and reading it after every poll cost the GEMM 1 to 1.5 %.
+//
+// The forms with `since` share one limit, counted from wait_start(): once it has passed, *since is WAIT_OVER, and this
+// and every later wait of the thread return after a poll, so that a loop can look at it once a round instead of
+// after every wait.  What is done in between works on stale data; the caller drops it and reports.  A warp that
+// waits takes issue slots from the warps it waits for: the loop is as few instructions as it can be.
+constexpr uint32_t WAIT_OVER = 31;
+// The clock's upper half in units of 32; the low five bits count failed polls.  At least two units, so that no valid
+// value is WAIT_OVER or what a failed poll makes of it.
+__device__ __forceinline__ uint32_t wait_start() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%clock_hi;" : "=r"(t));
+  return (t < 2 ? 2u : t) << 5;
+}
 #define LOGOS_MBAR_TRY(P, BAR, PH) "mbarrier.try_wait.parity.shared::cta.b64 " P ", [" BAR "], " PH ";\n\t"
+#define LOGOS_MBAR_REGS "{\n\t.reg .pred p, q, r, s;\n\t.reg .u32 t;\n"
 #define LOGOS_MBAR_AGAIN                                                                                     \
   "@p bra DONE;\n\t"                                                                                         \
-  "setp.ne.u32 s, %0, 0;\n\t"                                                                                \
-  "@s add.u32 %0, %0, -1;\n\t"                                                                               \
+  "add.u32 %0, %0, 1;\n\t"                                                                                   \
+  "and.b32 t, %0, 31;\n\t"                                                                                   \
+  "setp.ne.u32 s, t, 0;\n\t"                                                                                 \
+  "@s bra POLL;\n\t"                                                                                         \
+  "setp.eq.u32 s, %0, 32;\n\t"                                                                               \
+  "@s bra OVER;\n\t"                                                                                         \
+  "add.u32 %0, %0, -32;\n\t"                                                                                 \
+  "mov.u32 t, %%clock_hi;\n\t"                                                                               \
+  "shl.b32 t, t, 5;\n\t"                                                                                     \
+  "sub.s32 t, t, %0;\n\t"                                                                                    \
+  "setp.lt.s32 s, t, 64;\n\t"                                                                                \
   "@s bra POLL;\n"                                                                                           \
+  "OVER:\n\tmov.u32 %0, 31;\n"                                                                              \
   "DONE:\n\t}"
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t* polls) {
-  asm volatile("{\n\t.reg .pred p, s;\nPOLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_AGAIN
-               : "+r"(*polls)
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, uint32_t* since) {
+  asm volatile(LOGOS_MBAR_REGS "POLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_AGAIN
+               : "+r"(*since)
                : "r"(bar), "r"(parity)
                : "memory");
 }
 // Two or three barriers polled together: their latencies overlap.
-__device__ __forceinline__ void mbar_wait2(uint32_t bar0, uint32_t ph0, uint32_t bar1, uint32_t ph1, uint32_t* polls) {
-  asm volatile("{\n\t.reg .pred p, q, s;\nPOLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_TRY("q", "%3", "%4")
+__device__ __forceinline__ void mbar_wait2(uint32_t bar0, uint32_t ph0, uint32_t bar1, uint32_t ph1, uint32_t* since) {
+  asm volatile(LOGOS_MBAR_REGS "POLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_TRY("q", "%3", "%4")
                "and.pred p, p, q;\n\t" LOGOS_MBAR_AGAIN
-               : "+r"(*polls)
+               : "+r"(*since)
                : "r"(bar0), "r"(ph0), "r"(bar1), "r"(ph1)
                : "memory");
 }
 __device__ __forceinline__ void mbar_wait3(uint32_t bar0, uint32_t ph0, uint32_t bar1, uint32_t ph1, uint32_t bar2, uint32_t ph2,
-                                           uint32_t* polls) {
-  asm volatile("{\n\t.reg .pred p, q, r, s;\nPOLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_TRY("q", "%3", "%4")
+                                           uint32_t* since) {
+  asm volatile(LOGOS_MBAR_REGS "POLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") LOGOS_MBAR_TRY("q", "%3", "%4")
                LOGOS_MBAR_TRY("r", "%5", "%6") "and.pred p, p, q;\n\tand.pred p, p, r;\n\t" LOGOS_MBAR_AGAIN
-               : "+r"(*polls)
+               : "+r"(*since)
                : "r"(bar0), "r"(ph0), "r"(bar1), "r"(ph1), "r"(bar2), "r"(ph2)
                : "memory");
 }
-// A single wait with a budget of its own; false when it gave up.
+// A single wait with a limit of its own, counted from its 32nd failed poll; false when it gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t polls = kWaitPolls;
-  mbar_wait(smem_u32(bar), parity, &polls);
-  return polls != 0;
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p, s;\n\t.reg .u32 n, t, e;\n\tmov.u32 n, 0;\n"
+               "POLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2")
+               "@p bra DONE;\n\t"
+               "add.u32 n, n, 1;\n\t"
+               "and.b32 t, n, 31;\n\t"
+               "setp.ne.u32 s, t, 0;\n\t"
+               "@s bra POLL;\n\t"
+               "mov.u32 t, %%clock_hi;\n\t"
+               "setp.eq.u32 s, n, 32;\n\t"
+               "@s mov.u32 e, t;\n\t"
+               "sub.u32 t, t, e;\n\t"
+               "setp.lt.u32 s, t, 2;\n\t"
+               "@s bra POLL;\n"
+               "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok)
+               : "r"(smem_u32(bar)), "r"(parity)
+               : "memory");
+  return ok != 0;
 }
 
 __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {

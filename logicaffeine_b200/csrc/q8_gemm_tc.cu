@@ -406,7 +406,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   const int units = prior_status != 0 ? 0 : (p.pairs + p.solos) * p.splits * p.mtiles;
 
   bool ok = true;
-  uint32_t polls = kWaitPolls;   // see mbar_wait; a new budget every unit
+  uint32_t since = wait_start();   // see mbar_wait; a new limit every unit
 
   // Every role walks the same sequence of groups: units, stages, the unit's tiles, halves.
   if (warp < 4) {
@@ -423,12 +423,12 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       Ring<SC_SLOTS> c;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const TcUnit it = tc_unit(p, u);
-        polls = kWaitPolls;
+        since = wait_start();
         for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
           for (int j = it.tile; j < it.tile + it.ntile; ++j) {
             const int block = j * p.stages_total + i;   // of a tile-major array
             const uint32_t bar = raw_full + 8 * r.slot;
-            mbar_wait(raw_empty + 8 * r.slot, r.ph ^ 1u, &polls);
+            mbar_wait(raw_empty + 8 * r.slot, r.ph ^ 1u, &since);
             if (elect_one()) {
               mbar_arrive_expect_tx(bar, RAW_BYTES + SC_BYTES);
               // row-major weights: tile (row, stage) of a [N][K] map; tile-major: 128 rows of 128 bytes at
@@ -444,7 +444,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             r.next();
             c.next();
           }
-          if (polls == 0) {
+          if (since == WAIT_OVER) {
             if (lane == 0) tc_report(p.status, 2010, i, it.nst);
             ok = false;
           }
@@ -457,18 +457,18 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       Ring<ACT_SLOTS> r;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const TcUnit it = tc_unit(p, u);
-        polls = kWaitPolls;
+        since = wait_start();
         const int m0 = it.mtile * T;
         for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
           const uint32_t bar = act_full + 8 * r.slot;
-          mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &polls);
+          mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &since);
           if (elect_one()) {
             mbar_arrive_expect_tx(bar, Cfg::ACT_BYTES);
             tma_load_4d_hint(act + r.slot * Cfg::ACT_BYTES, &map_a, bar, 0, m0, 2 * i, 0, pol);
           }
           __syncwarp();
           r.next();
-          if (polls == 0) {
+          if (since == WAIT_OVER) {
             if (lane == 0) tc_report(p.status, 2020, i, it.nst);
             ok = false;
           }
@@ -487,7 +487,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       Ring<ENTRIES, 2> rd(half % ENTRIES);                         // the entry
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const TcUnit it = tc_unit(p, u);
-        polls = kWaitPolls;
+        since = wait_start();
         for (int i = 0; i < it.nst; ++i) {
           const uint64_t bdesc0 = bdesc_first + (uint32_t)(ra.slot * (Cfg::ACT_BYTES >> 4));   // start address field: no carry out of it
           for (int j = 0; j < it.ntile; ++j) {
@@ -495,9 +495,9 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             const uint32_t free_bar = acc_empty + 8 * PER * re.slot, full_bar = acc_full + 8 * PER * rf.slot;
 #pragma unroll
             for (int k = 0; k < PER; ++k) {
-              if (k > 0) mbar_wait(free_bar + 8 * k, re.ph, &polls);
-              else if (j == 0) mbar_wait3(act_full + 8 * ra.slot, ra.ph, ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
-              else mbar_wait2(ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &polls);
+              if (k > 0) mbar_wait(free_bar + 8 * k, re.ph, &since);
+              else if (j == 0) mbar_wait3(act_full + 8 * ra.slot, ra.ph, ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &since);
+              else mbar_wait2(ta_full + 8 * rt.slot, rt.ph, free_bar, re.ph, &since);
               tc_fence_after();
               const uint32_t d0 = tmem_base + Cfg::ACC_COL0 + rd.slot * Cfg::ENTRY_COLS + k * IB * T;
               if (elect_one()) {
@@ -529,7 +529,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             rd.next();
           }
           ra.next();
-          if (polls == 0) {
+          if (since == WAIT_OVER) {
             if (lane == 0) tc_report(p.status, 2030, i, it.nst);
             ok = false;
             break;
@@ -551,12 +551,12 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     Ring<TA_SLOTS, 2> a(0, 1u);   // a stage takes slots a and a + 1
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
-      polls = kWaitPolls;
+      since = wait_start();
       const int count = it.nst * it.ntile;
       for (int i = 0; i < count && ok; ++i) {
         // everything the stage needs in one wait, all its loads together, one wait for its stores: a round of
         // latency costs as much as fifty instructions
-        mbar_wait3(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, ta_empty + 8 * (a.slot + 1), a.ph, &polls);
+        mbar_wait3(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, ta_empty + 8 * (a.slot + 1), a.ph, &since);
         tc_fence_after();
         uint4 wv[8];
 #pragma unroll
@@ -586,7 +586,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         mbar_arrive_if(ta_full + 8 * (a.slot + 1), lane == 0);
         a.next();
         r.next();
-        if (polls == 0) {
+        if (since == WAIT_OVER) {
           if (lane == 0) tc_report(p.status, 2040, i, count);
           ok = false;
         }
@@ -624,7 +624,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         step(ent, 1, ENTRIES);
         const uint32_t at1 = t_lane + col + ent * Cfg::ENTRY_COLS;
         step(ent, 1, ENTRIES);
-        mbar_wait2(acc_full + 8 * grp, ph, acc_full + 8 * (grp + 1), ph, &polls);
+        mbar_wait2(acc_full + 8 * grp, ph, acc_full + 8 * (grp + 1), ph, &since);
         tc_fence_after();
         uint32_t b[4 * hc];
         tc_ld_cols<hc>(at0, b);
@@ -640,7 +640,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 4; ++k) add_cols<hc>(sum, s[k], b + k * hc);
       } else {
-        if (PER == 1) mbar_wait2(acc_full + 8 * grp, ph, acc_full + 8 * (grp + 1), ph, &polls);
+        if (PER == 1) mbar_wait2(acc_full + 8 * grp, ph, acc_full + 8 * (grp + 1), ph, &since);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const uint32_t at = t_lane + col + ent * Cfg::ENTRY_COLS;
@@ -648,7 +648,7 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
           for (int k = 0; k < PER; ++k) {
             const uint32_t bar = 8 * (PER * (grp + h) + k);
-            if (PER > 1) mbar_wait(acc_full + bar, ph, &polls);
+            if (PER > 1) mbar_wait(acc_full + bar, ph, &since);
             if (PER > 1 || h == 0) tc_fence_after();
             if (h == 0 && k == 0) scales();
             drain_blocks<hc, IB, T>(sum, at + k * IB * T, s + h * 2 + k * IB, [&] {
@@ -668,18 +668,18 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     int u = blockIdx.x;
     for (; u < pair_units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
-      polls = kWaitPolls;
+      since = wait_start();
       float2 acc[pair_cols / 2];
 #pragma unroll
       for (int x = 0; x < pair_cols / 2; ++x) acc[x] = make_float2(0.f, 0.f);
-      for (int i = 0; i < it.nst && polls != 0; ++i) {
+      for (int i = 0; i < it.nst && since != WAIT_OVER; ++i) {
         drain_stage(pair_cols, acc, th * pair_cols, two);
         step(ent, 2 % ENTRIES, ENTRIES);            // past the other tile's two groups
         step(rc, 2, SC_SLOTS);
         grp ^= 4;
         ph ^= (uint32_t)(grp < 4);
       }
-      if (polls == 0) {
+      if (since == WAIT_OVER) {
         if (lane == 0) tc_report(p.status, 2050, 0, it.nst);
         ok = false;
         break;
@@ -694,18 +694,18 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     grp -= 2 * g;
     for (; u < units && ok; u += gridDim.x) {
       const TcUnit it = tc_unit(p, u);
-      polls = kWaitPolls;
+      since = wait_start();
       float2 acc[solo_cols / 2];
 #pragma unroll
       for (int x = 0; x < solo_cols / 2; ++x) acc[x] = make_float2(0.f, 0.f);
       const uint32_t col = (SHARE * g + th) * solo_cols;
-      for (int i = 0; i < it.nst && polls != 0; ++i) {
+      for (int i = 0; i < it.nst && since != WAIT_OVER; ++i) {
         drain_stage(solo_cols, acc, col, one);
         step(rc, 1, SC_SLOTS);
         step(grp, 2, GROUPS);
         ph ^= (uint32_t)(grp == 0);
       }
-      if (polls == 0) {
+      if (since == WAIT_OVER) {
         if (lane == 0) tc_report(p.status, 2051, 0, it.nst);
         ok = false;
         break;

@@ -3,6 +3,7 @@ oracle on the same seeded inputs.  Integer, index and KV-cache results are
 compared bit for bit; f32-accumulated results within a relative L2 error of
 1e-3 (the stated tolerance; observed values are around 1e-6)."""
 import os
+import shutil
 import subprocess
 import sys
 import textwrap
@@ -576,3 +577,19 @@ def test_attention_in_a_dependent_launch_scope(llm, oracle):
         for got, want in zip(_sequences_in_a_scope(llm, oracle, True), plain):
             for g, w in zip(got, want):
                 assert np.array_equal(g, w)
+
+
+def test_waits_inside_kernels_end_in_seconds(tmp_path):
+    """A wait for a barrier that nothing completes returns and says so, in seconds: the limit is of time, whatever a
+    poll takes."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    exe = str(tmp_path / "wait_limit")
+    subprocess.run([nvcc, "-ccbin", "/usr/bin/g++", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3",
+                    "--expt-relaxed-constexpr", "-I", os.path.join(here, "..", "logicaffeine_b200", "csrc"), "-o", exe,
+                    os.path.join(here, "wait_limit.cu")], check=True, capture_output=True)
+    lines = subprocess.run([exe], check=True, capture_output=True, text=True, timeout=120).stdout.split("\n")
+    for form, line in enumerate(lines[:2]):
+        f, ms, gave_up = line.split()
+        assert int(f) == form and int(gave_up) == 1, line
+        assert 1000 < float(ms) < 12000, line   # 2^32 to 2^33 cycles: 2.2 to 4.4 s at 1965 MHz
