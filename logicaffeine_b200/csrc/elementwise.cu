@@ -343,7 +343,7 @@ tp_residual_rmsnorm_kernel(float* __restrict__ h, const TpFusedArgs t, int parts
 template <bool BF16>
 __global__ void __launch_bounds__(256)
 gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const float* __restrict__ s, float* __restrict__ tiled,
-                 int64_t n, int64_t kb, int64_t ktiles, int64_t act_blocks) {
+                 int64_t n, int64_t kb, int64_t ktiles, int64_t act_blocks, unsigned* misfit, unsigned call) {
   // count8: groups of eight of the planes; rows of the planes are whole K tiles, rows of `a` kb * 32 values
   pdl_trigger();
   if ((int64_t)blockIdx.x < act_blocks) {
@@ -370,6 +370,22 @@ gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const flo
       const float4 v0 = __ldg(reinterpret_cast<const float4*>(a) + 2 * src), v1 = __ldg(reinterpret_cast<const float4*>(a) + 2 * src + 1);
       x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
       x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
+    }
+    if (tiled) {   // sixteen threads hold a row's values of a K tile
+      // An fp16 plane is off by up to 2^-25 below fp16's normal range, two planes by up to 2^-36: from the largest value
+      // on that is 2^-17 of it (results are rounded to 2^-9) and 2^-24.
+      constexpr float least = BF16 ? 0x1p-8f : 0x1p-12f;
+      const unsigned tile = 0xffffu << (threadIdx.x & 16);
+      float most = 0.f;
+      bool beyond = false;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        most = fmaxf(most, fabsf(x[j]));
+        beyond |= !(fabsf(x[j]) <= 65504.f);   // NaN too
+      }
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) most = fmaxf(most, __shfl_xor_sync(tile, most, d));
+      if (beyond || (most > 0.f && most < least)) *misfit = call;
     }
     __half hi[8], lo[8];
 #pragma unroll
@@ -587,16 +603,16 @@ logos_status_t launch_embed(const int32_t* tokens, const int8_t* q, const float*
 }
 
 logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t m, const float* s,
-                                float* tiled_or_null, int64_t n, int64_t k, cudaStream_t st) {
+                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call, cudaStream_t st) {
   if (k % 32 || (reinterpret_cast<uintptr_t>(a) & 15u))
     return fail(LOGOS_ERROR, "gemm_prep: K must be a multiple of 32 and the activations 16-byte aligned");
   const int64_t ktiles = (k + 127) / 128, count8 = m * ktiles * 16;
   const int64_t act_blocks = (count8 + 255) / 256, scale_blocks = tiled_or_null ? (n * ktiles + 255) / 256 : 0;
   const dim3 grid((unsigned)(act_blocks + scale_blocks));
   if (a_dtype == LOGOS_BF16)
-    gemm_prep_kernel<true><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks);
+    gemm_prep_kernel<true><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call);
   else
-    gemm_prep_kernel<false><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks);
+    gemm_prep_kernel<false><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call);
   count_launch(LK_ELEMWISE);
   return check_launch("gemm_prep_kernel");
 }

@@ -225,6 +225,45 @@ def test_q8_gemm_residual_of_several_token_tiles(llm, oracle, m, n, k):
     assert rel_l2(O.bf16_to_f32(c), O.bf16_to_f32(ref)) < 1e-3
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 128, 160), (17, 300, 1056), (64, 3584, 2368), (100, 19000, 160)])   # K splits and none
+def test_q8_gemm_activations_that_fp16_planes_do_not_hold(llm, oracle, m, n, k):
+    """K that is no multiple of 128: magnitudes past fp16's range, tiny ones and NaN give what f32 arithmetic gives, for
+    every epilogue, a residual in place among them, whatever the calls before and after had."""
+    O = oracle
+    a = O.synth_fill(O.F32, 2, 6, 10, 0, m * k, 0.0, 1.0).reshape(m, k)
+    q = O.synth_fill(O.I8, 0, 6, 11, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 6, 12, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    aux = O.f32_to_bf16(O.synth_fill(O.F32, 2, 6, 13, 0, m * n, 0.0, 1.0).reshape(m, n))
+    plain = llm.q8GemmF32Host(a, q, s)
+    large, tiny, nan = a.copy(), a * np.float32(1e-7), a.copy()
+    large[m - 1, k - 1] = 3e5
+    nan[m // 2, 5] = np.nan
+    for x in (large, tiny, nan):
+        rows = np.isfinite(x).all(axis=1)
+        got = llm.q8GemmF32Host(x, q, s)
+        want = O.q8_gemm_f32(np.where(np.isnan(x), np.float32(0), x), O.F32, q, s)
+        for r in np.flatnonzero(rows):
+            # f32 sums over k terms in another order: about sqrt(k) roundings of 2^-24
+            assert rel_l2(got[r], want[r]) < 2e-6
+        assert np.isnan(got[~rows]).all()
+        assert np.array_equal(llm.q8GemmF32Host(a, q, s), plain)
+        xb = O.f32_to_bf16(x)
+        for epi in (0, 1, 2):
+            got = O.bf16_to_f32(llm.q8GemmHost(xb, q, s, epilogue=epi, aux=aux if epi == 1 else None))
+            want = O.bf16_to_f32(llm.q8GemmHost(xb, q, s, epilogue=epi, aux=aux if epi == 1 else None, simt=True))
+            for r in np.flatnonzero(rows):
+                assert rel_l2(got[r], want[r]) < 3e-3   # bf16 results: half a last place is 2^-9 of the value
+            assert np.isnan(got[~rows]).all()
+        da, dq, ds, dc = (_dev(llm, v) for v in (xb, q, s, aux))
+        llm.q8Gemm(da, dq, ds, dc, m, n, k, 1, dc)
+        got = O.bf16_to_f32(dc.download(np.uint16, (m, n)))
+        want = O.bf16_to_f32(llm.q8GemmHost(xb, q, s, epilogue=1, aux=aux, simt=True))
+        for r in np.flatnonzero(rows):
+            assert rel_l2(got[r], want[r]) < 3e-3
+        assert np.isnan(got[~rows]).all()
+    assert llm.kernelStatus() == 0
+
+
 def _in_a_process_of_its_own(code):
     """Runs `code` after the imports it needs in a fresh process, whose library scratch is empty."""
     here = os.path.dirname(os.path.abspath(__file__))
