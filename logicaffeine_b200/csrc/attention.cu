@@ -569,6 +569,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
               }
             }
           }
+          fence_proxy_async_smem();   // the next tile's loads write here
           __syncwarp();
         }
 
@@ -727,6 +728,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           if (d == 0) *reinterpret_cast<float2*>(p.part_ml + (pi + r) * 2) = make_float2(mstar, L);
         }
       }
+      fence_proxy_async_smem();   // the scratch is a ring stage: the next tile's loads write there
       asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");   // everyone has read the scratch and qs
       if (lane == 0) mbar_arrive(&bar_empty[st]);
       if (!whole) {

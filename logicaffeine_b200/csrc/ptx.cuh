@@ -36,7 +36,7 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) { mbar_
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// generic-proxy writes -> visible to the async proxy (TMA, tcgen05.mma operand reads)
+// this thread's writes to shared memory come before what the async proxy (TMA) does there after a later barrier
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
