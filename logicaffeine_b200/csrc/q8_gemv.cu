@@ -168,7 +168,7 @@ logos_status_t launch_q8_gemv(const int8_t* q, const float* s, const float* x, f
     return LOGOS_OK;
   }
   // two rows a warp unless that would leave more than half of the warps without any; the larger CTA where x fits
-  // beside its rings (K up to 16384), past K = 29696 x stays in global memory
+  // beside its rings (K up to 16384), past K = 30208 x stays in global memory
   const int64_t sms = sm_count(device);
   const int rows = n <= sms * GEMV_WARPS ? 1 : 2;
   const int64_t groups = (n + rows - 1) / rows;
