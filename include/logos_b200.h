@@ -143,7 +143,7 @@ LOGOS_API logos_status_t logos_dev_free(logos_handle_t h);
 LOGOS_API logos_status_t logos_kernel_status(int32_t device, int32_t* out_code);
 
 /* Kernel launches this process has made through the library, by kind:
- * out8 = {q8_gemv, q8_gemm tcgen05, q8_gemm SIMT, attention, attention merge,
+ * out8 = {q8_gemv, q8_gemm tcgen05, q8_gemm SIMT, attention, 0,
  * norm/element-wise, synth/quantize, 0}.  Evidence that the CUDA path ran. */
 LOGOS_API logos_status_t logos_launch_counts(int64_t* out8);
 
@@ -393,7 +393,7 @@ LOGOS_API logos_status_t logos_llm_load_weights(logos_handle_t model, const char
  * holds no whole matrix). */
 LOGOS_API logos_status_t logos_llm_save_weights(logos_handle_t model, const char* path);
 /* One greedy step with CUDA events around every launch group; ms_by_class_out
- * receives 4 doubles: Q8 GEMMs, attention (+merge), norms/element-wise, and
+ * receives 4 doubles: Q8 GEMMs, attention, norms/element-wise, and
  * tensor-parallel exchange.  Advances the model like logos_llm_decode_step. */
 LOGOS_API logos_status_t logos_llm_profile_step(logos_handle_t model, double* ms_by_class_out);
 LOGOS_API logos_status_t logos_llm_free(logos_handle_t model);

@@ -3,7 +3,7 @@
 // One step, per layer (all sequences in lock step):
 //   residual add + RMSNorm -> 16-bit x          (one kernel; also folds split-K partials)
 //   Q8 GEMM  x -> [q | k | v]  (f32)
-//   RoPE + KV append + GQA attention           (one kernel + merge) -> 16-bit
+//   RoPE + KV append + GQA attention           (one kernel) -> 16-bit
 //   Q8 GEMM  o_proj  -> f32 partials           [all-reduce when tensor parallel]
 //   residual add + RMSNorm -> 16-bit x
 //   Q8 GEMM  gate/up with the SwiGLU epilogue -> 16-bit

@@ -190,12 +190,6 @@ struct Ring {
 
 __device__ __forceinline__ float silu_f(float g) { return __fdiv_rn(g, 1.0f + expf(-g)); }
 
-__device__ __forceinline__ float load_aux(const TcParams& p, int64_t i) {
-  if (p.c_dtype == LOGOS_F16) return __half2float(reinterpret_cast<const __half*>(p.aux)[i]);
-  if (p.c_dtype == LOGOS_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.aux)[i]);
-  return reinterpret_cast<const float*>(p.aux)[i];
-}
-
 // two int8 (bytes of w ^ 0x80808080, i.e. of q + 128 as unsigned bytes) -> packed fp16 pair, exact
 __device__ __forceinline__ uint32_t cvt_pair(uint32_t w_xor80, uint32_t selector) {
   uint32_t bits = __byte_perm(w_xor80, 0x64646464u, selector);   // 0x64bb = 1024 + (q + 128)
@@ -327,11 +321,12 @@ __device__ __forceinline__ void store_tile(const TcParams& p, const float2* acc,
   } else if (n < p.n) {
     const int64_t at = m0 * p.ldc + n;
     if (p.epilogue == EPI_RESIDUAL) {
-      int64_t i = at;
-      put_rows<HC>(p, at, rows, [&](int x) {
-        const float v = __fadd_rn(sum(x), load_aux(p, i));
-        i += p.ldc;
-        return v;
+      const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(p.aux) + at;   // only bf16 results have a residual
+      __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.c) + at;
+      each_row<HC>(rows, [&](int x) {
+        *d = __float2bfloat16_rn(__fadd_rn(sum(x), __bfloat162float(*r)));
+        r += p.ldc;
+        d += p.ldc;
       });
     } else {
       put_rows<HC>(p, at, rows, [&](int x) { return sum(x); });
@@ -883,6 +878,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   p.stages_total = (int)stages;
   p.s_tiled = s_tiled;
   p.wait_scales = g.s_tiled;
+  if (g.epilogue == EPI_RESIDUAL && g.c_dtype != LOGOS_BF16) return fail(LOGOS_ERROR, "q8_gemm: a residual goes with bf16 results");
   const int64_t mtiles = (g.m + T - 1) / T;
   const int64_t units = (int64_t)(plan.pairs + plan.solos) * plan.splits * mtiles;
   if (units > INT32_MAX / 4 || tiles * stages > INT32_MAX / TC_ROWS) return fail(LOGOS_OUT_OF_BOUNDS, "q8_gemm: too many work units");

@@ -102,8 +102,8 @@ def launchCounts():
     """Kernel launches made through the library so far, by kind."""
     out = (C.c_int64 * 8)()
     call("logos_launch_counts", out)
-    names = ("q8_gemv", "q8_gemm_tc", "q8_gemm_simt", "attention", "attention_merge", "elementwise", "synth")
-    return dict(zip(names, (int(v) for v in out)))
+    names = ("q8_gemv", "q8_gemm_tc", "q8_gemm_simt", "attention", None, "elementwise", "synth")
+    return {name: int(v) for name, v in zip(names, out) if name}
 
 
 def _h(buf):
