@@ -26,8 +26,8 @@
 //   * a small batch is bound by the chain from the predecessor's end to the output: in a decode step
 //     what is older than it (lengths, cached rows) is read, and the work cut, before the wait for
 //     the predecessor (AttnArgs::early_reads); every row of the query and the new K/V is one round of loads; the fold is three.
-// Measured, before -> after these two: 32 sequences of 4096, 28/4 heads of 128: 69.3 -> 62.2 us
-// (6.4 TB/s); seven ragged sequences 18.4 -> 14.3 us; a decode step of the 0.5B shape at batch 16
+// Measured, before -> after these two: 32 sequences of 4096, 28/4 heads of 128: 69.3 -> 62.7 us
+// (4.3 TB/s, launch and ramp included); seven ragged sequences 18.4 -> 14.3 us; a decode step of the 0.5B shape at batch 16
 // 954 -> 887 us (24 layers).
 #include "ops.cuh"
 #include "q8_gemm_tc.cuh"

@@ -37,6 +37,9 @@
 // warps, few and coarse hand-offs, ring positions kept as 32-bit shared addresses, and registers moved
 // from the other warps to the drain warps.
 //
+// Registers are what 96 tokens run out of: the kernel spills 112 to 164 bytes a thread there (`-Xptxas -v`), up to 40
+// elsewhere.
+//
 // HBM roofline: 1.125 bytes per weight (int8 + f32/32); activations and outputs are small next to
 // that at decode batch sizes.  With many tokens the FMA and tensor pipes are the bound.
 #include "q8_gemm_tc.cuh"
@@ -786,9 +789,12 @@ struct TcPlan {
   int t, splits, pairs, solos;
 };
 
-// Cycles of one K stage of a pair and of a single tile, by tokens per tile (timings of this kernel), of the
-// pipeline fill plus the last epilogue, and of a unit's epilogue.  They decide only who computes what: the
-// order of a sum depends on the K splits alone.
+// Cycles of one K stage of a pair and of a single tile, by tokens per tile, of the pipeline fill plus the last
+// epilogue, and of a unit's epilogue.  They decide only who computes what: the order of a sum depends on the K splits
+// alone.  The table was made with an earlier form of this kernel; timed again (calls in a row, by the slope between
+// K = 4096 and 12288, at 1965 MHz, one plane / two): singles 879/861, 879/1051, 1150/1574, 1620/2119, pairs
+// 1967/1917, 1804/2092, 2338/3018, 2914/3676.  From 64 tokens on it stands between what one plane and two cost; whether a table
+// for each makes better choices has not been tried.
 struct TcCost {
   int t, pair, solo;
 };

@@ -52,8 +52,8 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 
 // A warp takes R neighbouring rows (a group); groups go round the CTAs first, so that a small matrix still
 // uses every SM.  The ring runs on from one group to the next.  Measured before (eight loads a lane in flight in
-// registers, four CTAs an SM) -> now: 152064 x 5120 197 -> 148 us (5.9 TB/s), 151936 x 896 72 -> 37 us,
-// 27648 x 5120 43 -> 33 us, 5120 x 27648 154 -> 41 us, 300 x 16384 13.6 -> 8.3 us.  Four rows at a time
+// registers, four CTAs an SM) -> now: 152064 x 5120 197 -> 148 us (5.9 TB/s), 151936 x 896 72 -> 38 us,
+// 27648 x 5120 43 -> 33 us, 5120 x 27648 154 -> 45 us, 300 x 16384 13.6 -> 8.4 us.  Four rows at a time
 // measured 166 us on the first, one row 164 us.
 template <int R, bool X_IN_SMEM>
 __global__ void __launch_bounds__(GEMV_WARPS * 32, 1)
