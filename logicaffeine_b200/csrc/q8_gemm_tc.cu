@@ -37,7 +37,7 @@
 // warps, few and coarse hand-offs, ring positions kept as 32-bit shared addresses, and registers moved
 // from the other warps to the drain warps.
 //
-// Registers are what 96 tokens run out of: the kernel spills 112 to 164 bytes a thread there (`-Xptxas -v`), up to 40
+// Registers are what 96 tokens run out of: the kernel spills 112 to 172 bytes a thread there (`-Xptxas -v`), up to 40
 // elsewhere.
 //
 // HBM roofline: 1.125 bytes per weight (int8 + f32/32); activations and outputs are small next to
