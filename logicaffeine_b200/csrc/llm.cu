@@ -1,6 +1,8 @@
 // Batched Qwen-architecture greedy decode on Q8 weights.
 //
 // One step, per layer (all sequences in lock step):
+// (small models and batches: norm + qkv, attention, o_proj + residual, norm + gate/up + SwiGLU, down_proj + residual, a
+// kernel each, see q8_narrow.cu)
 //   residual add + RMSNorm -> 16-bit x          (one kernel; also folds split-K partials)
 //   Q8 GEMM  x -> [q | k | v]  (f32)
 //   RoPE + KV append + GQA attention           (one kernel) -> 16-bit
@@ -532,6 +534,40 @@ logos_status_t step_tail(Model* m, int parts, bool sample, bool log_tokens, cons
   return LOGOS_OK;
 }
 
+// Whether a layer's products run in the kernels that hold the norms, SwiGLU and the residual adds too (q8_narrow.cu):
+// where they take the shapes, up to 16 sequences (one token tile).  us a step of the 0.5B shape, the kernels of
+// q8_gemm_tc.cu and these: batch 1 904 / 621, 8 905 / 629, 16 900 / 763, 32 1000 / 995.
+bool narrow_layers(const Model* m) {
+  const logos_llm_config_t& c = m->cfg;
+  if (m->tp.degree > 1 || c.batch > 16) return false;
+  const Layer& L = m->layers[0];
+  for (const Q8Mat* w : {&L.wqkv, &L.wo, &L.wgu, &L.wd}) {
+    const bool norm = w == &L.wqkv || w == &L.wgu;
+    if (!w->tiled || !narrow_applicable(c.batch, w->n, w->k, norm, m->device)) return false;
+  }
+  return true;
+}
+
+// h (+= a * w), or c = rmsnorm(h) * w in one of its two forms
+logos_status_t narrow_product(Model* m, const Q8Mat& w, int out, int64_t gain_row, float* c, const ActOut& planes) {
+  ProfScope ps(m, PROF_GEMM);
+  NarrowArgs g;
+  g.q = w.q; g.s = w.s;
+  g.m = m->cfg.batch; g.n = w.n; g.k = w.k;
+  g.out = out;
+  if (out == NARROW_RESIDUAL) {
+    g.a = planes;
+    g.c = m->h;
+  } else {
+    g.h_in = m->h; g.gain = m->gains + gain_row * m->cfg.hidden; g.eps = m->cfg.rms_eps; g.act_mode = m->cfg.act_dtype;
+    g.c = c;
+    g.planes = planes;
+  }
+  g.device = m->device;
+  m->launch_counter += 1;
+  return launch_q8_narrow(g, m->stream);
+}
+
 // One lock-step decode step on the model's stream.  tokens_in: [B] device.
 // prompt_len ([B] device, ragged prompts only) with prompt_step: sequences whose prompt is over
 // (prompt_step >= prompt_len[i]) run through the step without advancing - their K/V row lands at
@@ -545,9 +581,9 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
   m->launch_counter = 0;
   // Every kernel of a step keeps the dependent-launch contract (common.cuh): before it has waited for its
   // predecessor a kernel touches weights only, and the attention the lengths and cached rows too.  What writes those
-  // (the end of the step before, or this step's attention of another layer, another cache) is over when
-  // the attention starts: the norm before the qkv product waits for its predecessor before it lets
-  // anything start, and the predecessor (embedding or down product) is later than they are.
+  // (the end of the step before, or this step's attention of another layer, another cache) is over when the
+  // attention starts: the embedding waits for the end of the step before, before it lets anything start, and no
+  // kernel of a step starts before the embedding has done so.
   PdlScope pdl(pdl_enabled());
   {
     ProfScope ps(m, PROF_ELEMWISE);
@@ -555,12 +591,15 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
   }
   m->launch_counter += 1;
   int parts = 0;
+  const bool narrow = narrow_layers(m);
   for (int64_t l = 0; l < c.layers; ++l) {
     Layer& L = m->layers[(size_t)l];
     int qkv_parts = 1;
-    LOGOS_TRY(norm_step(m, parts, 2 * l));
-    m->launch_counter += 1;
-    {
+    if (narrow) {
+      LOGOS_TRY(narrow_product(m, L.wqkv, NARROW_F32, 2 * l, m->qkv, ActOut()));
+    } else {
+      LOGOS_TRY(norm_step(m, parts, 2 * l));
+      m->launch_counter += 1;
       GemmArgs g;
       g.a = m->xn.hi; g.a_lo = m->xn.lo; g.a_dtype = LOGOS_F16; g.lda = H;
       g.q = L.wqkv.q; g.s = L.wqkv.s; g.q_tiled = L.wqkv.tiled;
@@ -593,6 +632,13 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
       m->launch_counter += 1;
     }
     LOGOS_TRY(debug_check(m, "attention", l));
+    if (narrow) {
+      LOGOS_TRY(narrow_product(m, L.wo, NARROW_RESIDUAL, 0, nullptr, m->att));
+      LOGOS_TRY(narrow_product(m, L.wgu, NARROW_SWIGLU, 2 * l + 1, nullptr, m->ffn));
+      LOGOS_TRY(narrow_product(m, L.wd, NARROW_RESIDUAL, 0, nullptr, m->ffn));
+      LOGOS_TRY(debug_check(m, "narrow products", l));
+      continue;
+    }
     LOGOS_TRY(gemm_partials(m, m->att, L.wo, &parts));
     LOGOS_TRY(debug_check(m, "o_proj gemm", l));
     LOGOS_TRY(norm_step(m, parts, 2 * l + 1));

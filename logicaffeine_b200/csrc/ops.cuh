@@ -70,6 +70,30 @@ int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device);
 // Whether the tcgen05 kernel accepts this call (else the SIMT kernel runs).
 bool gemm_tc_applicable(const GemmArgs& g);
 
+// ---- products of a small model's decode step (q8_narrow.cu): tile-major weights, few tokens, and in the same kernel what
+// comes before or after the product
+enum NarrowOut : int {
+  NARROW_F32 = 0,       // c[m][n] = rmsnorm(h_in) * w
+  NARROW_SWIGLU = 1,    // planes[m][n / 2] = swiglu(rmsnorm(h_in) * w), rows (2j, 2j + 1) = (gate_j, up_j)
+  NARROW_RESIDUAL = 2,  // c[m][n] += a * w
+};
+struct NarrowArgs {
+  const int8_t* q = nullptr;   // tile-major (launch_q8_retile)
+  const float*  s = nullptr;
+  int64_t       m = 0, n = 0, k = 0;
+  const float*  h_in = nullptr;   // [m][k] f32 (the norm forms)
+  const float*  gain = nullptr;   // [k]
+  float         eps = 0.f;
+  int           act_mode = LOGOS_F32;   // how normalised rows are rounded (see ActOut)
+  ActOut        a;                // planes [m][k] (NARROW_RESIDUAL)
+  int           out = NARROW_F32;
+  float*        c = nullptr;
+  ActOut        planes;
+  int           device = 0;
+};
+logos_status_t launch_q8_narrow(const NarrowArgs& a, cudaStream_t st);
+bool narrow_applicable(int64_t m, int64_t n, int64_t k, bool norm, int device);
+
 // ---- attention (attention.cu)
 // The attention kernel's arrival counters, whatever the call's extents: one per CTA of its persistent grid and one more
 constexpr int64_t ATT_COUNTER_BYTES = 4096;
