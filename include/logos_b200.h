@@ -184,9 +184,8 @@ LOGOS_API logos_status_t logos_q8_gemv(logos_handle_t q /*i8 [N][K]*/, logos_han
  * epilogue 0: plain.  1: C = bf16(acc + aux[m,n]) with aux bf16 [M][N] (residual).
  * 2: rows of q interleave gate (even) and up (odd); C is [M][N/2] =
  *    bf16( silu(acc_gate) * acc_up ).
- * The stand-alone operators logos_q8_gemm, logos_q8_gemm_f32 and logos_gqa_decode_attn(_fused)
- * keep activation planes, split-K and split-KV partials in one library-owned scratch block per
- * device, grown on demand and shared by every caller on that device: calls that use it must
+ * The stand-alone operators logos_q8_gemm and logos_q8_gemm_f32 keep activation planes and
+ * split-K partials in one library-owned scratch block per device (logos_gqa_decode_attn_fused its arrival counter in another), grown on demand and shared by every caller on that device: calls that use it must
  * be ordered on the GPU (one stream, or events).  A model (logos_llm_*) owns its own. */
 LOGOS_API logos_status_t logos_q8_gemm(logos_handle_t a /*bf16 [M][K]*/, logos_handle_t q, logos_handle_t s,
                              logos_handle_t c /*bf16*/, int64_t m, int64_t n, int64_t k,
@@ -232,24 +231,18 @@ LOGOS_API logos_status_t logos_gqa_decode_attn(logos_handle_t q, logos_handle_t 
  * call an operator: a serving process that hands the whole GPU to its own KV-cache and
  * weight arena at start-up (a later cudaMalloc from inside the library would fail or
  * fragment that arena), or a decode loop with a latency budget that an allocation's
- * device-wide synchronisation would break.  The partial results of (sequence, KV head) pairs
- * that the kernel's persistent grid cuts go to a fixed 6 MiB array inside the library image
- * instead of library-allocated scratch, so every GPU that loads the library holds those 6 MiB
- * until the process exits.  What the kernel needs depends on the GPU, not on the shape: two
- * slots of 16 * (d + 2) floats per CTA, two CTAs per SM (4.7 MiB on a
- * 148-SM B200 at d = 128), and 4 KiB of counters;
- * a GPU with so many SMs that this exceeds the array is refused with LOGOS_OUT_OF_BOUNDS and
- * a message giving both sizes, and so is a call with more than 2048 sequences (the limit of
- * both attention entry points: a CTA keeps the lengths in shared memory).
+ * device-wide synchronisation would break.  The kernel keeps nothing in global memory
+ * besides its result: the parts of a long sequence meet in the shared memories of a
+ * thread-block cluster.  What the two entry points differ in is the status word: this one's
+ * lies inside the library image.  A call with more than 2048 sequences is refused with
+ * LOGOS_OUT_OF_BOUNDS (the limit of both attention entry points).
  * The call itself makes no
- * cudaMalloc / cudaFree.  The first call on a device looks up the array's device address;
- * make that first call outside any stream capture.  All calls share the one array and one
- * status word.  Nothing is cleared between calls: the partials are always written before
- * they are read, the counters return to zero, and the status word is zero until a bounded wait inside the kernel gives up,
+ * cudaMalloc / cudaFree.  The first call on a device looks up the word's device address;
+ * make that first call outside any stream capture.  All calls share the one
+ * status word, which is zero until a bounded wait inside the kernel gives up,
  * after which calls on this entry point leave `o` untouched until logos_kernel_status has
  * reported and cleared the code (call logos_kernel_status once at start-up if it must not
- * allocate later).  Two calls that overlap on the GPU race on the array: keep calls on this
- * entry point ordered, for instance on one stream. */
+ * allocate later). */
 LOGOS_API logos_status_t logos_gqa_decode_attn_fixed_scratch(logos_handle_t q, logos_handle_t k_cache,
                                      logos_handle_t v_cache, logos_handle_t seq_len, logos_handle_t o,
                                      int64_t b, int64_t h_q, int64_t h_kv, int64_t d, int64_t l_max,

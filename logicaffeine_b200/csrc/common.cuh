@@ -79,7 +79,7 @@ logos_status_t buf_ptr(logos_handle_t h, int64_t elems, const char* name, T** ou
 }
 
 // Per-device scratch the library owns, for the stand-alone operators (activation planes and
-// split-K partials of logos_q8_gemm*, split-KV partials of logos_gqa_decode_attn*).  One block
+// split-K partials of logos_q8_gemm*).  One block
 // per (device, slot), shared by every caller on that device: calls that use it must be ordered
 // on the GPU (one stream, or the caller's own events).  Grows on demand, outside any stream
 // capture; outgrown blocks are kept until the process exits.  A model never uses it: what a
@@ -89,13 +89,10 @@ logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out);
 // captured, or there is no memory left for it.
 bool scratch_try(int32_t device, int slot, int64_t bytes, cudaStream_t st, void** out);
 
-// Arrival counters of the stand-alone attention calls, one block per device (every call asks for the same size), zeroed
-// when it is allocated; the kernels leave them at zero.  Ordered like scratch_get's blocks.
+// Arrival counters of the attention calls that advance the lengths, one block per device (every call asks for the same
+// size), zeroed when it is allocated; the kernels leave them at zero.  Ordered like scratch_get's blocks.
 logos_status_t counters_get(int32_t device, int64_t bytes, void** out);
-// Counters that someone else owns (a model): a kernel that gave up leaves them in the middle of a count, so
-// counters_reset zeroes all of a device's once such a failure has been read.
-void counters_register(int32_t device, void* ptr, int64_t bytes);
-void counters_unregister(void* ptr);
+// A kernel that gave up may leave them in the middle of a count: zeroes them once such a failure has been read.
 logos_status_t counters_reset(int32_t device);
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize of `kernel` on the current device, raised to `bytes` once instead of

@@ -84,9 +84,6 @@ struct Model {
   float* partials = nullptr; // [max_splits][B][H]
   float* dpart = nullptr;    // split-K partials of the GEMMs with a direct output (qkv, gate/up)
   int64_t dpart_floats = 0;
-  void*  attn_scratch = nullptr;  // split-KV partials of the attention kernel: owned here, so the captured step
-  int64_t attn_scratch_bytes = 0; // never points at the library's shared scratch
-  void*  attn_arrive = nullptr;   // its arrival counters
   // tensor parallelism with peer-addressable memory: partials, xn planes and flag words live in
   // one block per rank that every rank maps; the all-reduce is folded into residual + RMSNorm
   TpSymm symm;
@@ -170,7 +167,6 @@ void destroy(Model* m) {
   m->step_graph = nullptr;
   tp_symm_free(&m->symm);
   tp_destroy(&m->tp);
-  if (m->attn_arrive) counters_unregister(m->attn_arrive);
   for (void* p : m->allocs) cudaFree(p);
   if (m->pf.block) cudaFree(m->pf.block);
   if (m->prompt) cudaFree(m->prompt);
@@ -357,15 +353,6 @@ logos_status_t build(Model* m, const void* nccl_id) {
     const int64_t need_gu = s_gu > 1 ? (int64_t)s_gu * B * 2 * m->f_local : 0;
     m->dpart_floats = need_qkv > need_gu ? need_qkv : need_gu;
     if (m->dpart_floats > 0) LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->dpart), m->dpart_floats * 4));
-  }
-  {
-    AttnArgs a;
-    a.b = B; a.h_q = m->hq_local; a.h_kv = m->hkv_local; a.d = D; a.l_max = c.l_max; a.device = m->device;
-    m->attn_scratch_bytes = attn_scratch_bytes(a);
-    LOGOS_TRY(dmalloc(m, &m->attn_scratch, m->attn_scratch_bytes));
-    LOGOS_TRY(dmalloc(m, &m->attn_arrive, ATT_COUNTER_BYTES));
-    LOGOS_CUDA_TRY(cudaMemsetAsync(m->attn_arrive, 0, ATT_COUNTER_BYTES, m->stream));
-    counters_register(m->device, m->attn_arrive, ATT_COUNTER_BYTES);
   }
   LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->logits), B * c.vocab * 4));
   m->history_cap = c.l_max;
@@ -626,8 +613,6 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
       a.b = B; a.h_q = m->hq_local; a.h_kv = m->hkv_local; a.d = D; a.l_max = c.l_max;
       a.scale = 1.0f / sqrtf((float)D);
       a.device = m->device;
-      a.ext_scratch = m->attn_scratch; a.ext_scratch_bytes = m->attn_scratch_bytes;
-      a.ext_arrive = m->attn_arrive;
       LOGOS_TRY(launch_gqa_decode_attn(a, st));
       m->launch_counter += 1;
     }

@@ -95,8 +95,8 @@ logos_status_t launch_q8_narrow(const NarrowArgs& a, cudaStream_t st);
 bool narrow_applicable(int64_t m, int64_t n, int64_t k, bool norm, int device);
 
 // ---- attention (attention.cu)
-// The attention kernel's arrival counters, whatever the call's extents: one per CTA of its persistent grid and one more
-constexpr int64_t ATT_COUNTER_BYTES = 4096;
+// The attention kernel's arrival counter (calls that advance the lengths)
+constexpr int64_t ATT_COUNTER_BYTES = 256;
 struct AttnArgs {
   // query: either f16 [B][Hq][D] (q_f16) or f32 rows inside a wider matrix
   // (q_f32, row stride q_ld floats per sequence, head h at column h*D).
@@ -131,13 +131,7 @@ struct AttnArgs {
   int64_t       b = 0, h_q = 0, h_kv = 0, d = 0, l_max = 0;
   float         scale = 1.f;
   int           device = 0;
-  // Caller-provided scratch for the split-KV partials and the status word (both device
-  // addresses).  Null = the library's own per-device scratch, allocated on first use and shared
-  // by every stand-alone call on the device (a model passes its own: a captured step must not
-  // point at memory another caller can outgrow).
-  void*         ext_scratch = nullptr;
-  int64_t       ext_scratch_bytes = 0;
-  void*         ext_arrive = nullptr;      // with ext_scratch: ATT_COUNTER_BYTES of counters, zero before the first call
+  // Caller-provided status word (device address).  Null = the per-device one.
   int*          ext_status = nullptr;
   // Lengths and cached rows may be read before the previous kernel of the stream has completed.  Only for a caller
   // that knows every kernel which writes them to be over by then, as a decode step does; in a scope of the
@@ -145,9 +139,6 @@ struct AttnArgs {
   bool          early_reads = false;
 };
 logos_status_t launch_gqa_decode_attn(const AttnArgs& a, cudaStream_t st);
-// Bytes of split-KV scratch a call with these extents (b, h_q, h_kv, d, l_max, device) needs:
-// what a caller that passes ext_scratch has to provide (the counters come on top).
-int64_t attn_scratch_bytes(const AttnArgs& a);
 logos_status_t launch_kv_append_rope(__half* k_cache, __half* v_cache, const __half* k_new, const __half* v_new,
                                      const float* rope, int32_t* seq_len, int64_t b, int64_t h_kv, int64_t d,
                                      int64_t l_max, int device, cudaStream_t st);

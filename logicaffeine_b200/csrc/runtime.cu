@@ -181,7 +181,6 @@ struct Counters {
   int32_t device;
   void*   ptr;
   int64_t bytes;
-  bool    own;     // the library's block of the device
 };
 std::mutex g_counters_mu;
 std::vector<Counters> g_counters;
@@ -190,7 +189,7 @@ std::vector<Counters> g_counters;
 logos_status_t counters_get(int32_t device, int64_t bytes, void** out) {
   std::lock_guard<std::mutex> lk(g_counters_mu);
   for (const Counters& c : g_counters)
-    if (c.own && c.device == device) {
+    if (c.device == device) {
       *out = c.ptr;
       return LOGOS_OK;
     }
@@ -203,21 +202,9 @@ logos_status_t counters_get(int32_t device, int64_t bytes, void** out) {
     return cuda_fail(e, "cudaMemset (arrival counters)");
   }
   LOGOS_CUDA_TRY(cudaDeviceSynchronize());        // zero before a launch on any stream
-  g_counters.push_back({device, p, bytes, true});
+  g_counters.push_back({device, p, bytes});
   *out = p;
   return LOGOS_OK;
-}
-void counters_register(int32_t device, void* ptr, int64_t bytes) {
-  std::lock_guard<std::mutex> lk(g_counters_mu);
-  g_counters.push_back({device, ptr, bytes, false});
-}
-void counters_unregister(void* ptr) {
-  std::lock_guard<std::mutex> lk(g_counters_mu);
-  for (size_t i = 0; i < g_counters.size(); ++i)
-    if (g_counters[i].ptr == ptr) {
-      g_counters.erase(g_counters.begin() + (long)i);
-      return;
-    }
 }
 logos_status_t counters_reset(int32_t device) {
   std::lock_guard<std::mutex> lk(g_counters_mu);

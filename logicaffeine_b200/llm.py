@@ -172,8 +172,8 @@ def gqaDecodeAttn(q, k_cache, v_cache, seq_len, o, b, h_q, h_kv, d, l_max, softm
 
 
 def gqaDecodeAttnFixedScratch(q, k_cache, v_cache, seq_len, o, b, h_q, h_kv, d, l_max, softmax_scale, stream=None):
-    """gqaDecodeAttn for hosts that cannot let an operator allocate device memory: the split-KV partials use a
-    fixed 6 MiB array inside the library; larger shapes raise LogosError (OutOfBounds)."""
+    """gqaDecodeAttn for hosts that cannot let an operator allocate device memory: the kernel
+    keeps nothing in global memory, and the entry point's status word lies in the library image."""
     call("logos_gqa_decode_attn_fixed_scratch", q.handle, k_cache.handle, v_cache.handle, seq_len.handle, o.handle,
          int(b), int(h_q), int(h_kv), int(d), int(l_max), float(softmax_scale), _s(stream))
 

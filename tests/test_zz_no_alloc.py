@@ -3,10 +3,10 @@
 Some hosts cannot afford a device allocation inside an operator call: a server that gave
 the whole GPU to its own arena at start-up, or a decode loop whose latency budget has no
 room for the device-wide synchronisation an allocation implies.  For them
-logos_gqa_decode_attn_fixed_scratch keeps the partial results of the (sequence, KV head)
-pairs its persistent grid cuts in a fixed 6 MiB array inside the library.  It runs the same kernels as logos_gqa_decode_attn, so on the
-same inputs the two must agree bit for bit, call after call (the array keeps the previous
-call's contents), and a call beyond the stated maximum must be refused, not truncated.
+logos_gqa_decode_attn_fixed_scratch keeps its status word inside the library image and
+nothing else in global memory.  It runs the same kernels as logos_gqa_decode_attn, so on the
+same inputs the two must agree bit for bit, call after call, and a call beyond the stated
+maximum must be refused, not truncated.
 
 This file sorts last on purpose: if it fails under `pytest -x`, every other test has
 already run."""
@@ -25,7 +25,7 @@ def _inputs(O, b, hq, hkv, d, lmax, lens, seed):
 
 def test_fixed_scratch_attention_matches_the_allocating_entry_point_twice(llm, oracle):
     O = oracle
-    # two different shapes back to back: the second call finds the first call's partials in the array
+    # two different shapes back to back
     cases = [(4, 28, 4, 128, 700, [1, 64, 65, 699], 3), (3, 14, 2, 64, 300, [299, 130, 7], 4)]
     for b, hq, hkv, d, lmax, lens, seed in cases:
         q, kc, vc, seq = _inputs(O, b, hq, hkv, d, lmax, lens, seed)
@@ -59,7 +59,7 @@ def test_fixed_scratch_attention_matches_the_allocating_entry_point_twice(llm, o
 
 
 def test_fixed_scratch_refuses_what_does_not_fit(llm):
-    # the most sequences one call takes is 2048 (a CTA keeps one tile count per sequence in shared memory)
+    # the most sequences one call takes is 2048 (as it always was)
     b, hq, hkv, d, lmax = 2049, 2, 1, 64, 64
     q = llm.DeviceBuffer(b * hq * d * 2)
     cache = llm.DeviceBuffer(b * hkv * lmax * d * 2)
