@@ -670,11 +670,17 @@ logos_status_t launch_attn_t(const AttnArgs& a, cudaStream_t st) {
   if (!p.status) return fail(LOGOS_ERROR, "attention: no kernel status word");
 
   auto kernel = gqa_decode_attn_kernel<D>;
-  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), a.device, AttnSmem<D>::BYTES));
+  // Where there are SMs for all, a CTA asks for more than half of one's shared memory: a cluster's CTAs are packed onto an SM
+  // otherwise (three of head dimension 64 fit one).  A step of the 0.5B shape, batch 16 at 128 positions (96 CTAs) 748 -> 685 us,
+  // batch 8 591 -> 553; with more CTAs than SMs it only keeps them and the neighbouring kernels' CTAs apart: batch 16 at 1500
+  // positions (256 CTAs) 769 -> 963.
+  const int64_t ctas = a.b * a.h_kv * p.ranks;
+  const int smem = std::max(AttnSmem<D>::BYTES, ctas <= sm_count(a.device) ? 115 * 1024 : 0);
+  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), a.device, smem));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(a.b * a.h_kv * p.ranks));
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = AttnSmem<D>::BYTES;
+  cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
