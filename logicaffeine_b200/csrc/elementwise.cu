@@ -83,15 +83,18 @@ __global__ void embed_kernel(const int32_t* __restrict__ tokens, const int8_t* _
 // One CTA per row, 128-bit accesses: fold the split-K partials into the residual
 // stream in ascending order, keep the updated row on chip, reduce the sum of squares,
 // then write the normalised row as activation planes.  Rows of up to 8192 floats stay in
-// registers (IN_REGS): the kernel then uses no dynamic shared memory, so under a dependent
+// registers (PER float4 a thread): the kernel then uses no dynamic shared memory, so under a dependent
 // launch the next GEMM's CTAs, which take nearly a whole SM's shared memory, can start beside
-// it and fetch their first weights while the norm finishes.  Longer rows go through shared memory.
-template <bool IN_REGS>
+// it and fetch their first weights while the norm finishes.  Longer rows go through shared memory (PER = 0).
+// Memory-bound with many rows: a row of up to 2048 floats gets a CTA of just its threads, and the planes are written
+// eight bytes at a time (1088 rows of 896: 9.7 -> 5.6 us under ncu; four steps of eight layers of the 32B shape at batch 64
+// 11.71 -> 11.31 ms).
+template <int PER>
 __global__ void __launch_bounds__(512)
 residual_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ delta, int parts, int64_t part_stride,
                         const float* __restrict__ g, ActOut xn, int64_t hidden, float eps) {
   __shared__ float red[32];
-  extern __shared__ float4 row_cache4[];  // hidden floats (not IN_REGS)
+  extern __shared__ float4 row_cache4[];  // hidden floats (PER = 0)
   float* row_cache = reinterpret_cast<float*>(row_cache4);
   // h and the partials come from kernels of the same step: wait for them, and read them past L1
   pdl_wait();
@@ -99,14 +102,13 @@ residual_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ delta, 
   const int64_t row = blockIdx.x;
   float* hr = h + row * hidden;
   float ss = 0.f;
-  if (IN_REGS) {
-    constexpr int PER = 4;   // float4 per thread: 512 threads x 4 x 4 floats = 8192
-    const int64_t n4 = hidden >> 2;
+  if constexpr (PER > 0) {
+    const int n4 = (int)(hidden >> 2), step = blockDim.x;
     float4* hr4 = reinterpret_cast<float4*>(hr);
     float4 v[PER];
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-      const int64_t i = threadIdx.x + (int64_t)u * 512;
+      const int i = threadIdx.x + u * step;
       v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (i < n4) {
         v[u] = __ldcg(hr4 + i);
@@ -118,7 +120,7 @@ residual_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ delta, 
         if (parts > 0) hr4[i] = v[u];
       }
     }
-    // the same order of additions as the strided loop over the row: element i of thread t is t + 512 u
+    // the same order of additions as the strided loop over the row: element i of thread t is t + u * threads
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       ss = fmaf(v[u].x, v[u].x, ss); ss = fmaf(v[u].y, v[u].y, ss);
@@ -129,14 +131,11 @@ residual_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ delta, 
     const float4* g4 = reinterpret_cast<const float4*>(g);
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-      const int64_t i = threadIdx.x + (int64_t)u * 512;
+      const int i = threadIdx.x + u * step;
       if (i < n4) {
         const float4 gg = g4[i];
-        const int64_t e = row * hidden + 4 * i;
-        act_store(xn, e + 0, __fmul_rn(__fmul_rn(v[u].x, inv), gg.x));
-        act_store(xn, e + 1, __fmul_rn(__fmul_rn(v[u].y, inv), gg.y));
-        act_store(xn, e + 2, __fmul_rn(__fmul_rn(v[u].z, inv), gg.z));
-        act_store(xn, e + 3, __fmul_rn(__fmul_rn(v[u].w, inv), gg.w));
+        act_store4(xn, row * hidden + 4 * i, make_float4(__fmul_rn(__fmul_rn(v[u].x, inv), gg.x), __fmul_rn(__fmul_rn(v[u].y, inv), gg.y),
+                                                         __fmul_rn(__fmul_rn(v[u].z, inv), gg.z), __fmul_rn(__fmul_rn(v[u].w, inv), gg.w)));
       }
     }
     return;
@@ -622,13 +621,15 @@ logos_status_t launch_residual_rmsnorm(float* h, const float* delta, int parts, 
                                        cudaStream_t st) {
   if (rows == 0) return LOGOS_OK;
   if ((hidden & 3) == 0 && hidden <= 8192) {
-    LOGOS_CUDA_TRY(launch_kernel(residual_rmsnorm_kernel<true>, dim3((unsigned)rows), dim3(512), 0, st, h, delta, parts,
-                                 part_stride, g, xn, hidden, eps));
+    const bool one = hidden <= 2048;
+    const unsigned threads = one ? (unsigned)((hidden / 4 + 31) / 32 * 32) : 512u;
+    LOGOS_CUDA_TRY(launch_kernel(one ? residual_rmsnorm_kernel<1> : residual_rmsnorm_kernel<4>, dim3((unsigned)rows), dim3(threads), 0, st, h,
+                                 delta, parts, part_stride, g, xn, hidden, eps));
   } else {
     size_t smem = sizeof(float) * (size_t)hidden;
     if (smem > 48 * 1024)
-      LOGOS_CUDA_TRY(cudaFuncSetAttribute(residual_rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    LOGOS_CUDA_TRY(launch_kernel(residual_rmsnorm_kernel<false>, dim3((unsigned)rows), dim3(512), smem, st, h, delta, parts,
+      LOGOS_CUDA_TRY(cudaFuncSetAttribute(residual_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LOGOS_CUDA_TRY(launch_kernel(residual_rmsnorm_kernel<0>, dim3((unsigned)rows), dim3(512), smem, st, h, delta, parts,
                                  part_stride, g, xn, hidden, eps));
   }
   count_launch(LK_ELEMWISE);
