@@ -102,11 +102,14 @@ __device__ __forceinline__ void push8(uint32_t addr, float2 v, uint32_t bar) {
 }
 
 // Grid: x = unit groups x CTAs along K (a cluster), y = token tiles; a warp for every 64 columns.
+// Up to four tokens (TOK = 4) both planes of them are the eight columns of one MMA, hi 0 to 3 and lo 4 to 7: half the MMAs (a
+// step of the 0.5B shape at batch 1 498 -> 474 us).
 template <int TOK, int OUT>
 __global__ void __launch_bounds__(NW_THREADS)
 q8_narrow_kernel(const NarrowParams p) {
   constexpr bool NORM = OUT != NARROW_RESIDUAL;
-  constexpr int NT = TOK / 8;                                   // MMA columns
+  constexpr bool MERGED = TOK == 4;
+  constexpr int NT = MERGED ? 1 : TOK / 8;                      // MMAs side by side, of eight columns
   constexpr int PAIRS = NW_UNIT / 2 * TOK;                      // of a unit: two neighbouring output columns for a token
   constexpr int UNIT_PIECES = NW_WARPS * NW_PIECE;
   constexpr int COLS = 18;                                      // floats between the tokens of a warp's sums
@@ -163,7 +166,7 @@ q8_narrow_kernel(const NarrowParams p) {
     float4 v[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      const int t = g + 8 * j;
+      const int t = MERGED ? g & 3 : g + 8 * j;
       const float* src = p.h_in + (int64_t)(m0 + t) * p.k + col + t4 * 8;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -181,7 +184,7 @@ q8_narrow_kernel(const NarrowParams p) {
       float t = ss.x + ss.y;
       t += __shfl_xor_sync(0xffffffffu, t, 1);
       t += __shfl_xor_sync(0xffffffffu, t, 2);
-      if (t4 == 0) s_ss[warp][g + 8 * j] = t;
+      if (t4 == 0 && g + 8 * j < TOK) s_ss[warp][g + 8 * j] = t;
     }
     __syncthreads();
     float ss[NW_WARPS];
@@ -194,7 +197,7 @@ q8_narrow_kernel(const NarrowParams p) {
     const float inv_all = inv_sqrt(__fadd_rn(__fmul_rn(ss[0], p.inv_k), p.eps));   // of token `lane`
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      const float i1 = __shfl_sync(0xffffffffu, inv_all, g + 8 * j);
+      const float i1 = __shfl_sync(0xffffffffu, inv_all, MERGED ? g & 3 : g + 8 * j);
       const float2 inv = make_float2(i1, i1);
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
@@ -211,16 +214,22 @@ q8_narrow_kernel(const NarrowParams p) {
         plane_words(n[1], &bh[b][j].y, &bl[b][j].y);
         plane_words(n[2], &bh[b][j].z, &bl[b][j].z);
         plane_words(n[3], &bh[b][j].w, &bl[b][j].w);
+        if (MERGED && g >= 4) bh[b][j] = two ? bl[b][j] : make_uint4(0u, 0u, 0u, 0u);
       }
     }
   } else {
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      const int t = g + 8 * j;
+      const int t = MERGED ? g & 3 : g + 8 * j;
       const int64_t at = (int64_t)(m0 + t) * p.k + col + t4 * 8;
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
+        if (MERGED) {
+          const __half* plane = g < 4 ? p.a_hi : p.a_lo;
+          bh[b][j] = active && t < rows && plane ? __ldcg(reinterpret_cast<const uint4*>(plane + at + b * 32)) : zero;
+          continue;
+        }
         bh[b][j] = active && t < rows ? __ldcg(reinterpret_cast<const uint4*>(p.a_hi + at + b * 32)) : zero;
         bl[b][j] = active && t < rows && two ? __ldcg(reinterpret_cast<const uint4*>(p.a_lo + at + b * 32)) : zero;
       }
@@ -264,7 +273,7 @@ q8_narrow_kernel(const NarrowParams p) {
           for (int j = 0; j < NT; ++j) f(b, j);
       };
       each([&](int b, int j) { d[b][j][0] = d[b][j][1] = d[b][j][2] = d[b][j][3] = 0.f; });
-      if (two) {
+      if (two && !MERGED) {
         each([&](int b, int j) { mma_f16_16816(d[b][j], a[b][0], bl[b][j].x, bl[b][j].y); });
         each([&](int b, int j) { mma_f16_16816(d[b][j], a[b][1], bl[b][j].z, bl[b][j].w); });
         each([&](int b, int j) {
@@ -281,7 +290,9 @@ q8_narrow_kernel(const NarrowParams p) {
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
           const float* sc = x < 2 ? sc0 : sc1;
-          sums[(8 * j + 2 * t4 + (x & 1)) * COLS + g + (x < 2 ? 0 : 8)] = fmaf(sc[1], d[1][j][x], __fmul_rn(sc[0], d[0][j][x]));
+          float v = fmaf(sc[1], d[1][j][x], __fmul_rn(sc[0], d[0][j][x]));
+          if (MERGED) v = fmaf(__shfl_xor_sync(0xffffffffu, v, 2), 4.8828125e-4f, v);   // hi + lo * 2^-11
+          if (!MERGED || t4 < 2) sums[(8 * j + 2 * t4 + (x & 1)) * COLS + g + (x < 2 ? 0 : 8)] = v;
         }
     }
   } else {   // a warp without columns: zeros
@@ -341,7 +352,7 @@ struct NarrowPlan {
 
 NarrowPlan narrow_plan(int64_t m, int64_t n, int64_t k, int sms) {
   NarrowPlan pl;
-  pl.tok = m <= 8 ? 8 : 16;
+  pl.tok = m <= 4 ? 4 : m <= 8 ? 8 : 16;
   const int64_t slices = k / 64, units = (n + NW_UNIT - 1) / NW_UNIT, chunks = (m + pl.tok - 1) / pl.tok;
   pl.ranks = (int)((slices + NW_WARPS - 1) / NW_WARPS);
   const int64_t most = std::max<int64_t>(1, sms / (pl.ranks * chunks));   // groups that run at once
@@ -389,6 +400,15 @@ logos_status_t launch_t(const NarrowArgs& a, const NarrowPlan& pl, cudaStream_t 
   return check_launch("q8_narrow_kernel");
 }
 
+template <int TOK>
+logos_status_t launch_tok(const NarrowArgs& a, const NarrowPlan& pl, cudaStream_t st) {
+  switch (a.out) {
+    case NARROW_F32: return launch_t<TOK, NARROW_F32>(a, pl, st);
+    case NARROW_SWIGLU: return launch_t<TOK, NARROW_SWIGLU>(a, pl, st);
+    default: return launch_t<TOK, NARROW_RESIDUAL>(a, pl, st);
+  }
+}
+
 }  // namespace
 
 bool narrow_applicable(int64_t m, int64_t n, int64_t k, bool norm, int device) {
@@ -401,9 +421,11 @@ logos_status_t launch_q8_narrow(const NarrowArgs& a, cudaStream_t st) {
   const bool norm = a.out != NARROW_RESIDUAL;
   if (!narrow_applicable(a.m, a.n, a.k, norm, a.device)) return fail(LOGOS_ERROR, "q8_narrow: extents out of its range");
   const NarrowPlan pl = narrow_plan(a.m, a.n, a.k, sm_count(a.device));
-  if (a.out == NARROW_F32) return pl.tok == 8 ? launch_t<8, NARROW_F32>(a, pl, st) : launch_t<16, NARROW_F32>(a, pl, st);
-  if (a.out == NARROW_SWIGLU) return pl.tok == 8 ? launch_t<8, NARROW_SWIGLU>(a, pl, st) : launch_t<16, NARROW_SWIGLU>(a, pl, st);
-  return pl.tok == 8 ? launch_t<8, NARROW_RESIDUAL>(a, pl, st) : launch_t<16, NARROW_RESIDUAL>(a, pl, st);
+  switch (pl.tok) {
+    case 4: return launch_tok<4>(a, pl, st);
+    case 8: return launch_tok<8>(a, pl, st);
+    default: return launch_tok<16>(a, pl, st);
+  }
 }
 
 }  // namespace logos

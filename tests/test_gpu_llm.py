@@ -61,11 +61,11 @@ def test_untied_head_and_head_dim_128(llm, oracle):
 
 
 # Layers whose products hold the norms, SwiGLU and the residual adds: two to sixteen warps along K, one to eight CTAs along it
-# (more than 1024 columns), units of 16 rows that do not fill the last CTA, batches around a token tile; the last two
+# (more than 1024 columns), units of 16 rows that do not fill the last CTA, batches around the token tiles of 4, 8 and 16; the last two
 # rows are just outside (hidden 1152, 17 sequences).  Bounds as in the test above: f32 sums in another order.
 @pytest.mark.parametrize("hidden,ffn,h_q,h_kv,head_dim,batch", [
     (128, 128, 2, 1, 64, 1), (256, 1152, 4, 2, 64, 8), (896, 8192, 14, 2, 64, 9), (1024, 2176, 8, 1, 128, 16),
-    (640, 4992, 7, 1, 128, 2), (1152, 1024, 4, 2, 64, 3), (256, 512, 4, 2, 64, 17)])
+    (640, 4992, 7, 1, 128, 2), (512, 640, 4, 2, 64, 4), (384, 256, 3, 3, 128, 5), (1152, 1024, 4, 2, 64, 3), (256, 512, 4, 2, 64, 17)])
 def test_layers_of_any_width_and_batch(llm, oracle, hidden, ffn, h_q, h_kv, head_dim, batch):
     O = oracle
     cfg = dict(SMALL, layers=2, hidden=hidden, ffn=ffn, h_q=h_q, h_kv=h_kv, head_dim=head_dim, batch=batch, vocab=512, l_max=32)
