@@ -104,7 +104,10 @@ int sm_count(int device);
 // Per-device status word in device memory: kernels store a non-zero code when
 // a bounded wait gives up.  0 = fine.
 int* kernel_status_ptr(int device);
+constexpr int KERNEL_STATUS_WORDS = 8;
 logos_status_t kernel_status_read(int device, int* out, bool clear);
+// the same for words that the caller has copied to the host already
+logos_status_t kernel_status_judge(int device, const int (&words)[KERNEL_STATUS_WORDS], int* out, bool clear);
 
 // ---------------------------------------------------------------- launch helpers
 logos_status_t check_launch(const char* kernel);

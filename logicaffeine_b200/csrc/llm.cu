@@ -103,6 +103,12 @@ struct Model {
   int64_t eager_sample_steps = 0;
   int32_t* prompt = nullptr;  // what a prompt pass indexes by (see prefill_chunked), or [T][B] tokens of the token-by-token pass
   int64_t  prompt_cap = 0;
+  // pinned: the status words, then the tokens of a decode_steps call where they fit.  Both come back before the call's one
+  // wait; a pageable destination and a status read of its own are a wait each.  Null: not to be had, done without.
+  struct Readback {
+    int status[KERNEL_STATUS_WORDS];
+    int32_t tokens[1024];
+  }* readback = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0.0;
   int64_t launches_per_step = 0;
@@ -171,6 +177,7 @@ void destroy(Model* m) {
   if (m->pf.block) cudaFree(m->pf.block);
   if (m->prompt) cudaFree(m->prompt);
   for (cudaEvent_t e : m->prof_events) cudaEventDestroy(e);
+  if (m->readback) cudaFreeHost(m->readback);
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
   if (m->stream) cudaStreamDestroy(m->stream);
@@ -245,6 +252,10 @@ logos_status_t build(Model* m, const void* nccl_id) {
   LOGOS_CUDA_TRY(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
   LOGOS_CUDA_TRY(cudaEventCreate(&m->ev0));
   LOGOS_CUDA_TRY(cudaEventCreate(&m->ev1));
+  if (cudaMallocHost(reinterpret_cast<void**>(&m->readback), sizeof(*m->readback)) != cudaSuccess) {
+    cudaGetLastError();
+    m->readback = nullptr;
+  }
   LOGOS_TRY(tp_init(&m->tp, g, r, nccl_id));
 
   m->layers.resize((size_t)c.layers);
@@ -1321,14 +1332,20 @@ logos_status_t logos_llm_decode_steps(logos_handle_t model, int64_t steps, int32
       }
     }
     LOGOS_CUDA_TRY(cudaEventRecord(m->ev1, m->stream));
+    Model::Readback* const back = m->readback;
+    const bool small = back && steps * B <= (int64_t)(sizeof(back->tokens) / 4);
     if (tokens_host_or_null)
-      LOGOS_CUDA_TRY(cudaMemcpyAsync(tokens_host_or_null, m->history, (size_t)(steps * B) * 4, cudaMemcpyDeviceToHost, m->stream));
+      LOGOS_CUDA_TRY(cudaMemcpyAsync(small ? back->tokens : tokens_host_or_null, m->history, (size_t)(steps * B) * 4, cudaMemcpyDeviceToHost, m->stream));
+    const int* status = back ? kernel_status_ptr(m->device) : nullptr;
+    if (status) LOGOS_CUDA_TRY(cudaMemcpyAsync(back->status, status, sizeof(back->status), cudaMemcpyDeviceToHost, m->stream));
     LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
+    if (tokens_host_or_null && small) memcpy(tokens_host_or_null, back->tokens, (size_t)(steps * B) * 4);
     float ms = 0.f;
     LOGOS_CUDA_TRY(cudaEventElapsedTime(&ms, m->ev0, m->ev1));
     m->last_ms = ms;
     int code = 0;
-    LOGOS_TRY(kernel_status_read(m->device, &code, false));
+    if (status) LOGOS_TRY(kernel_status_judge(m->device, back->status, &code, false));
+    else LOGOS_TRY(kernel_status_read(m->device, &code, false));
     if (code != 0) return fail(LOGOS_ERROR, "a device-side wait gave up (kernel status %d)", code);
     return LOGOS_OK;
   });

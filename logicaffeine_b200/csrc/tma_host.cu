@@ -92,8 +92,12 @@ logos_status_t kernel_status_read(int device, int* out, bool clear) {
   int* p = kernel_status_ptr(device);
   if (!p) return fail(LOGOS_ERROR, "no kernel status word (no CUDA device?)");
   LOGOS_CUDA_TRY(cudaSetDevice(device));
-  int words[8];
+  int words[KERNEL_STATUS_WORDS];
   LOGOS_CUDA_TRY(cudaMemcpy(words, p, sizeof(words), cudaMemcpyDeviceToHost));
+  return kernel_status_judge(device, words, out, clear);
+}
+
+logos_status_t kernel_status_judge(int device, const int (&words)[KERNEL_STATUS_WORDS], int* out, bool clear) {
   if (words[0] == 0) {
     // the word of the entry point that keeps its scratch inside the library image
     int sw[8];
@@ -113,7 +117,7 @@ logos_status_t kernel_status_read(int device, int* out, bool clear) {
                    std::to_string(words[4]) + " warp " + std::to_string(words[5]));
     if (clear) {
       LOGOS_TRY(counters_reset(device));
-      LOGOS_CUDA_TRY(cudaMemset(p, 0, sizeof(words)));
+      LOGOS_CUDA_TRY(cudaMemset(kernel_status_ptr(device), 0, sizeof(words)));
     }
   }
   return LOGOS_OK;
