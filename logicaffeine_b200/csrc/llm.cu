@@ -307,8 +307,8 @@ logos_status_t build(Model* m, const void* nccl_id) {
   }
   m->max_splits = 1;
   {
-    int s1 = gemm_pick_splits(B, H, m->nq, m->device);
-    int s2 = gemm_pick_splits(B, H, m->f_local, m->device);
+    int s1 = gemm_pick_splits(B, H, m->nq, m->device, true);
+    int s2 = gemm_pick_splits(B, H, m->f_local, m->device, true);
     m->max_splits = s1 > s2 ? s1 : s2;
   }
   LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->h), B * H * 4));
@@ -359,7 +359,7 @@ logos_status_t build(Model* m, const void* nccl_id) {
   {
     // qkv and gate/up split K too when their row tiles alone would leave most SMs idle (the
     // per-rank shapes of a TP group): room for the larger of the two sets of partials
-    const int s_qkv = gemm_pick_splits(B, m->nqkv, H, m->device), s_gu = gemm_pick_splits(B, 2 * m->f_local, H, m->device);
+    const int s_qkv = gemm_pick_splits(B, m->nqkv, H, m->device, true), s_gu = gemm_pick_splits(B, 2 * m->f_local, H, m->device, false);
     const int64_t need_qkv = s_qkv > 1 ? (int64_t)s_qkv * B * m->nqkv : 0;
     const int64_t need_gu = s_gu > 1 ? (int64_t)s_gu * B * 2 * m->f_local : 0;
     m->dpart_floats = need_qkv > need_gu ? need_qkv : need_gu;
@@ -408,7 +408,7 @@ __global__ void bump_len_kernel(int32_t* seq_len, int32_t* step_counter, int b, 
 logos_status_t gemm_direct(Model* m, const GemmArgs& g, int* unfolded_splits = nullptr) {
   ProfScope ps(m, PROF_GEMM);
   if (unfolded_splits) *unfolded_splits = 1;
-  int splits = gemm_pick_splits(g.m, g.n, g.k, m->device);
+  int splits = gemm_pick_splits(g.m, g.n, g.k, m->device, unfolded_splits != nullptr);
   if (splits > 1 && (int64_t)splits * g.m * g.n <= m->dpart_floats && gemm_tc_applicable(g)) {
     GemmArgs gp = g;
     gp.splits = splits;
@@ -441,7 +441,7 @@ logos_status_t gemm_partials(Model* m, const ActOut& a, const Q8Mat& w, int* spl
   g.q = w.q; g.s = w.s; g.q_tiled = w.tiled;
   g.m = B; g.n = w.n; g.k = w.k;
   g.device = m->device;
-  int splits = gemm_pick_splits(B, w.n, w.k, m->device);
+  int splits = gemm_pick_splits(B, w.n, w.k, m->device, true);
   if (splits > m->max_splits) splits = m->max_splits;
   if (splits > 1 && gemm_tc_applicable(g)) {
     g.splits = splits;

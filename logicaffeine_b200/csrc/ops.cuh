@@ -66,7 +66,8 @@ struct GemmArgs {
 };
 logos_status_t launch_q8_gemm(const GemmArgs& g, cudaStream_t st);
 // How many K-splits launch_q8_gemm would like for this shape (1 = none).
-int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device);
+// folded: the partials' consumer adds them up as it reads them.
+int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device, bool folded);
 // Whether the tcgen05 kernel accepts this call (else the SIMT kernel runs).
 bool gemm_tc_applicable(const GemmArgs& g);
 

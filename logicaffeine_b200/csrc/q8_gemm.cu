@@ -193,13 +193,18 @@ __global__ void __launch_bounds__(256) residual_kernel(const float* __restrict__
 // ties go to fewer splits (fewer partials to write and fold).  A row tile for each token tile of 64 is a
 // unit of its own: with many tokens there are enough.  The split count is also what fixes the order of a
 // sum, so that the same shape gives the same bits whatever the kernel's tiles.
-int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device) {
+// Where the consumer folds the partials as it reads them (`folded`: a decode step's norms and attention) a split costs no
+// launch: as few as three stages then, and the fixed part overlaps the predecessor's end, eight stage times.  With the
+// other rule / this one, us a step: 0.5B shape at batch 17 844 / 789, 64 1062 / 986; four layers of the 32B shape at batch 1
+// 731 / 695, 64 1182 / 1151.
+int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device, bool folded) {
   const int64_t tiles = ((n + 127) / 128) * std::max<int64_t>((m + 63) / 64, 1);
   const int64_t stages = k / 128;
   const int sms = sm_count(device);
-  if (tiles >= sms || stages < 8) return 1;
-  const int64_t fixed = 12;
-  const int64_t max_splits = std::min<int64_t>(stages / 4, 16);   // at least 4 stages (512 columns) per split
+  const int64_t least = folded ? 3 : 4;   // stages a split
+  if (tiles >= sms || stages < 2 * least) return 1;
+  const int64_t fixed = folded ? 8 : 12;
+  const int64_t max_splits = std::min<int64_t>(stages / least, 16);
   int best = 1;
   int64_t best_cost = INT64_MAX;
   for (int64_t sp = 1; sp <= max_splits; ++sp) {
@@ -262,7 +267,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   const int src_dtype = g.a_dtype;
   const int64_t stages = (g.k + 127) / 128;
   const bool retile = g.k % 128 != 0;
-  const int splits = gemm_pick_splits(g.m, g.n, g.k, g.device);
+  const int splits = gemm_pick_splits(g.m, g.n, g.k, g.device, false);
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   const int64_t lda = stages * 128;
   const int64_t plane_bytes = up(g.m * lda * 2);
