@@ -23,9 +23,9 @@
 //     the predecessor (AttnArgs::early_reads); every row of the query and the new K/V is one round of loads.
 // The form before this one was a persistent grid that cut the sequence of all pairs' tiles into 296 equal shares, with
 // the cut pairs' parts in global memory and an arrival counter for each share.  Measured, that one -> this one, with cold
-// caches and the events' 8 us (us, equal / ragged lengths): 64 sequences of 2048, 64/8 heads of 128 123 / 149 -> 111 / 76;
-// 32 of 4096, 28/4 76 / 62 -> 69 / 54; 7 of 2000, 14/2 of 64 27 / 24 -> 19 / 19; 16 of 128, 14/2 of 64 19 -> 16; one of 8000, 28/4 506 -> 25
-// (more than 64 parts went through a slow loop); 38 of 1300, 64/8 (8 pairs more than run at once) 69 / 86 -> 71 / 44.  Three
+// caches and the events' 8 us (us, equal / ragged lengths): 64 sequences of 2048, 64/8 heads of 128 123 / 149 -> 109 / 72;
+// 32 of 4096, 28/4 76 / 62 -> 69 / 48; 7 of 2000, 14/2 of 64 27 / 24 -> 19 / 18; 16 of 128, 14/2 of 64 19 -> 16; one of 8000, 28/4 506 -> 25
+// (more than 64 parts went through a slow loop); 38 of 1300, 64/8 (8 pairs more than run at once) 69 / 86 -> 67 / 45.  Three
 // ring stages at head dimension 128 against two: 64 of 1300, 64/8 86 -> 85, 25 of 2000, 28/4 41 -> 40.
 #include "ops.cuh"
 #include "q8_gemm_tc.cuh"

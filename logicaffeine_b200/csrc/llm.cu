@@ -534,7 +534,7 @@ logos_status_t step_tail(Model* m, int parts, bool sample, bool log_tokens, cons
 
 // Whether a layer's products run in the kernels that hold the norms, SwiGLU and the residual adds too (q8_narrow.cu):
 // where they take the shapes, up to 16 sequences (one token tile).  us a step of the 0.5B shape, the kernels of
-// q8_gemm_tc.cu and these: batch 1 904 / 621, 8 905 / 629, 16 900 / 763, 32 1000 / 995.
+// q8_gemm_tc.cu and these, with one attention for both: batch 1 904 / 621, 8 905 / 629, 16 900 / 763, 32 1000 / 995.
 bool narrow_layers(const Model* m) {
   const logos_llm_config_t& c = m->cfg;
   if (m->tp.degree > 1 || c.batch > 16) return false;
