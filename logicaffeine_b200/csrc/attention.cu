@@ -415,23 +415,6 @@ struct AttnSmem {
 };
 static_assert(2 * (AttnSmem<128>::BYTES + 1024) <= 228 * 1024, "two CTAs fit an SM");
 
-__device__ __forceinline__ uint32_t smem_of_rank(uint32_t addr, int rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  return a;
-}
-// 16 or 8 bytes into another CTA's shared memory, counted on a barrier there
-__device__ __forceinline__ void push16(uint32_t addr, float4 v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void push8(uint32_t addr, float2 v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
-               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar)
-               : "memory");
-}
-
 // Grid: (sequence, KV head) pairs x CTAs of a cluster.
 template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
@@ -584,7 +567,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   }
   if (parts == 1) return;
   asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
-  if (!mbar_wait(bar_parts, 0)) {
+  if (!mbar_wait_cluster(bar_parts, 0)) {
     if (lane == 0) atomicCAS(p.status, 0, 103);
     return;
   }

@@ -120,26 +120,54 @@ __device__ __forceinline__ void mbar_wait3(uint32_t bar0, uint32_t ph0, uint32_t
                : "memory");
 }
 // A single wait with a limit of its own, counted from its 32nd failed poll; false when it gave up.
+#define LOGOS_MBAR_SINGLE(TRY)                \
+  "{\n\t.reg .pred p, s;\n\t.reg .u32 n, t, e;\n\tmov.u32 n, 0;\n" \
+  "POLL:\n\t" TRY                             \
+  "@p bra DONE;\n\t"                          \
+  "add.u32 n, n, 1;\n\t"                      \
+  "and.b32 t, n, 31;\n\t"                     \
+  "setp.ne.u32 s, t, 0;\n\t"                  \
+  "@s bra POLL;\n\t"                          \
+  "mov.u32 t, %%clock_hi;\n\t"                \
+  "setp.eq.u32 s, n, 32;\n\t"                 \
+  "@s mov.u32 e, t;\n\t"                      \
+  "sub.u32 t, t, e;\n\t"                      \
+  "setp.lt.u32 s, t, 2;\n\t"                  \
+  "@s bra POLL;\n"                            \
+  "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile("{\n\t.reg .pred p, s;\n\t.reg .u32 n, t, e;\n\tmov.u32 n, 0;\n"
-               "POLL:\n\t" LOGOS_MBAR_TRY("p", "%1", "%2")
-               "@p bra DONE;\n\t"
-               "add.u32 n, n, 1;\n\t"
-               "and.b32 t, n, 31;\n\t"
-               "setp.ne.u32 s, t, 0;\n\t"
-               "@s bra POLL;\n\t"
-               "mov.u32 t, %%clock_hi;\n\t"
-               "setp.eq.u32 s, n, 32;\n\t"
-               "@s mov.u32 e, t;\n\t"
-               "sub.u32 t, t, e;\n\t"
-               "setp.lt.u32 s, t, 2;\n\t"
-               "@s bra POLL;\n"
-               "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+  asm volatile(LOGOS_MBAR_SINGLE(LOGOS_MBAR_TRY("p", "%1", "%2")) : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
+
+// ------------------------------------------------------------ clusters
+// A wait for what other CTAs of the cluster pushed into this one's shared memory: a push releases at cluster scope, and
+// only an acquire of that scope sees what it wrote (the plain form's is the CTA).
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(LOGOS_MBAR_SINGLE("mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t")
                : "=r"(ok)
                : "r"(smem_u32(bar)), "r"(parity)
                : "memory");
   return ok != 0;
+}
+// the address of this CTA's `addr` in the CTA of a rank
+__device__ __forceinline__ uint32_t smem_of_rank(uint32_t addr, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+// 16 or 8 bytes into another CTA's shared memory, counted on a barrier there
+__device__ __forceinline__ void push16(uint32_t addr, float4 v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void push8(uint32_t addr, float2 v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar)
+               : "memory");
 }
 
 __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {

@@ -90,17 +90,6 @@ __device__ __forceinline__ float inv_sqrt(float x) {
   const float y = rsqrtf(x), e = fmaf(-x * y, y, 1.0f);
   return fmaf(0.5f * y, e, y);
 }
-__device__ __forceinline__ uint32_t of_rank(uint32_t smem_addr, int rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
-  return a;
-}
-// eight bytes into another CTA's shared memory, counted on a barrier there
-__device__ __forceinline__ void push8(uint32_t addr, float2 v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
-               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar)
-               : "memory");
-}
 
 // Grid: x = unit groups x CTAs along K (a cluster), y = token tiles; a warp for every 64 columns.
 // Up to four tokens (TOK = 4) both planes of them are the eight columns of one MMA, hi 0 to 3 and lo 4 to 7: half the MMAs (a
@@ -318,7 +307,7 @@ q8_narrow_kernel(const NarrowParams p) {
   if (!NORM && ranks > 1) {
     cg::this_cluster().barrier_wait();
     if (rank != 0) {
-      const uint32_t to = of_rank(pushed + (rank - 1) * all * 8, 0), bar = of_rank(smem_u32(&s_bar), 0);
+      const uint32_t to = smem_of_rank(pushed + (rank - 1) * all * 8, 0), bar = smem_of_rank(smem_u32(&s_bar), 0);
       for (int e = tid; e < all; e += NW_THREADS) push8(to + e * 8, local(e), bar);
       return;
     }
@@ -326,7 +315,7 @@ q8_narrow_kernel(const NarrowParams p) {
   for (int e = tid; e < all; e += NW_THREADS) {
     float2 v = local(e);
     if (!NORM && ranks > 1) {
-      if (e == tid && !mbar_wait(&s_bar, 0)) atomicCAS(p.status, 0, 4010);
+      if (e == tid && !mbar_wait_cluster(&s_bar, 0)) atomicCAS(p.status, 0, 4010);
       for (int r = 1; r < ranks; ++r) {
         const uint2 o = lds_v2(pushed + ((r - 1) * all + e) * 8);
         v = add2(v, make_float2(__uint_as_float(o.x), __uint_as_float(o.y)));

@@ -1,6 +1,6 @@
 // Waits for barriers that nothing completes, until the limit of csrc/ptx.cuh ends them: prints a line
-// "<form> <milliseconds> <gave up>" for the form with a limit of its own and for the one with a limit shared by several
-// waits.  Barriers that are ready come first: those waits must not give up.
+// "<form> <milliseconds> <gave up>" for the form with a limit of its own, for the one with a limit shared by several
+// waits, and for the one that waits for other CTAs' pushes.  Barriers that are ready come first: those waits must not give up.
 #include "ptx.cuh"
 
 #include <cstdio>
@@ -21,6 +21,10 @@ __global__ void wait_limit(int form, int* out) {
     const bool ready = mbar_wait(&done_bar, 0);
     const bool ok = mbar_wait(&open_bar, 0);
     if (threadIdx.x == 0) out[0] = ready && !ok;
+  } else if (form == 2) {
+    const bool ready = mbar_wait_cluster(&done_bar, 0);
+    const bool ok = mbar_wait_cluster(&open_bar, 0);
+    if (threadIdx.x == 0) out[0] = ready && !ok;
   } else {
     uint32_t since = wait_start();
     mbar_wait2(done_a, 0, done_a, 0, &since);
@@ -34,7 +38,7 @@ __global__ void wait_limit(int form, int* out) {
 int main() {
   int *out = nullptr, gave_up = 0;
   if (cudaMalloc(&out, sizeof(int)) != cudaSuccess) return 2;
-  for (int form = 0; form < 2; ++form) {
+  for (int form = 0; form < 3; ++form) {
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
