@@ -433,6 +433,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   uint64_t* bar_empty = bar_full + STAGES;
   uint64_t* bar_parts = bar_empty + STAGES;
   int& s_bump = *reinterpret_cast<int*>(bar_parts + 1);
+  int& s_prior = *(&s_bump + 1);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = p.h_q / p.h_kv;
@@ -444,7 +445,8 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   // write any of them: everything waits.
   if (!p.early_reads) pdl_wait();
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
-  const int prior_status = *reinterpret_cast<volatile int*>(p.status);
+  // (one thread's value counts: the CTA takes one decision)
+  const int status = *reinterpret_cast<volatile int*>(p.status);
   const int len = __ldcg(p.seq_len + b);
   const int len0 = len < p.l_max ? len : p.l_max, len_eff = attn_len_eff(p, len0);
   const int tiles = (len_eff + ATT_TILE - 1) / ATT_TILE;
@@ -453,6 +455,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int per = parts > 0 ? (G + parts - 1) / parts : G;   // row slots a part
   const int mine = rank < parts ? (G - rank + parts - 1) / parts : 0;   // rows finished here: rank, rank + parts, ...
   if (tid == 0) {
+    s_prior = status;
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&bar_full[i], 1);
       mbar_init(&bar_empty[i], ATT_CWARPS);
@@ -462,6 +465,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     mbar_arrive_expect_tx(bar_parts, (parts > 1 ? parts - 1 : 0) * mine * (D * 4 + 8));
   }
   __syncthreads();
+  const bool prior = s_prior != 0;
   cg::cluster_group cluster = cg::this_cluster();
   cluster.barrier_arrive();   // "this CTA runs, its barrier stands": before anyone pushes into it
   const int64_t row_base = ((int64_t)b * p.h_kv + kvh) * p.l_max;
@@ -477,13 +481,18 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         if (l < p.l_max) p.seq_len[i] = l + 1;
       }
   }
+  // The last loads of tiles [t0, t): this CTA's shared memory is its own until they have landed.
+  auto drain = [&](int t) {
+    for (int i = max(0, t - t0 - STAGES); i < t - t0; ++i) mbar_wait(&bar_full[i % STAGES], (i / STAGES) & 1);
+  };
   if (warp == ATT_CWARPS) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0 && prior_status == 0) {
+    if (lane == 0 && !prior) {
       for (int t = t0; t < t1; ++t) {
         const int i = t - t0, st = i % STAGES;
         if (!mbar_wait(&bar_empty[st], ((i / STAGES) & 1) ^ 1)) {
           atomicExch(p.status, 101);
+          drain(t);
           break;
         }
         uint8_t* sb = stages + st * STAGE_BYTES;
@@ -499,103 +508,127 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   }
   pdl_wait();
   pdl_trigger();
-  if (warp == ATT_CWARPS || prior_status != 0) return;
+  if (warp == ATT_CWARPS) return;
   if (tiles == 0) {   // nothing to attend to: zeros
-    if (rank == 0)
+    if (rank == 0 && !prior)
       for (int e = tid; e < G * D; e += ATT_CTHREADS) store_out(p, ((int64_t)b * p.h_q + kvh * G) * D + e, 0.f);
     return;
   }
   if (rank >= parts) return;
 
   // ---------------------------------------------------------------- consumers
-  const int pos_new = len0;
-  const bool owns_new = p.fused && len0 < p.l_max && pos_new >= t0 * ATT_TILE && pos_new < t1 * ATT_TILE;
-  stage_query<D>(p, b, kvh, len0, owns_new, row_base, tid, qs, new_k, new_v);
-  asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
-  AttnState<D> w;
-  w.start(qs, lane);
-  bool ok = true;
-  int st = 0;
-  for (int t = t0; t < t1; ++t) {
-    const int i = t - t0;
-    st = i % STAGES;
-    if (!mbar_wait(&bar_full[st], (i / STAGES) & 1)) {
-      ok = false;
-      break;
+  // Whatever happens, a CTA pushes what its peers count on and takes what they push: nothing arrives in the memory of one
+  // that has left.  Without sums (a code was there, or a wait gave up) it pushes a mark in place of a row's sum of
+  // weights, which is never negative, and a row with a mark is not written.
+  constexpr float NO_SUMS = -1.f;
+  // Everything that peers push here has arrived.  Otherwise a peer is late (each of its waits is bounded): once the others have ended
+  // or are here too, what is still on its way arrives at once.
+  auto all_pushed = [&]() {
+    if (mbar_wait_cluster(bar_parts, 0)) return true;
+    atomicCAS(p.status, 0, 103);
+    cluster_meet();
+    mbar_wait_cluster(bar_parts, 0);
+    return false;
+  };
+  if (!prior) {
+    const int pos_new = len0;
+    const bool owns_new = p.fused && len0 < p.l_max && pos_new >= t0 * ATT_TILE && pos_new < t1 * ATT_TILE;
+    stage_query<D>(p, b, kvh, len0, owns_new, row_base, tid, qs, new_k, new_v);
+    asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
+    AttnState<D> w;
+    w.start(qs, lane);
+    bool ok = true;
+    int st = 0;
+    for (int t = t0; t < t1; ++t) {
+      const int i = t - t0;
+      st = i % STAGES;
+      if (!mbar_wait(&bar_full[st], (i / STAGES) & 1)) {
+        ok = false;
+        break;
+      }
+      uint8_t* kb = stages + st * STAGE_BYTES;
+      attn_tile<D>(p, w, kb, kb + NBOX * ATT_BOX_BYTES, warp, lane, t * ATT_TILE + 16 * warp, len_eff, owns_new, pos_new, new_k, new_v);
+      __syncwarp();
+      if (t + 1 < t1 && lane == 0) mbar_arrive(&bar_empty[st]);
     }
-    uint8_t* kb = stages + st * STAGE_BYTES;
-    attn_tile<D>(p, w, kb, kb + NBOX * ATT_BOX_BYTES, warp, lane, t * ATT_TILE + 16 * warp, len_eff, owns_new, pos_new, new_k, new_v);
-    __syncwarp();
-    if (t + 1 < t1 && lane == 0) mbar_arrive(&bar_empty[st]);
-  }
-  w.reduce_sums();
-  {
+    w.reduce_sums();
     int all_ok;
     asm volatile(
         "{\n\t.reg .pred q, r;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred r, 1, %2, q;\n\tselp.u32 %0, 1, 0, r;\n\t}"
         : "=r"(all_ok)
         : "r"((uint32_t)ok), "n"(ATT_CTHREADS)
         : "memory");
-    if (!all_ok) {
-      if (!ok && lane == 0) atomicExch(p.status, 102);
+    if (all_ok) {
+      float* mo = reinterpret_cast<float*>(stages + st * STAGE_BYTES);   // [warp][16][D]: every warp has read its rows of the last tile
+      w.put(mo, mml, warp, lane);
+      asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
+      if (parts > 1) cluster.barrier_wait();
+      const int64_t o0 = ((int64_t)b * p.h_q + kvh * G) * D;
+      for (int e = 4 * tid; e < G * D; e += 4 * ATT_CTHREADS) {
+        const int r = e / D, d = e - r * D;
+        float m, L;
+        const float4 acc = combine_warps<D>(mo, mml, r, d, &m, &L);
+        if (parts == 1) {
+          store_out4(p, o0 + e, acc, L);
+          continue;
+        }
+        const int to = r % parts;
+        const uint32_t at = smem_u32(pushed) + (rank * per + r / parts) * ROW_BYTES;
+        if (to == rank) {
+          *reinterpret_cast<float4*>(pushed + (rank * per + r / parts) * ROW_BYTES + d * 4) = acc;
+          if (d == 0) *reinterpret_cast<float2*>(pushed + (rank * per + r / parts) * ROW_BYTES + D * 4) = make_float2(m, L);
+        } else {
+          const uint32_t there = smem_of_rank(at, to), bar = smem_of_rank(smem_u32(bar_parts), to);
+          push16(there + d * 4, acc, bar);
+          if (d == 0) push8(there + D * 4, make_float2(m, L), bar);
+        }
+      }
+      if (parts == 1) return;
+      asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
+      if (!all_pushed()) return;
+      // the rows finished here, the parts in the order of their positions
+      for (int e = 4 * tid; e < mine * D; e += 4 * ATT_CTHREADS) {
+        const int slot = e / D, d = e - slot * D;
+        const uint8_t* row = pushed + slot * ROW_BYTES;
+        float2 ml[ATT_MAX_PARTS];
+        float m = -INFINITY;
+        bool whole = true;
+#pragma unroll
+        for (int i = 0; i < ATT_MAX_PARTS; ++i) {
+          ml[i] = i < parts ? *reinterpret_cast<const float2*>(row + i * per * ROW_BYTES + D * 4) : make_float2(-INFINITY, 0.f);
+          m = fmaxf(m, ml[i].x);
+          whole = whole && ml[i].y != NO_SUMS;
+        }
+        if (!whole) continue;
+        const float muse = (m == -INFINITY) ? 0.f : m;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float L = 0.f;
+#pragma unroll
+        for (int i = 0; i < ATT_MAX_PARTS; ++i)
+          if (i < parts) {
+            const float wgt = exp2f(ml[i].x - muse);
+            const float4 v = *reinterpret_cast<const float4*>(row + i * per * ROW_BYTES + d * 4);
+            acc.x = fmaf(v.x, wgt, acc.x); acc.y = fmaf(v.y, wgt, acc.y);
+            acc.z = fmaf(v.z, wgt, acc.z); acc.w = fmaf(v.w, wgt, acc.w);
+            L = fmaf(ml[i].y, wgt, L);
+          }
+        store_out4(p, o0 + (int64_t)(rank + slot * parts) * D + d, acc, L);
+      }
       return;
     }
-  }
-  float* mo = reinterpret_cast<float*>(stages + st * STAGE_BYTES);   // [warp][16][D]: every warp has read its rows of the last tile
-  w.put(mo, mml, warp, lane);
-  asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
-  if (parts > 1) cluster.barrier_wait();
-  const int64_t o0 = ((int64_t)b * p.h_q + kvh * G) * D;
-  for (int e = 4 * tid; e < G * D; e += 4 * ATT_CTHREADS) {
-    const int r = e / D, d = e - r * D;
-    float m, L;
-    const float4 acc = combine_warps<D>(mo, mml, r, d, &m, &L);
-    if (parts == 1) {
-      store_out4(p, o0 + e, acc, L);
-      continue;
-    }
-    const int to = r % parts;
-    const uint32_t at = smem_u32(pushed) + (rank * per + r / parts) * ROW_BYTES;
-    if (to == rank) {
-      *reinterpret_cast<float4*>(pushed + (rank * per + r / parts) * ROW_BYTES + d * 4) = acc;
-      if (d == 0) *reinterpret_cast<float2*>(pushed + (rank * per + r / parts) * ROW_BYTES + D * 4) = make_float2(m, L);
-    } else {
-      const uint32_t there = smem_of_rank(at, to), bar = smem_of_rank(smem_u32(bar_parts), to);
-      push16(there + d * 4, acc, bar);
-      if (d == 0) push8(there + D * 4, make_float2(m, L), bar);
-    }
+    if (!ok && lane == 0) atomicExch(p.status, 102);
+    if (tid == 0) drain(t1);   // the producer may be done and gone (one that is not drains what it has issued)
   }
   if (parts == 1) return;
-  asm volatile("bar.sync 1, %0;" ::"n"(ATT_CTHREADS) : "memory");
-  if (!mbar_wait_cluster(bar_parts, 0)) {
-    if (lane == 0) atomicCAS(p.status, 0, 103);
-    return;
+  cluster.barrier_wait();
+  for (int e = 4 * tid; e < G * D; e += 4 * ATT_CTHREADS) {
+    const int r = e / D, d = e - r * D, to = r % parts;
+    if (to == rank) continue;
+    const uint32_t there = smem_of_rank(smem_u32(pushed) + (rank * per + r / parts) * ROW_BYTES, to), bar = smem_of_rank(smem_u32(bar_parts), to);
+    push16(there + d * 4, make_float4(0.f, 0.f, 0.f, 0.f), bar);
+    if (d == 0) push8(there + D * 4, make_float2(0.f, NO_SUMS), bar);
   }
-  // the rows finished here, the parts in the order of their positions
-  for (int e = 4 * tid; e < mine * D; e += 4 * ATT_CTHREADS) {
-    const int slot = e / D, d = e - slot * D;
-    const uint8_t* row = pushed + slot * ROW_BYTES;
-    float2 ml[ATT_MAX_PARTS];
-    float m = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < ATT_MAX_PARTS; ++i) {
-      ml[i] = i < parts ? *reinterpret_cast<const float2*>(row + i * per * ROW_BYTES + D * 4) : make_float2(-INFINITY, 0.f);
-      m = fmaxf(m, ml[i].x);
-    }
-    const float muse = (m == -INFINITY) ? 0.f : m;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float L = 0.f;
-#pragma unroll
-    for (int i = 0; i < ATT_MAX_PARTS; ++i)
-      if (i < parts) {
-        const float wgt = exp2f(ml[i].x - muse);
-        const float4 v = *reinterpret_cast<const float4*>(row + i * per * ROW_BYTES + d * 4);
-        acc.x = fmaf(v.x, wgt, acc.x); acc.y = fmaf(v.y, wgt, acc.y);
-        acc.z = fmaf(v.z, wgt, acc.z); acc.w = fmaf(v.w, wgt, acc.w);
-        L = fmaf(ml[i].y, wgt, L);
-      }
-    store_out4(p, o0 + (int64_t)(rank + slot * parts) * D + d, acc, L);
-  }
+  all_pushed();
 }
 
 __global__ void bump_seq_len_kernel(int32_t* seq_len, int b, int l_max) {

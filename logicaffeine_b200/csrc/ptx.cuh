@@ -152,6 +152,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
                : "memory");
   return ok != 0;
 }
+// Returns once every thread of the cluster that has not ended is here.  Threads of a warp may come one by one.
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 // the address of this CTA's `addr` in the CTA of a rank
 __device__ __forceinline__ uint32_t smem_of_rank(uint32_t addr, int rank) {
   uint32_t a;
