@@ -73,7 +73,7 @@ struct AttnParams {
   const float*  rope;
   int32_t* seq_len;
   unsigned*     arrive;   // with bump: CTAs that have their length; zero before and after every launch (it wraps by itself)
-  int           bump;     // the last CTA to finish advances the lengths
+  int           bump;     // the last CTA to have its length advances the lengths
   int           early_reads;   // see AttnArgs
   void*         o;        // [B][Hq][D]
   int           o_dtype;
@@ -470,8 +470,9 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   cluster.barrier_arrive();   // "this CTA runs, its barrier stands": before anyone pushes into it
   const int64_t row_base = ((int64_t)b * p.h_kv + kvh) * p.l_max;
 
-  // the last CTA of the grid to have its length advances the lengths (before the producer starts: it may wait for the consumers)
-  if (p.bump) {
+  // the last CTA of the grid to have its length advances the lengths (before the producer starts: it may wait for the consumers),
+  // unless there is a code: nothing is appended then
+  if (p.bump && !prior) {
     pdl_wait();
     if (tid == 0) s_bump = arrive_inc(p.arrive, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();

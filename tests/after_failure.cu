@@ -1,0 +1,88 @@
+// What kernels do behind a failure: with a code in the status word, as a wait that gave up leaves it, a launch writes nothing,
+// and once the code is cleared the same launch writes its results.  Prints a line "<what> <changed behind the code> <changed after>" for each.
+#include "ops.cuh"
+#include "ptx.cuh"
+
+#include <cstdio>
+#include <cstring>
+#include <functional>
+#include <vector>
+
+using namespace logos;
+
+#define CHECK(x)                                                       \
+  do {                                                                 \
+    if (int e_ = (int)(x)) {                                           \
+      printf("%s: %d %s\n", #x, e_, last_error_text() ? last_error_text() : ""); \
+      return 2;                                                        \
+    }                                                                  \
+  } while (0)
+
+struct Buf {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+static Buf buf(size_t bytes, int dtype, int kind, int stream, float a, float b) {
+  Buf r;
+  r.bytes = bytes;
+  if (cudaMalloc(&r.p, bytes) != cudaSuccess) return r;
+  const int64_t size = dtype == LOGOS_F16 ? 2 : dtype == LOGOS_I8 ? 1 : 4;
+  launch_synth_fill(r.p, dtype, kind, 1, stream, 0, (int64_t)bytes / size, a, b, 0, nullptr);
+  return r;
+}
+
+static int run(const char* what, const std::vector<Buf>& written, const std::function<logos_status_t()>& launch) {
+  auto bytes = [&] {
+    std::vector<std::vector<char>> v;
+    for (const Buf& w : written) {
+      v.emplace_back(w.bytes);
+      cudaMemcpy(v.back().data(), w.p, w.bytes, cudaMemcpyDeviceToHost);
+    }
+    return v;
+  };
+  int* word = kernel_status_ptr(0);
+  const int code = 4242;
+  const auto before = bytes();
+  CHECK(cudaMemcpy(word, &code, sizeof(code), cudaMemcpyHostToDevice));
+  CHECK(launch());
+  CHECK(cudaDeviceSynchronize());
+  const auto behind = bytes();
+  int got = 0;
+  CHECK(kernel_status_read(0, &got, true));
+  if (got != code) return 3;
+  CHECK(launch());
+  CHECK(cudaDeviceSynchronize());
+  const auto after = bytes();
+  CHECK(kernel_status_read(0, &got, true));
+  if (got != 0) return 4;
+  bool all = true;
+  for (size_t i = 0; i < after.size(); ++i) all = all && after[i] != before[i];
+  printf("%s %d %d\n", what, (int)(behind != before), (int)all);
+  return 0;
+}
+
+static int attention(int d, int b) {
+  const int h_q = 14, h_kv = 2, l_max = 700;
+  const int64_t cache = (int64_t)b * h_kv * l_max * d;
+  AttnArgs a;
+  Buf q = buf(b * h_q * d * 2, LOGOS_F16, 2, 1, 0.f, 1.f), kn = buf(b * h_kv * d * 2, LOGOS_F16, 2, 2, 0.f, 1.f);
+  Buf k = buf(cache * 2, LOGOS_F16, 2, 3, 0.f, 1.f), v = buf(cache * 2, LOGOS_F16, 2, 4, 0.f, 1.f);
+  Buf rope = buf((size_t)l_max * d * 4, LOGOS_F32, 2, 5, 0.f, 1.f), o = buf(b * h_q * d * 2, LOGOS_F16, 2, 6, 0.f, 1.f);
+  Buf seq = buf(b * 4, LOGOS_F32, 2, 7, 0.f, 1.f);
+  std::vector<int> lens(b);
+  for (int i = 0; i < b; ++i) lens[i] = i * 600 / b;   // an empty sequence among them
+  CHECK(cudaMemcpy(seq.p, lens.data(), seq.bytes, cudaMemcpyHostToDevice));
+  a.q_f16 = (const __half*)q.p; a.k_new_f16 = a.v_new_f16 = (const __half*)kn.p;
+  a.k_cache = (__half*)k.p; a.v_cache = (__half*)v.p; a.rope = (const float*)rope.p; a.rotate_q = 1;
+  a.seq_len = (int32_t*)seq.p; a.bump_seq_len = 1; a.o = o.p;
+  a.b = b; a.h_q = h_q; a.h_kv = h_kv; a.d = d; a.l_max = l_max; a.scale = 0.1f;
+  return run("attention", {o, k, v, seq}, [&] { return launch_gqa_decode_attn(a, nullptr); });
+}
+
+int main() {
+  if (!kernel_status_ptr(0)) return 1;
+  for (int d : {64, 128})
+    for (int b : {1, 5, 200})   // clusters of up to eight CTAs, and of one
+      if (int rc = attention(d, b)) return rc;
+  return 0;
+}
