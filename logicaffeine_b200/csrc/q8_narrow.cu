@@ -107,6 +107,7 @@ q8_narrow_kernel(const NarrowParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float s_ss[NW_WARPS][TOK];
   __shared__ uint64_t s_bar;
+  __shared__ int s_prior;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
   const int ranks = NORM ? 1 : p.ranks, rank = NORM ? 0 : (int)(blockIdx.x % (unsigned)ranks);
@@ -121,6 +122,12 @@ q8_narrow_kernel(const NarrowParams p) {
   const int all = have * PAIRS;
 
   pdl_trigger();
+  // A code that an earlier kernel left: nothing is stored on top of it.  One thread reads and the CTA takes one decision; of a
+  // cluster the CTA that stores does, and the others push all the same, since it waits for what they push.  Read before the wait
+  // for the predecessor, as the kernels of q8_gemm_tc.cu do: all CTAs ask one L2 line for the word, and after the wait that is on
+  // the kernel's chain (a step of the 0.5B shape at batch 16 675 -> 688 us; 695 with every thread asking).
+  int status = 0;
+  if (tid == 0) status = *reinterpret_cast<volatile int*>(p.status);
   // ---- weights, scales, gains: nothing in a step writes them
   float4 gain[4];
   if (active) {
@@ -147,6 +154,7 @@ q8_narrow_kernel(const NarrowParams p) {
     }
     cg::this_cluster().barrier_arrive();   // "this CTA runs, its barrier stands": before anyone pushes into it
   }
+  if (tid == 0) s_prior = status;
   pdl_wait();
 
   // ---- fragments of the activations: a lane has columns 8 t4 .. 8 t4 + 7 of either block, for tokens g + 8 j
@@ -315,14 +323,20 @@ q8_narrow_kernel(const NarrowParams p) {
   for (int e = tid; e < all; e += NW_THREADS) {
     float2 v = local(e);
     if (!NORM && ranks > 1) {
-      if (e == tid && !mbar_wait_cluster(&s_bar, 0)) atomicCAS(p.status, 0, 4010);
+      if (e == tid && !mbar_wait_cluster(&s_bar, 0)) {
+        // a peer is late: once all have ended or are here, what is still on its way arrives at once
+        atomicCAS(p.status, 0, 4010);
+        cluster_meet();
+        mbar_wait_cluster(&s_bar, 0);
+        return;
+      }
       for (int r = 1; r < ranks; ++r) {
         const uint2 o = lds_v2(pushed + ((r - 1) * all + e) * 8);
         v = add2(v, make_float2(__uint_as_float(o.x), __uint_as_float(o.y)));
       }
     }
     const int n = column(e), t = token(e);
-    if (n >= p.n || t >= rows) continue;
+    if (n >= p.n || t >= rows || s_prior != 0) continue;
     const int64_t row = m0 + t;
     if (OUT == NARROW_SWIGLU) {
       act_store(p.planes, row * (p.n / 2) + n / 2, __fmul_rn(nw_silu(v.x), v.y));   // columns (2j, 2j + 1) are (gate_j, up_j)

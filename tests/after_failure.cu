@@ -79,8 +79,29 @@ static int attention(int d, int b) {
   return run("attention", {o, k, v, seq}, [&] { return launch_gqa_decode_attn(a, nullptr); });
 }
 
+static int narrow(int out, int m, int n, int k) {
+  NarrowArgs a;
+  Buf q = buf((size_t)(n + 127) / 128 * 128 * k, LOGOS_I8, 0, 1, 0.f, 0.f), s = buf((size_t)(n + 127) / 128 * 128 * (k / 32) * 4, LOGOS_F32, 1, 2, 1e-3f, 1e-2f);
+  Buf h = buf((size_t)m * k * 4, LOGOS_F32, 2, 3, 0.f, 1.f), gain = buf(k * 4, LOGOS_F32, 1, 4, 1.f, 1.f);
+  Buf hi = buf((size_t)m * k * 2, LOGOS_F16, 2, 5, 0.f, 1.f), c = buf((size_t)m * n * 4, LOGOS_F32, 2, 6, 0.f, 1.f);
+  Buf phi = buf((size_t)m * n, LOGOS_F16, 2, 7, 0.f, 1.f), plo = buf((size_t)m * n, LOGOS_F16, 2, 8, 0.f, 1.f);
+  a.q = (const int8_t*)q.p; a.s = (const float*)s.p; a.m = m; a.n = n; a.k = k;
+  a.h_in = (const float*)h.p; a.gain = (const float*)gain.p; a.eps = 1e-6f;
+  a.a.hi = a.a.lo = (__half*)hi.p;
+  a.out = out; a.c = (float*)c.p; a.planes.hi = (__half*)phi.p; a.planes.lo = (__half*)plo.p;
+  if (!narrow_applicable(m, n, k, out != NARROW_RESIDUAL, 0)) return 5;
+  return run(out == NARROW_F32 ? "norm" : out == NARROW_SWIGLU ? "norm+swiglu" : "residual",
+             out == NARROW_SWIGLU ? std::vector<Buf>{phi, plo} : std::vector<Buf>{c}, [&] { return launch_q8_narrow(a, nullptr); });
+}
+
 int main() {
   if (!kernel_status_ptr(0)) return 1;
+  for (int m : {1, 8, 16})
+    for (int out : {NARROW_F32, NARROW_SWIGLU, NARROW_RESIDUAL})
+      for (int k : {896, 4864}) {
+        if (out != NARROW_RESIDUAL && k > 1024) continue;
+        if (int rc = narrow(out, m, 896, k)) return rc;
+      }
   for (int d : {64, 128})
     for (int b : {1, 5, 200})   // clusters of up to eight CTAs, and of one
       if (int rc = attention(d, b)) return rc;
