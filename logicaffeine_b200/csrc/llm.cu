@@ -307,9 +307,9 @@ logos_status_t build(Model* m, const void* nccl_id) {
   }
   m->max_splits = 1;
   {
-    int s1 = gemm_pick_splits(B, H, m->nq, m->device, true);
-    int s2 = gemm_pick_splits(B, H, m->f_local, m->device, true);
-    m->max_splits = s1 > s2 ? s1 : s2;
+    // both rules where there are ranks: which of them holds (partials_folded) is known after the exchange's set-up
+    for (const bool folded : {true, g == 1})
+      for (const int64_t k : {m->nq, m->f_local}) m->max_splits = std::max(m->max_splits, gemm_pick_splits(B, H, k, m->device, folded));
   }
   LOGOS_TRY(dmalloc(m, reinterpret_cast<void**>(&m->h), B * H * 4));
   LOGOS_CUDA_TRY(cudaMemsetAsync(m->h, 0, (size_t)(B * H * 4), m->stream));   // a prompt pass may read rows that no step wrote
@@ -433,6 +433,10 @@ logos_status_t gemm_direct(Model* m, const GemmArgs& g, int* unfolded_splits = n
   return LOGOS_OK;
 }
 
+// Whether what reads the partials of o_proj and down_proj adds them up on the way: the norm, alone or with the exchange inside.
+// An all-reduce of a kernel's own wants one sum, which a kernel makes.
+bool partials_folded(const Model* m) { return m->tp.degree == 1 || m->tp_fused; }
+
 // GEMM producing f32 partials [splits][B][N] in m->partials; returns the split count.
 logos_status_t gemm_partials(Model* m, const ActOut& a, const Q8Mat& w, int* splits_out) {
   const int64_t B = m->cfg.batch;
@@ -441,7 +445,7 @@ logos_status_t gemm_partials(Model* m, const ActOut& a, const Q8Mat& w, int* spl
   g.q = w.q; g.s = w.s; g.q_tiled = w.tiled;
   g.m = B; g.n = w.n; g.k = w.k;
   g.device = m->device;
-  int splits = gemm_pick_splits(B, w.n, w.k, m->device, true);
+  int splits = gemm_pick_splits(B, w.n, w.k, m->device, partials_folded(m));
   if (splits > m->max_splits) splits = m->max_splits;
   if (splits > 1 && gemm_tc_applicable(g)) {
     g.splits = splits;
@@ -455,7 +459,7 @@ logos_status_t gemm_partials(Model* m, const ActOut& a, const Q8Mat& w, int* spl
     ProfScope ps(m, PROF_GEMM);
     LOGOS_TRY(launch_q8_gemm(g, m->stream));
   }
-  if (m->tp.degree > 1 && !m->tp_fused) {
+  if (!partials_folded(m)) {
     ProfScope ps(m, PROF_COMM);
     const int64_t count = B * w.n;
     if (splits > 1) {
