@@ -637,23 +637,44 @@ def test_waits_inside_kernels_end_in_seconds(tmp_path):
         assert 1000 < float(ms) < 12000, line   # 2^32 to 2^33 cycles: 2.2 to 4.4 s at 1965 MHz
 
 
-def test_kernels_behind_a_failure_write_nothing(tmp_path):
-    """With a code in the status word a kernel leaves its outputs, the cache and the lengths as they are; once the code has
-    been read and cleared the same launch writes them all."""
+@pytest.fixture(scope="module")
+def native(tmp_path_factory):
+    """Runs a program beside this file that is linked with the operators, and returns its output's lines."""
     here = os.path.dirname(os.path.abspath(__file__))
     csrc = os.path.join(here, "..", "logicaffeine_b200", "csrc")
+    out = str(tmp_path_factory.mktemp("native"))
     nvcc = [shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc", "-ccbin", "/usr/bin/g++", "-gencode", "arch=compute_100a,code=sm_100a",
             "-std=c++17", "-O3", "--expt-relaxed-constexpr", "-I", csrc]
-    sources = [os.path.join(here, "after_failure.cu")] + [os.path.join(csrc, f + ".cu") for f in (
-        "attention", "elementwise", "q8_gemm", "q8_gemm_tc", "q8_narrow", "runtime", "synth", "tma_host")]
-    objects = [str(tmp_path / (os.path.basename(s) + ".o")) for s in sources]
-    with ThreadPoolExecutor(len(sources)) as ex:
-        list(ex.map(lambda so: subprocess.run(nvcc + ["-c", so[0], "-o", so[1]], check=True, capture_output=True), zip(sources, objects)))
-    exe = str(tmp_path / "after_failure")
-    subprocess.run(nvcc + ["-o", exe] + objects + ["-ldl"], check=True, capture_output=True)
-    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
-    lines = r.stdout.split("\n")
-    assert r.returncode == 0 and len(lines) > 1, r.stdout
-    for line in lines[:-1]:
+
+    def compiled(sources):
+        objects = [os.path.join(out, os.path.basename(s) + ".o") for s in sources]
+        with ThreadPoolExecutor(len(sources)) as ex:
+            list(ex.map(lambda so: subprocess.run(nvcc + ["-c", so[0], "-o", so[1]], check=True, capture_output=True), zip(sources, objects)))
+        return objects
+
+    operators = compiled([os.path.join(csrc, f + ".cu") for f in ("attention", "elementwise", "q8_gemm", "q8_gemm_tc", "q8_narrow", "runtime",
+                                                                  "synth", "tma_host")])
+
+    def run(program):
+        exe = os.path.join(out, program)
+        subprocess.run(nvcc + ["-o", exe] + compiled([os.path.join(here, program + ".cu")]) + operators + ["-ldl"], check=True, capture_output=True)
+        r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stdout
+        return r.stdout.split("\n")[:-1]
+
+    return run
+
+
+def test_kernels_behind_a_failure_write_nothing(native):
+    """With a code in the status word a kernel leaves its outputs, the cache and the lengths as they are; once the code has
+    been read and cleared the same launch writes them all."""
+    lines = native("after_failure")
+    assert lines
+    for line in lines:
         what, behind, after = line.rsplit(" ", 2)
         assert (behind, after) == ("0", "1"), line
+
+
+def test_narrow_products_bit_for_bit(native):
+    lines = native("narrow_products")
+    assert lines and all(line.endswith(" 0") for line in lines), lines
