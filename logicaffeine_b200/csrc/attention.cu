@@ -3,8 +3,8 @@
 //
 // HBM-bound where the cache is large: every step streams the whole K and V history once (512 bytes per
 // position per KV head at D=128).  Latency-bound where it is small.  So:
-//   * a (sequence, KV head) pair is a cluster of one to eight CTAs, each of which takes an equal part of the pair's
-//     64-position K/V tiles: as many as two CTAs an SM leave room for, one where there are more pairs than that.  Clusters
+//   * a (sequence, KV head) pair is a cluster of one to eight CTAs (up to sixteen where sequences can be long), each of which takes an
+//     equal part of the pair's 64-position K/V tiles: as many as make the fewest and shortest rounds (attn_cut).  Clusters
 //     start as room comes free, so ragged lengths and several rounds of them even out by themselves;
 //   * a producer thread moves the tiles into a shared-memory ring with TMA tile loads (128-byte swizzle, no multicast)
 //     signalled on mbarriers; four consumer warps each own 16 positions of every tile;
@@ -21,12 +21,9 @@
 //     goes through global memory;
 //   * in a decode step what is older than it (lengths, cached rows) is read before the wait for
 //     the predecessor (AttnArgs::early_reads); every row of the query and the new K/V is one round of loads.
-// The form before this one was a persistent grid that cut the sequence of all pairs' tiles into 296 equal shares, with
-// the cut pairs' parts in global memory and an arrival counter for each share.  Measured, that one -> this one, with cold
-// caches and the events' 8 us (us, equal / ragged lengths): 64 sequences of 2048, 64/8 heads of 128 123 / 149 -> 109 / 72;
-// 32 of 4096, 28/4 76 / 62 -> 69 / 48; 7 of 2000, 14/2 of 64 27 / 24 -> 19 / 18; 16 of 128, 14/2 of 64 19 -> 16; one of 8000, 28/4 506 -> 25
-// (more than 64 parts went through a slow loop); 38 of 1300, 64/8 (8 pairs more than run at once) 69 / 86 -> 67 / 45.  Three
-// ring stages at head dimension 128 against two: 64 of 1300, 64/8 86 -> 85, 25 of 2000, 28/4 41 -> 40.
+// With cold caches and the events' 8 us (us): 64 sequences of 1024, 64/8 heads of 128 68; 32 of 4096, 28/4 66; 4 of 32768, 28/4 70;
+// 7 of up to 2000, 14/2 of 64 15; one of 4096, 64/8 19.  Three ring stages at head dimension 128 against two: 64 of 1300, 64/8 86 -> 85,
+// 25 of 2000, 28/4 41 -> 40.
 #include "ops.cuh"
 #include "q8_gemm_tc.cuh"
 #include "ptx.cuh"
@@ -34,8 +31,11 @@
 #include <cooperative_groups.h>
 #include <math.h>
 
+#include <limits.h>
+
 #include <algorithm>
 #include <mutex>
+#include <unordered_map>
 
 namespace logos {
 
@@ -50,7 +50,8 @@ constexpr int ATT_CTHREADS = ATT_CWARPS * 32;
 constexpr int ATT_THREADS = (ATT_CWARPS + 1) * 32;
 constexpr int ATT_BOX_BYTES = 64 * 128;  // 64 rows x 128 bytes
 constexpr int ATT_MAX_BATCH = 2048;      // sequences a call
-constexpr int ATT_MAX_PARTS = 8;         // a portable cluster
+constexpr int ATT_PUSHED_ROWS = 21;      // parts x ceil(group / parts), exact for up to 8 parts; of more, only counts that keep to it
+constexpr int ATT_WIDE = 16;             // CTAs of the largest cluster; the next has 8, as many as are portable
 
 struct AttnParams {
   const __half* q_f16;
@@ -79,7 +80,8 @@ struct AttnParams {
   int           o_dtype;
   ActOut        o_act;
   int           b, h_q, h_kv, l_max;
-  int           ranks;    // CTAs of a pair's cluster
+  int           ranks;    // CTAs of a pair's cluster; all of them have tiles from `all_from` tiles on, at most `few` below that
+  int           few, all_from;
   float         scale_log2;
   int*          status;
 };
@@ -408,15 +410,15 @@ struct AttnSmem {
   static constexpr int QS_STRIDE = D + 8;  // halfs; +16 bytes keeps ldmatrix rows on distinct banks
   static constexpr int STAGE_BYTES = 2 * (D / 64) * ATT_BOX_BYTES;
   static constexpr int STAGES = D == 64 ? 4 : 3;
-  static constexpr int PUSHED_ROWS = 21;                         // parts x ceil(group / parts): at most 21 of 16 and 8
+  static constexpr int PUSHED_ROWS = ATT_PUSHED_ROWS;
   static constexpr int ROW_BYTES = (D + 4) * 4;                  // sums, maximum, sum of weights, padding
   static constexpr int WORK = (16 * QS_STRIDE * 2 + 2 * D * 2 + ATT_CWARPS * 16 * 2 * 4 + 15) / 16 * 16;
   static constexpr int BYTES = STAGES * STAGE_BYTES + WORK + PUSHED_ROWS * ROW_BYTES + (2 * STAGES + 2) * 8;
 };
 static_assert(2 * (AttnSmem<128>::BYTES + 1024) <= 228 * 1024, "two CTAs fit an SM");
 
-// Grid: (sequence, KV head) pairs x CTAs of a cluster.
-template <int D>
+// Grid: (sequence, KV head) pairs x CTAs of a cluster, up to MAX_PARTS.
+template <int D, int MAX_PARTS>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
   using Smem = AttnSmem<D>;
@@ -450,7 +452,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int len = __ldcg(p.seq_len + b);
   const int len0 = len < p.l_max ? len : p.l_max, len_eff = attn_len_eff(p, len0);
   const int tiles = (len_eff + ATT_TILE - 1) / ATT_TILE;
-  const int parts = min(ranks, tiles);                       // CTAs with tiles
+  const int parts = tiles >= p.all_from ? ranks : min(p.few, tiles);   // CTAs with tiles
   const int t0 = rank < parts ? rank * tiles / parts : 0, t1 = rank < parts ? (rank + 1) * tiles / parts : 0;
   const int per = parts > 0 ? (G + parts - 1) / parts : G;   // row slots a part
   const int mine = rank < parts ? (G - rank + parts - 1) / parts : 0;   // rows finished here: rank, rank + parts, ...
@@ -591,28 +593,40 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       for (int e = 4 * tid; e < mine * D; e += 4 * ATT_CTHREADS) {
         const int slot = e / D, d = e - slot * D;
         const uint8_t* row = pushed + slot * ROW_BYTES;
-        float2 ml[ATT_MAX_PARTS];
+        constexpr int SOME = 8;   // parts whose maxima and sums are in registers
+        const auto of_part = [&](int i) { return *reinterpret_cast<const float2*>(row + i * per * ROW_BYTES + D * 4); };
+        float2 ml[SOME];
         float m = -INFINITY;
         bool whole = true;
 #pragma unroll
-        for (int i = 0; i < ATT_MAX_PARTS; ++i) {
-          ml[i] = i < parts ? *reinterpret_cast<const float2*>(row + i * per * ROW_BYTES + D * 4) : make_float2(-INFINITY, 0.f);
+        for (int i = 0; i < SOME; ++i) {
+          ml[i] = i < parts ? of_part(i) : make_float2(-INFINITY, 0.f);
           m = fmaxf(m, ml[i].x);
           whole = whole && ml[i].y != NO_SUMS;
         }
+        if constexpr (MAX_PARTS > SOME)
+#pragma unroll 1
+          for (int i = SOME; i < parts; ++i) {
+            m = fmaxf(m, of_part(i).x);
+            whole = whole && of_part(i).y != NO_SUMS;
+          }
         if (!whole) continue;
         const float muse = (m == -INFINITY) ? 0.f : m;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float L = 0.f;
+        const auto add = [&](int i, float2 of) {
+          const float wgt = exp2f(of.x - muse);
+          const float4 v = *reinterpret_cast<const float4*>(row + i * per * ROW_BYTES + d * 4);
+          acc.x = fmaf(v.x, wgt, acc.x); acc.y = fmaf(v.y, wgt, acc.y);
+          acc.z = fmaf(v.z, wgt, acc.z); acc.w = fmaf(v.w, wgt, acc.w);
+          L = fmaf(of.y, wgt, L);
+        };
 #pragma unroll
-        for (int i = 0; i < ATT_MAX_PARTS; ++i)
-          if (i < parts) {
-            const float wgt = exp2f(ml[i].x - muse);
-            const float4 v = *reinterpret_cast<const float4*>(row + i * per * ROW_BYTES + d * 4);
-            acc.x = fmaf(v.x, wgt, acc.x); acc.y = fmaf(v.y, wgt, acc.y);
-            acc.z = fmaf(v.z, wgt, acc.z); acc.w = fmaf(v.w, wgt, acc.w);
-            L = fmaf(ml[i].y, wgt, L);
-          }
+        for (int i = 0; i < SOME; ++i)
+          if (i < parts) add(i, ml[i]);
+        if constexpr (MAX_PARTS > SOME)
+#pragma unroll 1
+          for (int i = SOME; i < parts; ++i) add(i, of_part(i));
         store_out4(p, o0 + (int64_t)(rank + slot * parts) * D + d, acc, L);
       }
       return;
@@ -661,12 +675,84 @@ __global__ void kv_append_rope_kernel(__half* k_cache, __half* v_cache, const __
   }
 }
 
-// CTAs of a pair's cluster: as many as two CTAs an SM leave room for, since all pairs then run at once; no more than a
-// sequence can have tiles.  With more pairs than that one each (in turn): two for 300 pairs of 2000 positions, 8/1 heads of
-// 128, 96 -> 92 us, but 304 to 512 pairs of 1300, 64/8 heads, lost up to 13 % by it.
-int attn_ranks(const AttnArgs& a) {
-  const int64_t room = 2 * (int64_t)sm_count(a.device), tiles_max = (a.l_max + ATT_TILE - 1) / ATT_TILE;
-  return (int)std::min<int64_t>({ATT_MAX_PARTS, std::max<int64_t>(1, room / (a.b * a.h_kv)), tiles_max});
+// Clusters of 1 to 16 CTAs that run at once, with two CTAs an SM and with one.  A cluster lies within a GPC, so that is fewer than
+// the SMs would hold: of 8 CTAs 33 and 15 on a B200, of 7 37 and 15, of 16 14 and 7.
+struct ClusterRoom {
+  int two[ATT_WIDE + 1] = {}, one[ATT_WIDE + 1] = {};
+};
+constexpr int ATT_ONE_AN_SM = 115 * 1024;   // bytes of shared memory of which an SM has no two
+
+template <int D>
+logos_status_t cluster_room(int device, const ClusterRoom** out) {
+  static std::mutex mu;
+  static std::unordered_map<int, ClusterRoom> rooms;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = rooms.find(device);
+  if (it == rooms.end()) {
+    LOGOS_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_attn_kernel<D, ATT_WIDE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    ClusterRoom room;
+    for (int r = 1; r <= ATT_WIDE; ++r) {
+      auto kernel = r <= 8 ? gqa_decode_attn_kernel<D, 8> : gqa_decode_attn_kernel<D, ATT_WIDE>;
+      LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), device, std::max(AttnSmem<D>::BYTES, ATT_ONE_AN_SM)));
+      for (int* fit : {&room.two[r], &room.one[r]}) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)r;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)r);
+        cfg.blockDim = dim3(ATT_THREADS);
+        cfg.dynamicSmemBytes = (size_t)(fit == &room.two[r] ? AttnSmem<D>::BYTES : ATT_ONE_AN_SM);
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        LOGOS_CUDA_TRY(cudaOccupancyMaxActiveClusters(fit, kernel, &cfg));
+      }
+    }
+    it = rooms.emplace(device, room).first;
+  }
+  *out = &it->second;
+  return LOGOS_OK;
+}
+
+// How the pairs' tiles are cut.
+struct AttnCut {
+  int ranks = 1, few = 1, all_from = INT_MAX;   // see AttnParams
+  bool one_an_sm = false;
+};
+
+// What bounds a cut is its rounds: a cluster that does not run at once waits for one that does, and a last round of few clusters
+// takes nearly as long as a full one (0.9 of it, from 34 to 128 pairs of 32768).  So: rounds x (tiles of a part + 16, for what a round
+// has besides: start, ramp, exchange).  In a decode step the neighbouring kernels have CTAs on the SMs too, and a round that
+// needs nearly all of them waits: 32 pairs in clusters of 8, of which 33 fit, 1187 us a step of the 32B shape, of 7 1149.  The rule before took 2 x SMs / pairs CTAs without a look at what fits, and so
+// two rounds for 16 pairs (8 x 16 with one CTA an SM: 15 clusters fit) or 38 (7 x 38: 37 fit).  That one -> this one, us:
+//   28/4 heads of 128, 4 x 32768 101 -> 67; 64/8, 38 x 4096 148 -> 134; 14/2 of 64, 7 ragged ones up to 131072 121 -> 85;
+//   a step of the 0.5B shape at batch 8 and 450 positions 638 -> 564, 9 and 1500 771 -> 689, 24 and 128 921 -> 829; of the 32B shape
+//   (8 layers) at batch 2 and 2000 1294 -> 1255.
+AttnCut attn_cut(int64_t pairs, int64_t tiles_max, int group, bool in_step, const ClusterRoom& room) {
+  AttnCut c;
+  // More than eight CTAs, which are not portable, only where sequences can be long: such clusters start later (8/1 heads, 8 x 3000
+  // in a cache of 131073 17.8 -> 21 us; 8 x 131072 162 -> 99).  They are used from four tiles a CTA on.
+  const int64_t most = std::min<int64_t>(tiles_max, tiles_max >= 512 ? ATT_WIDE : 8);
+  // More pairs than run at once: parts shorten the last round, but want 16 tiles each, in the sequence at hand too.
+  const bool many = pairs > room.two[1];
+  double best = 0.;
+  for (int r = 1; r <= most; ++r) {
+    if (room.two[r] < 1 || r * ((group + r - 1) / r) > ATT_PUSHED_ROWS || (many && r > 1 && tiles_max < 16 * r)) continue;
+    const int64_t full = pairs / room.two[r], rest = pairs % room.two[r];
+    double rounds = (double)full + (rest ? std::max(0.9, (double)rest / room.two[r]) : 0.);
+    if (in_step && rounds > 0.93 && rounds <= 1.) rounds = 1.1;
+    const double cost = rounds * (double)((tiles_max + r - 1) / r + 16);
+    if (best > 0. && cost > best) continue;
+    best = cost;
+    c.ranks = r;
+  }
+  c.few = many ? 1 : std::min(c.ranks, 8);
+  if (c.ranks > c.few) c.all_from = (many ? 16 : 4) * c.ranks;
+  // Where all clusters run at once with a CTA an SM, a CTA asks for more than half of an SM's shared memory: a cluster's CTAs are packed
+  // onto an SM otherwise.  A step of the 0.5B shape, batch 16 at 128 positions (96 CTAs) 748 -> 685 us; with more CTAs than
+  // that it only keeps them and the neighbouring kernels' CTAs apart: batch 16 at 1500 positions (256 CTAs) 769 -> 963.
+  c.one_an_sm = pairs <= room.one[c.ranks];
+  return c;
 }
 
 template <int D>
@@ -695,23 +781,20 @@ logos_status_t launch_attn_t(const AttnArgs& a, cudaStream_t st) {
   p.early_reads = a.early_reads;
   p.o = a.o; p.o_dtype = a.o_dtype; p.o_act = a.o_act;
   p.b = (int)a.b; p.h_q = (int)a.h_q; p.h_kv = (int)a.h_kv; p.l_max = (int)a.l_max;
-  p.ranks = attn_ranks(a);
   p.scale_log2 = a.scale * 1.4426950408889634f;
   p.status = a.ext_status ? a.ext_status : kernel_status_ptr(a.device);
   if (!p.status) return fail(LOGOS_ERROR, "attention: no kernel status word");
 
-  auto kernel = gqa_decode_attn_kernel<D>;
-  // Where there are SMs for all, a CTA asks for more than half of one's shared memory: a cluster's CTAs are packed onto an SM
-  // otherwise (three of head dimension 64 fit one).  A step of the 0.5B shape, batch 16 at 128 positions (96 CTAs) 748 -> 685 us,
-  // batch 8 591 -> 553; with more CTAs than SMs it only keeps them and the neighbouring kernels' CTAs apart: batch 16 at 1500
-  // positions (256 CTAs) 769 -> 963.
-  const int64_t ctas = a.b * a.h_kv * p.ranks;
-  const int smem = std::max(AttnSmem<D>::BYTES, ctas <= sm_count(a.device) ? 115 * 1024 : 0);
-  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), a.device, smem));
+  const ClusterRoom* room = nullptr;
+  LOGOS_TRY(cluster_room<D>(a.device, &room));
+  const int64_t pairs = a.b * a.h_kv;
+  const AttnCut cut = attn_cut(pairs, (a.l_max + ATT_TILE - 1) / ATT_TILE, (int)(a.h_q / a.h_kv), a.early_reads, *room);
+  auto kernel = cut.ranks <= 8 ? gqa_decode_attn_kernel<D, 8> : gqa_decode_attn_kernel<D, ATT_WIDE>;
+  p.ranks = cut.ranks; p.few = cut.few; p.all_from = cut.all_from;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.gridDim = dim3((unsigned)(pairs * cut.ranks));
   cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.dynamicSmemBytes = (size_t)(cut.one_an_sm ? std::max(AttnSmem<D>::BYTES, ATT_ONE_AN_SM) : AttnSmem<D>::BYTES);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;

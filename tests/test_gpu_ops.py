@@ -422,7 +422,13 @@ def test_gqa_decode_attn_fused_kv_bit_exact(llm, oracle, b, hq, hkv, d, lmax, le
     (1, 2, 1, 64, 64 * 200, [64 * 200 - 2]),           # one pair cut into more parts than the list holds
     (1, 12, 2, 128, 64 * 70, [64 * 66 - 1]),           # more shares than tiles: some hold none
     (2, 16, 1, 64, 64 * 64, [64 * 63, 0]),             # 64 parts beside a pair of one tile
-    (40, 32, 8, 128, 200, [(37 * i) % 199 for i in range(40)]),   # more pairs than shares: whole and cut ones
+    (40, 32, 8, 128, 200, [(37 * i) % 199 for i in range(40)]),   # more pairs than run at once, of few tiles
+    (1, 16, 1, 128, 64 * 7, [64 * 7 - 2]),             # seven parts of sixteen rows: all of the exchange's room
+    (1, 15, 1, 64, 64 * 512, [64 * 512 - 2]),          # sixteen parts
+    (3, 16, 1, 64, 64 * 512, [64 * 64 - 3, 64 * 64 + 5, 100]),     # just below and above where all sixteen are used
+    (16, 16, 1, 64, 64 * 512, [64 * 39 + 62] + [64 * 40 + i for i in range(8)] + [9000] + [70 * i for i in range(6)]),   # ten parts, 20 rows
+    (16, 7, 1, 64, 64 * 512, [64 * 48 - 2, 64 * 48, 20000] + [301 * i for i in range(13)]),                             # twelve
+    (19, 16, 16, 64, 64 * 40, [64 * 32 - 2, 64 * 32, 64 * 40 - 2] + [11 * i for i in range(16)]),    # more pairs than run at once, two parts
 ])
 def test_gqa_decode_attn_cut_pairs_fold_the_same_every_time(llm, oracle, b, hq, hkv, d, lmax, lens):
     O = oracle
