@@ -114,7 +114,7 @@ logos_status_t check_launch(const char* kernel);
 
 // Process-wide count of kernel launches by kind (read through logos_launch_counts).
 enum LaunchKind : int {
-  LK_GEMV = 0, LK_GEMM_TC = 1, LK_GEMM_SIMT = 2, LK_ATTN = 3, LK_ELEMWISE = 5, LK_SYNTH = 6,   // 4: no kind any more
+  LK_GEMV = 0, LK_GEMM_TC = 1, LK_GEMM_SIMT = 2, LK_ATTN = 3, LK_ELEMWISE = 5, LK_SYNTH = 6,   // 4 is free
   LK_KINDS = 8
 };
 void count_launch(int kind, int64_t n = 1);

@@ -76,6 +76,28 @@ def test_layers_of_any_width_and_batch(llm, oracle, hidden, ffn, h_q, h_kv, head
     ref.close()
 
 
+# One activation plane in the products that hold the norms; the same tokens go into both models.  The bound is that of the prompt's
+# logits above: f32 sums in another order tip 16-bit roundings, and those the later ones.
+@pytest.mark.parametrize("act", ["F16", "BF16"])
+@pytest.mark.parametrize("batch", [1, 4, 8, 16])
+def test_one_activation_plane_in_a_step(llm, oracle, act, batch):
+    O = oracle
+    cfg = dict(SMALL, batch=batch)
+    toks = O.synth_fill(O.I32, 3, 6, 999, 0, batch * 9, 0.0, float(cfg["vocab"])).reshape(batch, 9)
+    ref = O.Llm(tp_degree=1, tp_rank=0, device=0, act_dtype=getattr(O, act), **cfg)
+    gpu = llm.Llm(act_dtype=getattr(O, act), **cfg)
+    ref.prefill(toks[:, :6])
+    gpu.prefill(toks[:, :6])
+    for step in range(6, 9):
+        ref.set_tokens(toks[:, step].copy())
+        gpu.setTokens(toks[:, step].copy())
+        ref.decode_step()
+        gpu.decodeStep()
+        assert rel_l2(gpu.readLogits(), ref.read_logits()) < 2e-2
+    gpu.free()
+    ref.close()
+
+
 def test_decode_is_repeatable_after_rewind(llm, oracle):
     O = oracle
     toks = np.arange(SMALL["batch"] * 6, dtype=np.int32).reshape(SMALL["batch"], 6) % SMALL["vocab"]

@@ -59,7 +59,7 @@ def test_fixed_scratch_attention_matches_the_allocating_entry_point_twice(llm, o
 
 
 def test_fixed_scratch_refuses_what_does_not_fit(llm):
-    # the most sequences one call takes is 2048 (as it always was)
+    # the most sequences one call takes is 2048, in every attention entry point
     b, hq, hkv, d, lmax = 2049, 2, 1, 64, 64
     q = llm.DeviceBuffer(b * hq * d * 2)
     cache = llm.DeviceBuffer(b * hkv * lmax * d * 2)
