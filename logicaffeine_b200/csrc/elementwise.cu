@@ -52,8 +52,7 @@ __global__ void swiglu_f32_kernel(const float* __restrict__ gate, const float* _
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < count; i += step) {
     float g = gate[i];
-    float sg = __fdiv_rn(g, 1.0f + expf(-g));
-    y[i] = __fmul_rn(sg, up[i]);
+    y[i] = __fmul_rn(silu_f(g), up[i]);
   }
 }
 

@@ -27,7 +27,6 @@ __device__ __forceinline__ void store_out(void* c, int dtype, int64_t i, float v
   else if (dtype == LOGOS_BF16) reinterpret_cast<__nv_bfloat16*>(c)[i] = __float2bfloat16_rn(v);
   else reinterpret_cast<float*>(c)[i] = v;
 }
-__device__ __forceinline__ float silu_f(float g) { return __fdiv_rn(g, 1.0f + expf(-g)); }
 
 constexpr int SIMT_TN = 32;  // weight rows per CTA
 constexpr int SIMT_TM = 32;  // tokens per CTA

@@ -191,17 +191,6 @@ struct Ring {
   }
 };
 
-__device__ __forceinline__ float silu_f(float g) { return __fdiv_rn(g, 1.0f + expf(-g)); }
-
-// two int8 (bytes of w ^ 0x80808080, i.e. of q + 128 as unsigned bytes) -> packed fp16 pair, exact
-__device__ __forceinline__ uint32_t cvt_pair(uint32_t w_xor80, uint32_t selector) {
-  uint32_t bits = __byte_perm(w_xor80, 0x64646464u, selector);   // 0x64bb = 1024 + (q + 128)
-  __half2 h = *reinterpret_cast<__half2*>(&bits);
-  const uint32_t bias_bits = 0x64806480u;                        // 1152 = 1024 + 128
-  __half2 r = __hsub2(h, *reinterpret_cast<const __half2*>(&bias_bits));
-  return *reinterpret_cast<uint32_t*>(&r);
-}
-
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier; both addresses and the
 // size are multiples of 16
 __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gmem_src, uint32_t bytes, uint32_t bar) {

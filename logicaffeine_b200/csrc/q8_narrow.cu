@@ -64,24 +64,8 @@ __device__ __forceinline__ uint2 lds_v2(uint32_t addr) {
   asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
   return v;
 }
-// bytes of q + 128 -> packed fp16 pair of q, exact (0x64bb = 1024 + byte)
-__device__ __forceinline__ uint32_t q_pair(uint32_t w, uint32_t selector) {
-  const uint32_t bits = __byte_perm(w, 0x64646464u, selector), bias = 0x64806480u;
-  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&bits), *reinterpret_cast<const __half2*>(&bias));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
-__device__ __forceinline__ float nw_silu(float g) { return __fdiv_rn(g, 1.0f + expf(-g)); }
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-// Two activations into a word of either plane, with act_store's arithmetic.
-__device__ __forceinline__ void plane_words(float2 x, uint32_t* hi, uint32_t* lo) {
-  x = make_float2(act_clamp(x.x), act_clamp(x.y));
-  const __half2 h = __floats2half2_rn(x.x, x.y);
-  const float2 l = __ffma2_rn(__half22float2(h), make_float2(-2048.f, -2048.f), __fmul2_rn(x, make_float2(2048.f, 2048.f)));
-  const __half2 lh = __floats2half2_rn(l.x, l.y);   // (x - h) * 2048: exact before this rounding
-  *hi = *reinterpret_cast<const uint32_t*>(&h);
-  *lo = *reinterpret_cast<const uint32_t*>(&lh);
 }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
 // sum / k, correctly rounded: with the reciprocal's rounded value at hand one step on the quotient's remainder gives that
@@ -208,10 +192,10 @@ q8_narrow_kernel(const NarrowParams p) {
         if (p.act_mode == LOGOS_BF16)
 #pragma unroll
           for (int i = 0; i < 4; ++i) n[i] = __bfloat1622float2(__floats2bfloat162_rn(n[i].x, n[i].y));
-        plane_words(n[0], &bh[b][j].x, &bl[b][j].x);
-        plane_words(n[1], &bh[b][j].y, &bl[b][j].y);
-        plane_words(n[2], &bh[b][j].z, &bl[b][j].z);
-        plane_words(n[3], &bh[b][j].w, &bl[b][j].w);
+        act_words(n[0], &bh[b][j].x, &bl[b][j].x);
+        act_words(n[1], &bh[b][j].y, &bl[b][j].y);
+        act_words(n[2], &bh[b][j].z, &bl[b][j].z);
+        act_words(n[3], &bh[b][j].w, &bl[b][j].w);
         if (MERGED && g >= 4) bh[b][j] = two ? bl[b][j] : make_uint4(0u, 0u, 0u, 0u);
       }
     }
@@ -257,10 +241,10 @@ q8_narrow_kernel(const NarrowParams p) {
         const uint32_t w0[2] = {w[2 * b].x, w[2 * b].y}, w1[2] = {w[2 * b + 1].x, w[2 * b + 1].y};
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          a[b][k][0] = q_pair(w0[k], 0x4140);
-          a[b][k][1] = q_pair(w1[k], 0x4140);
-          a[b][k][2] = q_pair(w0[k], 0x4342);
-          a[b][k][3] = q_pair(w1[k], 0x4342);
+          a[b][k][0] = cvt_pair(w0[k], 0x4140);
+          a[b][k][1] = cvt_pair(w1[k], 0x4140);
+          a[b][k][2] = cvt_pair(w0[k], 0x4342);
+          a[b][k][3] = cvt_pair(w1[k], 0x4342);
         }
       }
       float d[2][NT][4];
@@ -339,7 +323,7 @@ q8_narrow_kernel(const NarrowParams p) {
     if (n >= p.n || t >= rows || s_prior != 0) continue;
     const int64_t row = m0 + t;
     if (OUT == NARROW_SWIGLU) {
-      act_store(p.planes, row * (p.n / 2) + n / 2, __fmul_rn(nw_silu(v.x), v.y));   // columns (2j, 2j + 1) are (gate_j, up_j)
+      act_store(p.planes, row * (p.n / 2) + n / 2, __fmul_rn(silu_f(v.x), v.y));   // columns (2j, 2j + 1) are (gate_j, up_j)
     } else {
       float2* c = reinterpret_cast<float2*>(p.c + row * p.n + n);
       if (!NORM) v = add2(e == tid ? h0 : __ldcg(c), v);
