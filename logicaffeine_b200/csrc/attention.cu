@@ -689,9 +689,10 @@ logos_status_t cluster_room(int device, const ClusterRoom** out) {
   std::lock_guard<std::mutex> lk(mu);
   auto it = rooms.find(device);
   if (it == rooms.end()) {
-    LOGOS_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_attn_kernel<D, ATT_WIDE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // a size that the device or the driver does not take has no room; one CTA always has
     ClusterRoom room;
-    for (int r = 1; r <= ATT_WIDE; ++r) {
+    const int most = cudaFuncSetAttribute(gqa_decode_attn_kernel<D, ATT_WIDE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess ? ATT_WIDE : 8;
+    for (int r = 1; r <= most; ++r) {
       auto kernel = r <= 8 ? gqa_decode_attn_kernel<D, 8> : gqa_decode_attn_kernel<D, ATT_WIDE>;
       LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), device, std::max(AttnSmem<D>::BYTES, ATT_ONE_AN_SM)));
       for (int* fit : {&room.two[r], &room.one[r]}) {
@@ -705,9 +706,12 @@ logos_status_t cluster_room(int device, const ClusterRoom** out) {
         cfg.dynamicSmemBytes = (size_t)(fit == &room.two[r] ? AttnSmem<D>::BYTES : ATT_ONE_AN_SM);
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        LOGOS_CUDA_TRY(cudaOccupancyMaxActiveClusters(fit, kernel, &cfg));
+        if (cudaOccupancyMaxActiveClusters(fit, kernel, &cfg) != cudaSuccess) *fit = 0;
       }
     }
+    cudaGetLastError();
+    room.two[1] = std::max(room.two[1], 1);
+    room.one[1] = std::max(room.one[1], 1);
     it = rooms.emplace(device, room).first;
   }
   *out = &it->second;

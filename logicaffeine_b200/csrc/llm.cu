@@ -537,8 +537,13 @@ logos_status_t step_tail(Model* m, int parts, bool sample, bool log_tokens, cons
 }
 
 // Whether a layer's products run in the kernels that hold the norms, SwiGLU and the residual adds too (q8_narrow.cu):
-// where they take the shapes, up to 16 sequences (one token tile).  us a step of the 0.5B shape, the kernels of
-// q8_gemm_tc.cu and these, with one attention for both: batch 1 904 / 621, 8 905 / 629, 16 900 / 763, 32 1000 / 995.
+// where they take the shapes, up to 16 sequences (one token tile).  The line is that of the 0.5B shape.  us a step of 12 layers, the
+// kernels of q8_gemm_tc.cu / these, with the same attention and today's K splits, hidden and FFN:
+//   896, 4864    batch 1 342 / 245, 8 350 / 278, 16 357 / 342, 17 393 / 437, 32 405 / 451
+//   512, 2048    batch 1 316 / 170, 16 324 / 217, 32 362 / 255, 64 443 / 320
+//   1024, 4096   batch 1 359 / 239, 16 388 / 325, 32 445 / 433
+//   1024, 8192   batch 1 392 / 284, 8 404 / 334, 12 415 / 430, 16 416 / 441
+// Narrow layers would gain beyond it, and wide FFNs lose up to 6 % just below it.
 bool narrow_layers(const Model* m) {
   const logos_llm_config_t& c = m->cfg;
   if (m->tp.degree > 1 || c.batch > 16) return false;
