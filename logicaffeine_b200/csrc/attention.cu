@@ -435,7 +435,6 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   uint64_t* bar_empty = bar_full + STAGES;
   uint64_t* bar_parts = bar_empty + STAGES;
   int& s_bump = *reinterpret_cast<int*>(bar_parts + 1);
-  int& s_prior = *(&s_bump + 1);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = p.h_q / p.h_kv;
@@ -447,7 +446,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   // write any of them: everything waits.
   if (!p.early_reads) pdl_wait();
   // a kernel that gave up earlier left a code behind: do not start new work on top of it
-  // (one thread's value counts: the CTA takes one decision)
+  // (the CTA takes one decision: a code that any of its threads has read)
   const int status = *reinterpret_cast<volatile int*>(p.status);
   const int len = __ldcg(p.seq_len + b);
   const int len0 = len < p.l_max ? len : p.l_max, len_eff = attn_len_eff(p, len0);
@@ -457,7 +456,6 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int per = parts > 0 ? (G + parts - 1) / parts : G;   // row slots a part
   const int mine = rank < parts ? (G - rank + parts - 1) / parts : 0;   // rows finished here: rank, rank + parts, ...
   if (tid == 0) {
-    s_prior = status;
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&bar_full[i], 1);
       mbar_init(&bar_empty[i], ATT_CWARPS);
@@ -466,8 +464,7 @@ gqa_decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     fence_barrier_init();
     mbar_arrive_expect_tx(bar_parts, (parts > 1 ? parts - 1 : 0) * mine * (D * 4 + 8));
   }
-  __syncthreads();
-  const bool prior = s_prior != 0;
+  const bool prior = __syncthreads_or(status != 0);
   cg::cluster_group cluster = cg::this_cluster();
   cluster.barrier_arrive();   // "this CTA runs, its barrier stands": before anyone pushes into it
   const int64_t row_base = ((int64_t)b * p.h_kv + kvh) * p.l_max;
@@ -732,11 +729,16 @@ struct AttnCut {
 //   28/4 heads of 128, 4 x 32768 101 -> 67; 64/8, 38 x 4096 148 -> 134; 14/2 of 64, 7 ragged ones up to 131072 121 -> 85;
 //   a step of the 0.5B shape at batch 8 and 450 positions 638 -> 564, 9 and 1500 771 -> 689, 24 and 128 921 -> 829; of the 32B shape
 //   (8 layers) at batch 2 and 2000 1294 -> 1255.
-AttnCut attn_cut(int64_t pairs, int64_t tiles_max, int group, bool in_step, const ClusterRoom& room) {
+AttnCut attn_cut(int64_t pairs, int64_t tiles_max, int group, int d, bool in_step, const ClusterRoom& room) {
   AttnCut c;
   // More than eight CTAs, which are not portable, only where sequences can be long: such clusters start later (8/1 heads, 8 x 3000
   // in a cache of 131073 17.8 -> 21 us; 8 x 131072 162 -> 99).  They are used from four tiles a CTA on.
-  const int64_t most = std::min<int64_t>(tiles_max, tiles_max >= 512 ? ATT_WIDE : 8);
+  // In a step, short sequences at head dimension 64 get parts of two tiles at least: a tile takes 0.4 us there, no more than what a
+  // part costs the chain.  A step of the 0.5B shape at batch 16 and 128 positions 678 -> 663 us, 600 708 -> 696, batch 12 and 350 672 -> 663,
+  // 24 and 128 827 -> 816.  With fewer pairs the SMs are idle anyway (batch 1 at 260 469 -> 481), with more they are full
+  // of one tile's parts too (batch 48 at 350 1001 -> 1015).
+  const bool pays = !in_step || d != 64 || pairs < 8 || pairs > 56 || tiles_max >= 12;
+  const int64_t most = pays ? std::min<int64_t>(tiles_max, tiles_max >= 512 ? ATT_WIDE : 8) : std::max<int64_t>(1, tiles_max / 2);
   // More pairs than run at once: parts shorten the last round, but want 16 tiles each, in the sequence at hand too.
   const bool many = pairs > room.two[1];
   double best = 0.;
@@ -792,7 +794,7 @@ logos_status_t launch_attn_t(const AttnArgs& a, cudaStream_t st) {
   const ClusterRoom* room = nullptr;
   LOGOS_TRY(cluster_room<D>(a.device, &room));
   const int64_t pairs = a.b * a.h_kv;
-  const AttnCut cut = attn_cut(pairs, (a.l_max + ATT_TILE - 1) / ATT_TILE, (int)(a.h_q / a.h_kv), a.early_reads, *room);
+  const AttnCut cut = attn_cut(pairs, (a.l_max + ATT_TILE - 1) / ATT_TILE, (int)(a.h_q / a.h_kv), D, a.early_reads, *room);
   auto kernel = cut.ranks <= 8 ? gqa_decode_attn_kernel<D, 8> : gqa_decode_attn_kernel<D, ATT_WIDE>;
   p.ranks = cut.ranks; p.few = cut.few; p.all_from = cut.all_from;
   cudaLaunchConfig_t cfg = {};
