@@ -18,7 +18,7 @@
 //     pay for its allocation, hand-offs and read-back.
 // Measured on a B200, from the wait's return to the last store, 0.5B shape at 8 / 16 tokens (us): qkv 2.4 / 2.9, o_proj 1.5 / 2.0,
 // gate/up 4.4 / 5.8, down_proj 2.4 / 3.0 (the rounded norm factor and the status word came later: 0.1 together); a step at batch
-// 1 / 8 / 16 477 / 547 / 674 (with norm and GEMM kernels of their own see narrow_layers in llm.cu).
+// 1 / 8 / 16 477 / 546 / 663 (with norm and GEMM kernels of their own see narrow_layers in llm.cu).
 // Of gate/up's time 2.1 / 2.6 us are the products: mma.sync runs at one m16n8k16 in 4.3 cycles an SM.
 // Arithmetic as in q8_gemm_tc.cu: int8 -> fp16 exactly, activations in two fp16 planes, a Q8 block's products summed on
 // the tensor core (q * lo' first, times 2^-11, then q * hi), then sum += scale * partial in f32.
