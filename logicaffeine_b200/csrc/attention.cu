@@ -724,26 +724,29 @@ struct AttnCut {
 // What bounds a cut is its rounds: a cluster that does not run at once waits for one that does, and a last round of few clusters
 // takes nearly as long as a full one (0.9 of it, from 34 to 128 pairs of 32768).  So: rounds x (tiles of a part + 16, for what a round
 // has besides: start, ramp, exchange).  In a decode step the neighbouring kernels have CTAs on the SMs too, and a round that
-// needs nearly all of them waits: 32 pairs in clusters of 8, of which 33 fit, 1187 us a step of the 32B shape, of 7 1149.  The rule before took 2 x SMs / pairs CTAs without a look at what fits, and so
-// two rounds for 16 pairs (8 x 16 with one CTA an SM: 15 clusters fit) or 38 (7 x 38: 37 fit).  That one -> this one, us:
+// needs nearly all of them waits: 32 pairs in clusters of 8, of which 33 fit, 1187 us a step of the 32B shape, of 7 1149.
+// The rule before took 2 x SMs / pairs CTAs without a look at what fits, and so two rounds for 16 pairs (8 x 16 with
+// one CTA an SM: 15 clusters fit) or 38 (7 x 38: 37 fit).  That one -> this one, us:
 //   28/4 heads of 128, 4 x 32768 101 -> 67; 64/8, 38 x 4096 148 -> 134; 14/2 of 64, 7 ragged ones up to 131072 121 -> 85;
 //   a step of the 0.5B shape at batch 8 and 450 positions 638 -> 564, 9 and 1500 771 -> 689, 24 and 128 921 -> 829; of the 32B shape
 //   (8 layers) at batch 2 and 2000 1294 -> 1255.
 AttnCut attn_cut(int64_t pairs, int64_t tiles_max, int group, int d, bool in_step, const ClusterRoom& room) {
   AttnCut c;
-  // More than eight CTAs, which are not portable, only where sequences can be long: such clusters start later (8/1 heads, 8 x 3000
-  // in a cache of 131073 17.8 -> 21 us; 8 x 131072 162 -> 99).  They are used from four tiles a CTA on.
   // In a step, short sequences at head dimension 64 get parts of two tiles at least: a tile takes 0.4 us there, no more than what a
   // part costs the chain.  A step of the 0.5B shape at batch 16 and 128 positions 678 -> 663 us, 600 708 -> 696, batch 12 and 350 672 -> 663,
   // 24 and 128 827 -> 816.  With fewer pairs the SMs are idle anyway (batch 1 at 260 469 -> 481), with more they are full
   // of one tile's parts too (batch 48 at 350 1001 -> 1015).
   const bool pays = !in_step || d != 64 || pairs < 8 || pairs > 56 || tiles_max >= 12;
+  // More than eight CTAs, which are not portable, only where sequences can be long: such clusters start later (8/1 heads, 8 x 3000
+  // in a cache of 131073 17.8 -> 21 us; 8 x 131072 162 -> 99).  They are used from four tiles a CTA on.  In a step only the largest:
+  // 12 layers of the 0.5B shape in a cache of 33000, batch 4 at 3000 / 30000 positions 284 / 540 -> 293 / 453 us, but by clusters of 13
+  // batch 7 298 / 560 -> 312 / 523.
   const int64_t most = pays ? std::min<int64_t>(tiles_max, tiles_max >= 512 ? ATT_WIDE : 8) : std::max<int64_t>(1, tiles_max / 2);
   // More pairs than run at once: parts shorten the last round, but want 16 tiles each, in the sequence at hand too.
   const bool many = pairs > room.two[1];
   double best = 0.;
   for (int r = 1; r <= most; ++r) {
-    if (room.two[r] < 1 || r * ((group + r - 1) / r) > ATT_PUSHED_ROWS || (many && r > 1 && tiles_max < 16 * r)) continue;
+    if (room.two[r] < 1 || (in_step && r > 8 && r < ATT_WIDE) || r * ((group + r - 1) / r) > ATT_PUSHED_ROWS || (many && r > 1 && tiles_max < 16 * r)) continue;
     const int64_t full = pairs / room.two[r], rest = pairs % room.two[r];
     double rounds = (double)full + (rest ? std::max(0.9, (double)rest / room.two[r]) : 0.);
     if (in_step && rounds > 0.93 && rounds <= 1.) rounds = 1.1;
