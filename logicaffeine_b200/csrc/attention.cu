@@ -930,6 +930,7 @@ logos_status_t logos_gqa_decode_attn_fixed_scratch(logos_handle_t q, logos_handl
     cudaStream_t st = as_stream(stream_or_null);
     a.q_f16 = qp; a.k_cache = kc; a.v_cache = vc; a.seq_len = sl; a.o = op; a.o_dtype = LOGOS_F16;
     a.b = b; a.h_q = h_q; a.h_kv = h_kv; a.d = d; a.l_max = l_max; a.scale = softmax_scale; a.device = dev;
+    OrderedScope ordered(st);
     return launch_gqa_decode_attn(a, st);
   });
 }
@@ -990,7 +991,9 @@ static logos_status_t attn_abi(bool fused, logos_handle_t q, logos_handle_t k_ne
   }
   a.b = b; a.h_q = h_q; a.h_kv = h_kv; a.d = d; a.l_max = l_max; a.scale = scale; a.device = dev;
   LOGOS_CUDA_TRY(cudaSetDevice(dev));
-  return launch_gqa_decode_attn(a, as_stream(stream));
+  const cudaStream_t st = as_stream(stream);
+  OrderedScope ordered(st);
+  return launch_gqa_decode_attn(a, st);
 }
 
 logos_status_t logos_gqa_decode_attn(logos_handle_t q, logos_handle_t k_cache, logos_handle_t v_cache,

@@ -343,6 +343,8 @@ __global__ void __launch_bounds__(256)
 gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const float* __restrict__ s, float* __restrict__ tiled,
                  int64_t n, int64_t kb, int64_t ktiles, int64_t act_blocks, unsigned* misfit, unsigned call) {
   // count8: groups of eight of the planes; rows of the planes are whole K tiles, rows of `a` kb * 32 values
+  // The product behind this kernel reads weights without a wait of its own: it may start once all before this one has ended.
+  pdl_wait();
   pdl_trigger();
   if ((int64_t)blockIdx.x < act_blocks) {
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -607,10 +609,8 @@ logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64
   const int64_t ktiles = (k + 127) / 128, count8 = m * ktiles * 16;
   const int64_t act_blocks = (count8 + 255) / 256, scale_blocks = tiled_or_null ? (n * ktiles + 255) / 256 : 0;
   const dim3 grid((unsigned)(act_blocks + scale_blocks));
-  if (a_dtype == LOGOS_BF16)
-    gemm_prep_kernel<true><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call);
-  else
-    gemm_prep_kernel<false><<<grid, 256, 0, st>>>(a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call);
+  auto kernel = a_dtype == LOGOS_BF16 ? gemm_prep_kernel<true> : gemm_prep_kernel<false>;
+  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(256), 0, st, a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call));
   count_launch(LK_ELEMWISE);
   return check_launch("gemm_prep_kernel");
 }

@@ -256,9 +256,9 @@ using namespace logos;
 
 // The stand-alone operators' way to the tensor-core kernel: activations into fp16 planes (and, where K is not
 // a multiple of 128, scales into the tile-major form) by one small kernel, then the product, then the
-// fold of the K splits.  The launches after the first are dependent ones: each kernel sets up, and the
-// product fetches its first weights, while the one before it finishes.  Nothing here writes weights, and the
-// first kernel is an ordinary launch, so what ran before in the stream has ended.
+// fold of the K splits.  The launches are dependent ones: each kernel sets up, and the product fetches its first
+// weights, while the one before it finishes.  Nothing here writes weights, and the first kernel lets the product start
+// only once what ran before in the stream has ended.
 constexpr int64_t STAGED_BYTES = 64ll << 20;   // sums staged at a time, see below: half of L2
 
 static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) {
@@ -328,7 +328,10 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     f.tiles_m = (e.m + SIMT_TM - 1) / SIMT_TM;
     return f;
   };
-  LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, misfit, call, st));
+  {
+    OrderedScope ordered(st);
+    LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, misfit, call, st));
+  }
   g.lda = lda;
   g.a = planes.hi;
   g.a_lo = planes.lo;

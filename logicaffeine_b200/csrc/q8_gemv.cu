@@ -58,7 +58,7 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 template <int R, bool X_IN_SMEM>
 __global__ void __launch_bounds__(GEMV_WARPS * 32, 1)
 q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const float* __restrict__ x,
-               float* __restrict__ y, int64_t n, int64_t k) {
+               float* __restrict__ y, int64_t n, int64_t k, bool early) {
   constexpr int U = 4 / R;   // chunks of a row that a lane has in a stage
   extern __shared__ float4 xs4[];
   const int tid = threadIdx.x;
@@ -69,8 +69,9 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
   const int xchunks = X_IN_SMEM ? (chunks + 31) / 32 * 32 : 0;
   uint8_t* ring = reinterpret_cast<uint8_t*>(xs4 + xchunks * 4) + warp * (GEMV_DEPTH * GEMV_STAGE);
   const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
-  // Dependent launch: the weights are read before the previous kernel of the stream has
-  // finished (the caller's scope promises nothing in it writes them); x and y wait for it.
+  // In a caller's scope the weights are read before the previous kernel of the stream has finished (the scope promises
+  // that nothing in it writes them); x and y wait for it.
+  if (!early) pdl_wait();
   pdl_trigger();
   const int64_t groups = (n + R - 1) / R, step = (int64_t)gridDim.x * warps;
   int64_t lg = blockIdx.x + (int64_t)gridDim.x * warp;   // the load cursor
@@ -105,7 +106,7 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
   };
 #pragma unroll
   for (int i = 0; i < GEMV_DEPTH - 1; ++i) load();
-  pdl_wait();
+  if (early) pdl_wait();
   if (X_IN_SMEM) {
     const float4* xg = reinterpret_cast<const float4*>(x);
     for (int i = tid; i < chunks * 4; i += blockDim.x) xs4[xs4_index(i >> 2, i & 3)] = __ldcg(xg + i);
@@ -180,7 +181,7 @@ logos_status_t launch_q8_gemv(const int8_t* q, const float* s, const float* x, f
                         : (in_smem ? q8_gemv_kernel<1, true> : q8_gemv_kernel<1, false>);
   LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kern), device, GEMV_SMEM));
   LOGOS_CUDA_TRY(launch_kernel(kern, dim3((unsigned)std::min(groups, sms)), dim3(warps * 32), (size_t)(ring(warps) + (in_smem ? xb : 0)),
-                               st, q, s, x, y, n, k));
+                               st, q, s, x, y, n, k, pdl_early()));
   count_launch(LK_GEMV);
   return check_launch("q8_gemv_kernel");
 }
@@ -201,6 +202,8 @@ extern "C" logos_status_t logos_q8_gemv(logos_handle_t q, logos_handle_t s, logo
     LOGOS_TRY(buf_ptr<float>(x, k, "x", &xp));
     LOGOS_TRY(buf_ptr<float>(y, n, "y", &yp));
     LOGOS_CUDA_TRY(cudaSetDevice(dev));
-    return launch_q8_gemv(qp, sp, xp, yp, n, k, dev, as_stream(stream_or_null));
+    const cudaStream_t st = as_stream(stream_or_null);
+    OrderedScope ordered(st);
+    return launch_q8_gemv(qp, sp, xp, yp, n, k, dev, st);
   });
 }

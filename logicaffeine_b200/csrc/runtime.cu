@@ -64,8 +64,9 @@ logos_status_t cuda_fail(cudaError_t e, const char* what) {
 static std::atomic<int64_t> g_launches[LK_KINDS];
 void count_launch(int kind, int64_t n) { g_launches[kind].fetch_add(n, std::memory_order_relaxed); }
 
-thread_local bool g_pdl = false;
-bool pdl_active() { return g_pdl; }
+thread_local PdlMode g_pdl = PdlMode::Off;
+bool pdl_active() { return g_pdl != PdlMode::Off; }
+bool pdl_early() { return g_pdl == PdlMode::Early; }
 bool pdl_enabled() {
   static const bool on = [] {
     const char* e = getenv("LOGOS_B200_PDL");
@@ -73,8 +74,18 @@ bool pdl_enabled() {
   }();
   return on;
 }
-PdlScope::PdlScope(bool on) : prev(g_pdl) { g_pdl = on; }
+PdlScope::PdlScope(bool on) : prev(g_pdl) { g_pdl = on ? PdlMode::Early : PdlMode::Off; }
 PdlScope::~PdlScope() { g_pdl = prev; }
+OrderedScope::OrderedScope(cudaStream_t st) : prev(g_pdl) {
+  if (prev != PdlMode::Off || !pdl_enabled()) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (st != nullptr && st != cudaStreamLegacy && cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (capture == cudaStreamCaptureStatusNone) g_pdl = PdlMode::Ordered;
+}
+OrderedScope::~OrderedScope() { g_pdl = prev; }
 
 logos_status_t check_launch(const char* kernel) {
   cudaError_t e = cudaGetLastError();
@@ -399,8 +410,8 @@ logos_status_t logos_dev_free(logos_handle_t h) {
 // calls; returns the previous setting through prev_out when that is not null.
 extern "C" logos_status_t logos_dependent_launch_scope(int32_t on, int32_t* prev_out) {
   return logos::guarded([&]() -> logos_status_t {
-    if (prev_out) *prev_out = logos::g_pdl ? 1 : 0;
-    logos::g_pdl = on != 0;
+    if (prev_out) *prev_out = logos::pdl_early() ? 1 : 0;
+    logos::g_pdl = on ? logos::PdlMode::Early : logos::PdlMode::Off;
     return LOGOS_OK;
   });
 }

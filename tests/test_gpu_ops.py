@@ -627,6 +627,49 @@ def test_attention_in_a_dependent_launch_scope(llm, oracle):
                 assert np.array_equal(g, w)
 
 
+def _freshly_written(llm, wait):
+    """Products whose weights and activations the calls just before them write, on one stream; bits of all results."""
+    n, k, m, rounds = 1184, 4096, 40, 6
+    dq, ds, other = llm.DeviceBuffer(n * k), llm.DeviceBuffer(n * (k // 32) * 4), llm.DeviceBuffer(n * k)
+    dx, dxb, scratch = llm.DeviceBuffer(m * k * 4), llm.DeviceBuffer(m * k * 2), llm.DeviceBuffer(n * 4)
+    sizes = [n * 4, n * 4, m * n * 4, m * n * 2]
+    outs = [[llm.DeviceBuffer(b) for b in sizes] for _ in range(rounds)]
+    llm.synthFill(other, llm.I8, 0, 99, 1, 0, n * k, 0.0, 1.0)
+
+    def then():
+        if wait:
+            llm.devSync()
+
+    for i, (y0, y1, c0, c1) in enumerate(outs):
+        llm.synthFill(dx, llm.F32, 2, 60 + i, 3, 0, m * k, 0.0, 1.0)
+        llm.synthFill(dxb, llm.BF16, 2, 60 + i, 4, 0, m * k, 0.0, 1.0)
+        llm.synthFill(ds, llm.F32, 1, 60 + i, 2, 0, n * (k // 32), 1e-3, 1e-2)
+        llm.synthFill(dq, llm.I8, 0, 60 + i, 1, 0, n * k, 0.0, 1.0)
+        then()
+        if i % 2:                       # a call between the writer and one that reads its weights early
+            llm.q8Gemv(other, ds, dx, scratch, n, k)
+            prev = llm.dependentLaunchScope(True)
+            llm.q8Gemv(dq, ds, dx, y0, n, k)
+            llm.dependentLaunchScope(prev)
+            then()
+        for call in (lambda: llm.q8Gemv(dq, ds, dx, y0 if not i % 2 else y1, n, k), lambda: llm.q8GemmF32(dx, dq, ds, c0, m, n, k),
+                     lambda: llm.q8Gemm(dxb, dq, ds, c1, m, n, k)):
+            call()
+            then()
+    llm.devSync()
+    return [b.download(np.uint8, (size,)) for row in outs for b, size in zip(row, sizes)][: 4 * rounds]
+
+
+def test_operators_behind_calls_that_write_their_weights(llm, oracle):
+    """Outside a scope a product reads nothing before the calls ahead of it have ended, and a scope's early reads behind
+    such a product do not pass it."""
+    want = _freshly_written(llm, True)
+    for _ in range(3):
+        for i, (got, w) in enumerate(zip(_freshly_written(llm, False), want)):
+            if i % 4 != 1 or i // 4 % 2:   # (a second vector in odd rounds only)
+                assert np.array_equal(got, w), i
+
+
 def test_waits_inside_kernels_end_in_seconds(tmp_path):
     """A wait for a barrier that nothing completes returns and says so, in seconds: the limit is of time, whatever a
     poll takes."""
