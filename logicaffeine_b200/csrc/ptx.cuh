@@ -119,6 +119,22 @@ __device__ __forceinline__ void mbar_wait3(uint32_t bar0, uint32_t ph0, uint32_t
                : "r"(bar0), "r"(ph0), "r"(bar1), "r"(ph1), "r"(bar2), "r"(ph2)
                : "memory");
 }
+// The same for a converged warp and a barrier that is mostly ready when it is asked: one poll and a vote first, without a
+// loop.  A taken branch costs the loop above 30 of its 110 cycles on a ready barrier; where waits are long
+// (q8_gemm_tc_kernel at 64 tokens) the extra poll costs more than it saves, 1 to 3 %.
+__device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\t" LOGOS_MBAR_TRY("p", "%1", "%2") "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok;
+}
+__device__ __forceinline__ void mbar_wait_ready(uint32_t bar, uint32_t parity, uint32_t* since) {
+  if (__builtin_expect(!__all_sync(0xffffffffu, mbar_try(bar, parity)), 0)) mbar_wait(bar, parity, since);
+}
+__device__ __forceinline__ void mbar_wait3_ready(uint32_t bar0, uint32_t ph0, uint32_t bar1, uint32_t ph1, uint32_t bar2, uint32_t ph2,
+                                                 uint32_t* since) {
+  const uint32_t ready = mbar_try(bar0, ph0) & mbar_try(bar1, ph1) & mbar_try(bar2, ph2);
+  if (__builtin_expect(!__all_sync(0xffffffffu, ready), 0)) mbar_wait3(bar0, ph0, bar1, ph1, bar2, ph2, since);
+}
 // A single wait with a limit of its own, counted from its 32nd failed poll; false when it gave up.
 #define LOGOS_MBAR_SINGLE(TRY)                \
   "{\n\t.reg .pred p, s;\n\t.reg .u32 n, t, e;\n\tmov.u32 n, 0;\n" \

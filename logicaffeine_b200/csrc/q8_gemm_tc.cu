@@ -38,7 +38,7 @@
 // from the other warps to the drain warps.
 //
 // Registers are what 96 tokens run out of: the kernel spills 112 to 172 bytes a thread there (`-Xptxas -v`), up to 40
-// elsewhere.
+// elsewhere.  With many tokens and enough row tiles another form of it runs, see WideCfg.
 //
 // HBM roofline: 1.125 bytes per weight (int8 + f32/32); activations and outputs are small next to
 // that at decode batch sizes.  With many tokens the FMA and tensor pipes are the bound.
@@ -112,6 +112,36 @@ struct TcCfg {
   static_assert(SMEM <= 227 * 1024 && SMEM > 114 * 1024, "shared memory: one CTA per SM, since it takes all of tensor memory");
   static constexpr int ENTRY_COLS = 2 * T;
   static_assert(ACC_COL0 + ENTRIES * ENTRY_COLS <= (int)TMEM_COLS, "TMEM budget");
+};
+
+// The wide form, for many tokens: a unit is one row tile x 2 T tokens (x a K split), so that converted weights serve twice as
+// many tokens.  Half a stage is one slot of the operand ring and of the activation ring.
+template <int T, int LIMBS>
+struct WideCfg {
+  // One MMA of N = 2 T for both halves of the tokens, a block for each MMA warp, with one plane; an MMA warp for each
+  // half of the tokens with two, where a joint block would be complete only after twice the time.
+  static constexpr bool JOINT = LIMBS == 1;
+  static constexpr int ENTRIES = 2;                                // accumulator entries: blocks of 2 T columns
+  static constexpr int FULLS = JOINT ? ENTRIES : 2 * ENTRIES;      // hand-offs of a block: together, or each half of the tokens
+  static constexpr int ACT_BYTES = 2 * T * 128 * LIMBS;
+  static constexpr int ACT_SLOTS = T == 96 ? (LIMBS == 2 ? 3 : 5) : (LIMBS == 2 ? 4 : 6);
+  // Scales need no barriers of their own (see TcCfg): those of stage n are written once the converters have released stage
+  // n - RAW_SLOTS; its operand slots were free by then, so all MMAs of stage n - RAW_SLOTS - 2 were complete, and the last
+  // two of its blocks needed the entries of the first two, whose readers had that stage's scales.
+  static constexpr int SC_MORE = 3;                                // (one to spare)
+  static constexpr int RAW_SLOTS_FIT = (225 * 1024 - 2048 - ACT_SLOTS * ACT_BYTES - SC_MORE * SC_BYTES) / (RAW_BYTES + SC_BYTES);
+  static constexpr int RAW_SLOTS = RAW_SLOTS_FIT < 5 ? RAW_SLOTS_FIT : 5;
+  static constexpr int SC_SLOTS = RAW_SLOTS + SC_MORE;
+  static constexpr int CONV_WARP0 = 4, DRAIN_WARP0 = 8, DRAIN_WARPS = 8;   // four single-role warps, then these
+  static constexpr int THREADS = (DRAIN_WARP0 + DRAIN_WARPS) * 32;
+  // T sums a thread, and 48 (32) columns on their way to them.  Not one register of that may be spilled: with 9 % of the
+  // instructions spills the kernel took half as long again.
+  static constexpr int REGS_MISC = 64, REGS_CONV = 80, REGS_DRAIN = 184;
+  static_assert(4 * REGS_MISC + 4 * REGS_CONV + DRAIN_WARPS * REGS_DRAIN <= (DRAIN_WARP0 + DRAIN_WARPS) * (65536 / THREADS / 8 * 8), "register split");
+  static constexpr int ACC_COL0 = 4 * TA_SLOT_COLS;
+  static_assert(ACC_COL0 + ENTRIES * 2 * T <= (int)TMEM_COLS, "TMEM budget");
+  static constexpr size_t SMEM = 1024 + (size_t)RAW_SLOTS * RAW_BYTES + (size_t)ACT_SLOTS * ACT_BYTES + (size_t)SC_SLOTS * SC_BYTES + 1024;
+  static_assert(RAW_SLOTS >= 3 && SMEM <= 227 * 1024 && SMEM > 114 * 1024, "shared memory: one CTA per SM, since it takes all of tensor memory");
 };
 
 struct TcParams {
@@ -202,7 +232,10 @@ __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gmem_sr
 // N columns of a row into r[0 .. N)
 template <int N>
 __device__ __forceinline__ void tc_ld_cols(uint32_t taddr, uint32_t* r) {
-  if constexpr (N == 32) tc_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(r));
+  if constexpr (N > 32) {
+    tc_ld_cols<32>(taddr, r);
+    tc_ld_cols<N - 32>(taddr + 32, r + 32);
+  } else if constexpr (N == 32) tc_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(r));
   else if constexpr (N == 24) {
     tc_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(r));
     tc_ld_32x32b_x8(taddr + 16, *reinterpret_cast<uint32_t(*)[8]>(r + 16));
@@ -256,6 +289,23 @@ __device__ __forceinline__ void drain_blocks(float2* sum, uint32_t ta, const flo
       }
     }
   }
+}
+
+// 64 bytes of a row of weights in shared memory (four chunks) -> fp16 in an operand slot.  Exact: see cvt_pair.
+template <bool TILED>
+__device__ __forceinline__ void convert_half(const uint4 (&wv)[4], uint32_t t_dst) {
+  uint32_t o[32];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint32_t ws[4] = {wv[c].x, wv[c].y, wv[c].z, wv[c].w};
+#pragma unroll
+    for (int wi = 0; wi < 4; ++wi) {
+      const uint32_t w = TILED ? ws[wi] : ws[wi] ^ 0x80808080u;   // tile-major bytes hold q + 128 already
+      o[c * 8 + 2 * wi] = cvt_pair(w, 0x4140);
+      o[c * 8 + 2 * wi + 1] = cvt_pair(w, 0x4342);
+    }
+  }
+  tc_st_32x32b_x32(t_dst, o);
 }
 
 // A thread's HC sums of output column n, tokens m0 ..: a warp stores 32 consecutive columns of a token at a time.
@@ -710,6 +760,295 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   }
 }
 
+// The wide form (WideCfg).  The same arithmetic in the same order as the kernel above, so the same bits.
+//
+// What bounds it with many tokens: a block's sums go through registers once, 96 columns x 128 rows for each half of the
+// tokens, and two entries of tensor memory are all there is room for.  A block takes 500 cycles: 96 to 192 of MMA, about 160
+// until its completion is seen, two loads of 48 columns with the FMAs of the first half between them, and the MMA warp's
+// wake-up.  So eight drain warps with a whole channel's columns each instead of sixteen with half of them (hand-offs are what
+// costs: a poll of a ready barrier is 80 cycles, an arrival seven for each warp), the second load released before its FMAs.
+// Against pairs of row tiles (calls in a row, 1000 W, bf16 2048 x 37888 x 3584 / f32 4096 x 10240 x 5120, us): 965 -> 777 / 983 -> 852.
+// A joint MMA for both planes 872, two MMA warps for one plane 795; loads of 16 columns, each ahead of the FMAs of the one
+// before, 815 / 887.
+template <int T, int LIMBS, bool TILED>
+__global__ void __launch_bounds__(WideCfg<T, LIMBS>::THREADS, 1)
+q8_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_a,
+                    const __grid_constant__ CUtensorMap map_s, const TcParams p) {
+  using Cfg = WideCfg<T, LIMBS>;
+  constexpr bool JOINT = Cfg::JOINT;
+  constexpr int FULLS = Cfg::FULLS, ACT_SLOTS = Cfg::ACT_SLOTS, RAW_SLOTS = Cfg::RAW_SLOTS, SC_SLOTS = Cfg::SC_SLOTS;
+
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = (smem_u32(smem_raw) + 1023u) & ~1023u;       // [RAW_SLOTS] x 16 KB
+  const uint32_t act = raw + RAW_SLOTS * RAW_BYTES;                 // [ACT_SLOTS] x ACT_BYTES: [planes][2 T][64]
+  const uint32_t scl = act + ACT_SLOTS * Cfg::ACT_BYTES;            // [SC_SLOTS] x 2 KB
+  const uint32_t raw_full = scl + SC_SLOTS * SC_BYTES;              // barriers, 8 bytes each: [RAW_SLOTS]
+  const uint32_t raw_empty = raw_full + 8 * RAW_SLOTS;
+  const uint32_t act_full = raw_empty + 8 * RAW_SLOTS;              // [ACT_SLOTS]
+  const uint32_t act_empty = act_full + 8 * ACT_SLOTS;
+  const uint32_t ta_full = act_empty + 8 * ACT_SLOTS;               // [TA_SLOTS]
+  const uint32_t ta_empty = ta_full + 8 * TA_SLOTS;
+  const uint32_t acc_full = ta_empty + 8 * TA_SLOTS;                // [FULLS]
+  const uint32_t acc_empty = acc_full + 8 * FULLS;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int prior_status;
+
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  constexpr int NBARS = 2 * (RAW_SLOTS + ACT_SLOTS + TA_SLOTS + FULLS);
+  static_assert(NBARS <= 128, "one barrier a thread");
+  if (warp >= Cfg::CONV_WARP0 && tid - Cfg::CONV_WARP0 * 32 < NBARS) {
+    const int i = tid - Cfg::CONV_WARP0 * 32;
+    const uint32_t bar = raw_full + 8 * i;
+    uint32_t count = 1;                                                  // TMA and tcgen05.commit arrive once
+    if (bar >= raw_empty && bar < act_full) count = 4;                   // the converter warps
+    else if (bar >= act_empty && bar < ta_full) count = 2;               // a commit of each MMA warp
+    else if (bar >= ta_full && bar < ta_empty) count = 4;
+    else if (bar >= ta_empty && bar < acc_full) count = 2;
+    else if (bar >= acc_empty) count = JOINT ? Cfg::DRAIN_WARPS : Cfg::DRAIN_WARPS / 2;
+    mbar_init(bar, count);
+    fence_barrier_init();
+  }
+  if (tid == 0) prior_status = *reinterpret_cast<volatile int*>(p.status);   // as above
+  if (warp == 1 && lane == 0) {
+    prefetch_tensormap(&map_q);
+    prefetch_tensormap(&map_a);
+    if (!p.s_tiled) prefetch_tensormap(&map_s);
+  }
+  if (warp == 3) {
+    tmem_alloc(&tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  pdl_trigger();   // as above
+  const int units = prior_status != 0 ? 0 : p.solos * p.splits * p.mtiles;
+
+  bool ok = true;
+  uint32_t since = wait_start();
+
+  if (warp < Cfg::CONV_WARP0) {
+    regs_dec<Cfg::REGS_MISC>();
+    if (warp == 0) {
+      // ------------------------------------------------------------ weight and scale producer
+      if (p.wait_scales) pdl_wait();
+      const uint64_t pol = p.stream_once ? policy_evict_first() : policy_evict_normal();
+      Ring<RAW_SLOTS> r;
+      Ring<SC_SLOTS> c;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const TcUnit it = tc_unit(p, u);
+        since = wait_start();
+        for (int i = it.st_begin; i < it.st_begin + it.nst && ok; ++i) {
+          const int block = it.tile * p.stages_total + i;   // of a tile-major array
+          const uint32_t bar = raw_full + 8 * r.slot;
+          mbar_wait(raw_empty + 8 * r.slot, r.ph ^ 1u, &since);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar, RAW_BYTES + SC_BYTES);
+            if (TILED) tma_load_2d_hint(raw + r.slot * RAW_BYTES, &map_q, bar, 0, block * TC_ROWS, pol);
+            else tma_load_2d_hint(raw + r.slot * RAW_BYTES, &map_q, bar, i * TC_KSTAGE, it.tile * TC_ROWS, pol);
+            if (TILED || p.s_tiled) bulk_load(scl + c.slot * SC_BYTES, p.s + (int64_t)block * (TC_ROWS * 4), SC_BYTES, bar);
+            else tma_load_2d(scl + c.slot * SC_BYTES, &map_s, bar, i * 4, it.tile * TC_ROWS);
+          }
+          __syncwarp();
+          r.next();
+          c.next();
+          if (since == WAIT_OVER) {
+            if (lane == 0) tc_report(p.status, 2110, i, it.nst);
+            ok = false;
+          }
+        }
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------ activation producer, half a stage at a time
+      pdl_wait();  // the activations are the previous kernel's output
+      const uint64_t pol = policy_evict_last();
+      Ring<ACT_SLOTS> r;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const TcUnit it = tc_unit(p, u);
+        since = wait_start();
+        for (int i = 2 * it.st_begin; i < 2 * (it.st_begin + it.nst) && ok; ++i) {
+          const uint32_t bar = act_full + 8 * r.slot;
+          mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &since);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar, Cfg::ACT_BYTES);
+            tma_load_4d_hint(act + r.slot * Cfg::ACT_BYTES, &map_a, bar, 0, it.mtile * 2 * T, i, 0, pol);
+          }
+          __syncwarp();
+          r.next();
+          if (since == WAIT_OVER) {
+            if (lane == 0) tc_report(p.status, 2120, i, it.nst);
+            ok = false;
+          }
+        }
+      }
+      // the last commits land before the CTA ends
+      for (int i = 0; i < ACT_SLOTS && ok; ++i) {
+        mbar_wait(act_empty + 8 * r.slot, r.ph ^ 1u, &since);
+        r.next();
+      }
+    } else {
+      // ------------------------------------------------------------ MMA issuers
+      constexpr uint32_t idesc = make_idesc_f16(0, 0, TC_ROWS, JOINT ? 2 * T : T);
+      const int w = warp - 2;
+      const uint64_t bdesc_first = make_desc_sw128(act + (JOINT ? 0 : w * T * 128));
+      const uint32_t d_first = tmem_base + Cfg::ACC_COL0 + (JOINT ? 0 : w * T);
+      const uint32_t bars = JOINT ? 0u : 8u * Cfg::ENTRIES * w;
+      Ring<ACT_SLOTS> ra;
+      Ring<TA_SLOTS> rt;
+      uint32_t e_ph = 1;   // of both entries
+      // block k of a half stage, into entry k; whether it begins and ends this warp's part of it
+      auto block = [&](int k, bool first, bool last) {
+        const uint64_t bdesc0 = bdesc_first + (uint32_t)(ra.slot * (Cfg::ACT_BYTES >> 4) + k * 4);   // start address field: no carry out of it
+        const uint32_t a0 = tmem_base + rt.slot * TA_SLOT_COLS + k * 16, d0 = d_first + k * 2 * T;
+        if (first) mbar_wait3_ready(act_full + 8 * ra.slot, ra.ph, ta_full + 8 * rt.slot, rt.ph, acc_empty + bars + 8 * k, e_ph, &since);
+        else mbar_wait_ready(acc_empty + bars + 8 * k, e_ph, &since);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int v = 0; v < 2 * LIMBS; ++v) {   // d = q * lo' first, then d = q * hi + d * 2^-11
+            const int l = (LIMBS == 2) ? 1 - (v >> 1) : 0;
+            const uint64_t bdesc = bdesc0 + (uint32_t)((l * 2 * T * 128 + (v & 1) * 32) >> 4);
+            if (LIMBS == 2 && v == 2) tc_mma_f16_ts_scaled_d<11>(d0, a0 + (v & 1) * 8, bdesc, idesc);
+            else if (v == 0) tc_mma_f16_ts<false>(d0, a0 + (v & 1) * 8, bdesc, idesc);
+            else tc_mma_f16_ts<true>(d0, a0 + (v & 1) * 8, bdesc, idesc);
+          }
+          tc_commit(acc_full + bars + 8 * k);
+          if (last) {
+            tc_commit(ta_empty + 8 * rt.slot);
+            tc_commit(act_empty + 8 * ra.slot);
+          }
+        }
+        __syncwarp();
+      };
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const TcUnit it = tc_unit(p, u);
+        since = wait_start();
+        for (int i = 0; i < 2 * it.nst; ++i) {
+          if (JOINT) {
+            block(w, true, true);
+          } else {
+            block(0, true, false);
+            block(1, false, true);
+          }
+          e_ph ^= 1u;
+          rt.next();
+          ra.next();
+          if (since == WAIT_OVER) break;
+        }
+        if (since == WAIT_OVER) {
+          if (lane == 0) tc_report(p.status, 2130, 0, it.nst);
+          ok = false;
+        }
+      }
+    }
+  } else if (warp < Cfg::DRAIN_WARP0) {
+    // ------------------------------------------------------------ converters: int8 smem -> fp16 TMEM
+    regs_dec<Cfg::REGS_CONV>();
+    const int qd = warp & 3;
+    const uint32_t row = qd * 32 + lane;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16);
+    uint32_t off[4];   // chunks of the row's first half, see above
+#pragma unroll
+    for (int c = 0; c < 4; ++c) off[c] = raw + swz128(row, c);
+    Ring<RAW_SLOTS> r;
+    Ring<TA_SLOTS, 2> a(0, 1u);   // a stage takes slots a and a + 1
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const TcUnit it = tc_unit(p, u);
+      since = wait_start();
+      for (int i = 0; i < it.nst && since != WAIT_OVER; ++i) {
+        mbar_wait3_ready(raw_full + 8 * r.slot, r.ph, ta_empty + 8 * a.slot, a.ph, ta_empty + 8 * (a.slot + 1), a.ph, &since);
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint4 wv[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) wv[c] = lds_v4((off[c] ^ (h ? 64u : 0u)) + r.slot * RAW_BYTES);
+          convert_half<TILED>(wv, t_lane + (a.slot + h) * TA_SLOT_COLS);
+        }
+        mbar_arrive_if(raw_empty + 8 * r.slot, lane == 0);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_if(ta_full + 8 * a.slot, lane == 0);
+        mbar_arrive_if(ta_full + 8 * (a.slot + 1), lane == 0);
+        a.next();
+        r.next();
+      }
+      if (since == WAIT_OVER) {
+        if (lane == 0) tc_report(p.status, 2140, 0, it.nst);
+        ok = false;
+      }
+    }
+    for (int i = 0; i < TA_SLOTS / 2 && ok; ++i) {   // as for the activations
+      mbar_wait2(ta_empty + 8 * a.slot, a.ph, ta_empty + 8 * (a.slot + 1), a.ph, &since);
+      a.next();
+    }
+  } else {
+    // ------------------------------------------------------------ drain + epilogue
+    regs_inc<Cfg::REGS_DRAIN>();
+    const int qd = warp & 3;
+    const int g = (warp - Cfg::DRAIN_WARP0) >> 2;   // which half of the tokens
+    const uint32_t row = qd * 32 + lane;
+    const uint32_t col0 = tmem_base + ((uint32_t)(qd * 32) << 16) + Cfg::ACC_COL0 + g * T;
+    const uint32_t bars = JOINT ? 0u : 8u * Cfg::ENTRIES * g;
+    const uint32_t s_row = scl + row * 16;
+    constexpr int CH = T == 96 ? 48 : 32;           // columns of a load
+    int rc = 0;                                     // scale slot of the stage
+    uint32_t ph = 0;                                // of both entries
+    pdl_wait();  // before any write to global memory (nothing to drain before the activations are in anyway)
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      const TcUnit it = tc_unit(p, u);
+      since = wait_start();
+      float2 acc[T / 2];
+#pragma unroll
+      for (int x = 0; x < T / 2; ++x) acc[x] = make_float2(0.f, 0.f);
+      for (int i = 0; i < it.nst && since != WAIT_OVER; ++i) {
+        float s[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {               // the stage's blocks
+          const uint32_t bar = bars + 8 * (k & 1);
+          mbar_wait_ready(acc_full + bar, ph, &since);
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < T / CH; ++c) {
+            uint32_t b[CH];
+            tc_ld_cols<CH>(col0 + (k & 1) * 2 * T + c * CH, b);
+            if (k == 0 && c == 0) {
+              const uint4 sc = lds_v4(s_row + rc * SC_BYTES);
+              s[0] = __uint_as_float(sc.x); s[1] = __uint_as_float(sc.y); s[2] = __uint_as_float(sc.z); s[3] = __uint_as_float(sc.w);
+            }
+            tc_loaded(b);
+            if (c == T / CH - 1) {
+              tc_fence_before();
+              __syncwarp();
+              mbar_arrive_if(acc_empty + bar, lane == 0);
+            }
+            add_cols<CH>(acc + c * (CH / 2), s[k], b);
+          }
+          if (k & 1) ph ^= 1u;
+        }
+        if (++rc == SC_SLOTS) rc = 0;
+      }
+      if (since == WAIT_OVER) {
+        if (lane == 0) tc_report(p.status, 2150, 0, it.nst);
+        break;
+      }
+      store_tile<T>(p, acc, it.split, (int64_t)it.tile * TC_ROWS + row, (int64_t)(it.mtile * 2 + g) * T, lane);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 3) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
 // ---------------------------------------------------------------- host side
 // What a tensor map is a function of: address, extents, pitches and box.  Maps are encoded once and kept.
 struct MapKey {
@@ -776,6 +1115,7 @@ namespace {
 // How a product is cut up: tokens per tile, K splits, and the row tiles that run in pairs and alone.
 struct TcPlan {
   int t, splits, pairs, solos;
+  bool wide;   // the wide form: 2 t tokens a tile, row tiles alone
 };
 
 // Cycles of one K stage of a pair and of a single tile, by tokens per tile, of the pipeline fill plus the last
@@ -785,16 +1125,22 @@ struct TcPlan {
 // 1967/1917, 1804/2092, 2338/3018, 2914/3676.  From 64 tokens on it stands between what one plane and two cost; whether a table
 // for each makes better choices has not been tried.
 struct TcCost {
-  int t, pair, solo;
+  int t, pair, solo, unit;
 };
-constexpr TcCost kCosts[] = {{16, 1760, 1065}, {32, 1900, 1090}, {64, 2550, 1400}, {96, 3300, 1900}};
-constexpr int kFillCycles = 8000, kUnitCycles = 700;
+constexpr TcCost kCosts[] = {{16, 1760, 1065, 700}, {32, 1900, 1090, 700}, {64, 2550, 1400, 700}, {96, 3300, 1900, 700}};
+// Units of the wide form on the same scale, fitted to 74 shapes timed with each form (m 70 to 4096, n 896 to 55296, K 512 to 8192,
+// one plane and two): what the costs choose is 0.1 % slower than the best of the three in the mean, 4 % at worst.  Bf16 / f32, us,
+// the other form -> 128 tokens a unit, 192: 128 x 18944 x 3584 38.0 -> 30.8, 36.1 / 49.4 -> 39.8, 47.3; 192 50.0 -> 55.8, 38.3 / 64.4
+// -> 73.7, 52.0; 1024 248 -> 210, 207 / 324 -> 287, 275; few row tiles, 1024 x 896 x 4864: 28.6 -> 36.5, 44.6 / 32.8 -> 41.5, 47.8.
+// Up to 64 tokens half of a wide unit would be empty.
+constexpr TcCost kWideCosts[] = {{64, 0, 1860, 1200}, {96, 0, 2380, 2100}};
+constexpr int kFillCycles = 8000;
 
 // The slowest CTA's time when `pairs` pair items and `solos` single tiles run round robin on g CTAs.
 int64_t plan_cycles(const TcCost& c, int64_t pairs, int64_t solos, int64_t sp, int64_t mt, int64_t stages, int64_t g) {
   const int64_t pu = pairs * sp * mt, total = (pairs + solos) * sp * mt;
   const int64_t per = (stages + sp - 1) / sp;
-  const int64_t tp = per * c.pair + kUnitCycles, ts = per * c.solo + kUnitCycles;
+  const int64_t tp = per * c.pair + c.unit, ts = per * c.solo + c.unit;
   int64_t worst = 0;
   for (int64_t cta : {(int64_t)0, pu % g, pu % g - 1, total % g - 1}) {
     if (cta < 0 || cta >= g) continue;
@@ -806,7 +1152,7 @@ int64_t plan_cycles(const TcCost& c, int64_t pairs, int64_t solos, int64_t sp, i
 
 TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms) {
   const int64_t tl = (n + TC_ROWS - 1) / TC_ROWS, stages = (k + TC_KSTAGE - 1) / TC_KSTAGE;
-  TcPlan best{16, (int)sp, 0, (int)tl};
+  TcPlan best{16, (int)sp, 0, (int)tl, false};
   int64_t best_cost = INT64_MAX;
   for (const TcCost& c : kCosts) {
     // fewer tokens than half a larger tile never pay for it
@@ -820,7 +1166,16 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms) {
       const int64_t cost = plan_cycles(c, pairs, tl - 2 * pairs, sp, mt, stages, sms);
       if (cost < best_cost) {
         best_cost = cost;
-        best = TcPlan{c.t, (int)sp, (int)pairs, (int)(tl - 2 * pairs)};
+        best = TcPlan{c.t, (int)sp, (int)pairs, (int)(tl - 2 * pairs), false};
+      }
+    }
+  }
+  if (m > 64) {
+    for (const TcCost& c : kWideCosts) {
+      const int64_t cost = plan_cycles(c, 0, tl, sp, (m + 2 * c.t - 1) / (2 * c.t), stages, sms);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = TcPlan{c.t, (int)sp, 0, (int)tl, true};
       }
     }
   }
@@ -845,9 +1200,10 @@ TcPlan plan_for(int64_t m, int64_t n, int64_t k, int64_t splits, int device) {
   return e.plan;
 }
 
-template <int T, int LIMBS>
+template <int T, int LIMBS, bool WIDE = false>
 logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) {
-  using Cfg = TcCfg<T, LIMBS>;
+  using Cfg = std::conditional_t<WIDE, WideCfg<T, LIMBS>, TcCfg<T, LIMBS>>;
+  constexpr int TOKENS = WIDE ? 2 * T : T;   // of a token tile
   CUtensorMap mq, ma, ms;
   const int64_t stages = (g.k + TC_KSTAGE - 1) / TC_KSTAGE, tiles = (g.n + TC_ROWS - 1) / TC_ROWS;
   if (g.q_tiled) {
@@ -859,7 +1215,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   // [planes][halves of a stage][tokens][64]: the planes lie at any multiple of 16 bytes from each other
   LOGOS_TRY(cached_map_4d(&ma, g.a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 64, (uint64_t)g.m, (uint64_t)(2 * stages), LIMBS,
                           (uint64_t)g.lda * 2, 128, LIMBS == 2 ? (uint64_t)(reinterpret_cast<const char*>(g.a_lo) - static_cast<const char*>(g.a)) : 128,
-                          T, 2, LIMBS));
+                          TOKENS, WIDE ? 1 : 2, LIMBS));
   ms = ma;
   const bool s_tiled = g.q_tiled || g.s_tiled;
   if (!s_tiled)
@@ -874,20 +1230,23 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   p.s_tiled = s_tiled;
   p.wait_scales = g.s_tiled;
   if (g.epilogue == EPI_RESIDUAL && g.c_dtype != LOGOS_BF16) return fail(LOGOS_ERROR, "q8_gemm: a residual goes with bf16 results");
-  const int64_t mtiles = (g.m + T - 1) / T;
+  const int64_t mtiles = (g.m + TOKENS - 1) / TOKENS;
   const int64_t units = (int64_t)(plan.pairs + plan.solos) * plan.splits * mtiles;
   if (units > INT32_MAX / 4 || tiles * stages > INT32_MAX / TC_ROWS) return fail(LOGOS_OUT_OF_BOUNDS, "q8_gemm: too many work units");
   p.pairs = plan.pairs;
   p.solos = plan.solos;
   p.mtiles = (int)mtiles;
-  const int64_t groups = (mtiles + 11) / 12;   // about 12 token tiles x 12 row tiles of 256 run side by side
+  // about 12 token tiles x 12 pairs of row tiles run side by side, of the wide form 8 x 18 row tiles
+  const int64_t most = WIDE ? 8 : 12, groups = (mtiles + most - 1) / most;
   p.group = (int)((mtiles + groups - 1) / groups);
   p.stream_once = mtiles == 1;
   p.status = kernel_status_ptr(g.device);
   if (!p.status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   if (p.splits > p.stages_total) return fail(LOGOS_ERROR, "q8_gemm: more K splits than 128-column stages");
 
-  auto kernel = g.q_tiled ? q8_gemm_tc_kernel<T, LIMBS, true> : q8_gemm_tc_kernel<T, LIMBS, false>;
+  void (*kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const TcParams);
+  if constexpr (WIDE) kernel = g.q_tiled ? q8_gemm_wide_kernel<T, LIMBS, true> : q8_gemm_wide_kernel<T, LIMBS, false>;
+  else kernel = g.q_tiled ? q8_gemm_tc_kernel<T, LIMBS, true> : q8_gemm_tc_kernel<T, LIMBS, false>;
   LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kernel), g.device, (int)Cfg::SMEM));
   // persistent CTAs: one per SM at most, each takes units blockIdx.x, blockIdx.x + gridDim.x, ...
   const int sms = sm_count(g.device);
@@ -899,6 +1258,7 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
 
 template <int LIMBS>
 logos_status_t launch_plan(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) {
+  if (plan.wide) return plan.t == 64 ? launch_t<64, LIMBS, true>(g, plan, st) : launch_t<96, LIMBS, true>(g, plan, st);
   switch (plan.t) {
     case 16: return launch_t<16, LIMBS>(g, plan, st);
     case 32: return launch_t<32, LIMBS>(g, plan, st);

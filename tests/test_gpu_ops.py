@@ -164,6 +164,28 @@ def test_q8_gemm_tiles_tails_and_units(llm, oracle, m, n, k):
     assert llm.kernelStatus() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (128, 18944, 128),    # one full tile of 128 tokens, one stage
+    (129, 37000, 160),    # a tile of 192 that is mostly full, a K tail of one Q8 block, a last row tile of 8 rows
+    (192, 18946, 384),    # 192 full, an odd number of stages, two rows in the last row tile
+    (193, 37888, 288),    # a second tile of one token, several units a CTA
+    (450, 19000, 1152),   # tiles of 128 and a tail, more stages than any ring has slots
+])
+def test_q8_gemm_wide_units_give_the_same_bits(llm, oracle, m, n, k):
+    """Many tokens run in larger units than 64: the order of a sum, and so its bits, are those of 64 tokens at a time."""
+    O = oracle
+    a = O.synth_fill(O.F32, 2, 8, 10, 0, m * k, 0.0, 1.0).reshape(m, k)
+    q = O.synth_fill(O.I8, 0, 8, 11, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 8, 12, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    ab = O.f32_to_bf16(a)
+    c, cb, cs = llm.q8GemmF32Host(a, q, s), llm.q8GemmHost(ab, q, s), llm.q8GemmHost(ab, q, s, epilogue=2)
+    for i in range(0, m, 64):
+        assert np.array_equal(c[i:i + 64], llm.q8GemmF32Host(a[i:i + 64], q, s)), i
+        assert np.array_equal(cb[i:i + 64], llm.q8GemmHost(ab[i:i + 64], q, s)), i
+        assert np.array_equal(cs[i:i + 64], llm.q8GemmHost(ab[i:i + 64], q, s, epilogue=2)), i
+    assert llm.kernelStatus() == 0
+
+
 def test_q8_gemm_config1_slice(llm, oracle):
     """Config 1 shapes (M=64, K=3584) on a 2048-row slice of N, both kernels."""
     O = oracle
