@@ -749,3 +749,9 @@ def test_kernels_behind_a_failure_write_nothing(native):
 def test_narrow_products_bit_for_bit(native):
     lines = native("narrow_products")
     assert lines and not [line for line in lines if not line.endswith(" 0")]
+
+
+def test_short_division_of_swiglu_gives_the_same_bits(native):
+    """All gates that it takes (0, and every finite float of at least 2^-100) against the division that rounds correctly."""
+    taken, other = map(int, native("silu_gates")[0].split())
+    assert taken == 2 * (0x7f800000 - 0x0d800000) + 1 and other == 0
