@@ -266,11 +266,15 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   const int src_dtype = g.a_dtype;
   const int64_t stages = (g.k + 127) / 128;
   const bool retile = g.k % 128 != 0;
-  const int splits = gemm_pick_splits(g.m, g.n, g.k, g.device, false);
+  int splits = g.m > 64 ? gemm_many_splits(g.m, g.n, g.k, g.device) : gemm_pick_splits(g.m, g.n, g.k, g.device, false);
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   const int64_t lda = stages * 128;
   const int64_t plane_bytes = up(g.m * lda * 2);
   const int64_t scale_bytes = retile ? up((g.n + 127) / 128 * stages * 2048) : 0;
+  const int64_t own_bytes = (two_planes ? 2 : 1) * plane_bytes + scale_bytes + (retile ? 256 : 0);
+  void* scratch = nullptr;
+  // many tokens are worth splitting where there is room for the partial sums
+  if (g.m > 64 && splits > 1 && !scratch_try(g.device, 0, own_bytes + splits * g.m * g.n * (int64_t)sizeof(float), st, &scratch)) splits = 1;
   // The product kernel loads a residual row after row, which an SM with several tiles to do waits for every time: with
   // more tokens than its largest tile the sums are staged in f32 and a kernel of its own adds the residual, the same
   // bits.  A few token tiles at a time, so that the scratch stays small and the sums in L2.
@@ -280,8 +284,6 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   bool staged = g.epilogue == EPI_RESIDUAL && splits <= 1 && (retile || g.m > 96) && stage_rows > 0;
   const int64_t part_rows = staged ? std::min(g.m, stage_rows) : splits > 1 ? splits * g.m : 0;
   const int64_t part_bytes = part_rows * g.n * (int64_t)sizeof(float);
-  const int64_t own_bytes = (two_planes ? 2 : 1) * plane_bytes + scale_bytes + (retile ? 256 : 0);
-  void* scratch = nullptr;
   if (retile || staged) {
     // neither form is worth failing for: the CUDA-core kernel needs no scratch, and the residual can be added
     // in the product

@@ -1171,7 +1171,7 @@ constexpr TcCost kCosts[] = {{16, 1760, 1065, 700}, {32, 1900, 1090, 700}, {64, 
 // the other form -> 128 tokens a unit, 192: 128 x 18944 x 3584 38.0 -> 30.8, 36.1 / 49.4 -> 39.8, 47.3; 192 50.0 -> 55.8, 38.3 / 64.4
 // -> 73.7, 52.0; 1024 248 -> 210, 207 / 324 -> 287, 275; few row tiles, 1024 x 896 x 4864: 28.6 -> 36.5, 44.6 / 32.8 -> 41.5, 47.8.
 // Up to 64 tokens half of a wide unit would be empty.
-constexpr TcCost kWideCosts[] = {{64, 0, 1860, 1200}, {96, 0, 2380, 2100}};
+constexpr TcCost kWideCosts[] = {{64, 0, 1880, 1200}, {96, 0, 2380, 2100}};
 constexpr int kFillCycles = 8000;
 
 // The slowest CTA's time when `pairs` pair items and `solos` single tiles run round robin on g CTAs.
@@ -1188,7 +1188,7 @@ int64_t plan_cycles(const TcCost& c, int64_t pairs, int64_t solos, int64_t sp, i
   return worst + kFillCycles;
 }
 
-TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms) {
+TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms, int64_t* cycles = nullptr) {
   const int64_t tl = (n + TC_ROWS - 1) / TC_ROWS, stages = (k + TC_KSTAGE - 1) / TC_KSTAGE;
   TcPlan best{16, (int)sp, 0, (int)tl, false};
   int64_t best_cost = INT64_MAX;
@@ -1215,6 +1215,25 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms) {
         best_cost = cost;
         best = TcPlan{c.t, (int)sp, 0, (int)tl, true};
       }
+    }
+  }
+  if (cycles) *cycles = best_cost;
+  return best;
+}
+
+// See gemm_many_splits.  The fold of the splits on the costs' scale: its launch, and writing and reading the partial sums.
+int make_splits(int64_t m, int64_t n, int64_t k, int sms) {
+  const int64_t stages = k / TC_KSTAGE, most = std::min<int64_t>(stages / 4, 16);
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int64_t sp = 1; sp <= std::max<int64_t>(most, 1); ++sp) {
+    if (sp > 1 && sp * m * n > (16ll << 20)) break;
+    int64_t cost;
+    make_plan(m, n, k, sp, sms, &cost);
+    if (sp > 1) cost += 6000 + sp * m * n / 333;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = (int)sp;
     }
   }
   return best;
@@ -1319,6 +1338,19 @@ bool gemm_tc_applicable(const GemmArgs& g) {
       (reinterpret_cast<uintptr_t>(g.q) & 15u) || (reinterpret_cast<uintptr_t>(g.s) & 15u))
     return false;
   return true;
+}
+
+int gemm_many_splits(int64_t m, int64_t n, int64_t k, int device) {
+  if ((n + TC_ROWS - 1) / TC_ROWS >= sm_count(device)) return 1;
+  struct Entry {
+    int64_t m = -1, n = 0, k = 0;
+    int device = 0, splits = 1;
+  };
+  thread_local Entry cache[64];   // a pure function of the shape, as the plans are
+  const uint64_t h = ((uint64_t)m * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)n * 0xBF58476D1CE4E5B9ull) ^ ((uint64_t)k * 0x94D049BB133111EBull);
+  Entry& e = cache[(h ^ (h >> 29)) >> 7 & 63];
+  if (e.m != m || e.n != n || e.k != k || e.device != device) e = Entry{m, n, k, device, make_splits(m, n, k, sm_count(device))};
+  return e.splits;
 }
 
 logos_status_t launch_q8_gemm_tc(const GemmArgs& g, cudaStream_t st) {

@@ -186,6 +186,33 @@ def test_q8_gemm_wide_units_give_the_same_bits(llm, oracle, m, n, k):
     assert llm.kernelStatus() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (65, 130, 1536),      # the first count past the other rule, three splits of four stages
+    (129, 1000, 2080),    # a K tail of one Q8 block, splits of unequal length
+    (300, 520, 4096),     # several token tiles
+])
+def test_q8_gemm_many_tokens_in_k_splits(llm, oracle, m, n, k):
+    """Few row tiles and more than 64 tokens: every epilogue behind the fold, and the same bits from call to call."""
+    O = oracle
+    a = O.synth_fill(O.F32, 2, 9, 10, 0, m * k, 0.0, 1.0).reshape(m, k)
+    q = O.synth_fill(O.I8, 0, 9, 11, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 9, 12, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    before = llm.launchCounts()
+    c = llm.q8GemmF32Host(a, q, s)
+    after = llm.launchCounts()
+    # the preparation, the product, and the fold that only K splits have
+    assert after["q8_gemm_tc"] == before["q8_gemm_tc"] + 1 and after["elementwise"] == before["elementwise"] + 2
+    assert rel_l2(c, O.q8_gemm_f32(a, O.F32, q, s)) < 2e-6   # as above: sqrt(k) roundings of 2^-24, planes of 22 bits
+    assert np.array_equal(llm.q8GemmF32Host(a, q, s), c)
+    ab = O.f32_to_bf16(a)
+    aux = O.f32_to_bf16(O.synth_fill(O.F32, 2, 9, 13, 0, m * n, 0.0, 1.0).reshape(m, n))
+    for epilogue in (0, 1, 2):
+        got = llm.q8GemmHost(ab, q, s, epilogue=epilogue, aux=aux if epilogue == 1 else None)
+        # one rounding to bf16 of sums in another order: last-place differences of few elements
+        assert np.mean(got != O.q8_gemm(ab, q, s, epilogue, aux if epilogue == 1 else None)) < 0.01, epilogue
+    assert llm.kernelStatus() == 0
+
+
 def test_q8_gemm_config1_slice(llm, oracle):
     """Config 1 shapes (M=64, K=3584) on a 2048-row slice of N, both kernels."""
     O = oracle
