@@ -12,6 +12,7 @@
 #include "ops.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace logos {
 
@@ -29,13 +30,30 @@ __device__ __forceinline__ float byte_to_f32(uint32_t w_xor80, uint32_t selector
   return __uint_as_float(bits) - 8388736.0f;
 }
 
-__device__ __forceinline__ float dot4(uint32_t w, float4 x, float acc) {
-  uint32_t u = w ^ 0x80808080u;
-  acc = fmaf(byte_to_f32(u, 0x7650), x.x, acc);
-  acc = fmaf(byte_to_f32(u, 0x7651), x.y, acc);
-  acc = fmaf(byte_to_f32(u, 0x7652), x.z, acc);
-  acc = fmaf(byte_to_f32(u, 0x7653), x.w, acc);
+__device__ __forceinline__ float4 four_f32(uint32_t w) {
+  const uint32_t u = w ^ 0x80808080u;
+  return make_float4(byte_to_f32(u, 0x7650), byte_to_f32(u, 0x7651), byte_to_f32(u, 0x7652), byte_to_f32(u, 0x7653));
+}
+__device__ __forceinline__ float dot4(float4 w, float4 x, float acc) {
+  acc = fmaf(w.x, x.x, acc);
+  acc = fmaf(w.y, x.y, acc);
+  acc = fmaf(w.z, x.z, acc);
+  acc = fmaf(w.w, x.w, acc);
   return acc;
+}
+
+// four neighbouring values of x, past L1; x is what the previous kernel wrote
+__device__ __forceinline__ float4 load_x4(const float* x, int64_t i) { return __ldcg(reinterpret_cast<const float4*>(x) + i); }
+__device__ __forceinline__ float4 load_x4(const __nv_bfloat16* x, int64_t i) {
+  const uint2 v = __ldcg(reinterpret_cast<const uint2*>(x) + i);
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                     __uint_as_float(v.y & 0xffff0000u));
+}
+// sums of two neighbouring rows' (R = 2) or one row's product with one vector -> results, in T
+__device__ __forceinline__ void store_y(float* y, const float*, int, int64_t at, float v) { y[at] = v; }
+__device__ __forceinline__ void store_y(__nv_bfloat16* y, const __nv_bfloat16* aux, int epilogue, int64_t at, float v) {
+  if (epilogue == EPI_RESIDUAL) v = __fadd_rn(v, __bfloat162float(aux[at]));
+  y[at] = __float2bfloat16_rn(v);
 }
 
 // xs4 layout: chunk c (16 floats) is split into 4 float4; float4 j of chunk c
@@ -55,10 +73,12 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 // registers, four CTAs an SM) -> now: 152064 x 5120 197 -> 148 us (5.9 TB/s), 151936 x 896 72 -> 38 us,
 // 27648 x 5120 43 -> 33 us, 5120 x 27648 154 -> 45 us, 300 x 16384 13.6 -> 8.4 us.  Four rows at a time
 // measured 166 us on the first, one row 164 us.
-template <int R, bool X_IN_SMEM>
+// M vectors of x at a time (rows of an [M][K] matrix, in T), as the GEMM operators have for a few tokens: a weight is
+// converted once for all of them, and their results go through the GEMM's epilogues.
+template <int R, bool X_IN_SMEM, int M, typename T>
 __global__ void __launch_bounds__(GEMV_WARPS * 32, 1)
-q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const float* __restrict__ x,
-               float* __restrict__ y, int64_t n, int64_t k, bool early) {
+q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const T* __restrict__ x, T* y, int64_t n, int64_t k, bool early,
+               const T* aux, int epilogue) {
   constexpr int U = 4 / R;   // chunks of a row that a lane has in a stage
   extern __shared__ float4 xs4[];
   const int tid = threadIdx.x;
@@ -67,7 +87,7 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
   const int chunks = (int)(k >> 4);  // 16-element chunks per row
   const int kb = (int)(k >> 5);
   const int xchunks = X_IN_SMEM ? (chunks + 31) / 32 * 32 : 0;
-  uint8_t* ring = reinterpret_cast<uint8_t*>(xs4 + xchunks * 4) + warp * (GEMV_DEPTH * GEMV_STAGE);
+  uint8_t* ring = reinterpret_cast<uint8_t*>(xs4 + M * xchunks * 4) + warp * (GEMV_DEPTH * GEMV_STAGE);
   const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
   // In a caller's scope the weights are read before the previous kernel of the stream has finished (the scope promises
   // that nothing in it writes them); x and y wait for it.
@@ -108,15 +128,18 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
   for (int i = 0; i < GEMV_DEPTH - 1; ++i) load();
   if (early) pdl_wait();
   if (X_IN_SMEM) {
-    const float4* xg = reinterpret_cast<const float4*>(x);
-    for (int i = tid; i < chunks * 4; i += blockDim.x) xs4[xs4_index(i >> 2, i & 3)] = __ldcg(xg + i);
+#pragma unroll
+    for (int v = 0; v < M; ++v)
+      for (int i = tid; i < chunks * 4; i += blockDim.x) xs4[v * xchunks * 4 + xs4_index(i >> 2, i & 3)] = load_x4(x + v * k, i);
     __syncthreads();
   }
   int slot = 0;
   for (int64_t g = blockIdx.x + (int64_t)gridDim.x * warp; g < groups; g += step) {
-    float acc[R];
+    float acc[R][M];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int v = 0; v < M; ++v) acc[r][v] = 0.f;
     for (int c0 = 0; c0 < chunks; c0 += 32 * U) {
       __syncwarp();   // every lane is done with the stage that the next load overwrites
       load();
@@ -129,35 +152,87 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
         const int c = c0 + 32 * u + lane;
         if (c < chunks) {
           uint4 w[R];
-          float p[R];
+          float p[R][M];
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             w[r] = *reinterpret_cast<const uint4*>(st + (r * U + u) * 512 + lane * 16);
-            p[r] = 0.f;
+#pragma unroll
+            for (int v = 0; v < M; ++v) p[r][v] = 0.f;
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const float4 xv = X_IN_SMEM ? xs4[xs4_index(c, j)] : __ldcg(reinterpret_cast<const float4*>(x) + (int64_t)c * 4 + j);
+            float4 f[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) p[r] = dot4(j == 0 ? w[r].x : j == 1 ? w[r].y : j == 2 ? w[r].z : w[r].w, xv, p[r]);
+            for (int r = 0; r < R; ++r) f[r] = four_f32(j == 0 ? w[r].x : j == 1 ? w[r].y : j == 2 ? w[r].z : w[r].w);
+#pragma unroll
+            for (int v = 0; v < M; ++v) {
+              const float4 xv = X_IN_SMEM ? xs4[v * xchunks * 4 + xs4_index(c, j)] : load_x4(x + v * k, (int64_t)c * 4 + j);
+#pragma unroll
+              for (int r = 0; r < R; ++r) p[r][v] = dot4(f[r], xv, p[r][v]);
+            }
           }
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const float sc = *reinterpret_cast<const float*>(st + 2048 + (r * 16 * U + 16 * u + (lane >> 1)) * 4);
-            acc[r] = fmaf(sc, p[r], acc[r]);
+#pragma unroll
+            for (int v = 0; v < M; ++v) acc[r][v] = fmaf(sc, p[r][v], acc[r][v]);
           }
         }
       }
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int v = 0; v < M; ++v) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-      if (lane == 0 && g * R + r < n) y[g * R + r] = acc[r];
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[r][v] += __shfl_xor_sync(0xffffffffu, acc[r][v], o);
+      if (lane != v) continue;
+      if (R == 2 && epilogue == EPI_SWIGLU) {   // rows (2j, 2j + 1) are (gate_j, up_j)
+        store_y(y, aux, EPI_NONE, v * (n / 2) + g, __fmul_rn(silu_f(acc[0][v]), acc[R - 1][v]));
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (g * R + r < n) store_y(y, aux, epilogue, v * n + g * R + r, acc[r][v]);
+      }
     }
   }
 }
 
+
+}  // namespace
+
+namespace {
+
+int64_t ring_bytes(int warps) { return (int64_t)warps * GEMV_DEPTH * GEMV_STAGE; }
+int64_t x_bytes(int64_t m, int64_t k) { return m * ((k / 16 + 31) / 32 * 128) * (int64_t)sizeof(float4); }
+
+template <int M, typename T>
+logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64_t n, int64_t k, const T* aux, int epilogue, int device,
+                        cudaStream_t st) {
+  // two rows a warp unless that would leave more than half of the warps without any; the larger CTA where x fits
+  // beside its rings (K up to 16384 for one vector), past K = 30208 x stays in global memory (one vector only)
+  const int64_t sms = sm_count(device);
+  const int rows = n <= sms * GEMV_WARPS && epilogue != EPI_SWIGLU ? 1 : 2;
+  const int64_t groups = (n + rows - 1) / rows;
+  const int64_t xb = x_bytes(M, k);
+  const int warps = ring_bytes(GEMV_WARPS) + xb <= GEMV_SMEM ? GEMV_WARPS : GEMV_FEW_WARPS;
+  const bool in_smem = ring_bytes(warps) + xb <= GEMV_SMEM;
+  auto kern = rows == 2 ? q8_gemv_kernel<2, true, M, T> : q8_gemv_kernel<1, true, M, T>;
+  if constexpr (M == 1 && std::is_same_v<T, float>) {
+    if (!in_smem) kern = rows == 2 ? q8_gemv_kernel<2, false, M, T> : q8_gemv_kernel<1, false, M, T>;
+  }
+  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kern), device, GEMV_SMEM));
+  LOGOS_CUDA_TRY(launch_kernel(kern, dim3((unsigned)std::min(groups, sms)), dim3(warps * 32), (size_t)(ring_bytes(warps) + (in_smem ? xb : 0)),
+                               st, q, s, x, y, n, k, pdl_early(), aux, epilogue));
+  count_launch(LK_GEMV);
+  return check_launch("q8_gemv_kernel");
+}
+
+template <typename T>
+logos_status_t launch_rows(const int8_t* q, const float* s, const T* x, T* y, int64_t m, int64_t n, int64_t k, const T* aux, int epilogue,
+                           int device, cudaStream_t st) {
+  return m == 1 ? launch_m<1, T>(q, s, x, y, n, k, aux, epilogue, device, st) : launch_m<2, T>(q, s, x, y, n, k, aux, epilogue, device, st);
+}
 
 }  // namespace
 
@@ -168,22 +243,20 @@ logos_status_t launch_q8_gemv(const int8_t* q, const float* s, const float* x, f
     LOGOS_CUDA_TRY(cudaMemsetAsync(y, 0, sizeof(float) * n, st));
     return LOGOS_OK;
   }
-  // two rows a warp unless that would leave more than half of the warps without any; the larger CTA where x fits
-  // beside its rings (K up to 16384), past K = 30208 x stays in global memory
-  const int64_t sms = sm_count(device);
-  const int rows = n <= sms * GEMV_WARPS ? 1 : 2;
-  const int64_t groups = (n + rows - 1) / rows;
-  const int64_t xb = (k / 16 + 31) / 32 * 128 * (int64_t)sizeof(float4);
-  auto ring = [](int warps) { return (int64_t)warps * GEMV_DEPTH * GEMV_STAGE; };
-  const int warps = ring(GEMV_WARPS) + xb <= GEMV_SMEM ? GEMV_WARPS : GEMV_FEW_WARPS;
-  const bool in_smem = ring(warps) + xb <= GEMV_SMEM;
-  auto kern = rows == 2 ? (in_smem ? q8_gemv_kernel<2, true> : q8_gemv_kernel<2, false>)
-                        : (in_smem ? q8_gemv_kernel<1, true> : q8_gemv_kernel<1, false>);
-  LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kern), device, GEMV_SMEM));
-  LOGOS_CUDA_TRY(launch_kernel(kern, dim3((unsigned)std::min(groups, sms)), dim3(warps * 32), (size_t)(ring(warps) + (in_smem ? xb : 0)),
-                               st, q, s, x, y, n, k, pdl_early()));
-  count_launch(LK_GEMV);
-  return check_launch("q8_gemv_kernel");
+  return launch_m<1, float>(q, s, x, y, n, k, nullptr, EPI_NONE, device, st);
+}
+
+bool gemv_takes(int64_t m, int64_t n, int64_t k) {
+  if (m == 2 && n * k > (48ll << 20)) return false;
+  return (m == 1 || m == 2) && n >= 1 && k >= 128 && k % 128 == 0 && ring_bytes(GEMV_FEW_WARPS) + x_bytes(m, k) <= GEMV_SMEM;
+}
+
+logos_status_t launch_q8_gemv_tokens(const GemmArgs& g, cudaStream_t st) {
+  if (g.a_dtype == LOGOS_F32)
+    return launch_rows(g.q, g.s, static_cast<const float*>(g.a), static_cast<float*>(g.c), g.m, g.n, g.k, static_cast<const float*>(nullptr),
+                       EPI_NONE, g.device, st);
+  return launch_rows(g.q, g.s, static_cast<const __nv_bfloat16*>(g.a), static_cast<__nv_bfloat16*>(g.c), g.m, g.n, g.k,
+                     static_cast<const __nv_bfloat16*>(g.aux), g.epilogue, g.device, st);
 }
 
 }  // namespace logos

@@ -169,7 +169,7 @@ def test_q8_gemm_tiles_tails_and_units(llm, oracle, m, n, k):
     (129, 37000, 160),    # a tile of 192 that is mostly full, a K tail of one Q8 block, a last row tile of 8 rows
     (192, 18946, 384),    # 192 full, an odd number of stages, two rows in the last row tile
     (193, 37888, 288),    # a second tile of one token, several units a CTA
-    (450, 19000, 1152),   # tiles of 128 and a tail, more stages than any ring has slots
+    (460, 19000, 1152),   # tiles of 128 and a tail, more stages than any ring has slots
 ])
 def test_q8_gemm_wide_units_give_the_same_bits(llm, oracle, m, n, k):
     """Many tokens run in larger units than 64: the order of a sum, and so its bits, are those of 64 tokens at a time."""
@@ -261,6 +261,46 @@ def test_q8_gemv_edges(llm, oracle, n, k):
     # f32 sums of k terms in any order: k roundings of at most 2^-24 of the sum of magnitudes
     bound = k * 2.0 ** -24 * (np.abs(w) @ np.abs(x.astype(np.float64)))
     assert (np.abs(y - w @ x.astype(np.float64)) <= bound).all()
+
+
+@pytest.mark.parametrize("n,k", [
+    (2, 128), (301, 384),                     # one pair of rows; less than a stage a row, an odd number of rows
+    ("warps", 640), ("warps+2", 640),         # one row a warp while every SM's 24 warps suffice, then two
+    (66, 8192), (66, 8320), (66, 14848),      # two vectors beside the larger CTA's rings, and the smaller one's
+    (66, 14976), (66, 30208), (66, 30336),    # one vector still, two in the GEMM; one too
+    (8192, 6144), (8194, 6144),               # the most weights of two vectors
+])
+@pytest.mark.parametrize("m", [1, 2])
+def test_q8_gemm_of_one_or_two_tokens(llm, oracle, m, n, k):
+    """The GEMV kernel's form of the GEMM operators: every epilogue, f32 and bf16."""
+    O = oracle
+    if isinstance(n, str):
+        import torch
+        n = 24 * torch.cuda.get_device_properties(0).multi_processor_count + (2 if n.endswith("+2") else 0)
+    a = O.synth_fill(O.F32, 2, 7, 10, 0, m * k, 0.0, 1.0).reshape(m, k)
+    q = O.synth_fill(O.I8, 0, 7, 11, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 7, 12, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    before = llm.launchCounts()["q8_gemv"]
+    c = llm.q8GemmF32Host(a, q, s)
+    takes = k <= 30208 if m == 1 else k <= 14848 and n * k <= 48 << 20
+    assert llm.launchCounts()["q8_gemv"] == before + takes
+    w = q.astype(np.float64) * np.repeat(s.astype(np.float64), 32, axis=1)
+    # f32 sums of k terms in any order: k roundings of at most 2^-24 of the sum of magnitudes, and 22-bit planes in the GEMM
+    bound = (k + 8) * 2.0 ** -24 * (np.abs(a.astype(np.float64)) @ np.abs(w.T))
+    assert (np.abs(c - a.astype(np.float64) @ w.T) <= bound).all()
+    ab = O.f32_to_bf16(a)
+    aux = O.f32_to_bf16(O.synth_fill(O.F32, 2, 7, 13, 0, m * n, 0.0, 1.0).reshape(m, n))
+    for epilogue in (0, 1, 2) if n % 2 == 0 else (0, 1):
+        got = O.bf16_to_f32(llm.q8GemmHost(ab, q, s, epilogue=epilogue, aux=aux if epilogue == 1 else None))
+        want = O.bf16_to_f32(O.q8_gemm(ab, q, s, epilogue, aux if epilogue == 1 else None))
+        # two f32 sums of k terms, each off by at most k roundings of the sum of magnitudes, then rounded to bf16 (2^-8 of the value
+        # where they straddle); SwiGLU passes an error on times at most 1.1 (its slope) and the other factor
+        e = 2 * (k + 8) * 2.0 ** -24 * (np.abs(O.bf16_to_f32(ab).astype(np.float64)) @ np.abs(w.T))
+        if epilogue == 2:
+            exact = np.abs(O.bf16_to_f32(ab).astype(np.float64) @ w.T)
+            e = 1.1 * (e[:, ::2] * exact[:, 1::2] + e[:, 1::2] * exact[:, ::2] + e[:, ::2] * e[:, 1::2])
+        assert (np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + e).all() and np.mean(got != want) < 0.02, epilogue
+    assert llm.kernelStatus() == 0
 
 
 @pytest.mark.parametrize("m,n,k", [(96, 19000, 256), (97, 19001, 256), (193, 19004, 160), (100, 200, 128)])
