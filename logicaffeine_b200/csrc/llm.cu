@@ -64,6 +64,8 @@ struct PrefillWs {
   __half* q16 = nullptr;     // [rows][nq] rotated queries
   ActOut  att;               // [rows][nq]
   ActOut  ffn;               // [rows][f_local]
+  float*  split = nullptr;   // partial sums of K splits, an allocation of its own; null where there was no room for it
+  int64_t split_floats = 0;
 };
 
 struct Model {
@@ -175,6 +177,7 @@ void destroy(Model* m) {
   tp_destroy(&m->tp);
   for (void* p : m->allocs) cudaFree(p);
   if (m->pf.block) cudaFree(m->pf.block);
+  if (m->pf.split) cudaFree(m->pf.split);
   if (m->prompt) cudaFree(m->prompt);
   for (cudaEvent_t e : m->prof_events) cudaEventDestroy(e);
   if (m->readback) cudaFreeHost(m->readback);
@@ -668,7 +671,7 @@ logos_status_t step(Model* m, const int32_t* tokens_in, bool sample, bool log_to
 // h[b] = ws.h[row] + ws.delta[row] for the sequences whose last prompt position lies in the chunk that
 // starts at p0: the rows the end of the step (final norm, lm_head, token choice) runs on.
 __global__ void gather_last_rows_kernel(float* __restrict__ h, const float* __restrict__ src, const float* __restrict__ delta,
-                                        const int32_t* __restrict__ lens, const int32_t* __restrict__ seq_row0,
+                                        int parts, int64_t part_stride, const int32_t* __restrict__ lens, const int32_t* __restrict__ seq_row0,
                                         const int32_t* __restrict__ seq_count, int p0, int64_t hidden) {
   pdl_wait();
   pdl_trigger();
@@ -676,8 +679,11 @@ __global__ void gather_last_rows_kernel(float* __restrict__ h, const float* __re
   const int count = seq_count[b];
   if (count == 0 || lens[b] != p0 + count) return;
   const int64_t row = seq_row0[b] + count - 1;
-  for (int64_t e = threadIdx.x; e < hidden; e += blockDim.x)
-    h[b * hidden + e] = __fadd_rn(__ldcg(src + row * hidden + e), __ldcg(delta + row * hidden + e));
+  for (int64_t e = threadIdx.x; e < hidden; e += blockDim.x) {
+    float d = __ldcg(delta + row * hidden + e);
+    for (int i = 1; i < parts; ++i) d = __fadd_rn(d, __ldcg(delta + i * part_stride + row * hidden + e));
+    h[b * hidden + e] = __fadd_rn(__ldcg(src + row * hidden + e), d);
+  }
 }
 
 // Sequence state before the token choice that ends a prompt pass, a CTA a sequence: one that took a prompt stands at
@@ -761,6 +767,7 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
   if (w.block) {
     LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
     cudaFree(w.block);
+    if (w.split) cudaFree(w.split);
     w = PrefillWs();
   }
   char* base = nullptr;
@@ -787,6 +794,13 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
     planes[i]->lo = two ? reinterpret_cast<__half*>(base + o_lo[i]) : nullptr;
   }
   w.rows = want;
+  // up to sixteen splits of the widest product that is split, 64 MB at most; prompts go on without
+  w.split_floats = std::min<int64_t>(16 * want * std::max(H, m->nqkv), 16ll << 20);
+  if (cudaMalloc(reinterpret_cast<void**>(&w.split), (size_t)w.split_floats * 4) != cudaSuccess) {
+    cudaGetLastError();
+    w.split = nullptr;
+    w.split_floats = 0;
+  }
   return LOGOS_OK;
 }
 
@@ -882,17 +896,40 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
       g.device = m->device;
       return launch_q8_gemm(g, st);
     };
+    // The same with K splits where a matrix has few row tiles for these rows: into `parts` copies that the next norm adds up, or
+    // with a fold of its own (us: 1 x 100 tokens of the 0.5B shape 1963 -> 1633, 2 x 64 1993 -> 1494, 16 x 128 3990 -> 3890, two layers of the
+    // 32B shape 1 x 128 tokens 1189 -> 894, of which the wide GEMM units are a third).
+    int parts = 1;             // of the pending row-parallel product
+    const float* delta = w.delta;
+    auto gemm_split = [&](const ActOut& a, const Q8Mat& wt, int64_t k, GemmArgs g, bool folded) -> logos_status_t {
+      int sp = 1;
+      if (w.split && (!folded || m->tp.degree == 1) && wt.tiled)
+        sp = M > 64 ? gemm_many_splits(M, wt.n, k, m->device, folded) : gemm_pick_splits(M, wt.n, k, m->device, folded);
+      if (sp * M * wt.n > w.split_floats) sp = 1;
+      if (folded) {
+        parts = sp;
+        delta = sp > 1 ? w.split : w.delta;
+      }
+      if (sp <= 1) return gemm(a, wt, k, g);
+      const GemmArgs out = g;
+      g.c = nullptr;
+      g.splits = sp;
+      g.partials = w.split;
+      LOGOS_TRY(gemm(a, wt, k, g));
+      if (folded) return LOGOS_OK;
+      return launch_splitk_reduce(w.split, sp, out.c, out.c_dtype, out.c_act, out.ldc, nullptr, M, wt.n, EPI_NONE, st);
+    };
     auto reduce_delta = [&]() -> logos_status_t {
       if (m->tp.degree > 1) return tp_allreduce_sum_f32(&m->tp, w.delta, M * H, st);
       return LOGOS_OK;
     };
     for (int64_t l = 0; l < c.layers; ++l) {
       Layer& L = m->layers[(size_t)l];
-      LOGOS_TRY(launch_residual_rmsnorm(w.h, w.delta, l == 0 ? 0 : 1, M * H, m->gains + (2 * l) * H, w.xn, M, H, c.rms_eps, st));
+      LOGOS_TRY(launch_residual_rmsnorm(w.h, delta, l == 0 ? 0 : parts, M * H, m->gains + (2 * l) * H, w.xn, M, H, c.rms_eps, st));
       {
         GemmArgs g;
         g.c = w.qkv; g.c_dtype = LOGOS_F32; g.ldc = m->nqkv;
-        LOGOS_TRY(gemm(w.xn, L.wqkv, H, g));
+        LOGOS_TRY(gemm_split(w.xn, L.wqkv, H, g, false));
       }
       {
         PrefillAttnArgs a;
@@ -908,10 +945,10 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
       {
         GemmArgs g;
         g.c = w.delta; g.c_dtype = LOGOS_F32; g.ldc = H;
-        LOGOS_TRY(gemm(w.att, L.wo, m->nq, g));
+        LOGOS_TRY(gemm_split(w.att, L.wo, m->nq, g, true));
         LOGOS_TRY(reduce_delta());
       }
-      LOGOS_TRY(launch_residual_rmsnorm(w.h, w.delta, 1, M * H, m->gains + (2 * l + 1) * H, w.xn, M, H, c.rms_eps, st));
+      LOGOS_TRY(launch_residual_rmsnorm(w.h, delta, parts, M * H, m->gains + (2 * l + 1) * H, w.xn, M, H, c.rms_eps, st));
       {
         GemmArgs g;
         g.c_dtype = LOGOS_ACT_PLANES; g.c_act = w.ffn; g.ldc = m->f_local;
@@ -921,14 +958,14 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
       {
         GemmArgs g;
         g.c = w.delta; g.c_dtype = LOGOS_F32; g.ldc = H;
-        LOGOS_TRY(gemm(w.ffn, L.wd, m->f_local, g));
+        LOGOS_TRY(gemm_split(w.ffn, L.wd, m->f_local, g, true));
         LOGOS_TRY(reduce_delta());
       }
       LOGOS_TRY(debug_check(m, "prefill layer", l));
     }
     // the last position of every prompt that ends in this chunk: fold the pending delta
     LOGOS_CUDA_TRY(launch_kernel(gather_last_rows_kernel, dim3((unsigned)B), dim3(256), 0, st, m->h, (const float*)w.h,
-                                 (const float*)w.delta, (const int32_t*)lens_dev, row0_dev, count_dev, (int)ch.p0, H));
+                                 delta, parts, M * H, (const int32_t*)lens_dev, row0_dev, count_dev, (int)ch.p0, H));
     LOGOS_TRY(check_launch("gather_last_rows_kernel"));
   }
   // the ordinary end of a step for the sequences that took a prompt

@@ -70,6 +70,12 @@ logos_status_t launch_gemm_operator(const GemmArgs& g, cudaStream_t st);
 // How many K-splits launch_q8_gemm would like for this shape (1 = none).
 // folded: the partials' consumer adds them up as it reads them.
 int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device, bool folded);
+// K splits of a product of more than 64 tokens, whose fold is a launch (folded: the consumer's): what makes the kernel's own plan and the
+// fold cheapest together, by the plans' costs.  gemm_pick_splits counts units of 64 tokens, a form that many tokens do not
+// run in.  At most 64 MB of partial sums; one split where every SM has a row tile.  35 drawn shapes of 65 to 3411 tokens: 1 %
+// slower than the best count in the mean, by that rule 6.4 % (bf16 389 x 2048 x 16512 81.8 -> 60.4 us, 256 x 3584 x 18944 95.6 ->
+// 74.5, f32 173 x 2304 x 6016 24.8 -> 19.7).
+int gemm_many_splits(int64_t m, int64_t n, int64_t k, int device, bool folded);
 // Whether the tcgen05 kernel accepts this call (else the SIMT kernel runs).
 bool gemm_tc_applicable(const GemmArgs& g);
 // A stand-alone product of one or two tokens by the GEMV kernel: one launch instead of the preparation of activation planes,

@@ -266,7 +266,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   const int src_dtype = g.a_dtype;
   const int64_t stages = (g.k + 127) / 128;
   const bool retile = g.k % 128 != 0;
-  int splits = g.m > 64 ? gemm_many_splits(g.m, g.n, g.k, g.device) : gemm_pick_splits(g.m, g.n, g.k, g.device, false);
+  int splits = g.m > 64 ? gemm_many_splits(g.m, g.n, g.k, g.device, false) : gemm_pick_splits(g.m, g.n, g.k, g.device, false);
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   const int64_t lda = stages * 128;
   const int64_t plane_bytes = up(g.m * lda * 2);

@@ -1224,8 +1224,9 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms, int64_t* 
   return best;
 }
 
-// See gemm_many_splits.  The fold of the splits on the costs' scale: its launch, and writing and reading the partial sums.
-int make_splits(int64_t m, int64_t n, int64_t k, int sms) {
+// See gemm_many_splits.  The fold of the splits on the costs' scale: its launch (unless the consumer folds), and writing and
+// reading the partial sums.
+int make_splits(int64_t m, int64_t n, int64_t k, int sms, bool folded) {
   const int64_t stages = k / TC_KSTAGE, most = std::min<int64_t>(stages / 4, 16);
   int best = 1;
   int64_t best_cost = INT64_MAX;
@@ -1233,7 +1234,7 @@ int make_splits(int64_t m, int64_t n, int64_t k, int sms) {
     if (sp > 1 && sp * m * n > (16ll << 20)) break;
     int64_t cost;
     make_plan(m, n, k, sp, sms, &cost);
-    if (sp > 1) cost += 6000 + sp * m * n / 333;
+    if (sp > 1) cost += folded ? 1500 + sp * m * n / 600 : 6000 + sp * m * n / 333;
     if (cost < best_cost) {
       best_cost = cost;
       best = (int)sp;
@@ -1343,16 +1344,18 @@ bool gemm_tc_applicable(const GemmArgs& g) {
   return true;
 }
 
-int gemm_many_splits(int64_t m, int64_t n, int64_t k, int device) {
+int gemm_many_splits(int64_t m, int64_t n, int64_t k, int device, bool folded) {
   if ((n + TC_ROWS - 1) / TC_ROWS >= sm_count(device)) return 1;
   struct Entry {
     int64_t m = -1, n = 0, k = 0;
     int device = 0, splits = 1;
+    bool folded = false;
   };
   thread_local Entry cache[64];   // a pure function of the shape, as the plans are
   const uint64_t h = ((uint64_t)m * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)n * 0xBF58476D1CE4E5B9ull) ^ ((uint64_t)k * 0x94D049BB133111EBull);
   Entry& e = cache[(h ^ (h >> 29)) >> 7 & 63];
-  if (e.m != m || e.n != n || e.k != k || e.device != device) e = Entry{m, n, k, device, make_splits(m, n, k, sm_count(device))};
+  if (e.m != m || e.n != n || e.k != k || e.device != device || e.folded != folded)
+    e = Entry{m, n, k, device, make_splits(m, n, k, sm_count(device), folded), folded};
   return e.splits;
 }
 

@@ -440,3 +440,23 @@ def test_prompt_pass_with_seven_query_heads_per_kv_head_and_a_second_prompt(llm,
         ref.close()
     assert llm.kernelStatus() == 0
     gpu.free()
+
+
+@pytest.mark.parametrize("batch,t", [(1, 17), (2, 32), (1, 65), (3, 70)])   # up to 64 rows, and the rule above; one chunk and its last rows
+def test_prompts_of_few_rows_in_k_splits(llm, oracle, batch, t):
+    """Few rows and long K: qkv with a fold of its own, o_proj and down_proj folded by the norms and, after the last layer,
+    where the last rows are gathered."""
+    O = oracle
+    cfg = dict(layers=2, hidden=1536, h_q=12, h_kv=2, head_dim=128, ffn=4096, vocab=1024, l_max=128, batch=batch,
+               rms_eps=1e-6, rope_theta=1e6, tied_embeddings=1, seed=4, init_std=0.02)
+    toks = O.synth_fill(O.I32, 3, cfg["seed"], 900 + t, 0, batch * t, 0.0, float(cfg["vocab"])).reshape(batch, t)
+    ref = O.Llm(tp_degree=1, tp_rank=0, device=0, act_dtype=O.F32, **cfg)
+    ref.prefill(toks)
+    gpu = llm.Llm(**cfg)
+    gpu.prefill(toks)
+    assert rel_l2(gpu.readLogits(), ref.read_logits()) < 1e-4   # as above: f32 sums in another order over fp16 K and V
+    want = np.array([ref.decode_step().copy() for _ in range(6)])
+    assert np.array_equal(gpu.decodeSteps(6), want)
+    assert llm.kernelStatus() == 0
+    gpu.free()
+    ref.close()
