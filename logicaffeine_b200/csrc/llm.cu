@@ -64,8 +64,8 @@ struct PrefillWs {
   __half* q16 = nullptr;     // [rows][nq] rotated queries
   ActOut  att;               // [rows][nq]
   ActOut  ffn;               // [rows][f_local]
-  float*  split = nullptr;   // partial sums of K splits, an allocation of its own; null where there was no room for it
-  int64_t split_floats = 0;
+  float*  split = nullptr;   // [split_floats] partial sums of K splits
+  int64_t split_floats = 0;  // asked for; `split` is null where there was no room for it
 };
 
 struct Model {
@@ -177,7 +177,6 @@ void destroy(Model* m) {
   tp_destroy(&m->tp);
   for (void* p : m->allocs) cudaFree(p);
   if (m->pf.block) cudaFree(m->pf.block);
-  if (m->pf.split) cudaFree(m->pf.split);
   if (m->prompt) cudaFree(m->prompt);
   for (cudaEvent_t e : m->prof_events) cudaEventDestroy(e);
   if (m->readback) cudaFreeHost(m->readback);
@@ -739,15 +738,15 @@ logos_status_t prompt_words(Model* m, int64_t need) {
 // One block for the buffers of a chunk of up to `rows` rows.  When a later prompt fills a larger chunk than any before
 // it, it grows at least geometrically, up to `most` rows unless more are needed; the old block is freed once the
 // stream has left it.
-logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
+logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most, int64_t split_floats) {
   PrefillWs& w = m->pf;
-  if (w.rows >= rows) return LOGOS_OK;
+  if (w.rows >= rows && w.split_floats >= split_floats) return LOGOS_OK;
   const logos_llm_config_t& c = m->cfg;
   const int64_t H = c.hidden;
   const bool two = c.act_dtype == LOGOS_F32;
   const int64_t widths[3] = {H, m->nq, m->f_local};
-  int64_t total = 0, o_h = 0, o_delta = 0, o_qkv = 0, o_q16 = 0, o_hi[3], o_lo[3];
-  auto lay_out = [&](int64_t n) {
+  int64_t total = 0, o_h = 0, o_delta = 0, o_qkv = 0, o_q16 = 0, o_split = 0, o_hi[3], o_lo[3];
+  auto lay_out = [&](int64_t n, int64_t split) {
     total = 0;
     auto place = [&](int64_t bytes) {
       const int64_t at = total;
@@ -762,20 +761,27 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
       o_hi[i] = place(n * widths[i] * 2);
       o_lo[i] = two ? place(n * widths[i] * 2) : 0;
     }
+    o_split = place(split * 4);
   };
-  int64_t want = std::max(rows, std::min(2 * w.rows, most));
+  int64_t want = w.rows >= rows ? w.rows : std::max(rows, std::min(2 * w.rows, most));
+  split_floats = std::max(split_floats, w.split_floats);
+  int64_t split = split_floats;
   if (w.block) {
     LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
     cudaFree(w.block);
-    if (w.split) cudaFree(w.split);
     w = PrefillWs();
   }
   char* base = nullptr;
-  lay_out(want);
+  lay_out(want, split);
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&base), (size_t)total);
   if (e != cudaSuccess && want > rows) {
     cudaGetLastError();
-    lay_out(want = rows);
+    lay_out(want = rows, split);
+    e = cudaMalloc(reinterpret_cast<void**>(&base), (size_t)total);
+  }
+  if (e != cudaSuccess && split > 0) {   // prompts go on without splits
+    cudaGetLastError();
+    lay_out(want, split = 0);
     e = cudaMalloc(reinterpret_cast<void**>(&base), (size_t)total);
   }
   if (e != cudaSuccess) {
@@ -787,6 +793,8 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
   w.delta = reinterpret_cast<float*>(base + o_delta);
   w.qkv = reinterpret_cast<float*>(base + o_qkv);
   w.q16 = reinterpret_cast<__half*>(base + o_q16);
+  w.split = split > 0 ? reinterpret_cast<float*>(base + o_split) : nullptr;
+  w.split_floats = split_floats;
   ActOut* planes[3] = {&w.xn, &w.att, &w.ffn};
   for (int i = 0; i < 3; ++i) {
     planes[i]->mode = c.act_dtype;
@@ -794,14 +802,15 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most) {
     planes[i]->lo = two ? reinterpret_cast<__half*>(base + o_lo[i]) : nullptr;
   }
   w.rows = want;
-  // up to sixteen splits of the widest product that is split, 64 MB at most; prompts go on without
-  w.split_floats = std::min<int64_t>(16 * want * std::max(H, m->nqkv), 16ll << 20);
-  if (cudaMalloc(reinterpret_cast<void**>(&w.split), (size_t)w.split_floats * 4) != cudaSuccess) {
-    cudaGetLastError();
-    w.split = nullptr;
-    w.split_floats = 0;
-  }
   return LOGOS_OK;
+}
+
+// K splits of a prompt's product of `rows` rows whose partial sums fit 64 MB (folded: by its consumer; a rank's row-parallel products
+// stay whole, since the exchange wants one sum).
+int prompt_splits(const Model* m, int64_t rows, const Q8Mat& w, bool folded) {
+  if (!w.tiled || (folded && m->tp.degree > 1)) return 1;
+  const int sp = rows > 64 ? gemm_many_splits(rows, w.n, w.k, m->device, folded) : gemm_pick_splits(rows, w.n, w.k, m->device, folded);
+  return sp * rows * w.n <= (16ll << 20) ? sp : 1;
 }
 
 // The prompt pass proper: chunks of positions, every sequence's part of the chunk at once, so that each
@@ -846,7 +855,19 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
   };
   cut();
   while (most_rows > 0) {
-    const logos_status_t got = prefill_workspace(m, most_rows, target_rows);
+    int64_t split_floats = 0;
+    for (const Chunk& ch : chunks) {
+      if (m->layers.empty()) break;
+      const Layer& L = m->layers[0];
+      auto want = [&](const Q8Mat& wt, bool folded) {
+        const int64_t sp = prompt_splits(m, ch.rows, wt, folded);
+        if (sp > 1) split_floats = std::max(split_floats, sp * ch.rows * wt.n);
+      };
+      want(L.wqkv, false);
+      want(L.wo, true);
+      want(L.wd, true);
+    }
+    const logos_status_t got = prefill_workspace(m, most_rows, target_rows, split_floats);
     if (got == LOGOS_OK) break;
     // no room for chunks of this size: smaller ones, down to a position at a time
     const int64_t before = most_rows;
@@ -902,10 +923,7 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
     int parts = 1;             // of the pending row-parallel product
     const float* delta = w.delta;
     auto gemm_split = [&](const ActOut& a, const Q8Mat& wt, int64_t k, GemmArgs g, bool folded) -> logos_status_t {
-      int sp = 1;
-      if (w.split && (!folded || m->tp.degree == 1) && wt.tiled)
-        sp = M > 64 ? gemm_many_splits(M, wt.n, k, m->device, folded) : gemm_pick_splits(M, wt.n, k, m->device, folded);
-      if (sp * M * wt.n > w.split_floats) sp = 1;
+      const int sp = w.split ? prompt_splits(m, M, wt, folded) : 1;
       if (folded) {
         parts = sp;
         delta = sp > 1 ? w.split : w.delta;
