@@ -4,8 +4,16 @@
 
 using namespace logos;
 
+// Whether results go over the activations.  The GEMM has copied those into planes before it writes; of the GEMV kernel some
+// CTAs read them while others write already.
+static bool over_activations(const GemmArgs& g) {
+  const int64_t bytes = g.a_dtype == LOGOS_F32 ? 4 : 2;   // of results too
+  const char *a = static_cast<const char*>(g.a), *c = static_cast<const char*>(g.c);
+  return c < a + g.m * g.lda * bytes && a < c + g.m * g.ldc * bytes;
+}
+
 static logos_status_t launch_product(const GemmArgs& g, cudaStream_t st) {
-  if (!g.force_simt && gemv_takes(g.m, g.n, g.k)) {
+  if (!g.force_simt && gemv_takes(g.m, g.n, g.k) && !over_activations(g)) {
     OrderedScope ordered(st);
     return launch_q8_gemv_tokens(g, st);
   }

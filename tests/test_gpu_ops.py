@@ -303,6 +303,35 @@ def test_q8_gemm_of_one_or_two_tokens(llm, oracle, m, n, k):
     assert llm.kernelStatus() == 0
 
 
+@pytest.mark.parametrize("m", [1, 2, 3])
+@pytest.mark.parametrize("n,k", [(2048, 2048), (3072, 1024)])   # results of the activations' size, and of a larger one
+def test_q8_gemm_results_over_the_activations(llm, oracle, m, n, k):
+    """A product into the buffer that its activations are in, with the residual there too where it fits: what only kernels that
+    have read all activations before the first result is written can give."""
+    O = oracle
+    a = O.synth_fill(O.F32, 2, 17, 10, 0, m * n, 0.0, 1.0)   # the product's are the first m * k
+    q = O.synth_fill(O.I8, 0, 17, 11, 0, n * k).reshape(n, k)
+    s = O.synth_fill(O.F32, 1, 17, 12, 0, n * (k // 32), 1e-3, 1e-2).reshape(n, k // 32)
+    w = q.astype(np.float64) * np.repeat(s.astype(np.float64), 32, axis=1)
+    dq, ds, db = _dev(llm, q), _dev(llm, s), _dev(llm, a)
+    gemv = llm.launchCounts()["q8_gemv"]
+    llm.q8GemmF32(db, dq, ds, db, m, n, k)
+    x = a[:m * k].reshape(m, k).astype(np.float64)
+    # f32 sums of k terms in any order: k roundings of at most 2^-24 of the sum of magnitudes, and 22-bit planes
+    bound = (k + 8) * 2.0 ** -24 * (np.abs(x) @ np.abs(w.T))
+    assert (np.abs(db.download(np.float32, (m, n)) - x @ w.T) <= bound).all()
+    for epilogue in (0, 1, 2):
+        ab = O.f32_to_bf16(a)
+        db = _dev(llm, ab)
+        aux = ab.reshape(m, n) if epilogue == 1 else None
+        llm.q8Gemm(db, dq, ds, db, m, n, k, epilogue, db if epilogue == 1 else None)
+        got = db.download(np.uint16, (m, n // 2 if epilogue == 2 else n))
+        # one rounding to bf16 of sums in another order: last-place differences of few elements
+        assert np.mean(got != O.q8_gemm(ab[:m * k].reshape(m, k), q, s, epilogue, aux)) < 0.01, epilogue
+    assert llm.launchCounts()["q8_gemv"] == gemv   # its CTAs read activations while others write
+    assert llm.kernelStatus() == 0
+
+
 @pytest.mark.parametrize("m,n,k", [(96, 19000, 256), (97, 19001, 256), (193, 19004, 160), (100, 200, 128)])
 def test_q8_gemm_residual_of_several_token_tiles(llm, oracle, m, n, k):
     """Past one token tile the residual is added by a kernel of its own: ends of its vectors, and of the rule."""
