@@ -89,8 +89,8 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
   const int xchunks = X_IN_SMEM ? (chunks + 31) / 32 * 32 : 0;
   uint8_t* ring = reinterpret_cast<uint8_t*>(xs4 + M * xchunks * 4) + warp * (GEMV_DEPTH * GEMV_STAGE);
   const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
-  // In a caller's scope the weights are read before the previous kernel of the stream has finished (the scope promises
-  // that nothing in it writes them); x and y wait for it.
+  // early: the weights are read before the previous kernel of the stream has finished (q8_gemv in a caller's scope, which
+  // promises that nothing in it writes them); x and y wait for it.
   if (!early) pdl_wait();
   pdl_trigger();
   const int64_t groups = (n + R - 1) / R, step = (int64_t)gridDim.x * warps;
@@ -207,8 +207,8 @@ int64_t ring_bytes(int warps) { return (int64_t)warps * GEMV_DEPTH * GEMV_STAGE;
 int64_t x_bytes(int64_t m, int64_t k) { return m * ((k / 16 + 31) / 32 * 128) * (int64_t)sizeof(float4); }
 
 template <int M, typename T>
-logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64_t n, int64_t k, const T* aux, int epilogue, int device,
-                        cudaStream_t st) {
+logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64_t n, int64_t k, bool early, const T* aux, int epilogue,
+                        int device, cudaStream_t st) {
   // two rows a warp unless that would leave more than half of the warps without any; the larger CTA where x fits
   // beside its rings (K up to 16384 for one vector), past K = 30208 x stays in global memory (one vector only)
   const int64_t sms = sm_count(device);
@@ -223,15 +223,17 @@ logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64
   }
   LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kern), device, GEMV_SMEM));
   LOGOS_CUDA_TRY(launch_kernel(kern, dim3((unsigned)std::min(groups, sms)), dim3(warps * 32), (size_t)(ring_bytes(warps) + (in_smem ? xb : 0)),
-                               st, q, s, x, y, n, k, pdl_early(), aux, epilogue));
+                               st, q, s, x, y, n, k, early, aux, epilogue));
   count_launch(LK_GEMV);
   return check_launch("q8_gemv_kernel");
 }
 
+// The GEMM operators' first kernel waits in a caller's scope too.
 template <typename T>
 logos_status_t launch_rows(const int8_t* q, const float* s, const T* x, T* y, int64_t m, int64_t n, int64_t k, const T* aux, int epilogue,
                            int device, cudaStream_t st) {
-  return m == 1 ? launch_m<1, T>(q, s, x, y, n, k, aux, epilogue, device, st) : launch_m<2, T>(q, s, x, y, n, k, aux, epilogue, device, st);
+  return m == 1 ? launch_m<1, T>(q, s, x, y, n, k, false, aux, epilogue, device, st)
+                : launch_m<2, T>(q, s, x, y, n, k, false, aux, epilogue, device, st);
 }
 
 }  // namespace
@@ -243,7 +245,7 @@ logos_status_t launch_q8_gemv(const int8_t* q, const float* s, const float* x, f
     LOGOS_CUDA_TRY(cudaMemsetAsync(y, 0, sizeof(float) * n, st));
     return LOGOS_OK;
   }
-  return launch_m<1, float>(q, s, x, y, n, k, nullptr, EPI_NONE, device, st);
+  return launch_m<1, float>(q, s, x, y, n, k, pdl_early(), nullptr, EPI_NONE, device, st);
 }
 
 bool gemv_takes(int64_t m, int64_t n, int64_t k) {

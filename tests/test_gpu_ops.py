@@ -788,6 +788,39 @@ def test_operators_behind_calls_that_write_their_weights(llm, oracle):
                 assert np.array_equal(got, w), i
 
 
+def test_products_in_a_scope_behind_one_that_writes_their_scales(llm, oracle):
+    """q8_gemm of any number of tokens reads nothing before the calls ahead of it have ended, in a caller's scope too: here the
+    scales are the results of a long product that was still running when the scope was opened."""
+    n, k, nw, kw, m, rounds = 1184, 4096, 2368, 8192, 64, 4    # m * nw results are the n * k / 32 scales
+    dq, wq, ws = llm.DeviceBuffer(n * k), llm.DeviceBuffer(nw * kw), llm.DeviceBuffer(nw * (kw // 32) * 4)
+    wx, ds, dx, dxb = (llm.DeviceBuffer(b) for b in (m * kw * 4, m * nw * 4, 3 * k * 4, 3 * k * 2))
+    llm.synthFill(dq, llm.I8, 0, 5, 1, 0, n * k, 0.0, 1.0)
+    llm.synthFill(wq, llm.I8, 0, 5, 2, 0, nw * kw, 0.0, 1.0)
+    llm.synthFill(ws, llm.F32, 1, 5, 3, 0, nw * (kw // 32), 1e-5, 1e-4)
+    llm.synthFill(dx, llm.F32, 2, 5, 4, 0, 3 * k, 0.0, 1.0)
+    llm.synthFill(dxb, llm.BF16, 2, 5, 4, 0, 3 * k, 0.0, 1.0)
+
+    def results(wait):
+        outs = []
+        for i in range(rounds):
+            for tokens in (1, 2, 3):
+                c, cb = llm.DeviceBuffer(tokens * n * 4), llm.DeviceBuffer(tokens * n * 2)
+                for call in (lambda: llm.q8GemmF32(dx, dq, ds, c, tokens, n, k), lambda: llm.q8Gemm(dxb, dq, ds, cb, tokens, n, k)):
+                    llm.synthFill(wx, llm.F32, 2, 70 + 3 * i + tokens, 5, 0, m * kw, 0.0, 1.0)
+                    llm.q8GemmF32(wx, wq, ws, ds, m, nw, kw)
+                    if wait:
+                        llm.devSync()
+                    prev = llm.dependentLaunchScope(True)
+                    call()
+                    llm.dependentLaunchScope(prev)
+                outs += [(c, tokens * n * 4), (cb, tokens * n * 2)]
+        llm.devSync()
+        return [b.download(np.uint8, (size,)) for b, size in outs]
+
+    for got, want in zip(results(False), results(True)):
+        assert np.array_equal(got, want)
+
+
 def test_waits_inside_kernels_end_in_seconds(tmp_path):
     """A wait for a barrier that nothing completes returns and says so, in seconds: the limit is of time, whatever a
     poll takes."""
