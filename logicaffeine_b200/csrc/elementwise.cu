@@ -340,10 +340,13 @@ tp_residual_rmsnorm_kernel(float* __restrict__ h, const TpFusedArgs t, int parts
 // aligned), then four scales a thread: one row of a K tile.
 template <bool BF16>
 __global__ void __launch_bounds__(256)
-gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const float* __restrict__ s, float* __restrict__ tiled,
-                 int64_t n, int64_t kb, int64_t ktiles, int64_t act_blocks, unsigned* misfit, unsigned call) {
+gemm_prep_kernel(const void* a, ActOut o, int64_t count8, const float* s, float* tiled, int64_t n, int64_t kb, int64_t ktiles,
+                 int64_t act_blocks, unsigned* misfit, unsigned call) {
   // count8: groups of eight of the planes; rows of the planes are whole K tiles, rows of `a` kb * 32 values
   // The product behind this kernel reads weights without a wait of its own: it may start once all before this one has ended.
+  // Activations and scales can be what the kernel before has just written: no pointer here says read-only, whose loads need
+  // not see that.  (The scales by ordinary loads: a row's four come from one line, past L1 each fetched it for itself,
+  // 64 x 3584 x 2368 13.65 -> 14.01 us.)
   pdl_wait();
   pdl_trigger();
   if ((int64_t)blockIdx.x < act_blocks) {
@@ -359,7 +362,7 @@ gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const flo
     }
     if (!inside) {
     } else if (BF16) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a) + src);
+      const uint4 v = __ldcg(reinterpret_cast<const uint4*>(a) + src);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -367,7 +370,7 @@ gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const flo
         x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
       }
     } else {
-      const float4 v0 = __ldg(reinterpret_cast<const float4*>(a) + 2 * src), v1 = __ldg(reinterpret_cast<const float4*>(a) + 2 * src + 1);
+      const float4 v0 = __ldcg(reinterpret_cast<const float4*>(a) + 2 * src), v1 = __ldcg(reinterpret_cast<const float4*>(a) + 2 * src + 1);
       x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w;
       x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
     }
@@ -403,10 +406,10 @@ gemm_prep_kernel(const void* __restrict__ a, ActOut o, int64_t count8, const flo
   if (row >= n) return;
   float4 v;
   const float* src = s + row * kb + kt * 4;
-  v.x = __ldg(src);
-  v.y = kt * 4 + 1 < kb ? __ldg(src + 1) : 0.f;
-  v.z = kt * 4 + 2 < kb ? __ldg(src + 2) : 0.f;
-  v.w = kt * 4 + 3 < kb ? __ldg(src + 3) : 0.f;
+  v.x = src[0];
+  v.y = kt * 4 + 1 < kb ? src[1] : 0.f;
+  v.z = kt * 4 + 2 < kb ? src[2] : 0.f;
+  v.w = kt * 4 + 3 < kb ? src[3] : 0.f;
   reinterpret_cast<float4*>(tiled)[((row >> 7) * ktiles + kt) * 128 + (row & 127)] = v;
 }
 

@@ -788,6 +788,70 @@ def test_operators_behind_calls_that_write_their_weights(llm, oracle):
                 assert np.array_equal(got, w), i
 
 
+def _chained(llm, wait):
+    """Operators outside a scope whose inputs are the results of the calls just before them, over buffers that every round
+    uses again; all bits that the last rounds leave, and those of every round's ends."""
+    def sync(call, *args):
+        call(*args)
+        if wait:
+            llm.devSync()
+
+    def weights(i, n, k):
+        q, s = llm.DeviceBuffer(n * k), llm.DeviceBuffer(n * (k // 32) * 4)
+        llm.synthFill(q, llm.I8, 0, 40, 2 * i, 0, n * k, 0.0, 1.0)
+        llm.synthFill(s, llm.F32, 1, 40, 2 * i + 1, 0, n * (k // 32), 1e-4, 1e-3)
+        return q, s
+
+    rounds, b, hq, hkv, d, lmax = 5, 4, 8, 2, 64, 256
+    x0, y, s2, c, e = (llm.DeviceBuffer(4 * count) for count in (512, 3168, 2368 * 33, 3 * 2368, 3072))
+    xb, cb, hb, gb, o1, o2 = (llm.DeviceBuffer(2 * count) for count in (65 * 1024, 65 * 2177, 69 * 1536, 69 * 1024, 2048, 2048))
+    kc, vc = llm.DeviceBuffer(2 * b * hkv * lmax * d), llm.DeviceBuffer(2 * b * hkv * lmax * d)
+    tab, seq = _dev(llm, llm.ropeTable(lmax, d, 1e6)), _dev(llm, np.array([3, 64, 127, 200], np.int32))
+    wy, ws, w2, wd, we, wf = (weights(i, *shape) for i, shape in enumerate([(3168, 512), (2368 * 33, 512), (2368, 1056), (1024, 2368),
+                                                                          (512, 512), (640, 3072)]))
+    wc, wh, wg, wo, wp = (weights(10 + i, *shape) for i, shape in enumerate([(2177, 1024), (1536, 2048), (2048, 1536), (300, 1024), (700, 512)]))
+    dd = llm.DeviceBuffer(4 * 3072)
+    llm.synthFill(cb, llm.BF16, 2, 41, 1, 0, 65 * 2177, 0.0, 1.0)
+    for i, cache in enumerate((kc, vc)):
+        llm.synthFill(cache, llm.F16, 2, 41, 2 + i, 0, b * hkv * lmax * d, 0.0, 1.0)
+    ends = [[llm.DeviceBuffer(n) for n in (3072 * 4, 640 * 4, 2 * 300 * 2, 4 * 700 * 2)] for _ in range(rounds)]
+    llm.devSync()
+    for r, (end_e, end_f, end_o, end_p) in enumerate(ends):
+        llm.synthFill(x0, llm.F32, 2, 50 + r, 1, 0, 512, 0.0, 1.0)
+        llm.synthFill(xb, llm.BF16, 2, 50 + r, 2, 0, 65 * 1024, 0.0, 1.0)
+        # f32: vectors by the GEMV, activations and scales of a K that is no multiple of 128, then planes, then one token
+        sync(llm.q8Gemv, *wy, x0, y, 3168, 512)
+        sync(llm.q8Gemv, *ws, x0, s2, 2368 * 33, 512)
+        sync(llm.q8GemmF32, y, w2[0], s2, c, 3, 2368, 1056)
+        sync(llm.q8GemmF32, c, *wd, dd, 3, 1024, 2368)
+        sync(llm.q8GemmF32, dd, *we, e, 6, 512, 512)
+        sync(llm.q8GemmF32, e, *we, end_e, 6, 512, 512)
+        sync(llm.q8GemmF32, end_e, *wf, end_f, 1, 640, 3072)
+        # bf16: a residual in place with an odd number of columns, then products of what it left
+        sync(llm.q8Gemm, xb, *wc, cb, 65, 2177, 1024, 1, cb)
+        sync(llm.q8Gemm, cb, *wh, hb, 69, 1536, 2048)
+        sync(llm.q8Gemm, hb, *wg, gb, 69, 2048, 1536, 2)
+        # attention over those bits as f16 rows: append, attend, both in one call, and products of its result
+        sync(llm.kvAppendRope, kc, vc, gb, gb, tab, seq, b, hkv, d, lmax)
+        sync(llm.gqaDecodeAttn, gb, kc, vc, seq, o1, b, hq, hkv, d, lmax, 0.125)
+        sync(llm.gqaDecodeAttnFused, o1, gb, o1, kc, vc, tab, seq, o2, b, hq, hkv, d, lmax, 0.125)
+        sync(llm.q8Gemm, o2, *wo, end_o, 2, 300, 1024)
+        sync(llm.q8Gemm, o2, *wp, end_p, 4, 700, 512)
+    llm.devSync()
+    assert llm.kernelStatus() == 0
+    return [buf.download(np.uint8, (buf.nbytes,)) for buf in [y, s2, c, dd, e, cb, hb, gb, o1, o2, kc, vc, seq] + [x for row in ends for x in row]]
+
+
+def test_operators_behind_operators_that_write_their_operands(llm, oracle):
+    """An operator that starts while the one before it ends reads what that one wrote: activations, scales, residuals, cache
+    rows, lengths and queries."""
+    want = _chained(llm, True)
+    assert all(w.any() for w in want)
+    for _ in range(4):
+        for i, (got, w) in enumerate(zip(_chained(llm, False), want)):
+            assert np.array_equal(got, w), i
+
+
 def test_products_in_a_scope_behind_one_that_writes_their_scales(llm, oracle):
     """q8_gemm of any number of tokens reads nothing before the calls ahead of it have ended, in a caller's scope too: here the
     scales are the results of a long product that was still running when the scope was opened."""
