@@ -12,7 +12,6 @@
 #include "ops.cuh"
 
 #include <algorithm>
-#include <type_traits>
 
 namespace logos {
 
@@ -75,10 +74,10 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 // measured 166 us on the first, one row 164 us.
 // M vectors of x at a time (rows of an [M][K] matrix, in T), as the GEMM operators have for a few tokens: a weight is
 // converted once for all of them, and their results go through the GEMM's epilogues.
-template <int R, bool X_IN_SMEM, int M, typename T>
+template <int R, bool X_IN_SMEM, int M, typename T, bool STATUS>
 __global__ void __launch_bounds__(GEMV_WARPS * 32, 1)
 q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const T* __restrict__ x, T* y, int64_t n, int64_t k, bool early,
-               const T* aux, int epilogue) {
+               const T* aux, int epilogue, const int* status) {
   constexpr int U = 4 / R;   // chunks of a row that a lane has in a stage
   extern __shared__ float4 xs4[];
   const int tid = threadIdx.x;
@@ -127,11 +126,19 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
 #pragma unroll
   for (int i = 0; i < GEMV_DEPTH - 1; ++i) load();
   if (early) pdl_wait();
+  // The GEMM operators write nothing on top of an earlier failure (STATUS).  A thread of the last warp, which has the least of x
+  // to fetch, reads the code for all.  One token 768 x 2176 without it 2.44 us, so 2.52; by thread 0 2.8, by every thread 3.0.
+  const bool prior = STATUS && tid == (int)blockDim.x - 1 && __ldcg(status) != 0;
   if (X_IN_SMEM) {
 #pragma unroll
     for (int v = 0; v < M; ++v)
       for (int i = tid; i < chunks * 4; i += blockDim.x) xs4[v * xchunks * 4 + xs4_index(i >> 2, i & 3)] = load_x4(x + v * k, i);
-    __syncthreads();
+    if (!STATUS) {
+      __syncthreads();
+    } else if (__syncthreads_or(prior)) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      return;
+    }
   }
   int slot = 0;
   for (int64_t g = blockIdx.x + (int64_t)gridDim.x * warp; g < groups; g += step) {
@@ -206,9 +213,9 @@ namespace {
 int64_t ring_bytes(int warps) { return (int64_t)warps * GEMV_DEPTH * GEMV_STAGE; }
 int64_t x_bytes(int64_t m, int64_t k) { return m * ((k / 16 + 31) / 32 * 128) * (int64_t)sizeof(float4); }
 
-template <int M, typename T>
+template <int M, typename T, bool STATUS>
 logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64_t n, int64_t k, bool early, const T* aux, int epilogue,
-                        int device, cudaStream_t st) {
+                        const int* status, int device, cudaStream_t st) {
   // two rows a warp unless that would leave more than half of the warps without any; the larger CTA where x fits
   // beside its rings (K up to 16384 for one vector), past K = 30208 x stays in global memory (one vector only)
   const int64_t sms = sm_count(device);
@@ -217,13 +224,13 @@ logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64
   const int64_t xb = x_bytes(M, k);
   const int warps = ring_bytes(GEMV_WARPS) + xb <= GEMV_SMEM ? GEMV_WARPS : GEMV_FEW_WARPS;
   const bool in_smem = ring_bytes(warps) + xb <= GEMV_SMEM;
-  auto kern = rows == 2 ? q8_gemv_kernel<2, true, M, T> : q8_gemv_kernel<1, true, M, T>;
-  if constexpr (M == 1 && std::is_same_v<T, float>) {
-    if (!in_smem) kern = rows == 2 ? q8_gemv_kernel<2, false, M, T> : q8_gemv_kernel<1, false, M, T>;
+  auto kern = rows == 2 ? q8_gemv_kernel<2, true, M, T, STATUS> : q8_gemv_kernel<1, true, M, T, STATUS>;
+  if constexpr (!STATUS) {
+    if (!in_smem) kern = rows == 2 ? q8_gemv_kernel<2, false, M, T, false> : q8_gemv_kernel<1, false, M, T, false>;
   }
   LOGOS_TRY(allow_smem(reinterpret_cast<const void*>(kern), device, GEMV_SMEM));
   LOGOS_CUDA_TRY(launch_kernel(kern, dim3((unsigned)std::min(groups, sms)), dim3(warps * 32), (size_t)(ring_bytes(warps) + (in_smem ? xb : 0)),
-                               st, q, s, x, y, n, k, early, aux, epilogue));
+                               st, q, s, x, y, n, k, early, aux, epilogue, status));
   count_launch(LK_GEMV);
   return check_launch("q8_gemv_kernel");
 }
@@ -232,8 +239,10 @@ logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64
 template <typename T>
 logos_status_t launch_rows(const int8_t* q, const float* s, const T* x, T* y, int64_t m, int64_t n, int64_t k, const T* aux, int epilogue,
                            int device, cudaStream_t st) {
-  return m == 1 ? launch_m<1, T>(q, s, x, y, n, k, false, aux, epilogue, device, st)
-                : launch_m<2, T>(q, s, x, y, n, k, false, aux, epilogue, device, st);
+  const int* status = kernel_status_ptr(device);
+  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
+  return m == 1 ? launch_m<1, T, true>(q, s, x, y, n, k, false, aux, epilogue, status, device, st)
+                : launch_m<2, T, true>(q, s, x, y, n, k, false, aux, epilogue, status, device, st);
 }
 
 }  // namespace
@@ -245,7 +254,7 @@ logos_status_t launch_q8_gemv(const int8_t* q, const float* s, const float* x, f
     LOGOS_CUDA_TRY(cudaMemsetAsync(y, 0, sizeof(float) * n, st));
     return LOGOS_OK;
   }
-  return launch_m<1, float>(q, s, x, y, n, k, pdl_early(), nullptr, EPI_NONE, device, st);
+  return launch_m<1, float, false>(q, s, x, y, n, k, pdl_early(), nullptr, EPI_NONE, nullptr, device, st);
 }
 
 bool gemv_takes(int64_t m, int64_t n, int64_t k) {

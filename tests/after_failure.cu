@@ -26,7 +26,7 @@ static Buf buf(size_t bytes, int dtype, int kind, int stream, float a, float b) 
   Buf r;
   r.bytes = bytes;
   if (cudaMalloc(&r.p, bytes) != cudaSuccess) return r;
-  const int64_t size = dtype == LOGOS_F16 ? 2 : dtype == LOGOS_I8 ? 1 : 4;
+  const int64_t size = dtype == LOGOS_F16 || dtype == LOGOS_BF16 ? 2 : dtype == LOGOS_I8 ? 1 : 4;
   launch_synth_fill(r.p, dtype, kind, 1, stream, 0, (int64_t)bytes / size, a, b, 0, nullptr);
   return r;
 }
@@ -94,8 +94,34 @@ static int narrow(int out, int m, int n, int k) {
              out == NARROW_SWIGLU ? std::vector<Buf>{phi, plo} : std::vector<Buf>{c}, [&] { return launch_q8_narrow(a, nullptr); });
 }
 
+// A stand-alone product, results in place of the residual where there is one; `form` is what its plan makes of it.
+static int product(const char* form, int m, int n, int k, int dtype, int epilogue) {
+  const int size = dtype == LOGOS_F32 ? 4 : 2;
+  GemmArgs g;
+  Buf a = buf((size_t)m * k * size, dtype, 2, 1, 0.f, 1.f), q = buf((size_t)n * k, LOGOS_I8, 0, 2, 0.f, 0.f);
+  Buf s = buf((size_t)n * (k / 32) * 4, LOGOS_F32, 1, 3, 1e-3f, 1e-2f), c = buf((size_t)m * n * size, dtype, 2, 4, 0.f, 1.f);
+  if (!c.p) return 6;
+  g.a = a.p; g.a_dtype = dtype; g.lda = k;
+  g.q = (const int8_t*)q.p; g.s = (const float*)s.p;
+  g.c = c.p; g.c_dtype = dtype; g.ldc = epilogue == EPI_SWIGLU ? n / 2 : n;
+  if (epilogue == EPI_RESIDUAL) g.aux = c.p;
+  g.m = m; g.n = n; g.k = k; g.epilogue = epilogue;
+  if (int rc = run(form, {c}, [&] { return gemv_takes(m, n, k) ? launch_q8_gemv_tokens(g, nullptr) : launch_gemm_operator(g, nullptr); })) return rc;
+  for (const Buf& b : {a, q, s, c}) cudaFree(b.p);
+  return 0;
+}
+
 int main() {
   if (!kernel_status_ptr(0)) return 1;
+  for (int epilogue : {EPI_NONE, EPI_RESIDUAL, EPI_SWIGLU})
+    for (int dtype : {LOGOS_F32, LOGOS_BF16}) {
+      if (dtype == LOGOS_F32 && epilogue != EPI_NONE) continue;   // (f32 products have no epilogue)
+      for (int m : {1, 2})
+        if (int rc = product("gemv", m, 1024, 1024, dtype, epilogue)) return rc;
+      if (int rc = product("gemm", 40, 37888, 256, dtype, epilogue)) return rc;    // pairs of row tiles
+      if (epilogue == EPI_RESIDUAL) continue;                                      // (staged)
+      if (int rc = product("gemm", 384, 18944, 256, dtype, epilogue)) return rc;   // wide units
+    }
   for (int m : {1, 8, 16})
     for (int out : {NARROW_F32, NARROW_SWIGLU, NARROW_RESIDUAL})
       for (int k : {896, 4864}) {

@@ -916,8 +916,8 @@ def native(tmp_path_factory):
             list(ex.map(lambda so: subprocess.run(nvcc + ["-c", so[0], "-o", so[1]], check=True, capture_output=True), zip(sources, objects)))
         return objects
 
-    operators = compiled([os.path.join(csrc, f + ".cu") for f in ("attention", "elementwise", "q8_gemm", "q8_gemm_tc", "q8_narrow", "runtime",
-                                                                  "synth", "tma_host")])
+    operators = compiled([os.path.join(csrc, f + ".cu") for f in ("attention", "elementwise", "q8_gemm", "q8_gemm_tc", "q8_gemv", "q8_narrow",
+                                                                  "runtime", "synth", "tma_host")])
 
     def run(program):
         exe = os.path.join(out, program)
