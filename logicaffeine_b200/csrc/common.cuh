@@ -89,6 +89,9 @@ logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out);
 // captured, or there is no memory left for it.
 bool scratch_try(int32_t device, int slot, int64_t bytes, cudaStream_t st, void** out);
 
+// Whether `st` is being captured, as far as can be told: nothing may be allocated then.
+bool stream_capturing(cudaStream_t st);
+
 // Arrival counters of the attention calls that advance the lengths, one block per device (every call asks for the same
 // size), zeroed when it is allocated; the kernels leave them at zero.  Ordered like scratch_get's blocks.
 logos_status_t counters_get(int32_t device, int64_t bytes, void** out);
@@ -102,8 +105,8 @@ logos_status_t allow_smem(const void* kernel, int device, int bytes);
 int sm_count(int device);
 
 // Per-device status word in device memory: kernels store a non-zero code when
-// a bounded wait gives up.  0 = fine.
-int* kernel_status_ptr(int device);
+// a bounded wait gives up.  0 = fine.  Allocated when first asked for; without may_allocate null until then.
+int* kernel_status_ptr(int device, bool may_allocate = true);
 constexpr int KERNEL_STATUS_WORDS = 8;
 logos_status_t kernel_status_read(int device, int* out, bool clear);
 // the same for words that the caller has copied to the host already

@@ -128,7 +128,7 @@ q8_gemv_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, const 
   if (early) pdl_wait();
   // The GEMM operators write nothing on top of an earlier failure (STATUS).  A thread of the last warp, which has the least of x
   // to fetch, reads the code for all.  One token 768 x 2176 without it 2.44 us, so 2.52; by thread 0 2.8, by every thread 3.0.
-  const bool prior = STATUS && tid == (int)blockDim.x - 1 && __ldcg(status) != 0;
+  const bool prior = STATUS && status && tid == (int)blockDim.x - 1 && __ldcg(status) != 0;
   if (X_IN_SMEM) {
 #pragma unroll
     for (int v = 0; v < M; ++v)
@@ -239,8 +239,12 @@ logos_status_t launch_m(const int8_t* q, const float* s, const T* x, T* y, int64
 template <typename T>
 logos_status_t launch_rows(const int8_t* q, const float* s, const T* x, T* y, int64_t m, int64_t n, int64_t k, const T* aux, int epilogue,
                            int device, cudaStream_t st) {
-  const int* status = kernel_status_ptr(device);
-  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
+  // Without a word yet no kernel has given up; a capture, which cannot allocate one, goes on without.
+  const int* status = kernel_status_ptr(device, false);
+  if (!status && !stream_capturing(st)) {
+    status = kernel_status_ptr(device);
+    if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
+  }
   return m == 1 ? launch_m<1, T, true>(q, s, x, y, n, k, false, aux, epilogue, status, device, st)
                 : launch_m<2, T, true>(q, s, x, y, n, k, false, aux, epilogue, status, device, st);
 }

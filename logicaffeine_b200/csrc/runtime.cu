@@ -172,16 +172,18 @@ logos_status_t scratch_get(int32_t device, int slot, int64_t bytes, void** out) 
   return LOGOS_OK;
 }
 
+bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) == cudaSuccess) return capture != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 bool scratch_try(int32_t device, int slot, int64_t bytes, cudaStream_t st, void** out) {
   std::lock_guard<std::mutex> lk(g_scratch_mu);
   Scratch& s = scratch_of(device, slot);
   if (s.bytes < bytes) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    if (capture != cudaStreamCaptureStatusNone || scratch_grow(device, s, bytes) != cudaSuccess) return false;
+    if (stream_capturing(st) || scratch_grow(device, s, bytes) != cudaSuccess) return false;
   }
   *out = s.ptr;
   return true;

@@ -64,12 +64,13 @@ logos_status_t make_tensor_map_4d(CUtensorMap* out, const void* base, CUtensorMa
   return LOGOS_OK;
 }
 
-int* kernel_status_ptr(int device) {
+int* kernel_status_ptr(int device, bool may_allocate) {
   static std::mutex mu;
   static std::unordered_map<int, int*> words;
   std::lock_guard<std::mutex> lk(mu);
   auto it = words.find(device);
   if (it != words.end()) return it->second;
+  if (!may_allocate) return nullptr;
   // Device memory, not mapped host memory: every CTA reads this word once, and a read that
   // crosses PCIe costs about a microsecond and serialises.
   int prev = 0;

@@ -393,6 +393,31 @@ def _in_a_process_of_its_own(code):
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
 
 
+def test_q8_gemm_of_one_token_as_the_first_call_in_a_capture(llm):
+    """The GEMV form allocates nothing, so a process's first product can be inside a capture; the status word that it looks at
+    exists once a kernel that can give up has run."""
+    _in_a_process_of_its_own("""
+        import torch
+        n, k = 300, 512
+        a, q, s, c, want = (llm.DeviceBuffer(b) for b in (k * 4, n * k, n * (k // 32) * 4, n * 4, n * 4))
+        llm.synthFill(a, llm.F32, 2, 3, 3, 0, k)
+        llm.synthFill(q, llm.I8, 0, 3, 1, 0, n * k)
+        llm.synthFill(s, llm.F32, 1, 3, 2, 0, n * (k // 32), 1e-3, 1e-2)
+        llm.q8Gemv(q, s, a, want, n, k)
+        llm.devSync()
+        st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            llm.q8GemmF32(a, q, s, c, 1, n, k, stream=st.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        # the same kernel's sums
+        assert np.array_equal(c.download(np.uint32, (n,)), want.download(np.uint32, (n,)))
+        llm.q8GemmF32(a, q, s, c, 1, n, k)
+        assert np.array_equal(c.download(np.uint32, (n,)), want.download(np.uint32, (n,)))
+        assert llm.kernelStatus() == 0
+    """)
+
+
 @pytest.mark.parametrize("m,n", [(2048, 37888), (4100, 33000)])   # 310 MB of sums, and more than 2^27 of them
 def test_q8_gemm_residual_keeps_little_scratch(llm, m, n):
     _in_a_process_of_its_own("""
