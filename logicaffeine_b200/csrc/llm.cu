@@ -426,7 +426,7 @@ logos_status_t gemm_direct(Model* m, const GemmArgs& g, int* unfolded_splits = n
       return LOGOS_OK;
     }
     LOGOS_TRY(launch_splitk_reduce(m->dpart, splits, g.c, g.c_dtype, g.c_act, g.ldc, g.aux, g.m, g.n, g.epilogue,
-                                   m->stream));
+                                   m->device, m->stream));
     m->launch_counter += 1;
     return LOGOS_OK;
   }
@@ -935,7 +935,7 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
       g.partials = w.split;
       LOGOS_TRY(gemm(a, wt, k, g));
       if (folded) return LOGOS_OK;
-      return launch_splitk_reduce(w.split, sp, out.c, out.c_dtype, out.c_act, out.ldc, nullptr, M, wt.n, EPI_NONE, st);
+      return launch_splitk_reduce(w.split, sp, out.c, out.c_dtype, out.c_act, out.ldc, nullptr, M, wt.n, EPI_NONE, m->device, st);
     };
     auto reduce_delta = [&]() -> logos_status_t {
       if (m->tp.degree > 1) return tp_allreduce_sum_f32(&m->tp, w.delta, M * H, st);

@@ -6,7 +6,7 @@
 namespace logos {
 logos_status_t launch_q8_gemm_tc(const GemmArgs& g, cudaStream_t st);
 logos_status_t launch_splitk_reduce(const float* partials, int splits, void* c, int c_dtype, ActOut c_act,
-                                    int64_t ldc, const void* aux, int64_t m, int64_t n, int epilogue,
+                                    int64_t ldc, const void* aux, int64_t m, int64_t n, int epilogue, int device,
                                     cudaStream_t st);
 // Encoded 2-D tensor maps [d1][d0], cached by (address, shape, box, swizzle).
 logos_status_t cached_map(CUtensorMap* out, const void* base, CUtensorMapDataType dt, uint32_t elem, uint64_t d0,

@@ -119,8 +119,11 @@ int main() {
       for (int m : {1, 2})
         if (int rc = product("gemv", m, 1024, 1024, dtype, epilogue)) return rc;
       if (int rc = product("gemm", 40, 37888, 256, dtype, epilogue)) return rc;    // pairs of row tiles
-      if (epilogue == EPI_RESIDUAL) continue;                                      // (staged)
-      if (int rc = product("gemm", 384, 18944, 256, dtype, epilogue)) return rc;   // wide units
+      if (int rc = product("gemm", 384, 18944, 256, dtype, epilogue)) return rc;   // wide units, or a staged residual
+      if (int rc = product("gemm", 300, 512, 4096, dtype, epilogue)) return rc;    // K splits
+      // K that is no multiple of 128: the kernels behind the product may compute it again
+      if (int rc = product("gemm", 5, 512, 160, dtype, epilogue)) return rc;
+      if (int rc = product("gemm", 40, 512, 2080, dtype, epilogue)) return rc;
     }
   for (int m : {1, 8, 16})
     for (int out : {NARROW_F32, NARROW_SWIGLU, NARROW_RESIDUAL})
