@@ -55,7 +55,7 @@ struct Layer {
 
 // Buffers of the chunked prompt pass: one row per (sequence, position of the chunk).
 struct PrefillWs {
-  void*   block = nullptr;   // the one allocation they all lie in
+  void*   block = nullptr;   // the one allocation they all lie in (but see split_block)
   int64_t rows = 0;          // capacity
   float*  h = nullptr;       // [rows][H] residual stream
   float*  delta = nullptr;   // [rows][H] output of the last row-parallel GEMM, folded in by the next norm
@@ -65,7 +65,8 @@ struct PrefillWs {
   ActOut  att;               // [rows][nq]
   ActOut  ffn;               // [rows][f_local]
   float*  split = nullptr;   // [split_floats] partial sums of K splits
-  int64_t split_floats = 0;  // asked for; `split` is null where there was no room for it
+  int64_t split_floats = 0;
+  void*   split_block = nullptr;   // what `split` lies in since it outgrew its part of `block`
 };
 
 struct Model {
@@ -177,6 +178,7 @@ void destroy(Model* m) {
   tp_destroy(&m->tp);
   for (void* p : m->allocs) cudaFree(p);
   if (m->pf.block) cudaFree(m->pf.block);
+  if (m->pf.split_block) cudaFree(m->pf.split_block);
   if (m->prompt) cudaFree(m->prompt);
   for (cudaEvent_t e : m->prof_events) cudaEventDestroy(e);
   if (m->readback) cudaFreeHost(m->readback);
@@ -735,12 +737,41 @@ logos_status_t prompt_words(Model* m, int64_t need) {
   return LOGOS_OK;
 }
 
+constexpr int64_t MOST_SPLIT_FLOATS = 16ll << 20;   // partial sums of a prompt's product
+
+// Room for `need` partial sums where the workspace has less: a block of their own, twice as large as the last room, so that prompts
+// that grow settle it in a few steps without the workspace around it (one float more allocated all of it anew: 322 times
+// for prompts of 1, 2, ... 512 tokens of the 32B shape, now 12 times).  Without memory for it prompts go on with what there is, and ask
+// again.
+logos_status_t prefill_split_room(Model* m, int64_t need) {
+  PrefillWs& w = m->pf;
+  int64_t want = std::max(need, std::min(2 * w.split_floats, MOST_SPLIT_FLOATS));
+  void* block = nullptr;
+  cudaError_t e = cudaMalloc(&block, (size_t)want * 4);
+  if (e != cudaSuccess && want > need) {
+    cudaGetLastError();
+    e = cudaMalloc(&block, (size_t)(want = need) * 4);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return LOGOS_OK;
+  }
+  if (w.split_block) {
+    LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
+    cudaFree(w.split_block);
+  }
+  w.split_block = block;
+  w.split = static_cast<float*>(block);
+  w.split_floats = want;
+  return LOGOS_OK;
+}
+
 // One block for the buffers of a chunk of up to `rows` rows.  When a later prompt fills a larger chunk than any before
 // it, it grows at least geometrically, up to `most` rows unless more are needed; the old block is freed once the
 // stream has left it.
 logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most, int64_t split_floats) {
   PrefillWs& w = m->pf;
-  if (w.rows >= rows && w.split_floats >= split_floats) return LOGOS_OK;
+  if (w.rows >= rows) return w.split_floats >= split_floats ? LOGOS_OK : prefill_split_room(m, split_floats);
   const logos_llm_config_t& c = m->cfg;
   const int64_t H = c.hidden;
   const bool two = c.act_dtype == LOGOS_F32;
@@ -763,12 +794,12 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most, int64_t s
     }
     o_split = place(split * 4);
   };
-  int64_t want = w.rows >= rows ? w.rows : std::max(rows, std::min(2 * w.rows, most));
-  split_floats = std::max(split_floats, w.split_floats);
-  int64_t split = split_floats;
+  int64_t want = std::max(rows, std::min(2 * w.rows, most));
+  int64_t split = split_floats <= w.split_floats ? w.split_floats : std::max(split_floats, std::min(2 * w.split_floats, MOST_SPLIT_FLOATS));
   if (w.block) {
     LOGOS_CUDA_TRY(cudaStreamSynchronize(m->stream));
     cudaFree(w.block);
+    if (w.split_block) cudaFree(w.split_block);
     w = PrefillWs();
   }
   char* base = nullptr;
@@ -794,7 +825,7 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most, int64_t s
   w.qkv = reinterpret_cast<float*>(base + o_qkv);
   w.q16 = reinterpret_cast<__half*>(base + o_q16);
   w.split = split > 0 ? reinterpret_cast<float*>(base + o_split) : nullptr;
-  w.split_floats = split_floats;
+  w.split_floats = split;
   ActOut* planes[3] = {&w.xn, &w.att, &w.ffn};
   for (int i = 0; i < 3; ++i) {
     planes[i]->mode = c.act_dtype;
@@ -810,7 +841,7 @@ logos_status_t prefill_workspace(Model* m, int64_t rows, int64_t most, int64_t s
 int prompt_splits(const Model* m, int64_t rows, const Q8Mat& w, bool folded) {
   if (!w.tiled || (folded && m->tp.degree > 1)) return 1;
   const int sp = rows > 64 ? gemm_many_splits(rows, w.n, w.k, m->device, folded) : gemm_pick_splits(rows, w.n, w.k, m->device, folded);
-  return sp * rows * w.n <= (16ll << 20) ? sp : 1;
+  return sp * rows * w.n <= MOST_SPLIT_FLOATS ? sp : 1;
 }
 
 // The prompt pass proper: chunks of positions, every sequence's part of the chunk at once, so that each
@@ -923,7 +954,8 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
     int parts = 1;             // of the pending row-parallel product
     const float* delta = w.delta;
     auto gemm_split = [&](const ActOut& a, const Q8Mat& wt, int64_t k, GemmArgs g, bool folded) -> logos_status_t {
-      const int sp = w.split ? prompt_splits(m, M, wt, folded) : 1;
+      int sp = prompt_splits(m, M, wt, folded);
+      if (sp * M * wt.n > w.split_floats) sp = 1;   // no memory was left for them
       if (folded) {
         parts = sp;
         delta = sp > 1 ? w.split : w.delta;

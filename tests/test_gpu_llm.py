@@ -304,6 +304,25 @@ def test_prompts_that_grow_keep_no_outgrown_memory(llm, oracle):
     gpu.free()
 
 
+def test_prompts_that_grow_settle_their_workspace(llm):
+    """Prompts of ever more rows allocate now and then, not each: the workspace doubles, and so does the room for K splits, whose
+    need goes up with almost every row."""
+    cfg = dict(layers=1, hidden=5120, h_q=64, h_kv=8, head_dim=128, ffn=27648, vocab=1024, l_max=528, batch=1, rms_eps=1e-6,
+               rope_theta=1e6, tied_embeddings=1, seed=1, init_std=0.02)
+    gpu = llm.Llm(**cfg)
+    free = [llm.devMemInfo()[0]]
+    for t in range(8, 513, 8):
+        gpu.prefill(np.full((1, t), t, np.int32))
+        free.append(llm.devMemInfo()[0])
+    # a row is 0.3 MB of workspace and up to 0.3 MB of partial sums, the driver's blocks are 2 MB: seven doublings of the
+    # rows and some of the other show
+    assert sum(a != b for a, b in zip(free, free[1:])) <= 14, free
+    gpu.prefill(np.full((1, 512), 3, np.int32))
+    assert llm.devMemInfo()[0] == free[-1]
+    assert llm.kernelStatus() == 0
+    gpu.free()
+
+
 def test_a_longer_prompt_with_little_memory_left(llm, oracle):
     """A prompt for whose chunks there is no memory runs in smaller ones, and one after it in large ones again."""
     cfg = dict(SMALL, layers=1, hidden=1024, h_q=8, h_kv=2, head_dim=128, ffn=8192, batch=1, l_max=2100)
@@ -319,6 +338,28 @@ def test_a_longer_prompt_with_little_memory_left(llm, oracle):
     got = gpu.readLogits()
     rest.free()
     assert rel_l2(got, want) < 1e-4
+    gpu.prefill(toks)
+    assert np.array_equal(gpu.readLogits(), want)
+    assert llm.kernelStatus() == 0
+    gpu.free()
+
+
+def test_k_splits_come_back_once_there_is_memory_for_them(llm):
+    """A prompt that finds memory for its rows but not for its partial sums goes on without K splits; the same prompt later, with
+    memory for both, gives the bits that it gives a model which always had it."""
+    cfg = dict(SMALL, layers=1, hidden=1024, h_q=8, h_kv=2, head_dim=128, ffn=8192, batch=1, l_max=300)
+    toks = (np.arange(256, dtype=np.int32) * 37 % cfg["vocab"]).reshape(1, 256)
+    gpu = llm.Llm(**cfg)
+    gpu.prefill(toks)
+    want = gpu.readLogits()
+    gpu.free()
+    gpu = llm.Llm(**cfg)
+    gpu.prefill(toks[:, :4])
+    rest = llm.DeviceBuffer(llm.devMemInfo()[0] - (18 << 20))   # 256 rows take 15 MB, their partial sums 8
+    gpu.prefill(toks)
+    got = gpu.readLogits()
+    rest.free()
+    assert rel_l2(got, want) < 1e-4 and not np.array_equal(got, want)   # f32 sums in another order
     gpu.prefill(toks)
     assert np.array_equal(gpu.readLogits(), want)
     assert llm.kernelStatus() == 0
