@@ -1359,6 +1359,11 @@ int gemm_many_splits(int64_t m, int64_t n, int64_t k, int device, bool folded) {
   return e.splits;
 }
 
+int gemm_wide_tokens(int64_t m, int64_t n, int64_t k, int device) {
+  const TcPlan plan = plan_for(m, n, k, 1, device);
+  return plan.wide ? 2 * plan.t : 0;
+}
+
 logos_status_t launch_q8_gemm_tc(const GemmArgs& g, cudaStream_t st) {
   const TcPlan plan = plan_for(g.m, g.n, g.k, g.splits > 1 ? g.splits : 1, g.device);
   return g.a_lo ? launch_plan<2>(g, plan, st) : launch_plan<1>(g, plan, st);

@@ -5,6 +5,8 @@
 
 namespace logos {
 logos_status_t launch_q8_gemm_tc(const GemmArgs& g, cudaStream_t st);
+// Tokens of a unit of the wide form that a product without K splits runs in; 0: another form.
+int gemm_wide_tokens(int64_t m, int64_t n, int64_t k, int device);
 logos_status_t launch_splitk_reduce(const float* partials, int splits, void* c, int c_dtype, ActOut c_act,
                                     int64_t ldc, const void* aux, int64_t m, int64_t n, int epilogue, int device,
                                     cudaStream_t st);

@@ -164,13 +164,20 @@ def test_q8_gemm_tiles_tails_and_units(llm, oracle, m, n, k):
     assert llm.kernelStatus() == 0
 
 
-@pytest.mark.parametrize("m,n,k", [
-    (128, 18944, 128),    # one full tile of 128 tokens, one stage
-    (129, 37000, 160),    # a tile of 192 that is mostly full, a K tail of one Q8 block, a last row tile of 8 rows
-    (192, 18946, 384),    # 192 full, an odd number of stages, two rows in the last row tile
-    (193, 37888, 288),    # a second tile of one token, several units a CTA
-    (460, 19000, 1152),   # tiles of 128 and a tail, more stages than any ring has slots
-])
+# m, n, k and the tokens of the unit that it is for
+WIDE_UNITS = [
+    (128, 18944, 128, 128),    # one full tile of 128 tokens, one stage
+    (129, 37000, 160, 192),    # a tile of 192 that is mostly full, a K tail of one Q8 block, a last row tile of 8 rows
+    (192, 18946, 384, 0),      # two rows in the last row tile, which make pairs of 64 tokens the cheaper form
+    (193, 37888, 288, 128),    # a second tile of one token, several units a CTA
+    (460, 19000, 1152, 128),   # tiles of 128 and a tail, more stages than any ring has slots
+    (384, 18944, 1152, 192),   # two full tiles of 192, two units a CTA, more stages than any ring has slots
+    (387, 18944, 1024, 192),   # a third tile of three tokens (fewer are not the GEMM's), an even number of stages
+    (383, 18930, 1056, 192),   # tails of tokens, rows and K
+]
+
+
+@pytest.mark.parametrize("m,n,k", [shape[:3] for shape in WIDE_UNITS])
 def test_q8_gemm_wide_units_give_the_same_bits(llm, oracle, m, n, k):
     """Many tokens run in larger units than 64: the order of a sum, and so its bits, are those of 64 tokens at a time."""
     O = oracle
@@ -944,10 +951,10 @@ def native(tmp_path_factory):
     operators = compiled([os.path.join(csrc, f + ".cu") for f in ("attention", "elementwise", "q8_gemm", "q8_gemm_tc", "q8_gemv", "q8_narrow",
                                                                   "runtime", "synth", "tma_host")])
 
-    def run(program):
+    def run(program, *args):
         exe = os.path.join(out, program)
         subprocess.run(nvcc + ["-o", exe] + compiled([os.path.join(here, program + ".cu")]) + operators + ["-ldl"], check=True, capture_output=True)
-        r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+        r = subprocess.run([exe] + [str(a) for a in args], capture_output=True, text=True, timeout=120)
         assert r.returncode == 0, r.stdout
         return r.stdout.split("\n")[:-1]
 
@@ -962,6 +969,12 @@ def test_kernels_behind_a_failure_write_nothing(native):
     for line in lines:
         what, behind, after = line.rsplit(" ", 2)
         assert (behind, after) == ("0", "1"), line
+
+
+def test_forms_of_products_of_many_tokens(native):
+    """What the bits above are compared for does run in the wide form."""
+    lines = native("gemm_forms", *[x for shape in WIDE_UNITS for x in shape[:3]])
+    assert [int(line) for line in lines] == [shape[3] for shape in WIDE_UNITS]
 
 
 def test_narrow_products_bit_for_bit(native):
