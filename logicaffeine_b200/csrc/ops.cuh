@@ -63,6 +63,9 @@ struct GemmArgs {
   float*        partials = nullptr;
   int           device = 0;
   int           force_simt = 0;  // use the SIMT kernel even where the tensor-core one applies
+  // f32 results or partial sums go to a kernel that looks at the status word where they are NaN: a product that finds the code of
+  // an earlier failure puts that where its sums would be, and the kernel behind it writes nothing.
+  bool          mark_failure = false;
 };
 logos_status_t launch_q8_gemm(const GemmArgs& g, cudaStream_t st);
 // The stand-alone operators' form of it: row-major bf16 or f32 activations, planes and K splits in the library's scratch.
@@ -224,12 +227,10 @@ logos_status_t launch_tp_residual_rmsnorm(float* h, const TpFusedArgs& t, int pa
 // inside fp16's normal range, saturating outside; LOGOS_F32: two), and, where K is not a multiple of 128
 // (tiled_or_null set then and only then), scales [n][k/32] into the tile-major form
 // [row tile][K tile][128 rows][4], zero past K (rows past n are left alone: their products are dropped).  In the
-// latter form `call` is stored to misfit[0] if there are activations that the planes do not hold as the
-// CUDA-core kernel would use them: beyond fp16's range, NaN, or a whole K tile of a row below 2^-12 (bf16: 2^-8);
-// and to misfit[1] if the status word holds a code, something else if not.
+// latter form `call` is stored to *misfit if there are activations that the planes do not hold as the
+// CUDA-core kernel would use them: beyond fp16's range, NaN, or a whole K tile of a row below 2^-12 (bf16: 2^-8).
 logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t m, const float* s,
-                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call,
-                                const int* status, cudaStream_t st);
+                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call, cudaStream_t st);
 // Sampling state of a model, in device memory so that a captured step follows changes to it.
 struct SamplingParams {
   float inv_temperature;  // 1 / T

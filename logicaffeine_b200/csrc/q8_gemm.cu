@@ -103,11 +103,10 @@ __global__ void __launch_bounds__(256) q8_gemm_simt_kernel(const SimtArgs g) {
   simt_tile(g, blockIdx.x, blockIdx.y, blockIdx.z, as, qs);
 }
 
-// What the fp16 planes of a call do not hold (see launch_gemm_prep): the preparation stored `call` to words[0] then, and the
-// kernel that comes last computes the product again, epilogue included, instead of what it is for.  words[1] is `call` where
-// there was the code of an earlier failure.
+// What the fp16 planes of a call do not hold (see launch_gemm_prep): the preparation stored `call` to *word then, and the
+// kernel that comes last computes the product again, epilogue included, instead of what it is for.
 struct Misfit {
-  const unsigned* words = nullptr;   // null: nothing to look at
+  const unsigned* word = nullptr;   // null: nothing to look at
   unsigned call = 0;
   SimtArgs product = {};
   int64_t tiles_n = 0, tiles_m = 0;
@@ -119,32 +118,30 @@ __device__ __forceinline__ void redo_misfit(const Misfit& f) {
   for (int64_t t = blockIdx.x; t < f.tiles_n * f.tiles_m; t += gridDim.x)
     simt_tile(f.product, t % f.tiles_n, t / f.tiles_n, 0, as, qs);
 }
-__device__ __forceinline__ uint2 misfit_words(const Misfit& f) { return __ldcg(reinterpret_cast<const uint2*>(f.words)); }
+// The whole grid's part, unless there is the code of an earlier failure (one thread of a CTA reads it, all take one decision).
+__device__ __forceinline__ void redo_unless_failed(const Misfit& f, const int* status) {
+  if (!__syncthreads_or(threadIdx.x == 0 && __ldcg(status) != 0)) redo_misfit(f);
+}
 // Where no other kernel follows the product.
-__global__ void __launch_bounds__(256) q8_gemm_misfit_kernel(const Misfit f) {
+__global__ void __launch_bounds__(256) q8_gemm_misfit_kernel(const Misfit f, const int* status) {
   pdl_wait();
   pdl_trigger();
-  const uint2 words = misfit_words(f);
-  if (words.x == f.call && words.y != f.call) redo_misfit(f);
+  if (__ldcg(f.word) == f.call) redo_unless_failed(f, status);
 }
 
-// A product that finds the code of an earlier failure does nothing: what is in its place are another call's sums, and the kernel
-// behind it writes nothing either.  A preparation's words say so where there are any.  Else a thread of each CTA reads the code
-// before the wait for the product, which hides that (17 x 896 x 4864 9.41 -> 9.43 us; looked at where results are stored 10.0).
-// In place of the words that costs the second wave of CTAs 0.3 to 0.6 (64 x 3584 x 2368 13.6 -> 14.3, with the words 13.7).
-__device__ __forceinline__ bool after_failure(const int* status) { return __syncthreads_or(threadIdx.x == 0 && __ldcg(status) != 0); }
+// Sums come from a product that leaves NaN behind a failure and does nothing else (GemmArgs::mark_failure): only where a result is
+// NaN is the status word looked at.  One sector that every CTA reads costs products of few rows and many tokens 4 to 10 %.
+__device__ __forceinline__ bool unless_failed(float v, const int* status) { return v == v || __ldcg(status) == 0; }
 
-// Sum split-K partials in ascending split order, then apply the epilogue.  The misfit words are loaded beside the
+// Sum split-K partials in ascending split order, then apply the epilogue.  The misfit word is loaded beside the
 // partials and looked at after them.
 template <bool MISFIT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ partials, int splits, void* __restrict__ c, int c_dtype,
                                      ActOut c_act, int64_t ldc, const void* __restrict__ aux, int64_t m, int64_t n,
                                      int epilogue, const Misfit f, const int* status) {
-  const bool prior = !MISFIT && after_failure(status);
   pdl_wait();  // the partials are the previous kernel's output: wait for it, read them past L1
   pdl_trigger();
-  if (prior) return;
-  const uint2 words = MISFIT ? misfit_words(f) : make_uint2(0u, 0u);
+  const unsigned word = MISFIT ? __ldcg(f.word) : 0u;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool swiglu = epilogue == EPI_SWIGLU;
   const int64_t width = swiglu ? n / 2 : n;
@@ -165,26 +162,19 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partials, int spl
       if (epilogue == EPI_RESIDUAL) v = __fadd_rn(v, load_act(aux, c_dtype, at));
     }
   }
-  if (MISFIT && words.y == f.call) return;
-  if (MISFIT && words.x == f.call) redo_misfit(f);
-  else if (inside) store_out(c, c_dtype, at, v, c_act);
+  if (MISFIT && word == f.call) redo_unless_failed(f, status);
+  else if (inside && unless_failed(v, status)) store_out(c, c_dtype, at, v, c_act);
 }
 
 // c = staged sums + residual, bf16; HBM-bound, eight elements a thread.
 template <bool MISFIT>
 __global__ void __launch_bounds__(256) residual_kernel(const float* __restrict__ sums, const __nv_bfloat16* aux, __nv_bfloat16* c, int64_t count,
                                                        const Misfit f, const int* status) {
-  const bool prior = !MISFIT && after_failure(status);
   pdl_wait();
   pdl_trigger();
-  if (prior) return;
-  if (MISFIT) {
-    const uint2 words = misfit_words(f);
-    if (words.y == f.call) return;
-    if (words.x == f.call) {
-      redo_misfit(f);
-      return;
-    }
+  if (MISFIT && __ldcg(f.word) == f.call) {
+    redo_unless_failed(f, status);
+    return;
   }
   const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
   const bool vec = i + 8 <= count && !((reinterpret_cast<uintptr_t>(aux) | reinterpret_cast<uintptr_t>(c)) & 15u);
@@ -196,10 +186,13 @@ __global__ void __launch_bounds__(256) residual_kernel(const float* __restrict__
     uint4 o;
     __nv_bfloat16* oh = reinterpret_cast<__nv_bfloat16*>(&o);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) oh[j] = __float2bfloat16_rn(__fadd_rn(v[j], __bfloat162float(rh[j])));
+    for (int j = 0; j < 8; ++j) oh[j] = unless_failed(v[j], status) ? __float2bfloat16_rn(__fadd_rn(v[j], __bfloat162float(rh[j]))) : c[i + j];
     *reinterpret_cast<uint4*>(c + i) = o;
   } else {
-    for (int64_t j = i; j < count && j < i + 8; ++j) c[j] = __float2bfloat16_rn(__fadd_rn(__ldcg(sums + j), __bfloat162float(aux[j])));
+    for (int64_t j = i; j < count && j < i + 8; ++j) {
+      const float v = __ldcg(sums + j);
+      if (unless_failed(v, status)) c[j] = __float2bfloat16_rn(__fadd_rn(v, __bfloat162float(aux[j])));
+    }
   }
 }
 
@@ -234,12 +227,10 @@ int gemm_pick_splits(int64_t m, int64_t n, int64_t k, int device, bool folded) {
 }
 
 static logos_status_t launch_reduce(const float* partials, int splits, void* c, int c_dtype, ActOut c_act, int64_t ldc,
-                                    const void* aux, int64_t m, int64_t n, int epilogue, const Misfit& f, int device, cudaStream_t st) {
+                                    const void* aux, int64_t m, int64_t n, int epilogue, const Misfit& f, const int* status, cudaStream_t st) {
   int64_t total = (epilogue == EPI_SWIGLU) ? m * (n / 2) : m * n;
   if (total == 0) return LOGOS_OK;
-  const int* status = kernel_status_ptr(device);
-  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
-  LOGOS_CUDA_TRY(launch_kernel(f.words ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3((unsigned)((total + 255) / 256)),
+  LOGOS_CUDA_TRY(launch_kernel(f.word ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3((unsigned)((total + 255) / 256)),
                                dim3(256), 0, st, partials, splits, c, c_dtype, c_act, ldc, aux, m, n, epilogue, f, status));
   count_launch(LK_ELEMWISE);
   return check_launch("splitk_reduce_kernel");
@@ -248,7 +239,9 @@ static logos_status_t launch_reduce(const float* partials, int splits, void* c, 
 logos_status_t launch_splitk_reduce(const float* partials, int splits, void* c, int c_dtype, ActOut c_act,
                                     int64_t ldc, const void* aux, int64_t m, int64_t n, int epilogue, int device,
                                     cudaStream_t st) {
-  return launch_reduce(partials, splits, c, c_dtype, c_act, ldc, aux, m, n, epilogue, Misfit(), device, st);
+  const int* status = kernel_status_ptr(device);
+  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
+  return launch_reduce(partials, splits, c, c_dtype, c_act, ldc, aux, m, n, epilogue, Misfit(), status, st);
 }
 
 static SimtArgs simt_args(const GemmArgs& g) {
@@ -329,8 +322,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   // K that is no multiple of 128 was the CUDA-core kernel's alone, in f32 throughout.  What the planes do not hold is
   // still its, in the call's last kernel: the preparation marks the call by its number (nothing to clear: the word holds
   // another call's otherwise, and a replayed capture that finds its own mark does no more than the product
-  // again).  A kernel of its own after every product cost 2 us of 14; the folds load the word beside the partials, and the
-  // word beside it, which the preparation always writes: whether it found the code of a failure.
+  // again).  A kernel of its own after every product cost 2 us of 14; the folds load the word beside the partials.
   static std::atomic<unsigned> calls{0};
   unsigned* const misfit = retile ? reinterpret_cast<unsigned*>(at) : nullptr;
   const unsigned call = retile ? ++calls : 0;
@@ -344,18 +336,16 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     e.c = static_cast<char*>(e.c) + m0 * e.ldc * (e.c_dtype == LOGOS_BF16 ? 2 : 4);
     if (e.aux) e.aux = static_cast<const __nv_bfloat16*>(e.aux) + m0 * e.ldc;
     e.m = m;
-    f.words = misfit;
+    f.word = misfit;
     f.call = call;
     f.product = simt_args(e);
     f.tiles_n = (e.n + SIMT_TN - 1) / SIMT_TN;
     f.tiles_m = (e.m + SIMT_TM - 1) / SIMT_TM;
     return f;
   };
-  const int* status = kernel_status_ptr(g.device);
-  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   {
     OrderedScope ordered(st);
-    LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, misfit, call, status, st));
+    LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, misfit, call, st));
   }
   g.lda = lda;
   g.a = planes.hi;
@@ -366,16 +356,19 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     g.s_tiled = 1;
   }
   PdlScope pdl(pdl_active() || pdl_enabled());
+  const int* status = kernel_status_ptr(g.device);
+  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   if (splits <= 1 && !staged) {
     LOGOS_TRY(launch_q8_gemm(g, st));
     if (!retile) return LOGOS_OK;
     const Misfit f = again(0, g.m);
     const int64_t grid = std::min<int64_t>(f.tiles_n * f.tiles_m, 4ll * sm_count(g.device));
-    LOGOS_CUDA_TRY(launch_kernel(q8_gemm_misfit_kernel, dim3((unsigned)grid), dim3(256), 0, st, f));
+    LOGOS_CUDA_TRY(launch_kernel(q8_gemm_misfit_kernel, dim3((unsigned)grid), dim3(256), 0, st, f, status));
     count_launch(LK_GEMM_SIMT);
     return check_launch("q8_gemm_misfit_kernel");
   }
   GemmArgs gp = g;
+  gp.mark_failure = true;
   if (staged) {
     gp.c_dtype = LOGOS_F32;
     gp.epilogue = EPI_NONE;
@@ -388,7 +381,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
       LOGOS_TRY(launch_q8_gemm(gp, st));
       const int64_t count = gp.m * g.n;
       const Misfit f = again(m0, gp.m);
-      LOGOS_CUDA_TRY(launch_kernel(f.words ? residual_kernel<true> : residual_kernel<false>, dim3((unsigned)((count + 2047) / 2048)), dim3(256), 0, st,
+      LOGOS_CUDA_TRY(launch_kernel(f.word ? residual_kernel<true> : residual_kernel<false>, dim3((unsigned)((count + 2047) / 2048)), dim3(256), 0, st,
                                    reinterpret_cast<const float*>(at), reinterpret_cast<const __nv_bfloat16*>(g.aux) + m0 * g.n,
                                    reinterpret_cast<__nv_bfloat16*>(g.c) + m0 * g.n, count, f, status));
       count_launch(LK_ELEMWISE);
@@ -403,7 +396,7 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   gp.c_dtype = LOGOS_F32;
   gp.aux = nullptr;
   LOGOS_TRY(launch_q8_gemm(gp, st));
-  return launch_reduce(gp.partials, splits, g.c, g.c_dtype, ActOut(), g.ldc, g.aux, g.m, g.n, g.epilogue, again(0, g.m), g.device, st);
+  return launch_reduce(gp.partials, splits, g.c, g.c_dtype, ActOut(), g.ldc, g.aux, g.m, g.n, g.epilogue, again(0, g.m), status, st);
 }
 
 // Whether the operands of a stand-alone call can go to the tensor-core kernel once prepared (the planes and, where
