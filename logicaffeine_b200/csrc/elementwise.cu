@@ -341,16 +341,23 @@ tp_residual_rmsnorm_kernel(float* __restrict__ h, const TpFusedArgs t, int parts
 template <bool BF16>
 __global__ void __launch_bounds__(256)
 gemm_prep_kernel(const void* a, ActOut o, int64_t count8, const float* s, float* tiled, int64_t n, int64_t kb, int64_t ktiles,
-                 int64_t act_blocks, unsigned* misfit, unsigned call) {
+                 int64_t act_blocks, unsigned* misfit, unsigned call, float* sums, int64_t sum_count, const int* status) {
   // count8: groups of eight of the planes; rows of the planes are whole K tiles, rows of `a` kb * 32 values
   // The product behind this kernel reads weights without a wait of its own: it may start once all before this one has ended.
   // Activations and scales can be what the kernel before has just written: no pointer here says read-only, whose loads need
   // not see that.  (The scales by ordinary loads: a row's four come from one line, past L1 each fetched it for itself,
   // 64 x 3584 x 2368 13.65 -> 14.01 us.)
+  if (sums && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(status));
   pdl_wait();
   pdl_trigger();
-  if ((int64_t)blockIdx.x < act_blocks) {
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (sums && blockIdx.x == 0) {   // of its own, so that the code's load is beside the others' and not before them
+    if (__ldcg(status) != 0)
+      for (int64_t i = threadIdx.x; i < sum_count; i += 256) sums[i] = __uint_as_float(0x7fffffffu);
+    return;
+  }
+  const int64_t block = (int64_t)blockIdx.x - (sums ? 1 : 0);
+  if (block < act_blocks) {
+    const int64_t i = block * 256 + threadIdx.x;
     if (i >= count8) return;
     float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int64_t src = i;                      // group of eight of `a`
@@ -403,7 +410,7 @@ gemm_prep_kernel(const void* a, ActOut o, int64_t count8, const float* s, float*
     if (o.mode == LOGOS_F32) reinterpret_cast<uint4*>(o.lo)[i] = *reinterpret_cast<const uint4*>(lo);
     return;
   }
-  const int64_t i = ((int64_t)blockIdx.x - act_blocks) * 256 + threadIdx.x;   // (row, K tile), K tile fastest
+  const int64_t i = (block - act_blocks) * 256 + threadIdx.x;   // (row, K tile), K tile fastest
   const int64_t row = i / ktiles, kt = i - row * ktiles;
   if (row >= n) return;
   float4 v;
@@ -608,14 +615,16 @@ logos_status_t launch_embed(const int32_t* tokens, const int8_t* q, const float*
 }
 
 logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t m, const float* s,
-                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call, cudaStream_t st) {
+                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call,
+                                float* sums_or_null, int64_t count, const int* status, cudaStream_t st) {
   if (k % 32 || (reinterpret_cast<uintptr_t>(a) & 31u))
     return fail(LOGOS_ERROR, "gemm_prep: K must be a multiple of 32 and the activations 32-byte aligned");
   const int64_t ktiles = (k + 127) / 128, count8 = m * ktiles * 16;
   const int64_t act_blocks = (count8 + 255) / 256, scale_blocks = tiled_or_null ? (n * ktiles + 255) / 256 : 0;
-  const dim3 grid((unsigned)(act_blocks + scale_blocks));
+  const dim3 grid((unsigned)(act_blocks + scale_blocks + (sums_or_null ? 1 : 0)));
   auto kernel = a_dtype == LOGOS_BF16 ? gemm_prep_kernel<true> : gemm_prep_kernel<false>;
-  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(256), 0, st, a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call));
+  LOGOS_CUDA_TRY(launch_kernel(kernel, grid, dim3(256), 0, st, a, planes, count8, s, tiled_or_null, n, k / 32, ktiles, act_blocks, misfit, call,
+                               sums_or_null, count, status));
   count_launch(LK_ELEMWISE);
   return check_launch("gemm_prep_kernel");
 }

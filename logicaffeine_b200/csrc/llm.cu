@@ -421,11 +421,9 @@ logos_status_t gemm_direct(Model* m, const GemmArgs& g, int* unfolded_splits = n
     gp.c = nullptr;
     gp.c_dtype = LOGOS_F32;
     gp.aux = nullptr;
-    const bool unfolded = unfolded_splits && g.epilogue == EPI_NONE && g.ldc == g.n;
-    gp.mark_failure = !unfolded;
     LOGOS_TRY(launch_q8_gemm(gp, m->stream));
     m->launch_counter += 1;
-    if (unfolded) {
+    if (unfolded_splits && g.epilogue == EPI_NONE && g.ldc == g.n) {
       *unfolded_splits = splits;
       return LOGOS_OK;
     }
@@ -967,7 +965,6 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
       g.c = nullptr;
       g.splits = sp;
       g.partials = w.split;
-      g.mark_failure = !folded;
       LOGOS_TRY(gemm(a, wt, k, g));
       if (folded) return LOGOS_OK;
       return launch_splitk_reduce(w.split, sp, out.c, out.c_dtype, out.c_act, out.ldc, nullptr, M, wt.n, EPI_NONE, m->device, st);

@@ -63,9 +63,6 @@ struct GemmArgs {
   float*        partials = nullptr;
   int           device = 0;
   int           force_simt = 0;  // use the SIMT kernel even where the tensor-core one applies
-  // f32 results or partial sums go to a kernel that looks at the status word where they are NaN: a product that finds the code of
-  // an earlier failure puts that where its sums would be, and the kernel behind it writes nothing.
-  bool          mark_failure = false;
 };
 logos_status_t launch_q8_gemm(const GemmArgs& g, cudaStream_t st);
 // The stand-alone operators' form of it: row-major bf16 or f32 activations, planes and K splits in the library's scratch.
@@ -229,8 +226,11 @@ logos_status_t launch_tp_residual_rmsnorm(float* h, const TpFusedArgs& t, int pa
 // [row tile][K tile][128 rows][4], zero past K (rows past n are left alone: their products are dropped).  In the
 // latter form `call` is stored to *misfit if there are activations that the planes do not hold as the
 // CUDA-core kernel would use them: beyond fp16's range, NaN, or a whole K tile of a row below 2^-12 (bf16: 2^-8).
+// sums_or_null [count]: where the product will put sums for a kernel behind it.  With a code in the status word the product
+// does nothing, and NaN is put there, at which that kernel looks at the word (see q8_gemm.cu).
 logos_status_t launch_gemm_prep(const void* a, int a_dtype, ActOut planes, int64_t m, const float* s,
-                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call, cudaStream_t st);
+                                float* tiled_or_null, int64_t n, int64_t k, unsigned* misfit, unsigned call,
+                                float* sums_or_null, int64_t count, const int* status, cudaStream_t st);
 // Sampling state of a model, in device memory so that a captured step follows changes to it.
 struct SamplingParams {
   float inv_temperature;  // 1 / T

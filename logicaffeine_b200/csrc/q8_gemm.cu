@@ -129,8 +129,9 @@ __global__ void __launch_bounds__(256) q8_gemm_misfit_kernel(const Misfit f, con
   if (__ldcg(f.word) == f.call) redo_unless_failed(f, status);
 }
 
-// Sums come from a product that leaves NaN behind a failure and does nothing else (GemmArgs::mark_failure): only where a result is
-// NaN is the status word looked at.  One sector that every CTA reads costs products of few rows and many tokens 4 to 10 %.
+// Behind an earlier failure an operator's product does nothing, and its preparation has put NaN where its sums would be: only where
+// a result is NaN is the status word looked at.  Read by every CTA, that one sector cost products of few rows and many
+// tokens 2 to 10 %; NaN from the product's own kernel a prompt up to 1.7 %, by what the code for it did to the rest.
 __device__ __forceinline__ bool unless_failed(float v, const int* status) { return v == v || __ldcg(status) == 0; }
 
 // Sum split-K partials in ascending split order, then apply the epilogue.  The misfit word is loaded beside the
@@ -343,9 +344,12 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     f.tiles_m = (e.m + SIMT_TM - 1) / SIMT_TM;
     return f;
   };
+  const int* status = kernel_status_ptr(g.device);
+  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   {
     OrderedScope ordered(st);
-    LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, misfit, call, st));
+    LOGOS_TRY(launch_gemm_prep(src, src_dtype, planes, g.m, g.s, tiled, g.n, g.k, misfit, call,
+                               part_rows > 0 ? reinterpret_cast<float*>(at) : nullptr, part_rows * g.n, status, st));
   }
   g.lda = lda;
   g.a = planes.hi;
@@ -356,8 +360,6 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     g.s_tiled = 1;
   }
   PdlScope pdl(pdl_active() || pdl_enabled());
-  const int* status = kernel_status_ptr(g.device);
-  if (!status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   if (splits <= 1 && !staged) {
     LOGOS_TRY(launch_q8_gemm(g, st));
     if (!retile) return LOGOS_OK;
@@ -368,7 +370,6 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
     return check_launch("q8_gemm_misfit_kernel");
   }
   GemmArgs gp = g;
-  gp.mark_failure = true;
   if (staged) {
     gp.c_dtype = LOGOS_F32;
     gp.epilogue = EPI_NONE;

@@ -162,7 +162,6 @@ struct TcParams {
   int wait_scales;    // the scales are the previous kernel's output too
   int stream_once;    // one token tile: the weights are not read again
   int* status;
-  int mark_failure;   // see GemmArgs
 };
 
 struct TcUnit {
@@ -418,24 +417,6 @@ __device__ __forceinline__ void store_tile(const TcParams& p, const float2* acc,
   }
 }
 
-// What a CTA does behind an earlier failure, in place of its units of TOKENS tokens: one of its warps leaves NaN for the kernel
-// that adds up its sums.
-template <int TOKENS>
-__device__ __forceinline__ void mark_units(const TcParams& p, int lane) {
-  const int units = (p.pairs + p.solos) * p.splits * p.mtiles;
-  const int64_t ld = p.splits > 1 ? p.n : p.ldc;
-  for (int u = blockIdx.x; u < units; u += gridDim.x) {
-    const TcUnit it = tc_unit(p, u);
-    float* const out = p.splits > 1 ? p.partials + it.split * p.m * p.n : static_cast<float*>(p.c);
-    const int rows = it.ntile * TC_ROWS;
-#pragma unroll 1
-    for (int i = lane; i < TOKENS * rows; i += 32) {
-      const int64_t n = (int64_t)it.tile * TC_ROWS + i % rows, m = (int64_t)it.mtile * TOKENS + i / rows;
-      if (n < p.n && m < p.m) out[m * ld + n] = __uint_as_float(0x7fffffffu);
-    }
-  }
-}
-
 template <int T, int LIMBS, bool TILED>
 __global__ void __launch_bounds__(TcCfg<T, LIMBS>::THREADS, 1)
 q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_a,
@@ -550,7 +531,6 @@ q8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     } else if (warp == 1) {
       // ------------------------------------------------------------ activation producer
       pdl_wait();  // the activations are the previous kernel's output
-      if (prior_status != 0 && p.mark_failure) mark_units<T>(p, lane);
       const uint64_t pol = policy_evict_last();
       Ring<ACT_SLOTS> r;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
@@ -925,7 +905,6 @@ q8_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     } else if (warp == 1) {
       // ------------------------------------------------------------ activation producer, half a stage at a time
       pdl_wait();  // the activations are the previous kernel's output
-      if (prior_status != 0 && p.mark_failure) mark_units<2 * T>(p, lane);
       const uint64_t pol = policy_evict_last();
       Ring<ACT_SLOTS> r;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
@@ -1323,7 +1302,6 @@ logos_status_t launch_t(const GemmArgs& g, const TcPlan& plan, cudaStream_t st) 
   p.group = (int)((mtiles + groups - 1) / groups);
   p.stream_once = mtiles == 1;
   p.status = kernel_status_ptr(g.device);
-  p.mark_failure = g.mark_failure;
   if (!p.status) return fail(LOGOS_ERROR, "q8_gemm: no kernel status word");
   if (p.splits > p.stages_total) return fail(LOGOS_ERROR, "q8_gemm: more K splits than 128-column stages");
 
