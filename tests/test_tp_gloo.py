@@ -184,3 +184,12 @@ def test_folded_exchange_scheme_equals_allreduce_then_norm(oracle, tmp_path):
         assert np.array_equal(r[i]["hi"].view(np.uint16), hi.view(np.uint16))   # every rank holds every row
         assert np.array_equal(r[i]["lo"].view(np.uint16), lo.view(np.uint16))
         assert np.array_equal(r[i]["h_own"], total[i * (B // world):(i + 1) * (B // world)])  # only the owner's rows of h
+
+
+def test_importing_the_worker_leaves_its_importer_alive():
+    """The GPU tests import the worker's configurations; its end after 150 seconds is for the ranks that run it."""
+    import subprocess
+    code = "import faulthandler, sys; sys.path[:0] = %r\narmed = []\nfaulthandler.dump_traceback_later = lambda *a, **k: armed.append(a)\n" \
+           "import tp_worker\nassert not armed" % [os.path.join(ROOT, "tests"), ROOT]
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=240)
+    assert r.returncode == 0, r.stderr

@@ -11,7 +11,8 @@ import os
 import sys
 import time
 
-faulthandler.dump_traceback_later(150, exit=True)  # never outlive the test that started us
+if __name__ == "__main__":
+    faulthandler.dump_traceback_later(150, exit=True)  # never outlive the test that started us (which imports this file too)
 os.environ.setdefault("NCCL_NVLS_ENABLE", "0")
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
