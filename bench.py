@@ -33,10 +33,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 WORKLOADS = {
-    # BASELINE.json configs[4]
+    # throughput decode of the 32B shape
     "qwen32b-b64": dict(layers=64, hidden=5120, h_q=64, h_kv=8, head_dim=128, ffn=27648, vocab=152064, batch=64,
                         tied_embeddings=0, ctx=2048),
-    # BASELINE.json configs[3]
+    # decode of the 0.5B shape
     "qwen0.5b-b16": dict(layers=24, hidden=896, h_q=14, h_kv=2, head_dim=64, ffn=4864, vocab=151936, batch=16,
                          tied_embeddings=1, ctx=128),
     # a small shape for quick checks of the script itself

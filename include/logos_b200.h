@@ -184,6 +184,7 @@ LOGOS_API logos_status_t logos_q8_gemv(logos_handle_t q /*i8 [N][K]*/, logos_han
  * epilogue 0: plain.  1: C = bf16(acc + aux[m,n]) with aux bf16 [M][N] (residual).
  * 2: rows of q interleave gate (even) and up (odd); C is [M][N/2] =
  *    bf16( silu(acc_gate) * acc_up ).
+ * aux may be c.  Where K is a multiple of 128, c may lie over a (here and in logos_q8_gemm_f32): all of a has been read by then.
  * The stand-alone operators logos_q8_gemm and logos_q8_gemm_f32 keep activation planes and
  * split-K partials in one library-owned scratch block per device (logos_gqa_decode_attn_fused its arrival counter in another), grown on demand and shared by every caller on that device: calls that use it must
  * be ordered on the GPU (one stream, or events).  A model (logos_llm_*) owns its own. */

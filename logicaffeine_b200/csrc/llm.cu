@@ -949,8 +949,8 @@ logos_status_t prefill_chunked(Model* m, const int32_t* tokens_host, int64_t t, 
       return launch_q8_gemm(g, st);
     };
     // The same with K splits where a matrix has few row tiles for these rows: into `parts` copies that the next norm adds up, or
-    // with a fold of its own (us: 1 x 100 tokens of the 0.5B shape 1963 -> 1633, 2 x 64 1993 -> 1494, 16 x 128 3990 -> 3890, two layers of the
-    // 32B shape 1 x 128 tokens 1189 -> 894, of which the wide GEMM units are a third).
+    // with a fold of its own (us, without -> with: 100 tokens of the 0.5B shape 1824 -> 1411, 512 2724 -> 2382, 1088 4150 -> 4032; three
+    // layers of the 32B shape, 128 tokens 1419 -> 1038, 1088 7723 -> 7401).
     int parts = 1;             // of the pending row-parallel product
     const float* delta = w.delta;
     auto gemm_split = [&](const ActOut& a, const Q8Mat& wt, int64_t k, GemmArgs g, bool folded) -> logos_status_t {

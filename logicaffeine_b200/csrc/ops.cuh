@@ -79,8 +79,8 @@ int gemm_many_splits(int64_t m, int64_t n, int64_t k, int device, bool folded);
 // Whether the tcgen05 kernel accepts this call (else the SIMT kernel runs).
 bool gemm_tc_applicable(const GemmArgs& g);
 // A stand-alone product of one or two tokens by the GEMV kernel: one launch instead of the preparation of activation planes,
-// the product and the fold of its K splits, and f32 arithmetic throughout.  K a multiple of 128 (other K have a rule of
-// their own, see gemm_tensor) whose vectors fit beside the kernel's rings in shared memory, up to 30208 and 14848; two tokens
+// the product and the fold of its K splits, and f32 arithmetic throughout.  K a multiple of 128 (the kernel would take any K of whole
+// blocks; those stay with the GEMM and its rule for what planes do not hold, not timed) whose vectors fit beside the kernel's rings in shared memory, up to 30208 and 14848; two tokens
 // only of matrices whose stream the shared-memory reads of x do not hold up for long.  The GEMM / this, us: one token 768 x
 // 2176 10.3 / 4.4, 8064 x 3072 14.4 / 7.5, 152064 x 5120 181 / 171; two 896 x 2048 10.2 / 3.9, 10752 x 3072 16.8 / 11.5, 9216 x 6144 (57 M
 // weights) 20.6 / 19.4, 18944 x 3584 (68 M) 20.2 / 21.7, 5120 x 14848 26.7 / 33.1.

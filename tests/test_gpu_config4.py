@@ -1,4 +1,4 @@
-"""BASELINE.json's config 4 at its own shapes: a Qwen2.5-32B-shaped model (hidden 5120, 64 query /
+"""Throughput decode at its own shapes: a Qwen2.5-32B-shaped model (hidden 5120, 64 query /
 8 KV heads of 128, FFN 27648, vocabulary 152064, batch 64) at reduced depth, so the CPU oracle
 can step it.  Greedy tokens and logits of the unsharded GPU model equal the oracle's, and the
 same model under tensor parallelism on 2, 4 and 8 GPUs (one process per rank, both ways of

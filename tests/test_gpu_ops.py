@@ -231,7 +231,7 @@ def test_q8_gemm_config1_slice(llm, oracle):
 
 
 def test_q8_gemm_config1_full_size(llm, oracle):
-    """Config 1 as BASELINE.json states it: M=64 tokens x K=3584 x N=18944 (Qwen-7B FFN up-proj),
+    """The FFN up-projection at its full size: M=64 tokens x K=3584 x N=18944 (Qwen-7B FFN up-proj),
     bf16 activations, bf16 output, compared with the oracle's bf16-rounded result and, before
     the rounding hides it, with the oracle's f32 sums."""
     O = oracle
@@ -310,7 +310,7 @@ def test_q8_gemm_of_one_or_two_tokens(llm, oracle, m, n, k):
     assert llm.kernelStatus() == 0
 
 
-@pytest.mark.parametrize("m", [1, 2, 3])
+@pytest.mark.parametrize("m", [1, 2, 3, 200])   # the GEMV's token counts, and the GEMM's without and with K splits
 @pytest.mark.parametrize("n,k", [(2048, 2048), (3072, 1024)])   # results of the activations' size, and of a larger one
 def test_q8_gemm_results_over_the_activations(llm, oracle, m, n, k):
     """A product into the buffer that its activations are in, with the residual there too where it fits: what only kernels that
@@ -630,7 +630,7 @@ def test_gqa_decode_attn_batches_of_several_threads(llm, oracle):
 
 
 def test_gqa_decode_attn_config2_full_size(llm, oracle):
-    """Config 2 as BASELINE.json states it: batch 32, 28 query / 4 KV heads, head_dim 128, 4096
+    """Decode attention at its full size: batch 32, 28 query / 4 KV heads, head_dim 128, 4096
     cached positions, one token appended per sequence with RoPE theta 1e6: the KV cache after the
     call is bit-equal to the oracle's, the lengths advance, the output is within tolerance."""
     O = oracle

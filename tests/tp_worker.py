@@ -27,7 +27,7 @@ CFG = dict(layers=3, hidden=256, h_q=8, h_kv=2, head_dim=64, ffn=512, vocab=1024
            rms_eps=1e-6, rope_theta=1e6, tied_embeddings=0, seed=9, init_std=0.02)
 
 
-# BASELINE.json's config 4 (Qwen2.5-32B-shaped, batch 64) at reduced depth and a short context: every GEMM
+# Throughput decode of the 32B shape (batch 64) at reduced depth and a short context: every GEMM
 # shape of the real model (N = 55296 gate/up, K = 27648 down with split-K, the 1188-tile lm_head, 80-tile qkv),
 # 8 sequences per rank at 8 ranks, in a model the CPU oracle steps in a few seconds
 CFG4 = dict(layers=2, hidden=5120, h_q=64, h_kv=8, head_dim=128, ffn=27648, vocab=152064, l_max=32, batch=64,
